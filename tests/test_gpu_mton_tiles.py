@@ -1,0 +1,37 @@
+"""The M x N tensor-core kernel with in-kernel decoded code tiles
+(distanceBatchMToN / distanceBatchMToNSymmetric, space_turbo_quant.h:588-615)
+at the edges of its tiles: row counts around its column widths (16 ... 256),
+code counts around its 128-code tiles, reductions shorter than one 64-value
+K block and longer than one accumulation chunk, every index width, zero rows
+and rows of very different norms.  Tolerance: DIST_RTOL of the term scale
+(conftest.py), the bar of every distance."""
+import numpy as np
+import pytest
+
+import oracle as O
+import turboquant as tq
+from conftest import asym_term_scale, dist_close, sym_term_scale
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dim,bits", [(16, 4), (20, 8), (32, 2), (64, 3), (100, 5), (128, 4), (384, 4),
+                                      (768, 8), (1000, 9), (1536, 4), (4096, 6)])
+@pytest.mark.parametrize("m,n", [(9, 1), (16, 127), (17, 128), (64, 129), (65, 300), (129, 257),
+                                 (256, 130), (257, 1025)])
+def test_tile_edges(cuda_ok, dim, bits, m, n):
+    rng = np.random.default_rng(dim * 7 + bits + 31 * m + n)
+    X = (rng.standard_normal((n, dim)) * rng.uniform(1e-2, 1e2, (n, 1))).astype(np.float32)
+    Q = (rng.standard_normal((m, dim)) * rng.uniform(1e-2, 1e2, (m, 1))).astype(np.float32)
+    X[n // 2] = 0.0
+    Q[m // 2] = 0.0
+    s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    cs = s.code_size_bytes()
+    codes, rows = o.encode_batch(X), o.encode_batch(Q)
+    err, ok = dist_close(s.distance_m_to_n(Q, codes), o.distance_m_to_n(Q, codes),
+                         asym_term_scale(Q, codes, cs, cs - 12))
+    assert ok, ("asymmetric", err.max())
+    err, ok = dist_close(s.distance_m_to_n_symmetric(rows, codes),
+                         o.distance_m_to_n_symmetric(rows, codes),
+                         sym_term_scale(rows, codes, cs, cs - 12))
+    assert ok, ("symmetric", err.max())

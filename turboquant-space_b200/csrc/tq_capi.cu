@@ -19,6 +19,7 @@
 #include <string>
 #include <vector>
 
+#include "tq_cgemm.h"
 #include "tq_exact.h"
 #include "tq_host.h"
 #include "tq_internal.h"
@@ -136,54 +137,44 @@ tq_status mton_precision_ok(tq_precision p, bool sym) {
 }
 
 // M x N driver.  The row side (m queries, or m codes for the symmetric form)
-// is prepared once; the column side is decoded and contracted in chunks:
-//   FP32, m < kScanRows:  the HBM-bound scan kernel per row (no planes);
-//   FP32 otherwise:       FP32 planes + CUDA-core SGEMM;
-//   SPLIT_BF16:           hi/lo BF16 planes + tcgen05 GEMM;
-//   SPLIT_BF16_DECODED:   the same row planes; the column tiles decoded from the
-//                         codes in shared memory (per-code scalars only in HBM);
-//   REFERENCE:            the reference build's own arithmetic, one pair per thread.
+// is prepared once; the column side is contracted code tile by code tile:
+//   REFERENCE:   the reference build's own arithmetic, one pair per thread;
+//   FP32:        the tensor-core kernel on FP16 pairs (tq_cgemm.cu), or the
+//                HBM-bound scan kernel per row where use_cg() says so;
+//   SPLIT_BF16, SPLIT_BF16_DECODED: the tensor-core kernel on BF16 pairs.
 // Every distance ends in the same epilogue d = max(0, r2 + c2 - 2 C r1 c1).
 class MtonRunner {
   public:
-    static constexpr size_t kScanRows = 32;
     static constexpr size_t kRowPlaneBytes = size_t(512) << 20;
-    static constexpr size_t kColPlaneBytes = size_t(1) << 30;
 
-    static size_t row_chunk(const tq_space *sp, bool sym, tq_precision prec) {
+    static size_t row_chunk(const tq_space *sp, bool sym) {
         const size_t K = sym ? sp->D : 2 * sp->D;
-        size_t rows = (kRowPlaneBytes / (K * 4)) & ~size_t(tq::kPlaneRowAlign - 1);
-        (void)prec;
-        return std::max<size_t>(tq::kPlaneRowAlign, rows);
+        return std::max<size_t>(128, (kRowPlaneBytes / (K * 4)) & ~size_t(127));
     }
 
-    MtonRunner(tq_space *sp, bool sym, tq_precision prec, size_t m)
+    // n: all the columns of the call (run_cols may take them in parts)
+    MtonRunner(tq_space *sp, bool sym, tq_precision prec, size_t m, size_t n)
         : sp_(sp), sym_(sym), prec_(prec), m_(m) {
-        K_ = sym ? (int)sp->D : 2 * (int)sp->D;
-        dec_ = prec == TQ_PRECISION_SPLIT_BF16_DECODED;
-        fmt_ = (prec == TQ_PRECISION_SPLIT_BF16 || dec_) ? tq::kPlaneBF16 : tq::kPlaneF32;
-        planes_ = prec != TQ_PRECISION_REFERENCE &&
-                  (prec == TQ_PRECISION_SPLIT_BF16 || dec_ || m >= kScanRows);
-        m_pad_ = round_up(m, tq::kPlaneRowAlign);
-        const size_t col_align = prec == TQ_PRECISION_SPLIT_BF16 ? 256 : 128;
-        nc_max_ = std::max(col_align, ((kColPlaneBytes / ((size_t)K_ * 4)) / col_align) * col_align);
+        bf16_ = prec == TQ_PRECISION_SPLIT_BF16 || prec == TQ_PRECISION_SPLIT_BF16_DECODED;
+        cg_ = bf16_ || (prec == TQ_PRECISION_FP32 && use_cg(n));
     }
 
     tq_status prepare_rows(const void *rows_dev, cudaStream_t s) {
-        if (prec_ == TQ_PRECISION_SPLIT_BF16 && (K_ % 64 != 0))
+        const size_t D = sp_->D, K = sym_ ? D : 2 * D;
+        if (prec_ == TQ_PRECISION_SPLIT_BF16 && K % 64 != 0)
             return fail(TQ_ERR_NOT_SUPPORTED,
                         "split-BF16 contraction needs a reduction length that is a multiple of 64 "
-                        "(padded dim %zu)", sp_->D);
-        if (dec_ && sp_->D % 64 != 0)
-            return fail(TQ_ERR_NOT_SUPPORTED,
-                        "decoded split-BF16 tiles need a padded dim that is a multiple of 64 (padded dim %zu)",
-                        sp_->D);
-        if (dec_ && !tq::tc_dist_dec_fits((int)sp_->code_size))
-            return fail(TQ_ERR_NOT_SUPPORTED,
-                        "decoded split-BF16 tiles: a tile of 128 codes of %zu bytes does not fit in shared "
-                        "memory beside the pipeline (use split_bf16)", sp_->code_size);
-        if (fmt_ == tq::kPlaneF32 && planes_ && (K_ % 16 != 0)) planes_ = false;
-        const size_t D = sp_->D;
+                        "(padded dim %zu)", D);
+        if (prec_ == TQ_PRECISION_SPLIT_BF16_DECODED) {
+            if (D % 64 != 0)
+                return fail(TQ_ERR_NOT_SUPPORTED,
+                            "decoded split-BF16 tiles need a padded dim that is a multiple of 64 (padded dim %zu)",
+                            D);
+            if (sp_->code_size > kDecMaxCode)
+                return fail(TQ_ERR_NOT_SUPPORTED,
+                            "decoded split-BF16 tiles: a tile of 128 codes of %zu bytes does not fit in shared "
+                            "memory beside the pipeline (use split_bf16)", sp_->code_size);
+        }
         if (!sym_) {  // prepared queries (the scan path uses them directly)
             TQ_CUDA(prep_.alloc(sizeof(float) * m_ * (2 * D + 2), s), "cudaMallocAsync(prepared)");
             q_rot_ = static_cast<float *>(prep_.p);
@@ -195,137 +186,51 @@ class MtonRunner {
         } else {
             codes_a_ = static_cast<const uint8_t *>(rows_dev);
         }
-        if (!planes_) return TQ_OK;
-        const size_t plane_bytes = m_pad_ * (size_t)K_ * 4;
-        TQ_CUDA(rows_.alloc(plane_bytes + 2 * 4 * m_pad_, s), "cudaMallocAsync(row planes)");
-        a0_ = rows_.p;
-        a1_ = static_cast<unsigned char *>(rows_.p) + plane_bytes / 2;
-        r1_ = reinterpret_cast<float *>(static_cast<unsigned char *>(rows_.p) + plane_bytes);
-        r2_ = r1_ + m_pad_;
+        if (!cg_) return TQ_OK;
+        const size_t plane = m_ * tq::cg_row_k(sp_->P, form()) * 2;  // a multiple of 128 bytes
+        TQ_CUDA(rows_.alloc(2 * plane + m_ * sizeof(float4) + sizeof(int), s), "cudaMallocAsync(row planes)");
+        auto *base = static_cast<unsigned char *>(rows_.p);
+        r_.hi = base;
+        r_.lo = base + plane;
+        r_.rs = reinterpret_cast<float4 *>(base + 2 * plane);
+        if (bf16_) {  // reported by finish(); FP32 is stream-ordered and reports through the status word
+            err_ = reinterpret_cast<int *>(r_.rs + m_);
+            TQ_CUDA(cudaMemsetAsync(err_, 0, sizeof(int), s), "memset");
+        }
         if (!sym_)
-            TQ_CUDA(tq::launch_planes_from_prepared(q_rot_, s_q_, norms_, m_, m_pad_, (int)D, fmt_, a0_,
-                                                    a1_, r1_, r2_, s),
-                    "row planes");
+            TQ_CUDA(tq::launch_cg_rows_prepared(sp_->P, q_rot_, s_q_, norms_, m_, fmt(), r_, s), "row planes");
         else
-            TQ_CUDA(tq::launch_planes_from_codes(sp_->P, sp_->T, codes_a_, m_, m_pad_, true, fmt_, a0_,
-                                                 a1_, r1_, r2_, s),
-                    "row planes");
+            TQ_CUDA(tq::launch_cg_rows_codes(sp_->P, sp_->T, codes_a_, m_, form(), fmt(), r_, s), "row planes");
         return TQ_OK;
     }
 
     // columns [0, n) of device codes -> out[i * ldo + j]
     tq_status run_cols(const uint8_t *codes, size_t n, float *out, size_t ldo, cudaStream_t s) {
-        if (dec_) return run_cols_decoded(codes, n, out, ldo, s);
-        if (!planes_) {
-            if (!sym_ && prec_ == TQ_PRECISION_REFERENCE)
-                TQ_CUDA(tq::launch_exact_mton(sp_->P, sp_->T.centroids, q_rot_, s_q_, norms_, m_, codes,
-                                              n, out, ldo, s),
-                        "reference-order m_to_n kernel");
-            else if (!sym_)
-                TQ_CUDA(tq::launch_mton_fp32(sp_->P, sp_->T, q_rot_, s_q_, norms_, m_, codes, n, out,
-                                             ldo, s),
-                        "m_to_n scan kernel");
-            else if (prec_ == TQ_PRECISION_REFERENCE)
-                TQ_CUDA(tq::launch_exact_mton_sym(sp_->P, sp_->T.centroids, codes_a_, m_, codes, n, out,
-                                                  ldo, s),
-                        "reference-order symmetric m_to_n kernel");
-            else
-                TQ_CUDA(tq::launch_mton_sym_fp32(sp_->P, sp_->T, codes_a_, m_, codes, n, out, ldo, s),
-                        "symmetric m_to_n scan kernel");
-            return TQ_OK;
-        }
-        if (!cols_.p) {
-            const size_t nc = std::min(nc_max_, round_up(n, prec_ == TQ_PRECISION_SPLIT_BF16 ? 256 : 128));
-            nc_alloc_ = nc;
-            const size_t plane_bytes = nc * (size_t)K_ * 4;
-            TQ_CUDA(cols_.alloc(plane_bytes + 2 * 4 * nc + 16, s), "cudaMallocAsync(column planes)");
-            b0_ = cols_.p;
-            b1_ = static_cast<unsigned char *>(cols_.p) + plane_bytes / 2;
-            c1_ = reinterpret_cast<float *>(static_cast<unsigned char *>(cols_.p) + plane_bytes);
-            c2_ = c1_ + nc;
-            err_ = reinterpret_cast<int *>(c2_ + nc);
-            TQ_CUDA(cudaMemsetAsync(err_, 0, sizeof(int), s), "memset");
-        }
-        const size_t col_align = prec_ == TQ_PRECISION_SPLIT_BF16 ? 256 : 128;
-        for (size_t n0 = 0; n0 < n; n0 += nc_alloc_) {
-            const size_t nc = std::min(nc_alloc_, n - n0);
-            const size_t nc_pad = round_up(nc, col_align);
-            TQ_CUDA(tq::launch_planes_from_codes(sp_->P, sp_->T, codes + n0 * sp_->code_size, nc,
-                                                 nc_pad, sym_, fmt_, b0_, b1_, c1_, c2_, s),
-                    "column planes");
-            if (fmt_ == tq::kPlaneF32)
-                TQ_CUDA(tq::launch_sgemm_dist(static_cast<const float *>(a0_),
-                                              static_cast<const float *>(b0_), K_, m_, m_pad_, nc,
-                                              nc_pad, r1_, r2_, c1_, c2_, out + n0, ldo, s),
-                        "FP32 GEMM kernel");
-            else
-                TQ_CUDA(tq::launch_tc_dist(a0_, a1_, b0_, b1_, K_,
-                                           sym_ ? K_ : tq::asym_lo_width((int)sp_->D), m_, m_pad_,
-                                           nc, nc_pad, r1_, r2_, c1_, c2_, out + n0, ldo, err_, s),
-                        "tcgen05 GEMM kernel");
-        }
-        return TQ_OK;
-    }
-
-    // The decoded form: per chunk of columns, the per-code scalars (16 bytes a
-    // code) and one tensor-core launch whose decoder warps turn each tile of 128
-    // codes into its B tiles in shared memory.  A tile's codes arrive by one bulk
-    // copy rounded up to 16 bytes; whole tiles are multiples of 16 bytes, and a
-    // ragged last tile whose bytes do not end on that boundary is read from a
-    // padded copy, so no copy reads past the caller's codes.
-    tq_status run_cols_decoded(const uint8_t *codes, size_t n, float *out, size_t ldo, cudaStream_t s) {
-        const size_t cs = sp_->code_size;
-        if (reinterpret_cast<uintptr_t>(codes) & 15)
+        if (prec_ == TQ_PRECISION_SPLIT_BF16_DECODED && (reinterpret_cast<uintptr_t>(codes) & 15))
             return fail(TQ_ERR_NOT_SUPPORTED, "decoded split-BF16 tiles need 16-byte aligned device codes");
-        if (!cols_.p) {
-            nc_alloc_ = std::min(round_up(n, 128), kDecCols);
-            tail_bytes_ = round_up(128 * cs, 16) + 16;
-            TQ_CUDA(cols_.alloc(4 * 4 * nc_alloc_ + 16 + tail_bytes_, s), "cudaMallocAsync(column scalars)");
-            c1_ = static_cast<float *>(cols_.p);
-            c2_ = c1_ + nc_alloc_;
-            fc_ = c2_ + nc_alloc_;
-            fs_ = fc_ + nc_alloc_;
-            err_ = reinterpret_cast<int *>(fs_ + nc_alloc_);
-            tail_ = reinterpret_cast<uint8_t *>(err_ + 4);
-            TQ_CUDA(cudaMemsetAsync(err_, 0, sizeof(int), s), "memset");
-        }
-        tq::DecSrc d;
-        d.cs = (int)cs;
-        d.nibble = sp_->P.nibble;
-        d.kbc = (int)(sp_->D / 64);
-        d.centroids = sp_->T.centroids;
-        d.levels = (int)sp_->levels;
-        auto launch = [&](const uint8_t *src, size_t cols, float *dst) -> tq_status {
-            const size_t cols_pad = round_up(cols, 128);
-            TQ_CUDA(tq::launch_dec_factors(sp_->P, src, cols, cols_pad, sym_, c1_, c2_, sym_ ? nullptr : fc_,
-                                           sym_ ? nullptr : fs_, s),
-                    "column scalars");
-            d.codes = src;
-            d.n = (unsigned)cols;
-            d.fc = sym_ ? nullptr : fc_;
-            d.fs = sym_ ? nullptr : fs_;
-            TQ_CUDA(tq::launch_tc_dist_dec(a0_, a1_, m_, m_pad_, d, cols_pad, K_, r1_, r2_, c1_, c2_, dst, ldo,
-                                           err_, s),
-                    "tcgen05 GEMM kernel (decoded tiles)");
-            return TQ_OK;
-        };
-        for (size_t n0 = 0; n0 < n; n0 += nc_alloc_) {
-            const size_t nc = std::min(nc_alloc_, n - n0);
-            const size_t rem = nc % 128;
-            const size_t n_main = (rem != 0 && (rem * cs) % 16 != 0) ? nc - rem : nc;
-            tq_status st;
-            if (n_main > 0 && (st = launch(codes + n0 * cs, n_main, out + n0)) != TQ_OK) return st;
-            if (n_main < nc) {
-                TQ_CUDA(cudaMemcpyAsync(tail_, codes + (n0 + n_main) * cs, (nc - n_main) * cs,
-                                        cudaMemcpyDeviceToDevice, s),
-                        "copy of the last tile");
-                if ((st = launch(tail_, nc - n_main, out + n0 + n_main)) != TQ_OK) return st;
-            }
-        }
+        if (cg_)
+            TQ_CUDA(tq::launch_cgemm(sp_->P, sp_->T, form(), fmt(), r_, m_, codes, n, out, ldo,
+                                     err_ ? err_ : sp_->T.status, s),
+                    "tcgen05 M x N kernel");
+        else if (!sym_ && prec_ == TQ_PRECISION_REFERENCE)
+            TQ_CUDA(tq::launch_exact_mton(sp_->P, sp_->T.centroids, q_rot_, s_q_, norms_, m_, codes,
+                                          n, out, ldo, s),
+                    "reference-order m_to_n kernel");
+        else if (!sym_)
+            TQ_CUDA(tq::launch_mton_fp32(sp_->P, sp_->T, q_rot_, s_q_, norms_, m_, codes, n, out,
+                                         ldo, s),
+                    "m_to_n scan kernel");
+        else if (prec_ == TQ_PRECISION_REFERENCE)
+            TQ_CUDA(tq::launch_exact_mton_sym(sp_->P, sp_->T.centroids, codes_a_, m_, codes, n, out,
+                                              ldo, s),
+                    "reference-order symmetric m_to_n kernel");
+        else
+            TQ_CUDA(tq::launch_mton_sym_fp32(sp_->P, sp_->T, codes_a_, m_, codes, n, out, ldo, s),
+                    "symmetric m_to_n scan kernel");
         return TQ_OK;
     }
 
-    // Reports a bounded wait that gave up inside the tensor-core kernel.
+    // Reports a bounded wait that gave up inside the split-BF16 kernel.
     tq_status finish(cudaStream_t s) {
         if (!err_) return TQ_OK;
         int h = 0;
@@ -334,24 +239,32 @@ class MtonRunner {
         if (h != 0) return fail(TQ_ERR_TIMEOUT, "tensor-core kernel: a pipeline wait timed out (code %d)", h);
         return TQ_OK;
     }
+    // The space's status word carries this call's errors (host entry points read it).
+    bool uses_status_word() const { return cg_ && !err_; }
 
   private:
-    static constexpr size_t kDecCols = size_t(1) << 24;  // columns per decoded launch
-    static size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+    // Code size up to which SPLIT_BF16_DECODED is offered: a tile of 128 codes
+    // beside two 64 KB stages in shared memory.
+    static constexpr size_t kDecMaxCode = 756;
+    // FP32: the tensor-core kernel, except where the scan kernel's single launch
+    // is faster (us a call, scan / tensor-core): one or two rows, whose decode
+    // is not shared (384-d 4-bit, 200,000 codes: 38 / 151 for one row, 111 / 151
+    // for two, 394 / 153 for eight), and few rows against few codes, where the
+    // row-plane launch shows (8 x 1,000: 32 / 36; 8 x 30,000: 76 / 46).
+    bool use_cg(size_t n) const {
+        if (sp_->D < 16 || m_ <= 2) return false;
+        return m_ > 8 || m_ * n * sp_->D > (size_t(1) << 24);
+    }
+    int form() const { return sym_ ? tq::kCgSym : tq::kCgAsym; }
+    int fmt() const { return bf16_ ? tq::kCgBF16 : tq::kCgFP16; }
     tq_space *sp_;
-    bool sym_, dec_ = false;
-    size_t tail_bytes_ = 0;
-    float *fc_ = nullptr, *fs_ = nullptr;
-    uint8_t *tail_ = nullptr;
+    bool sym_, bf16_ = false, cg_ = false;
     tq_precision prec_;
-    size_t m_, m_pad_ = 0, nc_max_ = 0, nc_alloc_ = 0;
-    int K_ = 0, fmt_ = 0;
-    bool planes_ = false;
-    Scratch prep_, rows_, cols_;
+    size_t m_;
+    Scratch prep_, rows_;
     float *q_rot_ = nullptr, *s_q_ = nullptr, *norms_ = nullptr;
     const uint8_t *codes_a_ = nullptr;
-    void *a0_ = nullptr, *a1_ = nullptr, *b0_ = nullptr, *b1_ = nullptr;
-    float *r1_ = nullptr, *r2_ = nullptr, *c1_ = nullptr, *c2_ = nullptr;
+    tq::CgRows r_;
     int *err_ = nullptr;
 };
 
@@ -809,10 +722,10 @@ tq_status tq_distance_m_to_n_device(const tq_space *sp, const float *queries, si
     if ((st = check_codes_align(codes, "codes")) != TQ_OK) return st;
     if ((st = check_dev(out, m * n * 4, "out")) != TQ_OK) return st;
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t mchunk = MtonRunner::row_chunk(sp, false, precision);
+    const size_t mchunk = MtonRunner::row_chunk(sp, false);
     for (size_t m0 = 0; m0 < m; m0 += mchunk) {
         const size_t mc = std::min(mchunk, m - m0);
-        MtonRunner r(const_cast<tq_space *>(sp), false, precision, mc);
+        MtonRunner r(const_cast<tq_space *>(sp), false, precision, mc, n);
         if ((st = r.prepare_rows(queries + m0 * sp->dim, s)) != TQ_OK) return st;
         if ((st = r.run_cols(codes, n, out + m0 * n, n, s)) != TQ_OK) return st;
         if ((st = r.finish(s)) != TQ_OK) return st;
@@ -834,10 +747,10 @@ tq_status tq_distance_m_to_n_symmetric_device(const tq_space *sp, const uint8_t 
     if ((st = check_codes_align(B, "codes_b")) != TQ_OK) return st;
     if ((st = check_dev(out, m * n * 4, "out")) != TQ_OK) return st;
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t mchunk = MtonRunner::row_chunk(sp, true, precision);
+    const size_t mchunk = MtonRunner::row_chunk(sp, true);
     for (size_t m0 = 0; m0 < m; m0 += mchunk) {
         const size_t mc = std::min(mchunk, m - m0);
-        MtonRunner r(const_cast<tq_space *>(sp), true, precision, mc);
+        MtonRunner r(const_cast<tq_space *>(sp), true, precision, mc, n);
         if ((st = r.prepare_rows(A + m0 * sp->code_size, s)) != TQ_OK) return st;
         if ((st = r.run_cols(B, n, out + m0 * n, n, s)) != TQ_OK) return st;
         if ((st = r.finish(s)) != TQ_OK) return st;
@@ -957,7 +870,7 @@ tq_status mton_host(tq_space *sp, bool sym, tq_precision prec, const void *rows_
     Scratch rows;
     TQ_CUDA(rows.alloc(row_bytes, sc), "cudaMallocAsync(rows)");
     TQ_CUDA(cudaMemcpyAsync(rows.p, rows_host, row_bytes, cudaMemcpyHostToDevice, sc), "H2D rows");
-    MtonRunner runner(sp, sym, prec, m);
+    MtonRunner runner(sp, sym, prec, m, n);
     tq_status st = runner.prepare_rows(rows.p, sc);
     if (st != TQ_OK) return st;
     const size_t cbytes = (per * cs + 15) & ~size_t(15);
@@ -1002,6 +915,7 @@ tq_status mton_host(tq_space *sp, bool sym, tq_precision prec, const void *rows_
         if (e != cudaSuccess && result == TQ_OK) result = cuda_fail(e, "m_to_n");
     }
     if (result == TQ_OK) result = runner.finish(sc);
+    if (result == TQ_OK && runner.uses_status_word()) result = take_status(sp, nullptr);
     for (int k = 0; k < 2; ++k) {
         cudaEventDestroy(uploaded[k]);
         cudaEventDestroy(computed[k]);

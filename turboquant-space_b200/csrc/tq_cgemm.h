@@ -1,0 +1,33 @@
+// tq_cgemm.h -- the M x N distances with in-kernel decoded code tiles (tq_cgemm.cu).
+#pragma once
+
+#include "tq_internal.h"
+
+namespace tq {
+
+enum CgForm { kCgAsym = 0, kCgSym = 1, kCgLight = 2 };  // queries / codes / codes + light QJL term
+enum CgFmt { kCgFP16 = 0, kCgBF16 = 1 };                // 16-bit type of the hi / lo pairs
+
+// The row operand: hi and lo planes of m x cg_row_k 16-bit values and four
+// scalars a row, all 16-byte aligned.
+struct CgRows {
+    void *hi = nullptr, *lo = nullptr;
+    float4 *rs = nullptr;
+};
+size_t cg_row_k(const Params &P, int form);
+
+// Prepared queries (kCgAsym) or codes (kCgSym, kCgLight) -> row operand.
+cudaError_t launch_cg_rows_prepared(const Params &P, const float *q_rot, const float *s_q,
+                                    const float *norms, size_t m, int fmt, const CgRows &r,
+                                    cudaStream_t st);
+cudaError_t launch_cg_rows_codes(const Params &P, const DevTables &T, const uint8_t *codes, size_t m,
+                                 int form, int fmt, const CgRows &r, cudaStream_t st);
+
+// out[i * ldo + j] = distance of row i to code j.  Codes 4-byte aligned, the
+// code size a multiple of 4 (every padded dim but 4).  `err` (device int) is
+// set non-zero if a bounded wait in the kernel gave up.
+cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt, const CgRows &rows,
+                         size_t m, const uint8_t *codes, size_t n, float *out, size_t ldo, int *err,
+                         cudaStream_t st);
+
+}  // namespace tq

@@ -1,49 +1,29 @@
-// tq_mton.h -- operand planes and contraction kernels of the M x N distances
-// (tq_mton.cu: decode + FP32 SGEMM; tq_tc.cu: split-BF16 tcgen05 GEMM).
+// tq_mton.h -- operand planes (tq_mton.cu) and tensor-core contractions
+// (tq_tc.cu) of the serving top-k and the split-TF32 QJL-corrected distances.
 #pragma once
 
 #include "tq_internal.h"
 
 namespace tq {
 
-constexpr int kPlaneF32 = 0;   // one FP32 plane
-constexpr int kPlaneBF16 = 1;  // hi and lo BF16 planes, x = hi + lo
-constexpr int kPlaneRowAlign = 128;
-
 // Columns of the BF16 lo plane of asymmetric code planes: the QJL half of
 // those planes is exact (+-1, see tq_mton.cu), so lo is stored for the
 // centroid half only, rounded up to a whole 64-wide K block.
 inline int asym_lo_width(int D) { return D % 64 == 0 ? D : 2 * D; }
 
-// Rows [0, rows) of `codes` -> planes of rows_pad x K (K = D symmetric, 2D
-// asymmetric), zero rows beyond `rows`; s1/s2 per-row scalars (rows_pad).
-// BF16 lo planes have K columns, asym_lo_width(D) for asymmetric planes.
+// Rows [0, rows) of `codes` -> hi (rows_pad x 2D) and lo (rows_pad x
+// asym_lo_width(D)) planes, zero rows beyond `rows`; s1/s2 per-row scalars.
 cudaError_t launch_planes_from_codes(const Params &P, const DevTables &T, const uint8_t *codes,
-                                     size_t rows, size_t rows_pad, bool sym, int fmt, void *plane0,
-                                     void *plane1, float *s1, float *s2, cudaStream_t st);
+                                     size_t rows, size_t rows_pad, void *plane0, void *plane1,
+                                     float *s1, float *s2, cudaStream_t st);
 
 // Prepared queries -> planes of rows_pad x 2D and r1 = |q|, r2 = |q|^2.
 cudaError_t launch_planes_from_prepared(const float *q_rot, const float *s_q, const float *norms,
-                                        size_t rows, size_t rows_pad, int D, int fmt, void *plane0,
+                                        size_t rows, size_t rows_pad, int D, void *plane0,
                                         void *plane1, float *r1, float *r2, cudaStream_t st);
 
-// out[i, j] = max(0, r2_i + c2_j - 2 (C_ij r1_i) c1_j), C = A B^T in FP32.
-cudaError_t launch_sgemm_dist(const float *A, const float *B, int K, size_t m, size_t m_pad,
-                              size_t n, size_t n_pad, const float *r1, const float *r2,
-                              const float *c1, const float *c2, float *out, size_t ldo,
-                              cudaStream_t st);
-
-// The same with C = Ah Bh^T + Ah Bl^T + Al Bh^T on tcgen05 tensor cores
-// (FP32 accumulators in tensor memory, promoted to an IEEE FP32 running sum
-// every few K blocks).  K % 64 == 0, m_pad % 128 == 0, n_pad % 128 == 0.  Bl has k_lo columns (k_lo % 64 == 0, k_lo <= K): B's lo
-// part is zero beyond them, where the Ah Bl^T product is skipped.  `err`
-// (device int) is set non-zero if a bounded wait in the kernel gave up.
-cudaError_t launch_tc_dist(const void *Ah, const void *Al, const void *Bh, const void *Bl, int K,
-                           int k_lo, size_t m, size_t m_pad, size_t n, size_t n_pad, const float *r1,
-                           const float *r2, const float *c1, const float *c2, float *out,
-                           size_t ldo, int *err, cudaStream_t st);
-
-// Top-k over a device-resident index: C = A B^T as above, reduced per row to the
+// Top-k over a device-resident index: C = Ah Bh^T + Ah Bl^T + Al Bh^T
+// with d = max(0, r2 + c2 - 2 (C r1) c1), reduced per row to the
 // k (<= kCandMax) smallest (distance, index) pairs, ties to the smaller index.
 // The row count is read from m_dev; `grid` CTAs split the rows into 128-row
 // blocks and the columns into slices.
@@ -75,11 +55,10 @@ struct DecSrc {
 };
 
 // Per-code scalars of the decoded-B kernels for rows [0, rows) of `codes`
-// (zero for rows up to rows_pad): asymmetric: c1 = scale gamma |x| (or |x|),
-// c2 = |x|^2, fc, fs as above; symmetric: c1 = sigma |x|, c2 = |x|^2 (fc, fs
-// may be null).
+// (zero for rows up to rows_pad): c1 = scale gamma |x| (or |x|),
+// c2 = |x|^2, fc, fs as above.
 cudaError_t launch_dec_factors(const Params &P, const uint8_t *codes, size_t rows, size_t rows_pad,
-                               bool sym, float *c1, float *c2, float *fc, float *fs, cudaStream_t st);
+                               float *c1, float *c2, float *fc, float *fs, cudaStream_t st);
 
 constexpr int kTopKMax = 16;   // results per row (k) of the serving path
 constexpr int kCandMax = 32;   // list length of the tensor-core top-k (candidates per row)
@@ -107,17 +86,6 @@ cudaError_t launch_tc_topk_dec(int variant, const void *Ah, const void *Al, size
 // Whether `variant` runs with decoded B tiles for codes of cs bytes (a tile of
 // 128 codes must fit in shared memory beside the variant's stages).
 bool tc_topk_dec_ok(int variant, int cs);
-// The M x N distances of launch_tc_dist with decoded B tiles (128 x 128 tiles,
-// two stages): columns [0, dec.n) of dec.codes, out[i * ldo + j] for i < m.
-// Asymmetric (dec.fc, dec.fs set): K = 2D, dec.kbc = D / 64, c1 / c2 / fc / fs
-// from launch_dec_factors; symmetric (dec.fc null): K = D, dec.kbc = D / 64,
-// A the symmetric row planes.  The last tile's copy reads the codes up to a
-// 16-byte boundary past code dec.n - 1: the caller guarantees that memory.
-cudaError_t launch_tc_dist_dec(const void *Ah, const void *Al, size_t m, size_t m_pad, const DecSrc &dec,
-                               size_t n_pad, int K, const float *r1, const float *r2, const float *c1,
-                               const float *c2, float *out, size_t ldo, int *err, cudaStream_t st);
-// Whether a tile of 128 codes of cs bytes fits launch_tc_dist_dec's shared memory.
-bool tc_dist_dec_fits(int cs);
 // Threshold collection over the corpus for the rows of A (row count *m_dev,
 // nothing unless it exceeds min_rows): every column whose tile distance (as the
 // top-k pass computes it) is at most thr[row] goes to coll_i[row * cap + ...],

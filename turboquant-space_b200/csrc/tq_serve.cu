@@ -254,7 +254,7 @@ cudaError_t enqueue_batch(tq_server *sv, Slot &sl, int rows_cap, int var, bool c
     if (e != cudaSuccess) return e;
     unsigned char *ah = static_cast<unsigned char *>(sl.d_ap);
     unsigned char *al = ah + (size_t)rows_cap * K * 2;
-    e = tq::launch_planes_from_prepared(q_rot, s_q, norms, rows_cap, rows_cap, (int)D, tq::kPlaneBF16,
+    e = tq::launch_planes_from_prepared(q_rot, s_q, norms, rows_cap, rows_cap, (int)D,
                                         ah, al, sl.d_r1, sl.d_r2, st);
     if (e != cudaSuccess) return e;
     // tensor-core pass: each row's kc best candidates by approximate distance
@@ -722,12 +722,12 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
             const size_t rows_pad = std::min(chunk, ix->n_pad - r0);
             const size_t rows = r0 < n ? std::min(rows_pad, n - r0) : 0;
             e = tq::launch_planes_from_codes(sp->P, sp->T, ix->codes + std::min(r0, n - 1) * sp->code_size,
-                                             rows, rows_pad, false, tq::kPlaneBF16, hi + r0 * K * 2,
+                                             rows, rows_pad, hi + r0 * K * 2,
                                              lo + r0 * (size_t)ix->K_lo * 2, ix->c1 + r0, ix->c2 + r0,
                                              nullptr);
         }
     } else if (e == cudaSuccess) {
-        e = tq::launch_dec_factors(sp->P, ix->codes, n, ix->n_pad, false, ix->c1, ix->c2, ix->fc, ix->fs,
+        e = tq::launch_dec_factors(sp->P, ix->codes, n, ix->n_pad, ix->c1, ix->c2, ix->fc, ix->fs,
                                    nullptr);
     }
     if (e == cudaSuccess) e = tq::launch_index_bound(sp->P, ix->codes, n, ix->bound, nullptr);

@@ -1,8 +1,8 @@
-// tq_tc.cu -- the tensor-core contractions of the M x N distances on sm_100a
-// (tcgen05 + TMA), with their epilogues fused: the split-BF16 asymmetric and
-// symmetric distances (tc_dist), their per-row top-k over a device-resident
-// index (tc_topk, the serving kernel) and the split-TF32 QJL-corrected
-// symmetric distances (tc_symq).
+// tq_tc.cu -- tensor-core contractions on sm_100a (tcgen05 + TMA) over operand
+// planes, with their epilogues fused: the per-row top-k of the split-BF16
+// asymmetric distances over a device-resident index (tc_topk, the serving
+// kernel) and the split-TF32 QJL-corrected symmetric distances (tc_symq).
+// The M x N distances themselves: tq_cgemm.cu.
 //
 // C = Ah Bh^T + Ah Bl^T + Al Bh^T over hi/lo operand planes (x = hi + lo,
 // see tq_mton.cu and tq_symq.cu), accumulated in FP32 in tensor memory.  A
@@ -39,15 +39,12 @@
 // Every mbarrier wait is bounded: after ~2 s it records an error code in
 // *err and the CTA winds down (frees its tensor memory) instead of waiting
 // forever.
-#include <cuda.h>
 #include <cuda_bf16.h>
-#include <cudaTypedefs.h>
 
 #include <cstdint>
-#include <mutex>
 
-#include "tq_async.cuh"
 #include "tq_mton.h"
+#include "tq_tc.cuh"
 
 namespace tq {
 namespace {
@@ -69,27 +66,6 @@ constexpr int TC_BAR_BYTES = 256;
 constexpr int TC_DEC_TAB_BYTES = 256 * 8 + 256 * 4;
 // error codes written to *err
 constexpr int kErrFull = 1, kErrEmpty = 2, kErrTmemFull = 3, kErrTmemEmpty = 4;
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y,
-                                            uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major, 128-byte-swizzled tile whose
-// rows are 128 bytes and whose 8-row groups are 1024 bytes apart.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFFu);  // start address
-    d |= (uint64_t)1u << 16;                  // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024u >> 4) << 32;        // stride byte offset: 8 rows x 128 B
-    d |= (uint64_t)1u << 46;                  // descriptor version (sm_100)
-    d |= (uint64_t)2u << 61;                  // layout: SWIZZLE_128B
-    return d;
-}
 
 // Instruction descriptor: FP32 accumulator, A and B of format `fmt` (1 =
 // BF16 for kind::f16, 2 = TF32 for kind::tf32), both K-major, M128 N128.
@@ -115,81 +91,6 @@ __device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a, uint64_t b, ui
             "l"(a), "l"(b), "r"(tc_idesc(1)), "r"(acc)
             : "memory");
     }
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-// 32 consecutive 32-bit columns of this warp's 32 tensor-memory lanes; the
-// _nw form leaves the wait (tcgen05.wait::ld) to the caller.
-__device__ __forceinline__ void tmem_ld32_nw(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-          "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-}
-// 16 consecutive 32-bit columns of this warp's lanes; the caller waits
-// (tcgen05.wait::ld) before reading them.
-__device__ __forceinline__ void tmem_ld16_nw(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-
-__device__ __forceinline__ void tmem_wait_ld() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-          "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
-        "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]),
-        "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
-        "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-}
-
-__device__ __forceinline__ void tmem_wait_st() {
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // The tensor maps of up to two K segments: [segment][Ah, Al, Bh, Bl].
@@ -646,62 +547,9 @@ struct GridTiles {
     }
 };
 
-// d = max(0, r2_i + c2_j - 2 (C_ij r1_i) c1_j), stored to out[i * ldo + j].
-struct DistEpi {
-    struct Params {
-        GridTiles g;
-        size_t m, n;
-        const float *r1, *r2, *c1, *c2;
-        float *out;
-        size_t ldo;
-    };
-    __device__ static int tiles(const Params &p) { return GridTiles::count(p.g.num_tiles); }
-    __device__ static void tile_at(const Params &p, int t, int &mb, int &nb) { p.g.at(t, mb, nb); }
-    struct State {
-        int rit;
-        bool vec;
-        __device__ State(const Params &p, int row_in_tile)
-            : rit(row_in_tile),
-              vec(((p.ldo & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0)) {}
-        __device__ void tile(const Params &p, int mb, int nb, uint32_t y0, uint32_t) {
-            const size_t row = (size_t)mb * TC_BM + rit;
-            const bool row_ok = row < p.m;
-            const float rr1 = row_ok ? __ldg(p.r1 + row) : 0.0f;
-            const float rr2 = row_ok ? __ldg(p.r2 + row) : 0.0f;
-            float *orow = p.out + row * p.ldo;
-#pragma unroll 1
-            for (int ch = 0; ch < TC_BN / 32; ++ch) {
-                float c[32];
-                ld_sum32(y0 + 32 * ch, c);
-                const size_t col0 = (size_t)nb * TC_BN + ch * 32;
-                if (!row_ok || col0 >= p.n) continue;
-                float dv[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const size_t col = col0 + j < p.n ? col0 + j : p.n - 1;
-                    const float ipt = __fmul_rn(__fmul_rn(c[j], rr1), __ldg(p.c1 + col));
-                    const float d = __fsub_rn(__fadd_rn(rr2, __ldg(p.c2 + col)), __fmul_rn(2.0f, ipt));
-                    dv[j] = d > 0.0f ? d : 0.0f;
-                }
-                if (vec && col0 + 32 <= p.n) {
-                    float4 *o4 = reinterpret_cast<float4 *>(orow + col0);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        o4[j] = make_float4(dv[4 * j], dv[4 * j + 1], dv[4 * j + 2], dv[4 * j + 3]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (col0 + j < p.n) orow[col0 + j] = dv[j];
-                }
-            }
-        }
-        __device__ void finish(const Params &) {}
-    };
-};
-
 // ---------------------------------------------------------------------------
-// tcw_kernel: the M x N distances and the serving top-k with 128 x 256 tiles
-// (epilogue policies WDist, WTopk).  A 128 x 128 tile
+// tcw_kernel: the serving top-k with 128 x 256 tiles (epilogue policies WTopk,
+// WTopkD, WThreshD).  A 128 x 128 tile
 // with three operand reads per K step needs more shared-memory bandwidth than
 // the SM has once the TMA writes are counted (128 B/clk of MMA operands + 85
 // B/clk of copies), which held tcp_kernel near half of the tensor cycles; a
@@ -710,7 +558,7 @@ struct DistEpi {
 // warps, two per lane quadrant, each thread one row and 128 of the columns.
 // The promotion loads a chunk in 16-column pieces, the next piece in flight
 // while the current one is added, so that the MMAs seldom wait for a chunk
-// buffer; the distances are written from the registers.  Otherwise as
+// buffer.  Otherwise as
 // tcp_kernel (promoted chunks of CH K blocks, bounded waits).
 // ---------------------------------------------------------------------------
 constexpr int TW_BN = 256;
@@ -1198,49 +1046,6 @@ struct ThreshEpi {
 
 // ---- epilogue policies of tcw_kernel: each thread holds one row's running
 // sums of TW_COLS columns (half h of the 256-column tile) in registers.
-struct WDist {
-    static constexpr bool kDirect = false;  // running sums promoted into registers
-    using Params = DistEpi::Params;
-    __device__ static int tiles(const Params &p) { return GridTiles::count(p.g.num_tiles); }
-    __device__ static void tile_at(const Params &p, int t, int &mb, int &nb) { p.g.at(t, mb, nb); }
-    struct State {
-        int rit, h;
-        bool vec;
-        __device__ State(const Params &p, int row_in_tile, int half)
-            : rit(row_in_tile), h(half),
-              vec(((p.ldo & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0)) {}
-        // d = max(0, r2 + c2 - 2 (C r1) c1) from the registers
-        __device__ void tile(const Params &p, int mb, int nb, const float (&y)[TW_COLS]) {
-            const size_t row = (size_t)mb * TC_BM + rit;
-            if (row >= p.m) return;
-            const float rr1 = __ldg(p.r1 + row), rr2 = __ldg(p.r2 + row);
-            float *orow = p.out + row * p.ldo;
-            const size_t cbase = (size_t)nb * TW_BN + TW_COLS * h;
-#pragma unroll
-            for (int g = 0; g < TW_COLS / 4; ++g) {  // groups of 4 columns
-                const size_t col0 = cbase + 4 * g;
-                if (col0 >= p.n) break;
-                float dv[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const size_t col = col0 + u < p.n ? col0 + u : p.n - 1;
-                    const float ipt = __fmul_rn(__fmul_rn(y[4 * g + u], rr1), __ldg(p.c1 + col));
-                    const float d = __fsub_rn(__fadd_rn(rr2, __ldg(p.c2 + col)), __fmul_rn(2.0f, ipt));
-                    dv[u] = d > 0.0f ? d : 0.0f;
-                }
-                if (vec && col0 + 4 <= p.n) {
-                    *reinterpret_cast<float4 *>(orow + col0) = make_float4(dv[0], dv[1], dv[2], dv[3]);
-                } else {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (col0 + u < p.n) orow[col0 + u] = dv[u];
-                }
-            }
-        }
-        __device__ void finish(const Params &) {}
-    };
-};
-
 // The top-k over 256-wide column tiles: each thread keeps the best k of its
 // half of the columns, so a (row, slice) has two partial lists, written to
 // part_d / part_i [((cta * 128 + row) * 2 + half)][kCandMax].  The list lives
@@ -1629,33 +1434,6 @@ __global__ void bounded_wait_selftest_kernel(int *err, long long budget_cycles) 
     }
 }
 
-// ---- host: tensor maps ------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    });
-    return fn;
-}
-
-bool make_map(CUtensorMap *map, const void *base, int K, size_t rows, int box_rows) {
-    auto fn = encode_fn();
-    if (!fn) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box,
-              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // FP32 planes (TF32 operands): K x rows, 32-value (128-byte) boxes, 128-byte swizzle.
 bool make_map_f32(CUtensorMap *map, const void *base, int K, size_t rows, int box_rows) {
     auto fn = encode_fn();
@@ -1696,19 +1474,6 @@ cudaError_t tcw_launch(const TcMaps &maps, const TcShape &sh, const typename W::
     if (e != cudaSuccess) return e;
     kern<<<grid, TW_THREADS, smem, st>>>(maps, sh, ep, err);
     return cudaGetLastError();
-}
-
-bool aligned16(std::initializer_list<const void *> ps) {
-    for (const void *p : ps)
-        if (reinterpret_cast<uintptr_t>(p) & 15) return false;
-    return true;
-}
-
-unsigned sm_grid(size_t tiles) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return (unsigned)(tiles < (size_t)sms ? tiles : (size_t)sms);
 }
 
 // BF16 planes of one K segment: A (K x m_pad), B hi (K x n_pad), B lo (k_lo x n_pad).
@@ -1914,68 +1679,6 @@ cudaError_t launch_topk_merge(const int *m_dev, int grid_ctas, int lists, const 
     topk_merge_kernel<<<blocks ? blocks : 1, 32 * wpb, 0, st>>>(m_dev, lists, grid_ctas, part_d,
                                                                 part_i, k, out_d, out_i);
     return cudaGetLastError();
-}
-
-cudaError_t launch_tc_dist(const void *Ah, const void *Al, const void *Bh, const void *Bl, int K,
-                           int k_lo, size_t m, size_t m_pad, size_t n, size_t n_pad,
-                           const float *r1, const float *r2, const float *c1, const float *c2,
-                           float *out, size_t ldo, int *err, cudaStream_t st) {
-    if (m == 0 || n == 0) return cudaSuccess;
-    if (K % TC_BK || k_lo % TC_BK || k_lo <= 0 || k_lo > K || m_pad % TC_BM || n_pad % TC_BN ||
-        m > m_pad || n > n_pad)
-        return cudaErrorInvalidValue;
-    if (!aligned16({Ah, Al, Bh, Bl})) return cudaErrorMisalignedAddress;
-    alignas(64) TcMaps mp;
-    TcShape sh{};
-    if (!bf16_maps(mp, sh, Ah, Al, m_pad, Bh, Bl, n_pad, K, k_lo)) return cudaErrorInvalidValue;
-    const unsigned num_mb = (unsigned)(m_pad / TC_BM);
-    const size_t tiles = (size_t)num_mb * (n_pad / TC_BN);
-    if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;
-    if (n_pad % TW_BN == 0) {
-        // 128 x 256 tiles (tcw_kernel): B maps with 256-row boxes
-        if (!make_map(&mp.m[0][2], Bh, K, n_pad, TW_BN) || !make_map(&mp.m[0][3], Bl, k_lo, n_pad, TW_BN))
-            return cudaErrorInvalidValue;
-        const size_t wtiles = (size_t)num_mb * (n_pad / TW_BN);
-        const DistEpi::Params ep{GridTiles{num_mb, (unsigned)wtiles}, m, n, r1, r2, c1, c2, out, ldo};
-        // Chunk length: asymmetric planes (B lo narrower than K: a query against
-        // codes) take 8 K blocks per chunk; symmetric planes, whose code-against-
-        // itself terms are squares of centroid values, 4 (their drift per chunk
-        // is larger against a BF16-pair floor of 5-7e-6).
-        if (k_lo < K) return tcw_launch<WDist, 8>(mp, sh, ep, err, sm_grid(wtiles), st);
-        return tcw_launch<WDist, 4>(mp, sh, ep, err, sm_grid(wtiles), st);
-    }
-    const DistEpi::Params ep{GridTiles{num_mb, (unsigned)tiles}, m, n, r1, r2, c1, c2, out, ldo};
-    return tcp_launch<false, 3, 4, true, DistEpi>(mp, sh, ep, err, sm_grid(tiles), st);
-}
-
-bool tc_dist_dec_fits(int cs) {
-    DecSrc d;
-    d.cs = cs;
-    return cs > 0 && with_code_buffers(d, 2).cbufs > 0;
-}
-
-cudaError_t launch_tc_dist_dec(const void *Ah, const void *Al, size_t m, size_t m_pad, const DecSrc &dec,
-                               size_t n_pad, int K, const float *r1, const float *r2, const float *c1,
-                               const float *c2, float *out, size_t ldo, int *err, cudaStream_t st) {
-    if (m == 0 || dec.n == 0) return cudaSuccess;
-    const bool sym = dec.fc == nullptr;
-    if (K % TC_BK || m_pad % TC_BM || n_pad % TC_BN || m > m_pad || dec.n > n_pad || !dec_ok(dec, K))
-        return cudaErrorInvalidValue;
-    // symmetric: the whole K is centroid values; asymmetric: centroid half + sign half
-    if (sym ? dec.kbc != K / TC_BK : (dec.kbc * 2 != K / TC_BK || !dec.fs)) return cudaErrorInvalidValue;
-    if (!aligned16({Ah, Al})) return cudaErrorMisalignedAddress;
-    alignas(64) TcMaps mp;
-    TcShape sh{};
-    if (!a_maps(mp, sh, Ah, Al, m_pad, K, dec.kbc)) return cudaErrorInvalidValue;
-    const unsigned num_mb = (unsigned)(m_pad / TC_BM);
-    const size_t tiles = (size_t)num_mb * (n_pad / TC_BN);
-    if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;
-    const DecSrc d = with_code_buffers(dec, 2);
-    if (d.cbufs == 0) return cudaErrorInvalidValue;  // the code tile does not fit beside the stages
-    const DistEpi::Params ep{GridTiles{num_mb, (unsigned)tiles}, m, dec.n, r1, r2, c1, c2, out, ldo};
-    // chunk lengths as the planes kernels: 8 K blocks asymmetric, 4 symmetric
-    if (sym) return tcp_launch<false, 2, 4, true, DistEpi, true>(mp, sh, ep, err, sm_grid(tiles), st, d);
-    return tcp_launch<false, 2, 8, true, DistEpi, true>(mp, sh, ep, err, sm_grid(tiles), st, d);
 }
 
 cudaError_t launch_tc_symq(const void *A1h, const void *A1l, const void *B1h, const void *B1l,
