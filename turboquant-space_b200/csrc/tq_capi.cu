@@ -247,13 +247,14 @@ class MtonRunner {
     // beside two 64 KB stages in shared memory.
     static constexpr size_t kDecMaxCode = 756;
     // FP32: the tensor-core kernel, except where the scan kernel's single launch
-    // is faster (us a call, scan / tensor-core): one or two rows, whose decode
-    // is not shared (384-d 4-bit, 200,000 codes: 38 / 151 for one row, 111 / 151
-    // for two, 394 / 153 for eight), and few rows against few codes, where the
+    // per row is faster (us a call, scan / tensor-core): few rows, which do not
+    // pay for the decode of every code (200,000 codes: 384-d 4-bit 38 / 105 for
+    // one row, 111 / 105 for two, 394 / 107 for eight; 768-d 8-bit 113 / 252 for
+    // two, 378 / 252 for eight), and few rows against few codes, where the
     // row-plane launch shows (8 x 1,000: 32 / 36; 8 x 30,000: 76 / 46).
     bool use_cg(size_t n) const {
-        if (sp_->D < 16 || m_ <= 2) return false;
-        return m_ > 8 || m_ * n * sp_->D > (size_t(1) << 24);
+        if (sp_->D < 16 || m_ <= (sp_->P.nibble ? 2 : 4)) return false;
+        return m_ > 8 || m_ * n * sp_->D > (size_t(1) << 25);
     }
     int form() const { return sym_ ? tq::kCgSym : tq::kCgAsym; }
     int fmt() const { return bf16_ ? tq::kCgBF16 : tq::kCgFP16; }

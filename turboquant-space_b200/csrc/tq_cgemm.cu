@@ -31,13 +31,22 @@
 //
 // Accumulation: the MMAs of a chunk of K blocks accumulate from zero in one of
 // two tensor-memory buffers (the tensor core's FP32 accumulation truncates
-// toward zero, about 2^-24 of the running sum an MMA); the epilogue warps add
+// toward zero, about 2^-24 of the running sum an MMA; a block's small products
+// run before its hi hi ones, while the sum is small); the epilogue warps add
 // each finished chunk into FP32 registers with IEEE adds while the other
 // buffer fills.
 //
+// CTA pairs: wide tiles (NT > 64) run on clusters of two CTAs, 256 codes by NT
+// rows, tcgen05.mma.cta_group::2: each CTA decodes its 128 codes and loads half
+// of the rows' tile, so a K block's shared-memory traffic per CTA (MMA operand
+// reads + copies + decode) is 162 KB in 1536 clocks, under the 128 B/clk that
+// one CTA alone (243 KB) exceeded.
+//
 // Persistent, one CTA per SM, 16 warps:
 //   warp 0       TMA producer of the row operand's K blocks
-//   warp 1       allocates tensor memory; one thread issues the MMAs
+//   warp 1       allocates tensor memory; one thread issues the MMAs (in the
+//                other CTA of a pair it reports that CTA's stages)
+//   warps 2, 3   load the tiles' code words into a small ring (cp.async)
 //   warps 4..    DW decoder warps
 //   the rest     epilogue warps (two per lane quadrant, or one for NT <= 64)
 // Every mbarrier wait is bounded and ends in a status code (tq_async.cuh).
@@ -45,6 +54,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "tq_cgemm.h"
 #include "tq_tc.cuh"
@@ -59,7 +69,9 @@ constexpr int CG_THREADS = 512;
 constexpr int CG_MAX_STAGES = 6;
 constexpr int CG_TAB_BYTES = 128 * 128;    // byte codes: 128 entries x 32 lanes x (hi | lo << 16)
 constexpr int CG_SMEM_MAX = 227 * 1024;
-constexpr int CG_FIXED = 1024 /* alignment */ + 256 /* barriers */;
+constexpr int CG_MAX_RING = 8;             // K blocks of code words in flight
+constexpr int CG_BAR_BYTES = 384;
+constexpr int CG_FIXED = 1024 /* alignment */ + CG_BAR_BYTES;
 constexpr int kErrFull = 1, kErrEmpty = 2, kErrTmemFull = 3, kErrTmemEmpty = 4;
 
 // FP16 scalings: |q_rot|, |s_q| <= 1 and |c| < 5 (Lloyd-Max of N(0,1), at most
@@ -86,7 +98,7 @@ struct CgArgs {
     int fmt, form;
     int KBm, KB;         // K blocks of the centroid part, of all
     int chm, chs;        // K blocks per accumulation chunk: centroid part, sign part
-    int NT, stages;      // row columns per tile, pipeline stages
+    int NT, stages, ring;  // row columns per tile, pipeline stages, code-word ring slots
     unsigned num_nt, num_tiles;
     size_t m;
     const float4 *rs;    // per row: r1, r2, s1, s2
@@ -97,18 +109,59 @@ struct CgArgs {
     int *err;
 };
 
-__device__ __forceinline__ void umma16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                       uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
+// 4-byte asynchronous copy (zeros for bytes = 0); the surrounding 128 bytes
+// are fetched into L2 with it (the next K blocks of the same code).
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global.L2::128B [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+                 : "memory");
 }
+// Arrives on `bar` once this thread's copies so far have landed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__device__ __forceinline__ int cg_chunk_end(const CgArgs &p, int c0) {
-    return c0 < p.KBm ? min(c0 + p.chm, p.KBm) : min(c0 + p.chs, p.KB);
+// The K blocks of a tile in the order they run: the asymmetric form's sign part
+// first, so that its one long chunk covers the previous tile's output; the
+// light form's last, since its sums are not added to the centroid part's.
+template <bool LIGHT>
+struct CgOrder {
+    int KBm, KB, ns;  // ns: sign blocks that run first
+    __device__ explicit CgOrder(const CgArgs &p) : KBm(p.KBm), KB(p.KB), ns(LIGHT ? 0 : p.KB - p.KBm) {}
+    __device__ bool cent(int kb) const { return LIGHT ? kb < KBm : kb >= ns; }
+    // block index within its part, and in the row planes (centroid part first)
+    __device__ int part(int kb) const { return LIGHT ? (kb < KBm ? kb : kb - KBm) : (kb < ns ? kb : kb - ns); }
+    __device__ int plane(int kb) const { return LIGHT ? kb : (kb < ns ? KBm + kb : kb - ns); }
+    // end of the accumulation chunk that starts at c0
+    __device__ int chunk_end(const CgArgs &p, int c0) const {
+        if (cent(c0)) return min(c0 + p.chm, LIGHT ? KBm : KB);
+        return min(c0 + p.chs, LIGHT ? KB : ns);
+    }
+};
+
+template <bool PAIR>
+__device__ __forceinline__ void tmem_alloc(uint32_t slot) {
+    if constexpr (PAIR) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+}
+template <bool PAIR>
+__device__ __forceinline__ void tmem_dealloc(uint32_t base) {
+    if constexpr (PAIR)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512) : "memory");
+    else
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512) : "memory");
+}
+template <bool PAIR>
+__device__ __forceinline__ void commit(uint32_t bar) {
+    if constexpr (PAIR) umma_commit_pair(bar);
+    else umma_commit(bar);
 }
 
 // One of the registers' byte tables of a nibble decoder: entries 0..7, the low
@@ -154,10 +207,25 @@ __device__ __forceinline__ uint4 byte_sign(uint32_t x0, uint32_t x1, uint32_t on
     return r;
 }
 
+// f(k, x) for at least the first `cols` of CPT columns of a chunk buffer, in
+// pieces of 32 (a piece past `cols` holds values that are not used).
+template <int CPT, class F>
+__device__ __forceinline__ void chunk_pieces(uint32_t X, int cols, F f) {
+#pragma unroll
+    for (int pc = 0; pc < CPT / 32; ++pc) {
+        if (32 * pc >= cols) break;
+        uint32_t x[32];
+        __syncwarp();
+        tmem_ld32(X + 32 * pc, x);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) f(32 * pc + j, __uint_as_float(x[j]));
+    }
+}
+
 // DW: decoder warps (warps 4 .. 4 + DW - 1); the other 12 - DW warps are the
 // epilogue: two column halves of 128 (DW = 4), or one of 64 (DW = 8).  Batches
 // of few rows are bound by the decoders, wide ones by the MMAs.
-template <int DW, bool NIB>
+template <int DW, bool NIB, bool LIGHT, bool PAIR>
 __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_constant__ CUtensorMap map_h,
                                                               const __grid_constant__ CUtensorMap map_l,
                                                               const CgArgs p) {
@@ -166,34 +234,42 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
     constexpr int CPT = DW == 4 ? 128 : 64;  // columns per epilogue thread, at most
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int stage_bytes = 2 * CG_A_BYTES + 2 * p.NT * 128;
+    const uint32_t rank = PAIR ? cluster_rank() : 0u;
+    const int bt_bytes = p.NT * (PAIR ? 64 : 128);  // this CTA's rows of one B tile
+    const int stage_bytes = 2 * CG_A_BYTES + 2 * bt_bytes;
     const uint32_t tiles0 = smem_u32(smem);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + p.stages * stage_bytes);
-    // bars: full[6], empty[6], xfull[2], xempty[2], drain; then the TMEM slot
+    // bars: full[6], empty[6], xfull[2], xempty[2], drain, cfull[8], cempty[8], pfull[6]; then the TMEM slot
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * CG_MAX_STAGES;
     const uint32_t xfull0 = empty0 + 8 * CG_MAX_STAGES, xempty0 = xfull0 + 16, drain = xempty0 + 16;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * CG_MAX_STAGES + 5);
-    uint32_t *btab = reinterpret_cast<uint32_t *>(smem + p.stages * stage_bytes + 256);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t cfull0 = drain + 8, cempty0 = cfull0 + 8 * CG_MAX_RING;
+    const uint32_t pfull0 = cempty0 + 8 * CG_MAX_RING;  // PAIR, rank 0: the other CTA's stage is full
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * CG_MAX_STAGES + 5 + 2 * CG_MAX_RING);
+    // the ring of code words, then the byte codes' table
+    constexpr int WPI = NIB ? 1 : 2;                 // words of 8 coordinates
+    constexpr int RING_BYTES = CG_BM * 32 * WPI;     // one K block's words
+    unsigned char *ring = smem + p.stages * stage_bytes + CG_BAR_BYTES;
+    const uint32_t ring0 = smem_u32(ring);
+    uint32_t *btab = reinterpret_cast<uint32_t *>(ring + p.ring * RING_BYTES);
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(full0 + 8 * s, 1 + DW);  // the producer and one lane of each decoder warp
             mbar_init(empty0 + 8 * s, 1);
+            mbar_init(pfull0 + 8 * s, 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(xfull0 + 8 * b, 1);
-            mbar_init(xempty0 + 8 * b, EW);
+            mbar_init(xempty0 + 8 * b, PAIR ? 2 * EW : EW);  // PAIR: rank 0's counts both CTAs'
+        }
+        for (int k = 0; k < p.ring; ++k) {
+            mbar_init(cfull0 + 8 * k, 64);  // every loader thread
+            mbar_init(cempty0 + 8 * k, DW);
         }
         mbar_init(drain, 1);
         mbar_init_fence();
     }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_u32(tmem_slot)),
-                     "r"(512)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    if (warp == 1) tmem_alloc<PAIR>(smem_u32(tmem_slot));
     if constexpr (!NIB) {
         // entry v of lane l at btab[32 v + l]: hi | lo << 16
         for (int i = threadIdx.x; i < 128 * 32; i += CG_THREADS) {
@@ -205,30 +281,35 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         }
     }
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) cluster_sync();  // the other CTA's barriers and tensor memory too
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const int KB = p.KB, KBm = p.KBm;
-    const unsigned grid = gridDim.x;
+    const int KB = p.KB;
+    const CgOrder<LIGHT> ord(p);
+    // tiles of this CTA (or pair): t0, t0 + grid, ...; this CTA's first code of tile t
+    const unsigned grid = PAIR ? gridDim.x >> 1 : gridDim.x, t0 = PAIR ? blockIdx.x >> 1 : blockIdx.x;
+    auto first_code = [&](unsigned t) {
+        return (size_t)(t % p.num_nt) * (PAIR ? 2 * CG_BM : CG_BM) + rank * CG_BM;
+    };
 
-    // Register shares (DW = 4): 48 + 96 + 2 x 184 = 4 x 128, the launch's total.
+    // Register shares (DW = 4): 64 + 80 + 2 x 184 = 4 x 128, the launch's total.
     if (warp < 4) {
-        if constexpr (DW == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+        if constexpr (DW == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
         if (warp == 0) {
             // ---------------- TMA producer: the rows' K blocks ----------------
             if (lane == 0) {
                 uint32_t s = 0, ph = 1;
                 uint32_t it = 0;
                 bool ok = true;
-                const uint32_t bytes = 2u * (uint32_t)p.NT * 128u;
-                for (unsigned t = blockIdx.x; t < p.num_tiles && ok; t += grid) {
-                    const int mb = (int)(t / p.num_nt);
+                for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
+                    const int row = (int)((t / p.num_nt) * p.NT + rank * (p.NT / 2));
                     for (int kb = 0; kb < KB; ++kb, ++it) {
                         if (!mbar_wait(empty0 + 8 * s, ph, p.err, kErrEmpty)) { ok = false; break; }
                         const uint32_t b = tiles0 + s * stage_bytes + 2 * CG_A_BYTES, fb = full0 + 8 * s;
-                        mbar_expect_tx(fb, bytes);
-                        tma_load_2d(b, &map_h, kb * CG_BK, mb * p.NT, fb);
-                        tma_load_2d(b + p.NT * 128, &map_l, kb * CG_BK, mb * p.NT, fb);
+                        mbar_expect_tx(fb, 2u * bt_bytes);
+                        tma_load_2d(b, &map_h, ord.plane(kb) * CG_BK, row, fb);
+                        tma_load_2d(b + bt_bytes, &map_l, ord.plane(kb) * CG_BK, row, fb);
                         if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
                     }
                 }
@@ -238,62 +319,123 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
                     mbar_drain(full0 + 8 * (j % p.stages), (j / p.stages) & 1u);
                 }
             }
+        } else if (warp == 1 && rank != 0) {
+            // ---------------- PAIR, rank 1: reports each full stage to rank 0 ----------------
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
+                for (int kb = 0; kb < KB; ++kb) {
+                    if (!mbar_wait_warp(full0 + 8 * s, ph, p.err, kErrFull)) { ok = false; break; }
+                    if (lane == 0) mbar_arrive_cluster(rank0_addr(pfull0 + 8 * s));
+                    if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
+                }
+            }
+            // the pair's last commit: nothing of rank 0's is under way to this CTA's barriers
+            if (lane == 0) mbar_drain(drain, 0);
+            __syncwarp();
         } else if (warp == 1) {
             // ---------------- MMA issuer ----------------
-            if (lane == 0) {
-                const uint32_t f = p.fmt == kCgFP16 ? 0u : 1u;
-                const uint32_t idesc = (1u << 4) | (f << 7) | (f << 10) | ((uint32_t)(p.NT >> 3) << 17) |
-                                       ((uint32_t)(CG_BM >> 4) << 24);
-                const bool one_sign = p.form == kCgLight;  // +-1 rows: their lo is zero
-                uint32_t s = 0, ph = 0, gc = 0;
-                bool ok = true;
-                for (unsigned t = blockIdx.x; t < p.num_tiles && ok; t += grid) {
-                    for (int c0 = 0, c1 = 0; c0 < KB && ok; c0 = c1, ++gc) {
-                        c1 = cg_chunk_end(p, c0);
-                        const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
-                        if (!mbar_wait(xempty0 + 8 * b, xph ^ 1u, p.err, kErrTmemEmpty)) { ok = false; break; }
+            // The whole warp runs the loop, so that descriptors stay in uniform
+            // registers; one elected lane issues.
+            const bool lead = elect_one();
+            const uint32_t f = p.fmt == kCgFP16 ? 0u : 1u;
+            const uint32_t idesc = (1u << 4) | (f << 7) | (f << 10) | ((uint32_t)(p.NT >> 3) << 17) |
+                                   ((uint32_t)((PAIR ? 2 * CG_BM : CG_BM) >> 4) << 24);
+            constexpr bool one_sign = LIGHT;  // +-1 rows: their lo is zero
+            const uint32_t ab = CG_A_BYTES >> 4, bb = (uint32_t)bt_bytes >> 4;
+            uint32_t s = 0, ph = 0, gc = 0;
+            bool ok = true;
+            for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
+                for (int c0 = 0, c1 = 0; c0 < KB && ok; c0 = c1, ++gc) {
+                    c1 = ord.chunk_end(p, c0);
+                    const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
+                    if (!(PAIR ? mbar_wait_cluster_warp(xempty0 + 8 * b, xph ^ 1u, p.err, kErrTmemEmpty)
+                               : mbar_wait_warp(xempty0 + 8 * b, xph ^ 1u, p.err, kErrTmemEmpty))) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t d = tmem_base + b * 256u;
+                    uint32_t acc = 0u;
+                    for (int kb = c0; kb < c1; ++kb) {
+                        if (!mbar_wait_warp(full0 + 8 * s, ph, p.err, kErrFull)) { ok = false; break; }
+                        if (PAIR && !mbar_wait_cluster_warp(pfull0 + 8 * s, ph, p.err, kErrFull)) { ok = false; break; }
                         tc_fence_after();
-                        const uint32_t d = tmem_base + b * 256u;
-                        uint32_t acc = 0u;
-                        for (int kb = c0; kb < c1; ++kb) {
-                            if (!mbar_wait(full0 + 8 * s, ph, p.err, kErrFull)) { ok = false; break; }
-                            tc_fence_after();
-                            const uint32_t ah = tiles0 + s * stage_bytes, al = ah + CG_A_BYTES;
-                            const uint32_t bh = al + CG_A_BYTES, bl = bh + p.NT * 128;
-                            const bool cent = kb < KBm;
+                        const uint32_t ah = sw128_desc_lo(tiles0 + s * stage_bytes), al = ah + ab;
+                        const uint32_t bh = al + ab, bl = bh + bb;
+                        if (lead) {
+                            // one MMA's K: 32 bytes.  The block's small products first: each
+                            // MMA truncates the sum, and it is small until hi hi joins.
+                            if (ord.cent(kb)) {
+#pragma unroll
+                                for (int kk = 0; kk < 4; ++kk) {
+                                    umma_f16<PAIR>(d, al + 2 * kk, bh + 2 * kk, idesc, acc);
+                                    acc = 1u;
+                                }
+#pragma unroll
+                                for (int kk = 0; kk < 4; ++kk) umma_f16<PAIR>(d, ah + 2 * kk, bl + 2 * kk, idesc, 1u);
+                            } else if (!one_sign) {
+#pragma unroll
+                                for (int kk = 0; kk < 4; ++kk) {
+                                    umma_f16<PAIR>(d, ah + 2 * kk, bl + 2 * kk, idesc, acc);
+                                    acc = 1u;
+                                }
+                            }
 #pragma unroll
                             for (int kk = 0; kk < 4; ++kk) {
-                                const uint32_t ko = kk * 32;  // one MMA's K: 32 bytes
-                                // the small products first, while the sum is smaller
-                                if (cent) {
-                                    umma16(d, sw128_desc(al + ko), sw128_desc(bh + ko), idesc, acc);
-                                    acc = 1u;
-                                }
-                                if (cent || !one_sign) {
-                                    umma16(d, sw128_desc(ah + ko), sw128_desc(bl + ko), idesc, acc);
-                                    acc = 1u;
-                                }
-                                umma16(d, sw128_desc(ah + ko), sw128_desc(bh + ko), idesc, acc);
+                                umma_f16<PAIR>(d, ah + 2 * kk, bh + 2 * kk, idesc, acc);
                                 acc = 1u;
                             }
-                            umma_commit(empty0 + 8 * s);
-                            if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
+                            commit<PAIR>(empty0 + 8 * s);
                         }
-                        if (ok) umma_commit(xfull0 + 8 * b);
+                        acc = 1u;
+                        if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
                     }
+                    if (ok && lead) commit<PAIR>(xfull0 + 8 * b);
                 }
-                // every MMA issued must be complete before the tensor memory is freed
-                umma_commit(drain);
+            }
+            // every MMA issued must be complete before the tensor memory is freed
+            if (lead) {
+                commit<PAIR>(drain);
                 mbar_drain(drain, 0);
             }
+            __syncwarp();
+        } else {
+            // ---------------- code loaders (warps 2, 3) ----------------
+            // The words of each K block go to a small ring by 4-byte cp.async (a
+            // code is only 4-byte aligned): lane l takes word l & 7 of rows
+            // 4 i + (l >> 3).  They are warps of their own because a decoder's
+            // proxy fence waits for its own loads in flight.
+            const int r0 = (warp - 2) * 64 + (lane >> 3), c = lane & 7;
+            uint32_t cs = 0, cph = 1;
+            bool ok = true;
+            for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
+                const size_t j0 = min(first_code(t), p.n - 1);
+                const uint8_t *base = p.codes + j0 * (size_t)p.cs;
+                const int last = (int)min((size_t)(CG_BM - 1), p.n - 1 - j0);  // rows past n repeat the last code
+                for (int kb = 0; kb < KB; ++kb) {
+                    if (!mbar_wait_warp(cempty0 + 8 * cs, cph, p.err, kErrEmpty)) { ok = false; break; }
+                    const uint32_t dst = ring0 + cs * RING_BYTES;
+                    const int o = ord.part(kb) * (32 * WPI) + 4 * c;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const int r = r0 + 4 * i;
+                        const uint8_t *src = base + min(r, last) * p.cs + o;
+#pragma unroll
+                        for (int q = 0; q < WPI; ++q)  // zero beyond the packed bytes (D < 64)
+                            cp_async4(dst + r * (32 * WPI) + 32 * q + 4 * c, src + 32 * q,
+                                      o + 32 * q < p.pb ? 4u : 0u);
+                    }
+                    cp_async_arrive(cfull0 + 8 * cs);
+                    if (++cs == (uint32_t)p.ring) { cs = 0; cph ^= 1u; }
+                }
+            }
+            cp_async_wait_all();
         }
     } else if (warp < 4 + DW) {
         // ---------------- decoders ----------------
         // Warp w decodes rows RPW w ..: lane l takes 16-byte chunk l & 7 (8
         // coordinates) of rows 4 i + (l >> 3), so eight lanes read a row's
         // consecutive words and write its 128 bytes without bank conflicts.
-        if constexpr (DW == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
-        constexpr int RPW = CG_BM / DW, ITEMS = RPW / 4, WPI = NIB ? 1 : 2;
+        if constexpr (DW == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+        constexpr int RPW = CG_BM / DW, ITEMS = RPW / 4;
         const int r0 = (warp - 4) * RPW + (lane >> 3), c = lane & 7;
         NibTab tab{};
         if constexpr (NIB) {
@@ -311,37 +453,29 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         }
         const uint32_t one = p.fmt == kCgFP16 ? 0x3C003C00u : 0x3F803F80u;
         const uint32_t *tl = btab + lane;
-        // the words of K block kb of tile t (zero beyond the packed bytes: D < 64)
-        auto load = [&](uint32_t (&w)[ITEMS][WPI], unsigned t, int kb) {
-            const size_t j0 = (size_t)(t % p.num_nt) * CG_BM;
-            const int o = ((kb < KBm ? kb : kb - KBm) * 8 + c) * 4 * WPI;
-#pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                size_t row = j0 + r0 + 4 * i;
-                if (row >= p.n) row = p.n - 1;
-                const uint8_t *src = p.codes + row * (size_t)p.cs + o;
-#pragma unroll
-                for (int q = 0; q < WPI; ++q)
-                    w[i][q] = o + 4 * q < p.pb ? __ldg(reinterpret_cast<const uint32_t *>(src) + q) : 0u;
-            }
-        };
-        uint32_t s = 0, ph = 1;
+        uint32_t s = 0, ph = 1, cs = 0, cph = 0;
         bool ok = true;
-        uint32_t w[ITEMS][WPI], nw[ITEMS][WPI];
-        if (blockIdx.x < p.num_tiles) load(w, blockIdx.x, 0);
-        for (unsigned t = blockIdx.x; t < p.num_tiles && ok; t += grid) {
+        for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
             for (int kb = 0; kb < KB; ++kb) {
-                // the next block's words are in flight while this one is decoded
-                if (kb + 1 < KB) load(nw, t, kb + 1);
-                else if (t + grid < p.num_tiles) load(nw, t + grid, 0);
-                if (!mbar_wait(empty0 + 8 * s, ph, p.err, kErrEmpty)) { ok = false; break; }
-                unsigned char *base = smem + s * stage_bytes;
-                const bool cent = kb < KBm;
+                if (!mbar_wait_warp(cfull0 + 8 * cs, cph, p.err, kErrFull)) { ok = false; break; }
+                uint32_t w[ITEMS][WPI];
+                const unsigned char *rb = ring + cs * RING_BYTES;
 #pragma unroll
                 for (int i = 0; i < ITEMS; ++i) {
-                    const int r = r0 + 4 * i;
-                    unsigned char *dst = base + r * 128 + ((c ^ (r & 7)) << 4);
-                    if (cent) {
+                    if constexpr (NIB) {
+                        w[i][0] = *reinterpret_cast<const uint32_t *>(rb + (r0 + 4 * i) * 32 + 4 * c);
+                    } else {
+                        const uint2 v = *reinterpret_cast<const uint2 *>(rb + (r0 + 4 * i) * 64 + 8 * c);
+                        w[i][0] = v.x;
+                        w[i][WPI - 1] = v.y;
+                    }
+                }
+                if (!mbar_wait_warp(empty0 + 8 * s, ph, p.err, kErrEmpty)) { ok = false; break; }
+                unsigned char *dst = smem + s * stage_bytes + r0 * 128;
+                const int sw = (c ^ (r0 & 7)) << 4;  // the chunk's place in a row; rows 4 apart flip bit 6
+                if (ord.cent(kb)) {
+#pragma unroll
+                    for (int i = 0; i < ITEMS; ++i) {
                         uint4 hi, lo;
                         if constexpr (NIB) {
                             nib_cent(w[i][0], tab, hi, lo);
@@ -355,23 +489,27 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
                             lo = make_uint4(__byte_perm(e[0], e[1], 0x7632u), __byte_perm(e[2], e[3], 0x7632u),
                                             __byte_perm(e[4], e[5], 0x7632u), __byte_perm(e[6], e[7], 0x7632u));
                         }
-                        *reinterpret_cast<uint4 *>(dst) = hi;
-                        *reinterpret_cast<uint4 *>(dst + CG_A_BYTES) = lo;
-                    } else {
+                        unsigned char *d = dst + 512 * i + (sw ^ ((i & 1) << 6));
+                        *reinterpret_cast<uint4 *>(d) = hi;
+                        *reinterpret_cast<uint4 *>(d + CG_A_BYTES) = lo;
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < ITEMS; ++i) {
                         uint4 v;
                         if constexpr (NIB) v = nib_sign(w[i][0], one);
                         else v = byte_sign(w[i][0], w[i][WPI - 1], one);
-                        *reinterpret_cast<uint4 *>(dst) = v;
+                        *reinterpret_cast<uint4 *>(dst + 512 * i + (sw ^ ((i & 1) << 6))) = v;
                     }
                 }
                 fence_proxy_async_smem();  // the generic stores before the MMAs' async reads
                 __syncwarp();
-                if (lane == 0) mbar_arrive(full0 + 8 * s);
+                if (lane == 0) {
+                    mbar_arrive(full0 + 8 * s);
+                    mbar_arrive(cempty0 + 8 * cs);
+                }
                 if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
-#pragma unroll
-                for (int i = 0; i < ITEMS; ++i)
-#pragma unroll
-                    for (int q = 0; q < WPI; ++q) w[i][q] = nw[i][q];
+                if (++cs == (uint32_t)p.ring) { cs = 0; cph ^= 1u; }
             }
         }
     } else {
@@ -383,8 +521,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         float y[CPT];
         uint32_t gc = 0;
         bool ok = true;
-        for (unsigned t = blockIdx.x; t < p.num_tiles && ok; t += grid) {
-            const size_t row = (size_t)(t % p.num_nt) * CG_BM + 32 * quad + lane;
+        for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
+            const size_t row = first_code(t) + 32 * quad + lane;
             const size_t col0 = (size_t)(t / p.num_nt) * p.NT + half * cpt;
             // the code's trailer [norm, gamma, sigma]
             float norm = 0.0f, gamma = 0.0f, sigma = 0.0f;
@@ -395,81 +533,72 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
                 sigma = __ldg(meta + 2);
             }
             for (int c0 = 0, c1 = 0; c0 < KB; c0 = c1, ++gc) {
-                c1 = cg_chunk_end(p, c0);
+                c1 = ord.chunk_end(p, c0);
                 const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
-                if (!mbar_wait(xfull0 + 8 * b, xph, p.err, kErrTmemFull)) { ok = false; break; }
+                if (!mbar_wait_warp(xfull0 + 8 * b, xph, p.err, kErrTmemFull)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t X = lanes + b * 256u;
-                // how a chunk joins the running sum: centroid chunks are added;
-                // a sign chunk as fma(x, scale gamma, y), y first scaled by
-                // sigma (asymmetric); the light form's one sign chunk is its
-                // clamped correction
-                const bool cent = c0 < KBm;
-                const float fy = (!cent && c0 == KBm) ? __fmul_rn(sigma, p.undo_c) : 1.0f;
-                const float fx = __fmul_rn(__fmul_rn(p.scale, gamma), p.undo_s);
-#pragma unroll
-                for (int pc = 0; pc < CPT / 16; ++pc) {
-                    if (16 * pc >= cpt) break;
-                    uint32_t x[16];
-                    __syncwarp();
-                    tmem_ld16_nw(X + 16 * pc, x);
-                    tmem_wait_ld();
-                    if (cent) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const float a = __uint_as_float(x[j]);
-                            y[16 * pc + j] = c0 == 0 ? a : __fadd_rn(y[16 * pc + j], a);
-                        }
-                    } else if (p.form == kCgAsym) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            y[16 * pc + j] = __fmaf_rn(__uint_as_float(x[j]), fx, __fmul_rn(y[16 * pc + j], fy));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const size_t col = col0 + 16 * pc + j < p.m ? col0 + 16 * pc + j : p.m - 1;
-                            const float4 r = __ldg(p.rs + col);
-                            const float ip = __fmul_rn(__fmul_rn(__fmul_rn(y[16 * pc + j], p.undo_c), r.z), sigma);
-                            const float corr = __fmul_rn(__fmul_rn(__uint_as_float(x[j]), r.w), gamma);
-                            const float lim = fabsf(ip);
-                            y[16 * pc + j] = __fadd_rn(ip, fmaxf(-lim, fminf(lim, corr)));
-                        }
+                // How a chunk joins the running sum.  Symmetric and light: centroid
+                // chunks are added (the light form's last chunk is its clamped
+                // correction).  Asymmetric: fma(x, f, y) with f = scale gamma for
+                // the sign part and sigma for the centroid part.
+                if (LIGHT || p.form == kCgSym) {
+                    if (c0 == 0) chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = x; });
+                    else if (!LIGHT || ord.cent(c0)) chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = __fadd_rn(y[k], x); });
+                }
+                if constexpr (!LIGHT) {
+                    if (p.form == kCgAsym) {
+                        const float fx = ord.cent(c0) ? __fmul_rn(sigma, p.undo_c)
+                                                      : __fmul_rn(__fmul_rn(p.scale, gamma), p.undo_s);
+                        if (c0 == 0) chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = __fmul_rn(x, fx); });
+                        else chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = __fmaf_rn(x, fx, y[k]); });
                     }
+                } else if (!ord.cent(c0)) {
+                    const float4 *rs = p.rs + col0;
+                    const int last = (int)min((size_t)cpt, p.m > col0 ? p.m - col0 : 1) - 1;
+                    chunk_pieces<CPT>(X, cpt, [&](int k, float x) {
+                        const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + min(k, last)) + 1);
+                        const float ip = __fmul_rn(__fmul_rn(__fmul_rn(y[k], p.undo_c), r.x), sigma);
+                        const float corr = __fmul_rn(__fmul_rn(x, r.y), gamma);
+                        const float lim = fabsf(ip);
+                        y[k] = __fadd_rn(ip, fmaxf(-lim, fminf(lim, corr)));
+                    });
                 }
                 __syncwarp();
                 tc_fence_before();
-                if (lane == 0) mbar_arrive(xempty0 + 8 * b);
+                if (lane == 0) {
+                    if (PAIR) mbar_arrive_cluster(rank0_addr(xempty0 + 8 * b));
+                    else mbar_arrive(xempty0 + 8 * b);
+                }
             }
             if (!ok) break;
             if (row >= p.n) continue;
-            // d = max(0, r2 + c2 - 2 (C r1) c1)
+            // d = max(0, r2 + c2 - 2 (C r1) c1); a NaN gives 0
             const float c2 = __fmul_rn(norm, norm);
-            const float c1 = p.form == kCgSym ? __fmul_rn(sigma, norm) : norm;
-            const float un = p.form == kCgSym ? p.undo_c : 1.0f;
+            const float c1 = p.form == kCgSym ? __fmul_rn(__fmul_rn(sigma, norm), p.undo_c) : norm;
             float *o = p.out + col0 * p.ldo + row;
+            const float4 *rs = p.rs + col0;
+            const int live = (int)min((size_t)cpt, col0 < p.m ? p.m - col0 : 0);
 #pragma unroll
-            for (int pc = 0; pc < CPT / 16; ++pc) {
-                if (16 * pc >= cpt) break;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const size_t col = col0 + 16 * pc + j;
-                    if (col < p.m) {
-                        const float2 r = __ldg(reinterpret_cast<const float2 *>(p.rs + col));
-                        const float ipt = __fmul_rn(__fmul_rn(__fmul_rn(y[16 * pc + j], un), r.x), c1);
-                        const float d = __fsub_rn(__fadd_rn(r.y, c2), __fmul_rn(2.0f, ipt));
-                        __stcs(o, d > 0.0f ? d : 0.0f);
-                    }
-                    o += p.ldo;
+            for (int k = 0; k < CPT; ++k) {
+                if (k % 16 == 0 && k >= live) break;
+                if (k < live) {
+                    const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + k));
+                    const float ipt = __fmul_rn(__fmul_rn(y[k], r.x), c1);
+                    __stcs(o, fmaxf(__fmaf_rn(-2.0f, ipt, __fadd_rn(r.y, c2)), 0.0f));
                 }
+                o += p.ldo;
             }
         }
     }
     tc_fence_before();
-    __syncthreads();
+    // PAIR: no CTA leaves while the other may still arrive on its barriers or
+    // read its shared memory
+    if constexpr (PAIR) cluster_sync();
+    else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512)
-                     : "memory");
+        tmem_dealloc<PAIR>(tmem_base);
     }
 }
 
@@ -592,10 +721,11 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.form = form;
     a.KBm = (P.D + CG_BK - 1) / CG_BK;
     a.KB = form == kCgSym ? a.KBm : 2 * a.KBm;
-    // Chunk lengths (K blocks).  FP16: 2, so that the truncation of one chunk
-    // (24 MMAs) stays below the rounding of an FP32 chain; BF16: 8 for queries
-    // and 4 for codes against codes, whose terms share a sign more often.
-    a.chm = fmt == kCgFP16 ? 2 : form == kCgAsym ? 8 : 4;
+    // Chunk lengths (K blocks).  FP16: 2 (1 where the whole part is 4 blocks or
+    // fewer), so that the truncation of one chunk stays below the rounding of an
+    // FP32 chain of the same length; BF16: 8 for queries and 4 for codes against
+    // codes, whose terms share a sign more often.
+    a.chm = fmt == kCgFP16 ? (a.KBm <= 4 ? 1 : 2) : form == kCgAsym ? 8 : 4;
     a.chs = form == kCgLight ? a.KBm : 16;  // +-1 by +-1 sums are exact integers
     a.m = m;
     a.rs = rows.rs;
@@ -607,43 +737,59 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.out = out;
     a.ldo = ldo;
     a.err = err;
-    const size_t nt = (n + CG_BM - 1) / CG_BM;
     // Columns per tile: the width that takes the least time by a rough count
     // of clocks: waves of 148 CTAs times a tile's K blocks, each the slower of
-    // its MMAs (11 per block on average over both parts, NT / 2 clocks each)
-    // and its decode (~650 clocks), plus the tile's epilogue.
-    int best = 256;
+    // its MMAs (10 per block on average over both parts, NT / 2 clocks each)
+    // and its decode, plus the tile's epilogue.  Wide tiles (128, 256) run on
+    // CTA pairs, 256 codes a tile.
+    auto code_tiles = [&](int NT) { return (n + (NT > 64 ? 255 : 127)) / (NT > 64 ? 256 : 128); };
     double best_t = 0.0;
     for (int NT = 256; NT >= 16; NT >>= 1) {
-        const size_t tiles = nt * ((m + NT - 1) / NT);
-        const double waves = (double)((tiles + 147) / 148);
-        const double mma = 5.5 * NT, dec = NT <= 64 ? 400.0 : 650.0;
-        const double tt = waves * (a.KB * std::max(mma, dec) + 2.0 * NT + 1000.0);
+        const size_t tiles = code_tiles(NT) * ((m + NT - 1) / NT), slots = NT > 64 ? 74 : 148;
+        const double waves = (double)((tiles + slots - 1) / slots);
+        const double mma = 5.0 * NT, dec = NT <= 64 ? 750.0 : 1000.0;
+        const double tt = waves * (a.KB * std::max(mma, dec) + 8.0 * NT + 1000.0);
         if (NT == 256 || tt < best_t) {
-            best = NT;
+            a.NT = NT;
             best_t = tt;
         }
     }
-    a.NT = best;
-    const int stage_bytes = 2 * CG_A_BYTES + 2 * a.NT * 128;
-    const int tab = P.nibble ? 0 : CG_TAB_BYTES;
-    a.stages = std::min(CG_MAX_STAGES, (CG_SMEM_MAX - CG_FIXED - tab) / stage_bytes);
-    const size_t smem = (size_t)a.stages * stage_bytes + CG_FIXED + tab;
-    const size_t tiles = nt * ((m + a.NT - 1) / a.NT);
+    const bool pair = a.NT > 64;
+    const int stage_bytes = 2 * CG_A_BYTES + 2 * a.NT * (pair ? 64 : 128);
+    const int tab = P.nibble ? 0 : CG_TAB_BYTES, ring_bytes = CG_BM * (P.nibble ? 32 : 64);
+    const int avail = CG_SMEM_MAX - CG_FIXED - tab;
+    a.stages = std::min(CG_MAX_STAGES, (avail - 2 * ring_bytes) / stage_bytes);
+    a.ring = std::min(CG_MAX_RING, (avail - a.stages * stage_bytes) / ring_bytes);
+    const size_t smem = (size_t)a.stages * stage_bytes + a.ring * ring_bytes + CG_FIXED + tab;
+    const size_t nt = code_tiles(a.NT), tiles = nt * ((m + a.NT - 1) / a.NT);
     if (tiles > 0x7FFFFFFFull || nt > 0x7FFFFFFFull) return cudaErrorInvalidValue;
     a.num_nt = (unsigned)nt;
     a.num_tiles = (unsigned)tiles;
     alignas(64) CUtensorMap mh, ml;
-    const int K = a.KB * CG_BK;
-    if (!make_map(&mh, rows.hi, K, m, a.NT) || !make_map(&ml, rows.lo, K, m, a.NT))
-        return cudaErrorInvalidValue;
-    const bool narrow = a.NT <= 64;
-    auto kern = P.nibble ? (narrow ? cgemm_kernel<8, true> : cgemm_kernel<4, true>)
-                         : (narrow ? cgemm_kernel<8, false> : cgemm_kernel<4, false>);
+    const int K = a.KB * CG_BK, box = pair ? a.NT / 2 : a.NT;
+    if (!make_map(&mh, rows.hi, K, m, box) || !make_map(&ml, rows.lo, K, m, box)) return cudaErrorInvalidValue;
+    const bool light = form == kCgLight;
+    auto pick = [&](auto wide, auto nib) {
+        constexpr bool W = decltype(wide)::value, N = decltype(nib)::value;
+        return light ? cgemm_kernel<W ? 4 : 8, N, true, W> : cgemm_kernel<W ? 4 : 8, N, false, W>;
+    };
+    using T_ = std::true_type;
+    using F_ = std::false_type;
+    auto kern = P.nibble ? (pair ? pick(T_{}, T_{}) : pick(F_{}, T_{})) : (pair ? pick(T_{}, F_{}) : pick(F_{}, F_{}));
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<sm_grid(tiles), CG_THREADS, smem, st>>>(mh, ml, a);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(pair ? 2 * sm_grid(tiles, 2) : sm_grid(tiles));
+    cfg.blockDim = dim3(CG_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = pair ? 2 : 1;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, mh, ml, a);
 }
 
 }  // namespace tq

@@ -35,6 +35,109 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
     return d;
 }
 
+// The same descriptor's low word (the high word is the constant kDescHi);
+// adding bytes / 16 moves the start address.
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t addr) {
+    return ((addr >> 4) & 0x3FFFu) | (1u << 16);
+}
+
+// D[d_tmem] (+)= A B of one K = 16 step (kind::f16), descriptors by their low
+// words.  PAIR: one tile over the two CTAs of a cluster (M = 256: each CTA's
+// A rows and tensor memory, half of B's rows from each), issued by rank 0.
+template <bool PAIR = false>
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                         uint32_t acc) {
+    if constexpr (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "mov.b64 da, {%1, %5};\n\t"
+            "mov.b64 db, {%2, %5};\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(acc), "r"(kDescHi)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "mov.b64 da, {%1, %5};\n\t"
+            "mov.b64 db, {%2, %5};\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(acc), "r"(kDescHi)
+            : "memory");
+}
+
+// ---- CTA pairs (clusters of two) ---------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// Commit of the pair's MMAs so far to the barrier at this offset in both CTAs.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            bar),
+        "h"((uint16_t)3)
+        : "memory");
+}
+// The address of rank 0's copy of this CTA's shared-memory object.
+__device__ __forceinline__ uint32_t rank0_addr(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+
+// One lane of a converged warp (always the same one).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r));
+    return r != 0;
+}
+
+// As mbar_wait, for a barrier that the other CTA of the cluster arrives on.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int *err, int code) {
+    const long long t0 = clock64();
+    for (uint32_t it = 1;; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if ((it & 1023u) == 0) {
+            if (*reinterpret_cast<volatile int *>(err) != 0) return false;
+            if (clock64() - t0 > kWaitCycles) {
+                atomicCAS(err, 0, code);
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint32_t bar, uint32_t parity, int *err, int code) {
+    return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, err, code));
+}
+
+// mbar_wait by a whole warp, one result for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int *err, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code));
+}
+
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
@@ -144,10 +247,12 @@ inline bool aligned16(std::initializer_list<const void *> ps) {
     return true;
 }
 
-inline unsigned sm_grid(size_t tiles) {
+// CTAs (or clusters of `per` CTAs) of a persistent launch: one CTA per SM, at most one per tile.
+inline unsigned sm_grid(size_t tiles, int per = 1) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    sms /= per;
     return (unsigned)(tiles < (size_t)sms ? tiles : (size_t)sms);
 }
 
