@@ -1,5 +1,6 @@
 """The M x N tensor-core kernel with in-kernel decoded code tiles
-(distanceBatchMToN / distanceBatchMToNSymmetric, space_turbo_quant.h:588-615)
+(distanceBatchMToN / distanceBatchMToNSymmetric / ...Light,
+space_turbo_quant.h:588-615, 634-647)
 at the edges of its tiles: row counts around its column widths (16 ... 256),
 code counts around its 128-code tiles, reductions shorter than one 64-value
 K block and longer than one accumulation chunk, every index width, zero rows
@@ -35,3 +36,7 @@ def test_tile_edges(cuda_ok, dim, bits, m, n):
                          o.distance_m_to_n_symmetric(rows, codes),
                          sym_term_scale(rows, codes, cs, cs - 12))
     assert ok, ("symmetric", err.max())
+    err, ok = dist_close(s.distance_m_to_n_symmetric_light(rows, codes),
+                         o.distance_m_to_n_symmetric_qjl(rows, codes, "light"),
+                         sym_term_scale(rows, codes, cs, cs - 12))
+    assert ok, ("light", err.max())

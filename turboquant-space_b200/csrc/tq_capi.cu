@@ -968,7 +968,10 @@ constexpr size_t kSymqTcChunkBytes = size_t(2048) << 20;  // TF32 pairs: fewer, 
 
 size_t sq_round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// Row planes built once (from row codes, or from a prepared code), column
+// The light variant runs on the M x N kernel with in-kernel decoded code tiles
+// (tq_cgemm.cu, FP16 pairs; both precisions, padded dims of at least 16, 4-byte
+// aligned codes): no column planes.  Otherwise:
+// row planes built once (from row codes, or from a prepared code), column
 // planes built per chunk; one two-accumulator contraction per chunk: the FP32
 // CUDA-core kernel, or (split-TF32) the FP32 planes split into hi/lo TF32
 // planes (K padded to 32, rows to 128 / 256) for the tcgen05 kernel.  Padded
@@ -984,6 +987,8 @@ struct SymqRunner {
     float *P1a = nullptr, *P2a = nullptr, *sa = nullptr;
     float *A1 = nullptr, *A2 = nullptr;  // hi then lo, m_pad x K1p / K2p each
     int *err = nullptr;
+    bool cg = false;
+    tq::CgRows cgr;
 
     SymqRunner(const tq_space *s, int md, bool split_tf32 = false)
         : sp(s), mode(md), tc(split_tf32 && s->D >= 64) {
@@ -1002,6 +1007,7 @@ struct SymqRunner {
         return TQ_OK;
     }
     tq_status prepare_rows(const uint8_t *A, size_t rows_, cudaStream_t s) {
+        if (cg) return prepare_rows_cg(A, rows_, s);
         if (tc) return prepare_rows_tc(A, rows_, s);
         tq_status st = alloc_rows(rows_, s);
         if (st != TQ_OK) return st;
@@ -1009,6 +1015,28 @@ struct SymqRunner {
                 "symmetric planes kernel");
         return TQ_OK;
     }
+    // Takes the light variant to the M x N kernel where the codes allow it
+    // (A, B: device pointers of the call).
+    void choose(const void *A, const void *B) {
+        cg = light() && sp->D >= 16 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 3) == 0;
+    }
+    tq_status prepare_rows_cg(const uint8_t *A, size_t rows_, cudaStream_t s) {
+        m = rows_;
+        const size_t plane = m * tq::cg_row_k(sp->P, tq::kCgLight) * 2;  // a multiple of 128 bytes
+        TQ_CUDA(rows.alloc(2 * plane + m * sizeof(float4) + sizeof(int), s), "cudaMallocAsync(row planes)");
+        auto *base = static_cast<unsigned char *>(rows.p);
+        cgr.hi = base;
+        cgr.lo = base + plane;
+        cgr.rs = reinterpret_cast<float4 *>(base + 2 * plane);
+        if (tc) {  // reported by finish(), as the TF32 kernel's; otherwise stream-ordered
+            err = reinterpret_cast<int *>(cgr.rs + m);
+            TQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s), "memset");
+        }
+        TQ_CUDA(tq::launch_cg_rows_codes(sp->P, sp->T, A, m, tq::kCgLight, tq::kCgFP16, cgr, s), "row planes");
+        return TQ_OK;
+    }
+    // The space's status word carries this call's errors (host entry points read it).
+    bool uses_status_word() const { return cg && !err; }
     // The row planes straight into hi/lo TF32 pairs (m_pad x K1p, m_pad x
     // K2p); the light variant's sign plane is exact and has no lo plane.
     tq_status prepare_rows_tc(const uint8_t *A, size_t rows_, cudaStream_t s) {
@@ -1036,6 +1064,12 @@ struct SymqRunner {
     }
     // out[:, 0:n] (leading dimension ldo) for n column codes
     tq_status run_cols(const uint8_t *B, size_t n, float *out, size_t ldo, cudaStream_t s) {
+        if (cg) {
+            TQ_CUDA(tq::launch_cgemm(sp->P, sp->T, tq::kCgLight, tq::kCgFP16, cgr, m, B, n, out, ldo,
+                                     err ? err : sp->T.status, s),
+                    "tcgen05 light symmetric kernel");
+            return TQ_OK;
+        }
         if (tc) return run_cols_tc(B, n, out, ldo, s);
         if (!per) {
             per = std::max<size_t>(64, kSymqChunkBytes / (sizeof(float) * row_floats()));
@@ -1170,6 +1204,7 @@ tq_status tq_distance_m_to_n_symmetric_qjl_device(const tq_space *sp, const uint
     if ((st = check_dev(out, m * n * 4, "out")) != TQ_OK) return st;
     cudaStream_t s = (cudaStream_t)stream;
     SymqRunner r(sp, mode, precision == TQ_PRECISION_SPLIT_TF32);
+    r.choose(A, B);
     if ((st = r.prepare_rows(A, m, s)) != TQ_OK) return st;
     if ((st = r.run_cols(B, n, out, n, s)) != TQ_OK) return st;
     return r.finish(s);
@@ -1195,6 +1230,7 @@ tq_status tq_distance_m_to_n_symmetric_qjl(const tq_space *csp, const uint8_t *c
     TQ_CUDA(dA.alloc(m * cs, s), "cudaMallocAsync(codes_a)");
     TQ_CUDA(cudaMemcpyAsync(dA.p, codes_a, m * cs, cudaMemcpyHostToDevice, s), "H2D codes_a");
     SymqRunner r(sp, mode, precision == TQ_PRECISION_SPLIT_TF32);
+    r.choose(nullptr, nullptr);  // staging buffers of our own, aligned
     if ((st = r.prepare_rows(static_cast<uint8_t *>(dA.p), m, s)) != TQ_OK) return st;
     size_t per = std::max<size_t>(1, std::min(kChunkBytes / cs, (kChunkBytes * 2) / (4 * m)));
     per = std::min(per, n);
@@ -1211,6 +1247,7 @@ tq_status tq_distance_m_to_n_symmetric_qjl(const tq_space *csp, const uint8_t *c
                 "D2H distances");
     }
     TQ_CUDA(cudaStreamSynchronize(s), "distance_m_to_n_symmetric (QJL)");
+    if (r.uses_status_word()) return take_status(sp, nullptr);
     return r.finish(s);
 }
 
