@@ -1,0 +1,42 @@
+"""The serving top-k's filter pass (kernel variant 6) at the edges of its tiles,
+thresholds and row blocks: corpora around one 256-code tile and around the
+sample of the first threshold, one large enough for the second threshold, row
+counts around the MMA's column steps and the 256-row blocks, nibble and byte
+codes, reductions of one block and of many, zero rows and rows of very
+different norms.  Results equal the stable argsort of the oracle's
+distances bit for bit, and no candidate lies outside the pass's error bound."""
+import numpy as np
+import pytest
+
+import oracle as O
+import turboquant as tq
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dim,bits,n", [(64, 4, 1), (32, 4, 255), (100, 8, 256), (384, 4, 257), (1000, 3, 3000),
+                                        (128, 8, 8191), (128, 2, 8193), (768, 8, 12_000), (64, 4, 340_000)])
+@pytest.mark.parametrize("m,k", [(1, 1), (31, 10), (33, 16), (129, 10), (300, 10)])
+def test_filter_edges(cuda_ok, dim, bits, n, m, k):
+    rng = np.random.default_rng(dim + 3 * bits + n + m)
+    X = (rng.standard_normal((n, dim)) * rng.uniform(0.5, 2.0, (n, 1))).astype(np.float32)
+    X[n // 3] = 0.0
+    Q = (rng.standard_normal((m, dim)) * rng.uniform(1e-2, 1e2, (m, 1))).astype(np.float32)
+    Q[m // 2] = 0.0 if m > 1 else Q[m // 2]
+    space, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    codes = space.encode_batch(X)
+    ref = o.distance_m_to_n(Q, codes)
+    idx = np.argsort(ref, axis=1, kind="stable")[:, :k]
+    ix = space.index(codes)
+    try:
+        with ix.serve(k=k, max_rows=384, slots=1, kernel_variant=6) as sv:
+            D, I = sv.submit(Q).wait()
+            st = sv.stats()
+    finally:
+        ix.close()
+    w = idx.shape[1]
+    np.testing.assert_array_equal(I[:, :w], idx)
+    np.testing.assert_array_equal(D[:, :w].view(np.uint32),
+                                  np.take_along_axis(ref, idx, 1).astype(np.float32).view(np.uint32))
+    assert np.all(I[:, w:] == -1)
+    assert st["bound_violations"] == 0

@@ -109,18 +109,6 @@ struct CgArgs {
     int *err;
 };
 
-// 4-byte asynchronous copy (zeros for bytes = 0); the surrounding 128 bytes
-// are fetched into L2 with it (the next K blocks of the same code).
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, uint32_t bytes) {
-    asm volatile("cp.async.ca.shared.global.L2::128B [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes)
-                 : "memory");
-}
-// Arrives on `bar` once this thread's copies so far have landed.
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 // The K blocks of a tile in the order they run: the asymmetric form's sign part
 // first, so that its one long chunk covers the previous tile's output; the
 // light form's last, since its sums are not added to the centroid part's.
@@ -139,25 +127,6 @@ struct CgOrder {
     }
 };
 
-template <bool PAIR>
-__device__ __forceinline__ void tmem_alloc(uint32_t slot) {
-    if constexpr (PAIR) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    } else {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-}
-template <bool PAIR>
-__device__ __forceinline__ void tmem_dealloc(uint32_t base) {
-    if constexpr (PAIR)
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512) : "memory");
-    else
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512) : "memory");
-}
 template <bool PAIR>
 __device__ __forceinline__ void commit(uint32_t bar) {
     if constexpr (PAIR) umma_commit_pair(bar);
@@ -187,24 +156,21 @@ __device__ __forceinline__ void nib_cent(uint32_t x, const NibTab &t, uint4 &hi,
     lo.w = __byte_perm(a, b, 0x7362u);
 }
 
-// The QJL bits of 8 units -> 8 values +-1 (`one` = a pair of +1).
-__device__ __forceinline__ uint4 nib_sign(uint32_t x, uint32_t one) {
-    const uint32_t y = ~x;
-    uint4 r;
-    r.x = one | ((y << 15) & 0x8000u) | ((y << 27) & 0x80000000u);
-    r.y = one | ((y << 7) & 0x8000u) | ((y << 19) & 0x80000000u);
-    r.z = one | ((y >> 1) & 0x8000u) | ((y << 11) & 0x80000000u);
-    r.w = one | ((y >> 9) & 0x8000u) | ((y << 3) & 0x80000000u);
-    return r;
+// The QJL bits of 8 units -> 8 values +-1 (`one` = a pair of +1, `pm` the high
+// bytes of -1 and +1): a PRMT picks four coordinates' high bytes by their
+// bits, two more put the low byte beside each.
+__device__ __forceinline__ uint4 nib_sign(uint32_t x, uint32_t one, uint32_t pm) {
+    const uint32_t s = x & 0x11111111u;
+    const uint32_t a = __byte_perm(pm, 0u, s), b = __byte_perm(pm, 0u, s >> 16);
+    return make_uint4(__byte_perm(a, one, 0x1404u), __byte_perm(a, one, 0x3424u), __byte_perm(b, one, 0x1404u),
+                      __byte_perm(b, one, 0x3424u));
 }
-__device__ __forceinline__ uint4 byte_sign(uint32_t x0, uint32_t x1, uint32_t one) {
-    const uint32_t y0 = ~x0, y1 = ~x1;
-    uint4 r;
-    r.x = one | ((y0 << 15) & 0x8000u) | ((y0 << 23) & 0x80000000u);
-    r.y = one | ((y0 >> 1) & 0x8000u) | ((y0 << 7) & 0x80000000u);
-    r.z = one | ((y1 << 15) & 0x8000u) | ((y1 << 23) & 0x80000000u);
-    r.w = one | ((y1 >> 1) & 0x8000u) | ((y1 << 7) & 0x80000000u);
-    return r;
+// The same for units of a byte each.
+__device__ __forceinline__ uint4 byte_sign(uint32_t x0, uint32_t x1, uint32_t one, uint32_t pm) {
+    return make_uint4(__byte_perm(one, pm, ((x0 << 4) & 0x1010u) | 0x4040u),
+                      __byte_perm(one, pm, ((x0 >> 12) & 0x1010u) | 0x4040u),
+                      __byte_perm(one, pm, ((x1 << 4) & 0x1010u) | 0x4040u),
+                      __byte_perm(one, pm, ((x1 >> 12) & 0x1010u) | 0x4040u));
 }
 
 // f(k, x) for at least the first `cols` of CPT columns of a chunk buffer, in
@@ -269,7 +235,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         mbar_init(drain, 1);
         mbar_init_fence();
     }
-    if (warp == 1) tmem_alloc<PAIR>(smem_u32(tmem_slot));
+    if (warp == 1) tmem_alloc512<PAIR>(smem_u32(tmem_slot));
     if constexpr (!NIB) {
         // entry v of lane l at btab[32 v + l]: hi | lo << 16
         for (int i = threadIdx.x; i < 128 * 32; i += CG_THREADS) {
@@ -452,6 +418,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             }
         }
         const uint32_t one = p.fmt == kCgFP16 ? 0x3C003C00u : 0x3F803F80u;
+        const uint32_t pm = p.fmt == kCgFP16 ? 0x3CBCu : 0x3FBFu;
         const uint32_t *tl = btab + lane;
         uint32_t s = 0, ph = 1, cs = 0, cph = 0;
         bool ok = true;
@@ -497,8 +464,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
 #pragma unroll
                     for (int i = 0; i < ITEMS; ++i) {
                         uint4 v;
-                        if constexpr (NIB) v = nib_sign(w[i][0], one);
-                        else v = byte_sign(w[i][0], w[i][WPI - 1], one);
+                        if constexpr (NIB) v = nib_sign(w[i][0], one, pm);
+                        else v = byte_sign(w[i][0], w[i][WPI - 1], one, pm);
                         *reinterpret_cast<uint4 *>(dst + 512 * i + (sw ^ ((i & 1) << 6))) = v;
                     }
                 }
@@ -598,7 +565,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
     else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc<PAIR>(tmem_base);
+        tmem_dealloc512<PAIR>(tmem_base);
     }
 }
 

@@ -26,6 +26,7 @@
 //
 // Every operation below is one IEEE FP32 rounding (explicit _rn intrinsics:
 // nvcc would otherwise contract a multiply and an add into an FMA).
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -286,6 +287,7 @@ struct RescoreArgs {
     bool al4;
     const float *bound;
     float kappa, kappa_t, bound_scale;
+    RescoreFilter filter;
     float *out_d;
     long long *out_i;
     int *fail_rows;
@@ -351,7 +353,20 @@ __global__ void __launch_bounds__(256) rescore_kernel(RescoreArgs a) {
         // rescan an open row (its own kappa, kappa_t >= kappa)
         const float terms = a.cmax * a.bound[0] * sq + a.bound[1] * ss;
         const float rest = 2.0f * qn * kDegenerateG * ss * a.bound[3] + kKappaEpi * (qn2 + a.bound[2]);
-        const float eps = a.bound_scale * (2.0f * qn * a.kappa * terms + rest);
+        float eps = a.bound_scale * (2.0f * qn * a.kappa * terms + rest);
+        bool complete = true;
+        if (a.filter.rowq) {
+            // the filter pass's own bound (tq_filter.cu); 1.0001 >= |q_rot|, 1.001 covers
+            // this evaluation, and its distances' epilogue counts double
+            const float4 w = a.filter.rowq[row];
+            const float M0 = a.filter.bound[0], M1 = a.filter.bound[1], M2 = a.filter.bound[2],
+                        M3 = a.filter.bound[3];
+            const float e = w.x * M0 + 1.0001f * M1 + w.y * M2 + w.w * M3 +
+                            (float)(a.filter.mmas + 1) * (1.0f / 1048576.0f) * (w.z * M0 + w.w * (M2 + M3)) +
+                            2e-6f * (M0 + M2);
+            eps = a.bound_scale * (2.0f * qn * 1.001f * e + 2.0f * kKappaEpi * (qn2 + a.bound[2]));
+            complete = a.filter.bad[row] == 0;
+        }
         const float eps_t = a.bound_scale * (2.0f * qn * a.kappa_t * terms + rest);
         const bool viol = ci != kNoIdx && !(fabsf(ad - ed) <= eps);
         const unsigned viol_mask = __ballot_sync(kFull, viol);
@@ -377,7 +392,7 @@ __global__ void __launch_bounds__(256) rescore_kernel(RescoreArgs a) {
         const float ek = __shfl_sync(kFull, d, a.k - 1);
         // fewer than kc codes in the corpus: every code is a candidate
         const bool all_in = ci_last == kNoIdx;
-        const bool certified = viol_mask == 0u && (all_in || ek < ad_last - eps);
+        const bool certified = complete && viol_mask == 0u && (all_in || ek < ad_last - eps);
         if (certified) {
             if (lane < a.k) {
                 a.out_d[(size_t)row * a.k + lane] = d;
@@ -656,30 +671,30 @@ __global__ void __launch_bounds__(256) tensor_select_kernel(
     }
 }
 
-// Open row f's query planes (K BF16 values a row, hi and lo) and scales to
-// row f of the tensor-core threshold pass's operands.
+// Open row f's prepared query as row f of the tensor-core threshold pass's
+// operands: hi and lo BF16 planes of [q_rot | s_q] (x = hi + lo) and its norms.
 __global__ void __launch_bounds__(256) gather_open_kernel(const int *__restrict__ counters,
                                                           const int *__restrict__ fail_rows,
-                                                          const uint4 *__restrict__ ah,
-                                                          const uint4 *__restrict__ al,
-                                                          const float *__restrict__ r1,
-                                                          const float *__restrict__ r2, int w16,
-                                                          uint4 *__restrict__ ah2,
-                                                          uint4 *__restrict__ al2,
+                                                          const float *__restrict__ q_rot,
+                                                          const float *__restrict__ s_q,
+                                                          const float *__restrict__ norms, int D,
+                                                          __nv_bfloat16 *__restrict__ ah2,
+                                                          __nv_bfloat16 *__restrict__ al2,
                                                           float *__restrict__ r1o,
                                                           float *__restrict__ r2o) {
     const int nf = counters[kCntFallbackRows];
     if (nf <= kTensorTierMinRows) return;
-    const size_t total = (size_t)nf * w16;
+    const size_t K = 2 * (size_t)D, total = (size_t)nf * K;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (size_t)gridDim.x * blockDim.x) {
-        const size_t f = t / w16, w = t % w16;
-        const size_t src = (size_t)fail_rows[f] * w16 + w;
-        ah2[t] = ah[src];
-        al2[t] = al[src];
-        if (w == 0) {
-            r1o[f] = r1[fail_rows[f]];
-            r2o[f] = r2[fail_rows[f]];
+        const size_t f = t / K, k = t % K, row = (size_t)fail_rows[f];
+        const float v = k < (size_t)D ? q_rot[row * D + k] : s_q[row * D + k - D];
+        const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+        ah2[t] = hi;
+        al2[t] = __float2bfloat16_rn(v - __bfloat162float(hi));
+        if (k == 0) {
+            r1o[f] = norms[2 * row + 1];
+            r2o[f] = norms[2 * row];
         }
     }
 }
@@ -978,14 +993,14 @@ cudaError_t launch_rescore(const Params &P, const float *centroids, float cmax, 
                            int kc, int k, const float *cand_d, const long long *cand_i,
                            const float *q_rot, const float *s_q, const float *norms,
                            const uint8_t *codes, size_t n, const float *bound, float kappa,
-                           float kappa_t, float bound_scale,
+                           float kappa_t, const RescoreFilter &filter, float bound_scale,
                            float *out_d, long long *out_i, int *fail_rows, float *thr, float *tthr,
                            int *counters, int max_rows, cudaStream_t st) {
     if (kc < 1 || kc > 32 || k < 1 || k > kc || k > kTopKMax || max_rows < 1 || !(kappa > 0.0f))
         return cudaErrorInvalidValue;
     const RescoreArgs a{P,     centroids, cmax,  m_dev,     kc,          k,     cand_d,
                         cand_i, q_rot,    s_q,   norms,     codes,       n,     codes_al4(P, codes),
-                        bound, kappa, kappa_t > kappa ? kappa_t : kappa, bound_scale, out_d, out_i,
+                        bound, kappa, kappa_t > kappa ? kappa_t : kappa, bound_scale, filter, out_d, out_i,
                         fail_rows, thr, tthr, counters};
     const unsigned blocks = (unsigned)((max_rows + 7) / 8);
     if (P.nibble)
@@ -997,20 +1012,15 @@ cudaError_t launch_rescore(const Params &P, const float *centroids, float cmax, 
 
 int fallback_ctas(int sms) { return 2 * (sms > 0 ? sms : 148); }
 
-cudaError_t launch_gather_open(const int *counters, const int *fail_rows, const void *ah,
-                               const void *al, const float *r1, const float *r2, int K,
-                               int max_rows, void *ah2, void *al2, float *r1o, float *r2o,
-                               cudaStream_t st) {
-    if (K % 8 || max_rows < 1) return cudaErrorInvalidValue;
-    const uintptr_t any = reinterpret_cast<uintptr_t>(ah) | reinterpret_cast<uintptr_t>(al) |
-                          reinterpret_cast<uintptr_t>(ah2) | reinterpret_cast<uintptr_t>(al2);
-    if (any & 15) return cudaErrorMisalignedAddress;
-    const int w16 = K / 8;  // 16-byte words of a BF16 row
-    const size_t total = (size_t)max_rows * w16;
+cudaError_t launch_gather_open(const int *counters, const int *fail_rows, const float *q_rot,
+                               const float *s_q, const float *norms, int D, int max_rows, void *ah2,
+                               void *al2, float *r1o, float *r2o, cudaStream_t st) {
+    if (max_rows < 1) return cudaErrorInvalidValue;
+    const size_t total = (size_t)max_rows * 2 * D;
     const unsigned blocks = (unsigned)std::min<size_t>((total + 255) / 256, 148 * 4);
     gather_open_kernel<<<blocks ? blocks : 1, 256, 0, st>>>(
-        counters, fail_rows, static_cast<const uint4 *>(ah), static_cast<const uint4 *>(al), r1, r2,
-        w16, static_cast<uint4 *>(ah2), static_cast<uint4 *>(al2), r1o, r2o);
+        counters, fail_rows, q_rot, s_q, norms, D, static_cast<__nv_bfloat16 *>(ah2),
+        static_cast<__nv_bfloat16 *>(al2), r1o, r2o);
     return cudaGetLastError();
 }
 

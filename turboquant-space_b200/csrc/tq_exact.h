@@ -48,21 +48,28 @@ constexpr int kTensorTierMinRows = 4;
 // relative error bound (tc_topk_kappa of the variant that produced the
 // candidates); kappa_t = that of the threshold pass over open rows (tthr is
 // e_k plus the bound with max(kappa, kappa_t)).
+// filter: set (rowq non-null) when the filter pass (tq_filter.cu) produced the
+// candidates: its bound replaces kappa's, and a row it marks bad stays open.
+struct RescoreFilter {
+    const float4 *rowq = nullptr;
+    const float *bound = nullptr;
+    const int *bad = nullptr;
+    int mmas = 0;
+};
 cudaError_t launch_rescore(const Params &P, const float *centroids, float cmax, const int *m_dev,
                            int kc, int k, const float *cand_d, const long long *cand_i,
                            const float *q_rot, const float *s_q, const float *norms,
                            const uint8_t *codes, size_t n, const float *bound, float kappa,
-                           float kappa_t, float bound_scale,
+                           float kappa_t, const RescoreFilter &filter, float bound_scale,
                            float *out_d, long long *out_i, int *fail_rows, float *thr, float *tthr,
                            int *counters, int max_rows, cudaStream_t st);
 
-// The open rows' query planes and scales, gathered to rows 0 .. nf-1 for the
-// tensor-core threshold pass (nothing unless nf = counters[0] exceeds
-// kTensorTierMinRows).  Planes: rows of K BF16 values.
-cudaError_t launch_gather_open(const int *counters, const int *fail_rows, const void *ah,
-                               const void *al, const float *r1, const float *r2, int K,
-                               int max_rows, void *ah2, void *al2, float *r1o, float *r2o,
-                               cudaStream_t st);
+// The open rows' prepared queries as BF16 hi / lo planes (2D values a row) and
+// norms in rows 0 .. nf-1, for the tensor-core threshold pass (nothing unless
+// nf = counters[0] exceeds kTensorTierMinRows).
+cudaError_t launch_gather_open(const int *counters, const int *fail_rows, const float *q_rot,
+                               const float *s_q, const float *norms, int D, int max_rows, void *ah2,
+                               void *al2, float *r1o, float *r2o, cudaStream_t st);
 
 // Device buffers of the fallback (R = max_rows open rows at most).
 struct FallbackBuffers {

@@ -58,6 +58,7 @@
 #include <vector>
 
 #include "tq_exact.h"
+#include "tq_filter.h"
 #include "tq_host.h"
 #include "tq_mton.h"
 
@@ -73,6 +74,7 @@ struct tq_index {
     uint8_t *codes = nullptr;  // the corpus itself (n x code_size), for the exact stages
     float *bound = nullptr;    // kBoundFloats index-wide maxima of the error bound
     float cmax = 0.0f;         // max |centroid|
+    tq::FilterIndex filter;    // the filter pass's per-code factors (variant 6)
     int device = -1;
 };
 
@@ -133,6 +135,7 @@ struct Slot {
     int *d_rows = nullptr;
     void *d_ap = nullptr;  // query planes: max_rows x K x 2 BF16 planes
     long long *d_oi = nullptr;
+    tq::FilterBuffers flt;  // the filter pass's (variant 6)
     std::vector<int> bucket_rows;
     std::vector<cudaGraphExec_t> graphs;
     std::vector<tq_request *> batch;  // requests in flight in this slot
@@ -177,8 +180,11 @@ struct tq_server {
 
 namespace {
 
-// Kernel variants that serve an index layout: any for planes, the decoded-B
-// ones for codes.
+// The filter pass (tq_filter.cu), which decodes its code tiles itself.
+constexpr int kFilterVariant = 6;
+
+// Kernel variants that may be fixed for an index layout: any for planes, the
+// decoded-B ones for codes.  (The tuner may take the filter for either.)
 bool variant_fits(const tq_index *ix, int v) {
     return ix->layout == TQ_INDEX_CODES ? tq::tc_topk_dec_ok(v, (int)ix->sp->code_size)
                                         : (v >= 0 && v < tq::tc_topk_variants());
@@ -254,9 +260,6 @@ cudaError_t enqueue_batch(tq_server *sv, Slot &sl, int rows_cap, int var, bool c
     if (e != cudaSuccess) return e;
     unsigned char *ah = static_cast<unsigned char *>(sl.d_ap);
     unsigned char *al = ah + (size_t)rows_cap * K * 2;
-    e = tq::launch_planes_from_prepared(q_rot, s_q, norms, rows_cap, rows_cap, (int)D,
-                                        ah, al, sl.d_r1, sl.d_r2, st);
-    if (e != cudaSuccess) return e;
     // tensor-core pass: each row's kc best candidates by approximate distance
     const bool planes = ix->layout == TQ_INDEX_PLANES;
     unsigned char *bh = planes ? static_cast<unsigned char *>(ix->planes) : nullptr;
@@ -273,9 +276,20 @@ cudaError_t enqueue_batch(tq_server *sv, Slot &sl, int rows_cap, int var, bool c
         dec.centroids = sp->T.centroids;
         dec.levels = sp->levels;
     }
-    e = cudaMemsetAsync(sl.d_gthr, 0xFF, (size_t)rows_cap * sizeof(unsigned long long), st);
+    const bool filter = var == kFilterVariant;
+    if (filter) {
+        e = tq::launch_filter(sp->P, sp->T, ix->filter, q_rot, s_q, norms, sl.d_m, rows_cap, sv->kc, sl.flt,
+                              sl.d_cd, sl.d_ci, sl.d_err, st);
+    } else {
+        e = tq::launch_planes_from_prepared(q_rot, s_q, norms, rows_cap, rows_cap, (int)D,
+                                            ah, al, sl.d_r1, sl.d_r2, st);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(sl.d_gthr, 0xFF, (size_t)rows_cap * sizeof(unsigned long long), st);
+    }
     if (e != cudaSuccess) return e;
-    if (planes)
+    if (filter)
+        ;
+    else if (planes)
         e = tq::launch_tc_topk(var, ah, al, rows_cap, bh, bl, ix->n_pad, (int)K, ix->K_lo, sl.d_m, ix->n,
                                sl.d_r1, sl.d_r2, ix->c1, ix->c2, sv->kc, sl.d_pd, sl.d_pi, sl.d_gthr,
                                sl.d_err, sv->grid, st);
@@ -284,8 +298,9 @@ cudaError_t enqueue_batch(tq_server *sv, Slot &sl, int rows_cap, int var, bool c
                                    sl.d_r1, sl.d_r2, ix->c1, ix->c2, sv->kc, sl.d_pd, sl.d_pi, sl.d_gthr,
                                    sl.d_err, sv->grid, st);
     if (e != cudaSuccess) return e;
-    e = tq::launch_topk_merge(sl.d_m, sv->grid, tq::tc_topk_lists(var), sl.d_pd, sl.d_pi, sv->kc,
-                              rows_cap, sl.d_cd, sl.d_ci, st);
+    if (!filter)
+        e = tq::launch_topk_merge(sl.d_m, sv->grid, tq::tc_topk_lists(var), sl.d_pd, sl.d_pi, sv->kc,
+                                  rows_cap, sl.d_cd, sl.d_ci, st);
     if (e != cudaSuccess) return e;
     // exact stages: rescoring + certificate, then the full pass for the rows
     // the certificate leaves open
@@ -295,6 +310,9 @@ cudaError_t enqueue_batch(tq_server *sv, Slot &sl, int rows_cap, int var, bool c
                            q_rot, s_q, norms, ix->codes, ix->n, ix->bound,
                            tq::tc_topk_kappa(var, (int)K, ix->K_lo),
                            tq::tc_topk_kappa(tq::tc_thresh_variant(!planes, ix->n_pad), (int)K, ix->K_lo),
+                           filter ? tq::RescoreFilter{sl.flt.rowq, ix->filter.bound, sl.flt.bad,
+                                                      tq::filter_mmas(sp->P)}
+                                  : tq::RescoreFilter{},
                            sv->bound_scale, sl.d_od,
                            sl.d_oi, sl.d_fail, sl.d_thr, sl.d_tthr, sl.d_cnt, rows_cap, st);
     if (e != cudaSuccess) return e;
@@ -303,8 +321,8 @@ cudaError_t enqueue_batch(tq_server *sv, Slot &sl, int rows_cap, int var, bool c
     if (e != cudaSuccess) return e;
     unsigned char *ah2 = static_cast<unsigned char *>(sl.d_ap2);
     unsigned char *al2 = ah2 + (size_t)rows_cap * K * 2;
-    e = tq::launch_gather_open(sl.d_cnt, sl.d_fail, ah, al, sl.d_r1, sl.d_r2, (int)K, rows_cap, ah2, al2,
-                               sl.d_r1o, sl.d_r2o, st);
+    e = tq::launch_gather_open(sl.d_cnt, sl.d_fail, q_rot, s_q, norms, (int)D, rows_cap, ah2, al2, sl.d_r1o,
+                               sl.d_r2o, st);
     if (e != cudaSuccess) return e;
     e = tq::launch_tc_thresh(ah2, al2, rows_cap, bh, bl, planes ? nullptr : &dec, ix->n_pad, (int)K,
                              ix->K_lo, sl.d_cnt + tq::kCntFallbackRows, tq::kTensorTierMinRows, ix->n,
@@ -364,6 +382,10 @@ tq_status slot_alloc(tq_server *sv, Slot &sl) {
     const size_t o_colld = take(R * tq::kCollectCap * 4), o_colli = take(R * tq::kCollectCap * 4);
     const size_t o_scan = take(R * 4), o_list = take(R * 4), o_ap2 = take(R * K * 4);
     const size_t o_r1o = take(R * 4), o_r2o = take(R * 4), o_gthr = take(R * 8);
+    const size_t o_fp = take(R * tq::filter_k(sp->P) * 2), o_rowq = take(R * 16), o_r12 = take(R * 8);
+    const size_t o_uv = take(R * 8), o_fthr = take(R * 4), o_samp = take(R * tq::kFilterSample * 4);
+    const size_t o_fcnt = take(R * 4), o_fld = take(R * tq::kFilterCap * 4);
+    const size_t o_fli = take(R * tq::kFilterCap * 4), o_bad = take(R * 4);
     TQ_CUDA(cudaMalloc(&sl.d_block, off), "cudaMalloc(slot)");
     TQ_CUDA(cudaMemset(sl.d_block, 0, off), "cudaMemset(slot)");
     auto *base = static_cast<unsigned char *>(sl.d_block);
@@ -396,6 +418,16 @@ tq_status slot_alloc(tq_server *sv, Slot &sl) {
     sl.d_r1o = reinterpret_cast<float *>(base + o_r1o);
     sl.d_r2o = reinterpret_cast<float *>(base + o_r2o);
     sl.d_gthr = reinterpret_cast<unsigned long long *>(base + o_gthr);
+    sl.flt.planes = base + o_fp;
+    sl.flt.rowq = reinterpret_cast<float4 *>(base + o_rowq);
+    sl.flt.r12 = reinterpret_cast<float2 *>(base + o_r12);
+    sl.flt.uv = reinterpret_cast<float2 *>(base + o_uv);
+    sl.flt.thr = reinterpret_cast<float *>(base + o_fthr);
+    sl.flt.samp = reinterpret_cast<float *>(base + o_samp);
+    sl.flt.cnt = reinterpret_cast<int *>(base + o_fcnt);
+    sl.flt.list_d = reinterpret_cast<float *>(base + o_fld);
+    sl.flt.list_i = reinterpret_cast<int *>(base + o_fli);
+    sl.flt.bad = reinterpret_cast<int *>(base + o_bad);
     for (int b = 128; b < sv->max_rows; b *= 2) sl.bucket_rows.push_back(b);
     sl.bucket_rows.push_back(sv->max_rows);
     return TQ_OK;
@@ -499,7 +531,7 @@ tq_status autotune(tq_server *sv, int fixed_variant) {
         double best = 1e30;
         for (int v = 0; v < nv; ++v) {
             if (fixed_variant >= 0 && v != fixed_variant) continue;
-            if (!variant_fits(sv->index, v)) continue;
+            if (!variant_fits(sv->index, v) && v != kFilterVariant) continue;
             TQ_CUDA(enqueue_batch(sv, s0, rows, v, false), "autotune warm-up");
             TQ_CUDA(cudaEventRecord(e0, s0.stream), "event");
             for (int si = 1; si < ns; ++si)
@@ -696,8 +728,8 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
     const size_t plane_bytes = planes ? ix->n_pad * (K + (size_t)ix->K_lo) * 2 : 0;
     const size_t code_bytes = round_up(n * sp->code_size, 256);
     const size_t nscal = planes ? 2 : 4;  // c1, c2 (+ fc, fs)
-    cudaError_t e = cudaMalloc(&ix->block, plane_bytes + nscal * ix->n_pad * 4 + code_bytes +
-                                               tq::kBoundFloats * 4 + 256);
+    cudaError_t e = cudaMalloc(&ix->block, plane_bytes + (nscal + 1) * ix->n_pad * 4 + code_bytes +
+                                               (tq::kBoundFloats + tq::kFilterBound) * 4 + 256);
     if (e != cudaSuccess) {
         delete ix;
         return cuda_fail(e, "cudaMalloc(index)");
@@ -710,8 +742,13 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
         ix->fc = ix->c2 + ix->n_pad;
         ix->fs = ix->fc + ix->n_pad;
     }
-    ix->codes = reinterpret_cast<uint8_t *>(ix->c1 + nscal * ix->n_pad);
+    ix->filter.rho = reinterpret_cast<uint32_t *>(ix->c1 + nscal * ix->n_pad);
+    ix->codes = reinterpret_cast<uint8_t *>(ix->filter.rho + ix->n_pad);
     ix->bound = reinterpret_cast<float *>(ix->codes + code_bytes);
+    ix->filter.codes = ix->codes;
+    ix->filter.n = n;
+    ix->filter.bound = ix->bound + tq::kBoundFloats;
+    ix->filter.alpha = tq::filter_alpha(sp->centroids.data(), sp->levels);
     e = cudaMemcpy(ix->codes, codes, n * sp->code_size,
                    codes_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
     if (planes) {
@@ -731,6 +768,7 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
                                    nullptr);
     }
     if (e == cudaSuccess) e = tq::launch_index_bound(sp->P, ix->codes, n, ix->bound, nullptr);
+    if (e == cudaSuccess) e = tq::launch_filter_index(sp->P, sp->T, ix->filter, nullptr);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         cudaFree(ix->block);
@@ -800,6 +838,7 @@ tq_status tq_server_create_ex(tq_index *ix, const tq_server_params *prm, tq_serv
     const size_t slot_bytes =
         R * (ix->sp->dim * 4 + (2 * D + 2) * 4 + K * 4 + 8 + (size_t)k * 12 + (size_t)kc * 12 + 4 +
              (size_t)sv->fb_ctas * k * 8) +
+        R * (tq::filter_k(ix->sp->P) * 2 + 4 * tq::kFilterSample + 8 * tq::kFilterCap + 64) +
         (size_t)sms * 128 * tq::kTopKListsMax * tq::kCandMax * 8 + 8192;
     const size_t fit = std::max<size_t>(1, (free_b / 2) / slot_bytes);
     slots = (int)std::min<size_t>((size_t)slots, fit);

@@ -549,7 +549,7 @@ struct GridTiles {
 
 // ---------------------------------------------------------------------------
 // tcw_kernel: the serving top-k with 128 x 256 tiles (epilogue policies WTopk,
-// WTopkD, WThreshD).  A 128 x 128 tile
+// WThreshD).  A 128 x 128 tile
 // with three operand reads per K step needs more shared-memory bandwidth than
 // the SM has once the TMA writes are counted (128 B/clk of MMA operands + 85
 // B/clk of copies), which held tcp_kernel near half of the tensor cycles; a
@@ -1121,108 +1121,6 @@ struct WTopk {
     };
 };
 
-// The top-k over 256-wide column tiles whose sums run over the whole K in one
-// tensor-memory buffer (no promoted chunks; `kDirect`): the epilogue threads
-// read their row's 128 columns of the finished tile from tensor memory in
-// 16-column pieces and keep a register list of the best kCandMax, as TopkEpi
-// does.  Two partial lists per (row, slice), as WTopk.  Without promotion
-// the 128 x 256 tile needs no running sums in registers, which is what leaves
-// the registers for the list.
-struct WTopkD {
-    static constexpr bool kDirect = true;
-    using Params = TopkEpi::Params;  // nb_tiles counts 256-wide tiles
-    __device__ static int tiles(const Params &p) { return TopkEpi::tiles(p); }
-    __device__ static void tile_at(const Params &p, int t, int &mb, int &nb) {
-        TopkEpi::tile_at(p, t, mb, nb);
-    }
-    struct State {
-        int rit, h, m;
-        bool valid;
-        float rr1 = 0.0f, rr2 = 0.0f;
-        float bd[kCandMax];
-        int bi[kCandMax];
-        __device__ State(const Params &p, int row_in_tile, int half) : rit(row_in_tile), h(half) {
-            int mb;
-            unsigned nb0, nb1;
-            m = *p.m_dev;
-            valid = TopkEpi::slice(p, mb, nb0, nb1);
-            const int row = valid ? mb * TC_BM + rit : 0;
-            if (valid && row < m) {
-                rr1 = __ldg(p.r1 + row);
-                rr2 = __ldg(p.r2 + row);
-            }
-#pragma unroll
-            for (int t = 0; t < kCandMax; ++t) {
-                bd[t] = INFINITY;
-                bi[t] = 0x7fffffff;
-            }
-        }
-        // X: this thread's lane and first column of the tile's sums
-        // as TopkEpi::State::tile, with the row's published bound (p.gthr)
-        __device__ void tile_tmem(const Params &p, int mb, int nb, uint32_t X) {
-            const int row = mb * TC_BM + rit;
-            const bool row_ok = row < m;
-            const size_t cbase = (size_t)nb * TW_BN + TW_COLS * h;
-            const unsigned long long g = (row_ok && p.gthr) ? ld_volatile_u64(p.gthr + row) : ~0ull;
-#pragma unroll 1
-            for (int ch = 0; ch < TW_COLS / 16; ++ch) {
-                uint32_t r[16];
-                __syncwarp();
-                tmem_ld16_nw(X + 16 * ch, r);  // warp-collective: every lane loads
-                tmem_wait_ld();
-                if (!row_ok) continue;
-                const size_t col0 = cbase + ch * 16;
-                const unsigned long long own = topk_key(bd[kCandMax - 1], bi[kCandMax - 1]);
-                const unsigned long long T = own < g ? own : g;
-                float c[16];
-                uint32_t pass = 0u;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const size_t col = col0 + j;
-                    const size_t cc = col < p.n ? col : p.n - 1;
-                    const float ipt = __fmul_rn(__fmul_rn(__uint_as_float(r[j]), rr1), __ldg(p.c1 + cc));
-                    float d = __fsub_rn(__fadd_rn(rr2, __ldg(p.c2 + cc)), __fmul_rn(2.0f, ipt));
-                    d = d > 0.0f ? d : 0.0f;
-                    c[j] = d;
-                    if (col < p.n && topk_key(d, (int)col) < T) pass |= 1u << j;
-                }
-                if (pass) {
-                    float sd[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) sd[j] = c[j];
-                    do {
-                        const int j = __ffs(pass) - 1;
-                        pass &= pass - 1u;
-                        const float d = sd[j];
-                        const int ci = (int)(col0 + (size_t)j);
-                        const unsigned long long kj = topk_key(d, ci);
-                        if (kj < topk_key(bd[kCandMax - 1], bi[kCandMax - 1]) && kj < g)
-                            reg_insert(bd, bi, d, ci);
-                    } while (pass);
-                }
-            }
-            if (row_ok && p.gthr) {
-                const unsigned long long own = topk_key(bd[kCandMax - 1], bi[kCandMax - 1]);
-                if (own < g) atomicMin(p.gthr + row, own);
-            }
-        }
-        __device__ void finish(const Params &p) {
-            if (!valid) return;
-            int mb;
-            unsigned nb0, nb1;
-            TopkEpi::slice(p, mb, nb0, nb1);
-            if (mb * TC_BM + rit >= m) return;
-            const size_t o = (((size_t)blockIdx.x * TC_BM + rit) * 2 + h) * kCandMax;
-#pragma unroll
-            for (int u = 0; u < kCandMax; ++u)
-                if (u < p.k) {
-                    p.part_d[o + u] = bd[u];
-                    p.part_i[o + u] = bi[u];
-                }
-        }
-    };
-};
-
 // The threshold collection (as ThreshEpi) over 256-wide column tiles whose
 // sums run over the whole K in one tensor-memory buffer, read in place.
 struct WThreshD {
@@ -1502,9 +1400,11 @@ constexpr int kTopkShapes[][4] = {
     {TC_BM, TC_BN, 3, 4},  // 3
     {TC_BM, TC_BN, 2, 8},  // 4
     {TC_BM, TW_BN, 2, 4},  // 5: tcw_kernel
-    {TC_BM, TW_BN, 2, 0},  // 6: tcw_kernel, the whole K in one accumulator (0: no chunks)
+    // 6: the filter pass (tq_filter.cu): 256 codes by up to 256 rows over a CTA
+    // pair, two tile buffers, the whole K in one accumulator (0: no chunks)
+    {2 * TC_BM, TW_BN, 2, 0},
 };
-constexpr int kWholeK = 1 << 16;  // chunk length of variant 6: longer than any K
+constexpr int kWholeK = 1 << 16;  // chunk length of the threshold pass: longer than any K
 }  // namespace
 
 int tc_topk_variants() { return (int)(sizeof(kTopkShapes) / sizeof(kTopkShapes[0])); }
@@ -1545,7 +1445,7 @@ cudaError_t launch_tc_topk(int variant, const void *Ah, const void *Al, size_t r
                            const int *m_dev, size_t n, const float *r1, const float *r2,
                            const float *c1, const float *c2, int k, float *part_d, int *part_i,
                            unsigned long long *gthr, int *err, int grid, cudaStream_t st) {
-    if (k < 1 || k > kCandMax || grid < 1 || variant < 0 || variant >= tc_topk_variants())
+    if (k < 1 || k > kCandMax || grid < 1 || variant < 0 || variant >= tc_topk_variants() || variant == 6)
         return cudaErrorInvalidValue;
     if (K % TC_BK || k_lo % TC_BK || k_lo <= 0 || k_lo > K || rows_pad % TC_BM || n_pad % TC_BN)
         return cudaErrorInvalidValue;
@@ -1559,7 +1459,6 @@ cudaError_t launch_tc_topk(int variant, const void *Ah, const void *Al, size_t r
         if (!make_map(&mp.m[0][2], Bh, K, n_pad, TW_BN) || !make_map(&mp.m[0][3], Bl, k_lo, n_pad, TW_BN))
             return cudaErrorInvalidValue;
         const TopkEpi::Params ep{m_dev, (unsigned)(n_pad / TW_BN), n, r1, r2, c1, c2, k, part_d, part_i, gthr};
-        if (variant == 6) return tcw_launch<WTopkD, kWholeK>(mp, sh, ep, err, (unsigned)grid, st);
         if (variant == 5) return tcw_launch<WTopk, 4>(mp, sh, ep, err, (unsigned)grid, st);
         return tcw_launch<WTopk, 8>(mp, sh, ep, err, (unsigned)grid, st);
     }

@@ -68,6 +68,38 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint32_t a_lo, uint32_
             : "memory");
 }
 
+// All 512 tensor-memory columns of this CTA (PAIR: of both CTAs of the pair, called by both).
+template <bool PAIR>
+__device__ __forceinline__ void tmem_alloc512(uint32_t slot) {
+    if constexpr (PAIR) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+}
+template <bool PAIR>
+__device__ __forceinline__ void tmem_dealloc512(uint32_t base) {
+    if constexpr (PAIR)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512) : "memory");
+    else
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512) : "memory");
+}
+// 4-byte asynchronous copy (zeros for bytes = 0); the surrounding 128 bytes
+// are fetched into L2 with it (the next K blocks of the same code).
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global.L2::128B [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+                 : "memory");
+}
+// Arrives on `bar` once this thread's copies so far have landed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ---- CTA pairs (clusters of two) ---------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -92,8 +124,13 @@ __device__ __forceinline__ uint32_t rank0_addr(uint32_t addr) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
     return r;
 }
+// Arrives on a barrier of the other CTA.  No wider release than the default:
+// what the arrival reports (operand tiles, tensor-memory reads) is complete in
+// the arriving CTA's own memories before it is sent (proxy fence and local
+// barrier, or tcgen05.wait and fence), and the MMAs that depend on it access
+// them there; a cluster-scope release costs about 1,000 clocks here.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 // One lane of a converged warp (always the same one).
