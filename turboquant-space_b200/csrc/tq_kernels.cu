@@ -18,15 +18,16 @@
 #include "tq_internal.h"
 #include "tq_rht.cuh"
 
+#include <algorithm>
 #include <cstdint>
 
 namespace tq {
 namespace {
 
 // Per-warp shared bytes of the encode kernel: vpw vectors of D+8 floats, vpw x D
-// quantizer indices, vpw staged codes.
+// quantizer indices, vpw staged codes (each part a multiple of 16 bytes).
 __host__ __device__ __forceinline__ int encode_warp_bytes(int D, int cs, int vpw) {
-    return vpw * 4 * (D + 8) + vpw * D + align16(vpw * cs);
+    return vpw * 4 * (D + 8) + align16(vpw * D) + align16(vpw * cs);
 }
 
 // ---------------------------------------------------------------------------
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(256) encode_kernel(const float *__restrict__ X
     unsigned char *wbase = smem + kTabBytes + warp * encode_warp_bytes(D, cs, VPW);
     float *buf = reinterpret_cast<float *>(wbase);
     uint8_t *idxb = wbase + VPW * 4 * VS;
-    uint8_t *stage = idxb + VPW * D;
+    uint8_t *stage = idxb + align16(VPW * D);
     const int g = lane >> 3;
     float *gbuf = buf + (g % VPW) * VS;
     const bool vec4 = ((P.dim & 3) == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
@@ -518,10 +519,11 @@ __device__ __forceinline__ void rht2(float *buf, int lane, float pre, uint32_t s
     __syncwarp();
 }
 
-// Rows per warp and warps per CTA of encode2.  Byte codes at D = 1024 (168
-// registers) run 3 rows per warp in one CTA of 12 warps per SM, three warps
-// per scheduler to hide the serial reduction chains; shared memory holds 8
-// warps of 4 rows.  Everything else: 4 rows per warp, CTAs of 4 warps.
+// Rows per warp and warps per CTA of encode2 on inputs that fill the machine.
+// Byte codes at D = 1024 (168 registers) run 3 rows per warp in one CTA of 12
+// warps per SM, three warps per scheduler to hide the serial reduction chains;
+// shared memory holds 8 warps of 4 rows.  Everything else: 4 rows per warp,
+// CTAs of 4 warps.  Small inputs run one row per warp (encode2_launch).
 template <int LOG_D, bool NIBBLE>
 __host__ __device__ constexpr int enc2_rpw() { return (LOG_D == 10 && !NIBBLE) ? 3 : 4; }
 template <int LOG_D, bool NIBBLE>
@@ -536,11 +538,10 @@ __host__ __device__ constexpr int encode2_warp_bytes_c() {
     return 4 * RPW * vec_row_floats<(1 << LOG_D)>() + RPW * (1 << LOG_D);
 }
 
-template <int LOG_D, bool NIBBLE>
+template <int LOG_D, bool NIBBLE, int RPW>
 __global__ void __launch_bounds__(32 * enc2_max_warps<LOG_D, NIBBLE>()) encode2_kernel(
     const float *__restrict__ X, size_t n, uint8_t *__restrict__ out, Params P, DevTables T) {
-    constexpr int RPW = enc2_rpw<LOG_D, NIBBLE>();  // rows per warp
-    constexpr int D = 1 << LOG_D;
+    constexpr int D = 1 << LOG_D;  // RPW: rows per warp
     constexpr int E = D / 32;
     constexpr int VS = vec_row_floats<D>();
     static_assert(E >= 8 && E <= 32, "encode2 covers D = 256..1024");
@@ -561,8 +562,8 @@ __global__ void __launch_bounds__(32 * enc2_max_warps<LOG_D, NIBBLE>()) encode2_
     float *buf = reinterpret_cast<float *>(wbase);
     uint32_t *idxw = reinterpret_cast<uint32_t *>(wbase + 4 * RPW * VS);  // [RPW][E/4][32]
     uint8_t *stage = wbase;  // vector 0's buffer, once phase G has transformed it
-    // 8-lane group g runs the reduction chains of row g; with 3 rows per warp
-    // group 3 repeats row 2's (its results are not used)
+    // 8-lane group g runs the reduction chains of row g; groups past the last
+    // row repeat its chains (their results are not used)
     const int g = lane >> 3;
     const int gv = g < RPW ? g : RPW - 1;
     // sign bits of this lane's layout-A elements lane*E .. lane*E + E-1
@@ -743,7 +744,7 @@ __global__ void __launch_bounds__(32 * enc2_max_warps<LOG_D, NIBBLE>()) encode2_
 }
 
 // ---------------------------------------------------------------------------
-// prepareQuery: one warp per query.
+// prepareQuery: one warp per query (padded dims other than 256..1024).
 // ---------------------------------------------------------------------------
 template <int LOG_D>
 __global__ void __launch_bounds__(256) prepare_kernel(const float *__restrict__ Q, size_t m,
@@ -762,7 +763,21 @@ __global__ void __launch_bounds__(256) prepare_kernel(const float *__restrict__ 
     float *buf = reinterpret_cast<float *>(smem + kTabBytes) + warp * VS;
     for (size_t qi = (size_t)blockIdx.x * nwarps + warp; qi < m; qi += (size_t)gridDim.x * nwarps) {
         const float *src = Q + qi * (size_t)P.dim;
-        for (int i = lane; i < D; i += 32) buf[swz(i)] = (i < P.dim) ? src[i] : 0.0f;
+        constexpr int PER = D >= 32 ? D / 32 : 1, CH = PER < 16 ? PER : 16;
+#pragma unroll 1
+        for (int c0 = 0; c0 < PER; c0 += CH) {  // CH loads in flight
+            float x[CH];
+#pragma unroll
+            for (int t = 0; t < CH; ++t) {
+                const int i = lane + 32 * (c0 + t);
+                x[t] = i < P.dim ? __ldg(src + i) : 0.0f;
+            }
+#pragma unroll
+            for (int t = 0; t < CH; ++t) {
+                const int i = lane + 32 * (c0 + t);
+                if (i < D) buf[swz(i)] = x[t];
+            }
+        }
         __syncwarp();
         // |q|^2: the reference's batch drivers evaluate this loop as a plain
         // sequential sum (:443-445).  Lane 0 keeps the order; the squares of
@@ -788,6 +803,81 @@ __global__ void __launch_bounds__(256) prepare_kernel(const float *__restrict__ 
         fwht_from<LOG_D, 0, false>(buf, lane, 1.0f, s_qjl, P.wht_scale);
         float *sq = s_q + qi * (size_t)D;
         for (int i = lane; i < D; i += 32) sq[i] = buf[swz(i)];
+        if (lane == 0) {
+            norms[2 * qi] = qn2;
+            norms[2 * qi + 1] = qn;
+        }
+        __syncwarp();
+    }
+}
+
+// prepareQuery for D = 256, 512, 1024, with the transforms of encode2 (rht2:
+// the same roundings as fwht_from).  A single query is a serial chain of
+// latencies, so the row's loads are all in flight at once, and |q|^2 (a plain
+// sequential sum) reads four values a shared-memory load and waits only on its
+// adds: 4 clocks an element.
+template <int LOG_D>
+__global__ void __launch_bounds__(128) prepare2_kernel(const float *__restrict__ Q, size_t m,
+                                                       float *__restrict__ q_rot,
+                                                       float *__restrict__ s_q,
+                                                       float *__restrict__ norms, Params P,
+                                                       DevTables T) {
+    constexpr int D = 1 << LOG_D, E = D / 32, VS = vec_row_floats<D>();
+    __shared__ __align__(16) float s_buf[4][VS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *buf = s_buf[warp];
+    // sign bits of this lane's layout-A elements lane*E .. lane*E + E-1
+    const int bit0 = lane * E;
+    const uint32_t emask = (E >= 32) ? 0xffffffffu : ((1u << E) - 1u);
+    const uint32_t rbits = (__ldg(T.rot_mask + (bit0 >> 5)) >> (bit0 & 31)) & emask;
+    const uint32_t qbits = (__ldg(T.qjl_mask + (bit0 >> 5)) >> (bit0 & 31)) & emask;
+    for (size_t qi = (size_t)blockIdx.x * 4 + warp; qi < m; qi += (size_t)gridDim.x * 4) {
+        const float *src = Q + qi * (size_t)P.dim;
+        float x[E];
+#pragma unroll
+        for (int t = 0; t < E; ++t) x[t] = 32 * t + lane < P.dim ? __ldg(src + 32 * t + lane) : 0.0f;
+#pragma unroll
+        for (int t = 0; t < E; ++t) buf[PadLayout<E>::elem(32 * t + lane)] = x[t];
+        __syncwarp();
+        // |q|^2: the reference's batch drivers evaluate this loop as a plain
+        // sequential sum (:443-445); the zeros past dim leave it unchanged
+        float qn2 = 0.0f;
+        const int chunks = (P.dim + 3) >> 2;
+        int c = 0;
+#pragma unroll 1
+        for (; c + 8 <= chunks; c += 8) {
+            float4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const float4 *>(buf + PadLayout<E>::chunk(c + i));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                qn2 = __fadd_rn(qn2, __fmul_rn(v[i].x, v[i].x));
+                qn2 = __fadd_rn(qn2, __fmul_rn(v[i].y, v[i].y));
+                qn2 = __fadd_rn(qn2, __fmul_rn(v[i].z, v[i].z));
+                qn2 = __fadd_rn(qn2, __fmul_rn(v[i].w, v[i].w));
+            }
+        }
+        for (; c < chunks; ++c) {
+            const float4 v = *reinterpret_cast<const float4 *>(buf + PadLayout<E>::chunk(c));
+            qn2 = __fadd_rn(qn2, __fmul_rn(v.x, v.x));
+            qn2 = __fadd_rn(qn2, __fmul_rn(v.y, v.y));
+            qn2 = __fadd_rn(qn2, __fmul_rn(v.z, v.z));
+            qn2 = __fadd_rn(qn2, __fmul_rn(v.w, v.w));
+        }
+        const float qn = __fsqrt_rn(qn2);
+        const float qinv = (qn2 > f32_bits(kNormSqFloorBits)) ? __fdiv_rn(1.0f, qn) : 0.0f;
+        rht2<E, true>(buf, lane, qinv, rbits, P.wht_scale, x);
+        float *qr = q_rot + qi * (size_t)D;
+#pragma unroll
+        for (int t = 0; t < E; ++t) {
+            qr[32 * t + lane] = x[t];
+            buf[PadLayout<E>::elem(32 * t + lane)] = x[t];
+        }
+        __syncwarp();
+        rht2<E, false>(buf, lane, 1.0f, qbits, P.wht_scale, x);
+        float *sq = s_q + qi * (size_t)D;
+#pragma unroll
+        for (int t = 0; t < E; ++t) sq[32 * t + lane] = x[t];
         if (lane == 0) {
             norms[2 * qi] = qn2;
             norms[2 * qi + 1] = qn;
@@ -1706,20 +1796,19 @@ int sm_count() {
 
 constexpr int kSmemBudget = 227 * 1024;
 
-template <int LOG_D, bool NIBBLE>
-cudaError_t encode2_launch(const Params &P, const DevTables &T, const float *X, size_t n,
-                           uint8_t *out, cudaStream_t st) {
-    constexpr int RPW = enc2_rpw<LOG_D, NIBBLE>();
+template <int LOG_D, bool NIBBLE, int RPW>
+cudaError_t encode2_run(const Params &P, const DevTables &T, const float *X, size_t n, uint8_t *out,
+                        int max_warps, cudaStream_t st) {
     const int per_warp = encode2_warp_bytes_c<LOG_D, RPW>();
     int warps = (kSmemBudget - kTabBytes - crep_bytes(P)) / per_warp;
-    if (warps > enc2_max_warps<LOG_D, NIBBLE>()) warps = enc2_max_warps<LOG_D, NIBBLE>();
+    if (warps > max_warps) warps = max_warps;
     if (warps < 1) return cudaErrorInvalidConfiguration;
     const size_t smem = (size_t)kTabBytes + crep_bytes(P) + (size_t)warps * per_warp;
-    cudaError_t e = cudaFuncSetAttribute(encode2_kernel<LOG_D, NIBBLE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto kern = encode2_kernel<LOG_D, NIBBLE, RPW>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, encode2_kernel<LOG_D, NIBBLE>, 32 * warps, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     const size_t groups = (n + RPW - 1) / RPW;
@@ -1727,7 +1816,44 @@ cudaError_t encode2_launch(const Params &P, const DevTables &T, const float *X, 
     const size_t cap = (size_t)sm_count() * per_sm;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    encode2_kernel<LOG_D, NIBBLE><<<(unsigned)blocks, 32 * warps, smem, st>>>(X, n, out, P, T);
+    kern<<<(unsigned)blocks, 32 * warps, smem, st>>>(X, n, out, P, T);
+    return cudaGetLastError();
+}
+
+// Rows up to which an encode runs one row per warp: 8 a multiprocessor.  A warp
+// takes its rows' transforms one after the other, so fewer rows a warp end
+// sooner while multiprocessors are idle.
+size_t encode_small_rows() { return (size_t)sm_count() * 8; }
+
+template <int LOG_D, bool NIBBLE>
+cudaError_t encode2_launch(const Params &P, const DevTables &T, const float *X, size_t n,
+                           uint8_t *out, cudaStream_t st) {
+    if (n <= encode_small_rows()) return encode2_run<LOG_D, NIBBLE, 1>(P, T, X, n, out, 2, st);
+    return encode2_run<LOG_D, NIBBLE, enc2_rpw<LOG_D, NIBBLE>()>(P, T, X, n, out,
+                                                                 enc2_max_warps<LOG_D, NIBBLE>(), st);
+}
+
+template <int LOG_D, int VPW>
+cudaError_t encode_run(const Params &P, const DevTables &T, const float *X, size_t n, uint8_t *out,
+                       int max_warps, cudaStream_t st) {
+    auto kern = encode_kernel<LOG_D, VPW>;
+    const int per_warp = encode_warp_bytes(1 << LOG_D, P.cs, VPW);
+    int warps = (kSmemBudget - kTabBytes) / per_warp;
+    if (warps > max_warps) warps = max_warps;
+    if (warps < 1) return cudaErrorInvalidConfiguration;
+    const size_t smem = (size_t)kTabBytes + (size_t)warps * per_warp;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) per_sm = 1;
+    const size_t groups = (n + VPW - 1) / VPW;
+    size_t blocks = (groups + warps - 1) / warps;
+    const size_t cap = (size_t)sm_count() * per_sm;
+    if (blocks > cap) blocks = cap;
+    if (blocks < 1) blocks = 1;
+    kern<<<(unsigned)blocks, 32 * warps, smem, st>>>(X, n, out, P, T);
     return cudaGetLastError();
 }
 
@@ -1735,30 +1861,13 @@ template <int LOG_D>
 struct EncodeRun {
     static cudaError_t run(const Params &P, const DevTables &T, const float *X, size_t n,
                            uint8_t *out, cudaStream_t st) {
-        if constexpr (LOG_D >= 8 && LOG_D <= 10)
+        if constexpr (LOG_D >= 8 && LOG_D <= 10) {
             return P.nibble ? encode2_launch<LOG_D, true>(P, T, X, n, out, st)
                             : encode2_launch<LOG_D, false>(P, T, X, n, out, st);
-        constexpr int VPW = LOG_D >= 11 ? 2 : 4;
-        auto kern = encode_kernel<LOG_D, VPW>;
-        const int D = 1 << LOG_D;
-        const int per_warp = encode_warp_bytes(D, P.cs, VPW);
-        int warps = (kSmemBudget - kTabBytes) / per_warp;
-        if (warps > 8) warps = 8;
-        if (warps < 1) return cudaErrorInvalidConfiguration;
-        const size_t smem = (size_t)kTabBytes + (size_t)warps * per_warp;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
-        if (e != cudaSuccess) return e;
-        if (per_sm < 1) per_sm = 1;
-        const size_t groups = (n + VPW - 1) / VPW;
-        size_t blocks = (groups + warps - 1) / warps;
-        const size_t cap = (size_t)sm_count() * per_sm;
-        if (blocks > cap) blocks = cap;
-        if (blocks < 1) blocks = 1;
-        kern<<<(unsigned)blocks, 32 * warps, smem, st>>>(X, n, out, P, T);
-        return cudaGetLastError();
+        } else {
+            if (n <= encode_small_rows()) return encode_run<LOG_D, 1>(P, T, X, n, out, 2, st);
+            return encode_run<LOG_D, LOG_D >= 11 ? 2 : 4>(P, T, X, n, out, 8, st);
+        }
     }
 };
 
@@ -1766,6 +1875,12 @@ template <int LOG_D>
 struct PrepareRun {
     static cudaError_t run(const Params &P, const DevTables &T, const float *Q, size_t m,
                            float *q_rot, float *s_q, float *norms, cudaStream_t st) {
+        if constexpr (LOG_D >= 8 && LOG_D <= 10) {
+            const size_t blocks = std::min((m + 3) / 4, (size_t)sm_count() * 8);
+            prepare2_kernel<LOG_D><<<(unsigned)std::max<size_t>(blocks, 1), 128, 0, st>>>(Q, m, q_rot, s_q, norms,
+                                                                                          P, T);
+            return cudaGetLastError();
+        }
         const int D = 1 << LOG_D;
         int warps = (kSmemBudget - kTabBytes) / (4 * (D + 8));
         if (warps > 8) warps = 8;
