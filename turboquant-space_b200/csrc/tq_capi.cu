@@ -759,6 +759,51 @@ tq_status tq_distance_m_to_n_symmetric_device(const tq_space *sp, const uint8_t 
     return TQ_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+constexpr size_t kSmallResult = size_t(256) << 10;
+
+// distance_1_to_n of few host codes: one stream, one allocation, and one copy
+// back that brings the status word with the distances.  A re-ranking of 1,000
+// codes is all fixed costs: the two-stream form's second buffer, event and
+// streams' waits and its separate status read took 24 of 79 us.
+tq_status scan_host_small(tq_space *sp, const float *query, const uint8_t *codes, size_t n, float *out,
+                          cudaStream_t s) {
+    const size_t dim = sp->dim, D = sp->D, cs = sp->code_size;
+    const size_t o_prep = (dim * 4 + 15) & ~size_t(15), o_codes = o_prep + ((2 * D + 2) * 4 + 15) / 16 * 16;
+    const size_t o_out = o_codes + ((n * cs + 15) & ~size_t(15)), bytes = o_out + (n + 1) * 4;
+    Scratch buf;
+    TQ_CUDA(buf.alloc(bytes, s), "cudaMallocAsync(scan)");
+    auto *b = static_cast<unsigned char *>(buf.p);
+    float *dq = reinterpret_cast<float *>(b), *q_rot = reinterpret_cast<float *>(b + o_prep);
+    float *s_q = q_rot + D, *norms = s_q + D, *d_out = reinterpret_cast<float *>(b + o_out);
+    uint8_t *d_codes = b + o_codes;
+    std::vector<float> host;
+    try {
+        host.resize(n + 1);
+    } catch (const std::bad_alloc &) {
+        return fail(TQ_ERR_OUT_OF_MEMORY, "distance_1_to_n: host memory");
+    }
+    TQ_CUDA(cudaMemcpyAsync(dq, query, dim * 4, cudaMemcpyHostToDevice, s), "H2D query");
+    TQ_CUDA(tq::launch_prepare(sp->P, sp->T, dq, 1, q_rot, s_q, norms, s), "prepare kernel");
+    TQ_CUDA(cudaMemcpyAsync(d_codes, codes, n * cs, cudaMemcpyHostToDevice, s), "H2D codes");
+    TQ_CUDA(tq::launch_scan_1_to_n(sp->P, sp->T, q_rot, s_q, norms, d_codes, n, d_out, s), "scan kernel");
+    TQ_CUDA(cudaMemcpyAsync(d_out + n, sp->T.status, sizeof(int), cudaMemcpyDeviceToDevice, s), "status");
+    TQ_CUDA(cudaMemcpyAsync(host.data(), d_out, (n + 1) * 4, cudaMemcpyDeviceToHost, s), "D2H distances");
+    TQ_CUDA(cudaStreamSynchronize(s), "distance_1_to_n");
+    int code = 0;
+    std::memcpy(&code, &host[n], sizeof(int));
+    if (code != 0) return take_status(sp, nullptr);
+    std::memcpy(out, host.data(), n * 4);
+    return TQ_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 // ---- host-pointer entry points ---------------------------------------------
 // Inputs are streamed through the GPU in chunks of ~256 MB on two streams that
 // alternate, so the copies of one chunk overlap the kernels of the other.
@@ -810,6 +855,7 @@ tq_status tq_distance_1_to_n(const tq_space *csp, const float *query, const uint
     size_t per = std::max<size_t>(1, kChunkBytes / cs);
     per = std::min(per, n);
     cudaStream_t s0 = sp->host_stream[0];
+    if (n * sizeof(float) <= kSmallResult && n <= per) return scan_host_small(sp, query, codes, n, out, s0);
     Scratch qs;
     TQ_CUDA(qs.alloc(sizeof(float) * (sp->dim + 2 * sp->D + 2), s0), "cudaMallocAsync(query)");
     float *dq = static_cast<float *>(qs.p), *q_rot = dq + sp->dim, *s_q = q_rot + sp->D,

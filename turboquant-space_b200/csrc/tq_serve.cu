@@ -41,6 +41,9 @@
 //              stable argsort of the reference's distances, whatever the
 //              batch they ran in.
 #include <cuda_runtime.h>
+#ifdef __linux__
+#include <sys/prctl.h>
+#endif
 
 #include <algorithm>
 #include <atomic>
@@ -610,6 +613,10 @@ void finish_request(tq_server *sv, tq_request *r, double t) {
 void worker_loop(tq_server *sv) {
     DeviceGuard g(sv->index->device);
     const int k = sv->k;
+#ifdef __linux__
+    prctl(PR_SET_TIMERSLACK, 1000UL);  // this thread's sleeps end within 1 us (the default adds 50)
+#endif
+    double launched_ms = now_ms();
     std::unique_lock<std::mutex> lk(sv->mu);
     while (true) {
         bool any_busy = false;
@@ -677,11 +684,17 @@ void worker_loop(tq_server *sv) {
             }
             sl.busy = true;
             any_busy = true;
+            launched_ms = now_ms();
             ++sv->batches;
         }
         if (any_busy) {
+            // Poll at about 1/16 of the time the youngest batch has run, 5 to 50 us:
+            // a short batch's results wait a few microseconds, a long one costs
+            // few wake-ups.
+            const double ran_us = (now_ms() - launched_ms) * 1e3;
+            const int us = (int)std::min(50.0, std::max(5.0, ran_us / 16));
             lk.unlock();
-            std::this_thread::sleep_for(std::chrono::microseconds(50));
+            std::this_thread::sleep_for(std::chrono::microseconds(us));
             lk.lock();
         } else {
             sv->cv.wait_for(lk, std::chrono::milliseconds(5),

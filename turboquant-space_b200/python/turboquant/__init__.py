@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 
 import numpy as np
 
@@ -40,8 +41,18 @@ def _dlpack_cuda(obj) -> bool:
         return False
 
 
+def _plain_cuda(obj) -> bool:
+    """A plain strided torch CUDA tensor, read through its own attributes: the
+    interface's dict is built anew (1.4 us) at every look at it."""
+    t = sys.modules.get("torch")
+    return (t is not None and type(obj) is t.Tensor and obj.is_cuda and not obj.requires_grad
+            and obj.layout is t.strided and not obj.is_neg())
+
+
 def _is_device(obj) -> bool:
-    return hasattr(obj, "__cuda_array_interface__") or _dlpack_cuda(obj)
+    if type(obj) is np.ndarray:
+        return False
+    return _plain_cuda(obj) or hasattr(obj, "__cuda_array_interface__") or _dlpack_cuda(obj)
 
 
 def _as_cai(obj):
@@ -141,6 +152,9 @@ def _contig(shape, strides, itemsize):
 
 
 def _float_dev(obj, expected_last, name, expected_ndim):
+    if _plain_cuda(obj) and obj.dtype is _torch().float32 and obj.is_contiguous() \
+            and obj.dim() == expected_ndim and obj.shape[-1] == expected_last:
+        return obj.data_ptr(), obj.shape
     ptr, shape, typestr, strides = _cai(obj)
     if typestr not in ("<f4", "=f4", "f4"):
         raise ValueError(f"{name}: expected float32")
@@ -156,6 +170,10 @@ def _float_dev(obj, expected_last, name, expected_ndim):
 
 
 def _codes_dev(obj, cs, bad_type_msg="codes must be uint8"):
+    if _plain_cuda(obj) and obj.dtype is _torch().uint8 and obj.is_contiguous():
+        total = obj.numel()
+        if total % cs == 0:
+            return obj.data_ptr(), total // cs
     ptr, shape, typestr, strides = _cai(obj)
     if typestr[-1] != "1":
         raise ValueError(bad_type_msg)
@@ -169,6 +187,10 @@ def _codes_dev(obj, cs, bad_type_msg="codes must be uint8"):
 
 def _stream_and_device(obj):
     torch = _torch()
+    if _plain_cuda(obj):
+        dev = obj.device
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        return (raw(dev.index) if raw else torch.cuda.current_stream(dev).cuda_stream), dev
     obj = _as_cai(obj)
     dev = obj.device if isinstance(getattr(obj, "device", None), torch.device) \
         else torch.device("cuda", torch.cuda.current_device())
