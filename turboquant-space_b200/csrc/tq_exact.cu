@@ -273,6 +273,76 @@ __device__ __forceinline__ void load_centroids(float *sc, const float *centroids
     __syncthreads();
 }
 
+// hsum8 of values held one a lane, value j in lane base + j of an 8-lane run.
+__device__ __forceinline__ float hsum8_lanes(float v, int base, int lane) {
+    const int j = base + (lane & 3);
+    const float w = __fadd_rn(__shfl_sync(kFull, v, j), __shfl_sync(kFull, v, j + 4));
+    const float e = __fadd_rn(__shfl_sync(kFull, w, base), __shfl_sync(kFull, w, base + 2));
+    const float o = __fadd_rn(__shfl_sync(kFull, w, base + 1), __shfl_sync(kFull, w, base + 3));
+    return __fadd_rn(e, o);
+}
+
+// exact_b4 (D >= 64) of four codes by a warp: lane t keeps running sum t of each,
+// which takes bytes t, t + 32, ...; the same operations in the same order.  All
+// lanes get the results.
+__device__ __forceinline__ void warp_exact_b4(const float *sc, const float *__restrict__ q,
+                                              const float *__restrict__ s, float qn2, float qn, float scale,
+                                              int nb, const uint8_t *const (&code)[4], bool al4, int lane,
+                                              float (&d)[4]) {
+    float A[4] = {0.0f, 0.0f, 0.0f, 0.0f}, S[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float xn[4], g[4], sig[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        xn[c] = ld_f32(code[c] + nb, al4);
+        g[c] = ld_f32(code[c] + nb + 4, al4);
+        sig[c] = ld_f32(code[c] + nb + 8, al4);
+    }
+#pragma unroll 4
+    for (int k = lane; k < nb; k += 32) {
+        const float2 qq = __ldg(reinterpret_cast<const float2 *>(q) + k);
+        const float2 ss = __ldg(reinterpret_cast<const float2 *>(s) + k);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const unsigned byte = __ldg(code[c] + k), lo = byte & 15u, hi = byte >> 4;
+            const float ph = __fmul_rn(qq.y, sc[hi >> 1]);
+            A[c] = __fadd_rn(A[c], __fmaf_rn(qq.x, sc[lo >> 1], ph));
+            S[c] = __fadd_rn(S[c], __fadd_rn(sgn_s(ss.x, lo & 1u), sgn_s(ss.y, hi & 1u)));
+        }
+    }
+    const int j = lane & 7;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float V = __fadd_rn(__fadd_rn(__shfl_sync(kFull, A[c], 16 + j), __shfl_sync(kFull, A[c], 24 + j)),
+                                  __fadd_rn(__shfl_sync(kFull, A[c], j), __shfl_sync(kFull, A[c], 8 + j)));
+        const float W = __fadd_rn(__fadd_rn(__shfl_sync(kFull, S[c], 16 + j), __shfl_sync(kFull, S[c], 24 + j)),
+                                  __fadd_rn(__shfl_sync(kFull, S[c], j), __shfl_sync(kFull, S[c], 8 + j)));
+        const float ip = hsum8_lanes(V, 0, lane), dot = hsum8_lanes(W, 0, lane);
+        float t = __fmul_rn(__fmul_rn(scale, g[c]), dot);
+        t = __fmul_rn(__fmaf_rn(ip, sig[c], t), xn[c]);
+        d[c] = finish_dist(t, xn[c], qn2, qn);
+    }
+}
+
+// exact_b8 (D >= 8) of four codes by a warp: lane j of each 8-lane run keeps
+// running sum j of its run's code.  All lanes of a run get its result.
+__device__ __forceinline__ float warp_exact_b8(const float *sc, const float *__restrict__ q,
+                                               const float *__restrict__ s, float qn2, float qn, float scale,
+                                               int D, const uint8_t *__restrict__ code, bool al4, int lane) {
+    float A = 0.0f, S = 0.0f;
+#pragma unroll 8
+    for (int i = lane & 7; i < D; i += 8) {
+        const unsigned u = code[i];
+        A = __fmaf_rn(sc[u >> 1], __ldg(q + i), A);
+        S = __fadd_rn(S, sgn_s(__ldg(s + i), u & 1u));
+    }
+    const int base = lane & 24;
+    const float xn = ld_f32(code + D, al4), g = ld_f32(code + D + 4, al4);
+    const float sig = ld_f32(code + D + 8, al4);
+    const float ip = __fmul_rn(hsum8_lanes(A, base, lane), sig), dot = hsum8_lanes(S, base, lane);
+    const float t = __fmul_rn(__fmaf_rn(__fmul_rn(g, scale), dot, ip), xn);
+    return finish_dist(t, xn, qn2, qn);
+}
+
 struct RescoreArgs {
     Params P;
     const float *centroids;
@@ -295,7 +365,11 @@ struct RescoreArgs {
     int *counters;
 };
 
-// One warp per query row, lane l on candidate l.
+// One CTA of eight warps per query row.  A code's running sums are spread over
+// lanes (32 for nibble codes, 8 for byte codes), four candidates a warp: a
+// thread per candidate walked its code alone, 38 us of dependent loads at
+// 384-d for any number of rows, against 10 for 5 rows and 32 for 1,024.  Warp 0 then certifies and
+// sorts, lane l on candidate l.
 //
 // The certificate.  Let d'_j be the tensor pass's distance of code j and d_j
 // the reference's.  If |d'_j - d_j| <= eps for every j, a code outside the kc
@@ -323,24 +397,37 @@ struct RescoreArgs {
 template <bool NIBBLE>
 __global__ void __launch_bounds__(256) rescore_kernel(RescoreArgs a) {
     __shared__ float sc[kMaxLevels];
-    load_centroids(sc, a.centroids, a.P.levels);
+    __shared__ float s_ed[32], s_sum[2][8];
     const int m = *a.m_dev;
-    const int D = a.P.D, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < m; row += gridDim.x * wpb) {
+    if ((int)blockIdx.x >= m) return;
+    load_centroids(sc, a.centroids, a.P.levels);
+    const int D = a.P.D, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row = blockIdx.x;
+    {
         const float *q = a.q_rot + (size_t)row * D, *s = a.s_q + (size_t)row * D;
         const float qn2 = a.norms[2 * row], qn = a.norms[2 * row + 1];
-        float ad = INFINITY, ed = INFINITY;
-        int ci = kNoIdx;
-        if (lane < a.kc) {
-            const long long id = a.cand_i[(size_t)row * a.kc + lane];
-            if (id >= 0 && (size_t)id < a.n) {
-                ci = (int)id;
-                ad = a.cand_d[(size_t)row * a.kc + lane];
-                ed = exact_dist<NIBBLE>(a.P, sc, q, s, qn2, qn, a.codes + (size_t)ci * a.P.cs, a.al4);
-            }
+        const long long *cand = a.cand_i + (size_t)row * a.kc;
+        // candidate c's code (any code stands in for a missing one: its distance is not used)
+        auto code_of = [&](int c) {
+            const long long id = c < a.kc ? cand[c] : 0;
+            return a.codes + (size_t)(id >= 0 && (size_t)id < a.n ? id : 0) * a.P.cs;
+        };
+        if (NIBBLE && D >= 64) {
+            const uint8_t *code[4];
+            float d[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) code[c] = code_of(4 * warp + c);
+            warp_exact_b4(sc, q, s, qn2, qn, a.P.scale, a.P.pb, code, a.al4, lane, d);
+            if (lane < 4) s_ed[4 * warp + lane] = lane == 0 ? d[0] : lane == 1 ? d[1] : lane == 2 ? d[2] : d[3];
+        } else if (!NIBBLE && D >= 8) {
+            const int c = 4 * warp + (lane >> 3);
+            const float d = warp_exact_b8(sc, q, s, qn2, qn, a.P.scale, D, code_of(c), a.al4, lane);
+            if ((lane & 7) == 0) s_ed[c] = d;
+        } else if (warp == 0) {
+            s_ed[lane] = exact_dist<NIBBLE>(a.P, sc, q, s, qn2, qn, code_of(lane), a.al4);
         }
         float sq = 0.0f, ss = 0.0f;
-        for (int i = lane; i < D; i += 32) {
+        for (int i = threadIdx.x; i < D; i += 256) {
             sq += fabsf(q[i]);
             ss += fabsf(s[i]);
         }
@@ -348,6 +435,28 @@ __global__ void __launch_bounds__(256) rescore_kernel(RescoreArgs a) {
         for (int off = 16; off > 0; off >>= 1) {
             sq += __shfl_xor_sync(kFull, sq, off);
             ss += __shfl_xor_sync(kFull, ss, off);
+        }
+        if (lane == 0) {
+            s_sum[0][warp] = sq;
+            s_sum[1][warp] = ss;
+        }
+        __syncthreads();
+        if (warp != 0) return;
+        sq = ss = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            sq += s_sum[0][w];
+            ss += s_sum[1][w];
+        }
+        float ad = INFINITY, ed = INFINITY;
+        int ci = kNoIdx;
+        if (lane < a.kc) {
+            const long long id = cand[lane];
+            if (id >= 0 && (size_t)id < a.n) {
+                ci = (int)id;
+                ad = a.cand_d[(size_t)row * a.kc + lane];
+                ed = s_ed[lane];
+            }
         }
         // eps for this pass's candidates; eps_t for the threshold pass that may
         // rescan an open row (its own kappa, kappa_t >= kappa)
@@ -1002,7 +1111,7 @@ cudaError_t launch_rescore(const Params &P, const float *centroids, float cmax, 
                         cand_i, q_rot,    s_q,   norms,     codes,       n,     codes_al4(P, codes),
                         bound, kappa, kappa_t > kappa ? kappa_t : kappa, bound_scale, filter, out_d, out_i,
                         fail_rows, thr, tthr, counters};
-    const unsigned blocks = (unsigned)((max_rows + 7) / 8);
+    const unsigned blocks = (unsigned)max_rows;
     if (P.nibble)
         rescore_kernel<true><<<blocks, 256, 0, st>>>(a);
     else

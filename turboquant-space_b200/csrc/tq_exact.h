@@ -32,7 +32,7 @@ constexpr int kCollectCap = 1024;
 // costs for five).
 constexpr int kTensorTierMinRows = 4;
 
-// Candidate rescoring: one warp per query row (row count read from m_dev).
+// Candidate rescoring: one CTA per query row (row count read from m_dev).
 // cand_d / cand_i hold each row's kc (<= 32) tensor-pass candidates, ascending
 // by (approximate distance, index), index -1 past the corpus.  Each candidate
 // is rescored with the reference's own arithmetic; the row's k best by
