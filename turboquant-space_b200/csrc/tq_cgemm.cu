@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
-            mbar_init(full0 + 8 * s, 1 + DW);  // the producer and one lane of each decoder warp
+            mbar_init(full0 + 8 * s, 1 + 4);  // the producer and the block's four decoder warps
             mbar_init(empty0 + 8 * s, 1);
             mbar_init(pfull0 + 8 * s, 1);
         }
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         }
         for (int k = 0; k < p.ring; ++k) {
             mbar_init(cfull0 + 8 * k, 64);  // every loader thread
-            mbar_init(cempty0 + 8 * k, DW);
+            mbar_init(cempty0 + 8 * k, 4);
         }
         mbar_init(drain, 1);
         mbar_init_fence();
@@ -397,12 +397,16 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         }
     } else if (warp < 4 + DW) {
         // ---------------- decoders ----------------
-        // Warp w decodes rows RPW w ..: lane l takes 16-byte chunk l & 7 (8
-        // coordinates) of rows 4 i + (l >> 3), so eight lanes read a row's
-        // consecutive words and write its 128 bytes without bank conflicts.
+        // Four warps decode a K block, 32 rows each: lane l takes 16-byte chunk
+        // l & 7 (8 coordinates) of rows 4 i + (l >> 3), so eight lanes read a
+        // row's consecutive words and write its 128 bytes without bank
+        // conflicts.  Eight warps are two groups that take every other block:
+        // a block's waits, loads and fence are latencies in series, which the
+        // groups overlap (8 x 200k, 768-d 8-bit: 255 -> 242 us; 384-d 4-bit: 100 ->
+        // 95 us; 40 x 50k, 1536-d 4-bit: 129 -> 118 us).
         if constexpr (DW == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
-        constexpr int RPW = CG_BM / DW, ITEMS = RPW / 4;
-        const int r0 = (warp - 4) * RPW + (lane >> 3), c = lane & 7;
+        constexpr int GROUPS = DW / 4, ITEMS = 8;
+        const int r0 = ((warp - 4) & 3) * 32 + (lane >> 3), c = lane & 7;
         NibTab tab{};
         if constexpr (NIB) {
 #pragma unroll
@@ -420,10 +424,14 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         const uint32_t one = p.fmt == kCgFP16 ? 0x3C003C00u : 0x3F803F80u;
         const uint32_t pm = p.fmt == kCgFP16 ? 0x3CBCu : 0x3FBFu;
         const uint32_t *tl = btab + lane;
-        uint32_t s = 0, ph = 1, cs = 0, cph = 0;
+        // block `it` of the CTA: stage it % stages and ring slot it % ring (both
+        // counts are 2 or more)
+        const uint32_t group = GROUPS == 2 ? (uint32_t)(warp - 4) >> 2 : 0u;
+        uint32_t s = group, ph = 1, cs = group, cph = 0, it = 0;
         bool ok = true;
         for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
-            for (int kb = 0; kb < KB; ++kb) {
+            for (int kb = 0; kb < KB; ++kb, ++it) {
+                if (GROUPS == 2 && (it & 1u) != group) continue;
                 if (!mbar_wait_warp(cfull0 + 8 * cs, cph, p.err, kErrFull)) { ok = false; break; }
                 uint32_t w[ITEMS][WPI];
                 const unsigned char *rb = ring + cs * RING_BYTES;
@@ -475,8 +483,10 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
                     mbar_arrive(full0 + 8 * s);
                     mbar_arrive(cempty0 + 8 * cs);
                 }
-                if (++s == (uint32_t)p.stages) { s = 0; ph ^= 1u; }
-                if (++cs == (uint32_t)p.ring) { cs = 0; cph ^= 1u; }
+                s += GROUPS;
+                if (s >= (uint32_t)p.stages) { s -= p.stages; ph ^= 1u; }
+                cs += GROUPS;
+                if (cs >= (uint32_t)p.ring) { cs -= p.ring; cph ^= 1u; }
             }
         }
     } else {
@@ -714,7 +724,7 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     for (int NT = 256; NT >= 16; NT >>= 1) {
         const size_t tiles = code_tiles(NT) * ((m + NT - 1) / NT), slots = NT > 64 ? 74 : 148;
         const double waves = (double)((tiles + slots - 1) / slots);
-        const double mma = 5.0 * NT, dec = NT <= 64 ? 750.0 : 1000.0;
+        const double mma = 5.0 * NT, dec = NT <= 64 ? 600.0 : 1000.0;
         const double tt = waves * (a.KB * std::max(mma, dec) + 8.0 * NT + 1000.0);
         if (NT == 256 || tt < best_t) {
             a.NT = NT;
