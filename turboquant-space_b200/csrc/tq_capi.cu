@@ -332,6 +332,7 @@ tq_status tq_space_create(size_t dim, int bits, uint64_t rot_seed, uint64_t qjl_
         P.lutq = 0;
         P.qlut_k = 0;
         P.qflag = 0;
+        P.qshift = 0;
         if (tq::build_quant_lut(sp->boundaries, tq::kQlutBuckets, tq::kQlutMaxK, sp->qlut)) {
             P.lutq = 1;
             P.qlut_k = sp->qlut.k;
@@ -340,6 +341,7 @@ tq_status tq_space_create(size_t dim, int bits, uint64_t rot_seed, uint64_t qjl_
             // one boundary at most per bucket and lo < 128: bit 7 can flag the
             // buckets that hold one (the others need no comparison)
             P.qflag = (P.qlut_k == 1 && sp->levels <= 128) ? 1 : 0;
+            if (P.qflag) P.qshift = tq::coarse_shift(sp->qlut, P.nb);
         }
 
         // device binding (optional: without a GPU the space answers geometry

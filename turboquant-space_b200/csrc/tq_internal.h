@@ -39,6 +39,7 @@ struct Params {
     int qlut_k;        // boundaries compared per bucket
     int qflag;         // 1: T.qlutf holds lo | 0x80 for the buckets that hold a boundary
                        //    (levels <= 128, qlut_k = 1)
+    int qshift;        // > 0 (P.qflag): 2^qshift neighbouring buckets hold one boundary at most
     float qlut_s;      // bucket(v) = clamp(fma(v, qlut_s, qlut_c), 0, NB-1)
     float qlut_c;
     float scale;       // sqrt(pi/2)/sqrt(D)            space_turbo_quant.h:265
@@ -60,6 +61,10 @@ struct DevTables {
 // ---- kernel launchers (tq_kernels.cu); all stream-ordered -------------------
 cudaError_t launch_encode(const Params &P, const DevTables &T, const float *X, size_t n,
                           uint8_t *out, cudaStream_t st);
+// Encode for padded dims 256 .. 1024 and P.qshift > 0, rows in registers
+// (tq_encode.cu); launch_encode takes it for inputs that fill the device.
+cudaError_t launch_encode_regs(const Params &P, const DevTables &T, const float *X, size_t n, uint8_t *out,
+                               int sms, cudaStream_t st);
 cudaError_t launch_prepare(const Params &P, const DevTables &T, const float *Q, size_t m,
                            float *q_rot, float *s_q, float *norms, cudaStream_t st);
 cudaError_t launch_scan_1_to_n(const Params &P, const DevTables &T, const float *q_rot,

@@ -317,32 +317,6 @@ __global__ void __launch_bounds__(256) encode_kernel(const float *__restrict__ X
 // accesses, the layout-B accesses and the 8-lane reduction chains are free of
 // bank conflicts without per-access index arithmetic.
 // ---------------------------------------------------------------------------
-typedef unsigned long long u64;
-
-__device__ __forceinline__ u64 fadd2(u64 a, u64 b) {
-    u64 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ u64 fsub2(u64 a, u64 b) {
-    u64 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ u64 fmul2(u64 a, u64 b) {
-    u64 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ u64 mk2(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void un2(u64 v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 // Vector buffer layout of encode2: element e at e + 4 (e >> 5), i.e. every
 // 32-float row is followed by 4 floats of padding.  The layout-A float4
 // accesses (lane l: elements E l .. E l + E - 1), the layout-B accesses
@@ -519,15 +493,15 @@ __device__ __forceinline__ void rht2(float *buf, int lane, float pre, uint32_t s
     __syncwarp();
 }
 
-// Rows per warp and warps per CTA of encode2 on inputs that fill the machine.
-// Byte codes at D = 1024 (168 registers) run 3 rows per warp in one CTA of 12
-// warps per SM, three warps per scheduler to hide the serial reduction chains;
-// shared memory holds 8 warps of 4 rows.  Everything else: 4 rows per warp,
-// CTAs of 4 warps.  Small inputs run one row per warp (encode2_launch).
-template <int LOG_D, bool NIBBLE>
-__host__ __device__ constexpr int enc2_rpw() { return (LOG_D == 10 && !NIBBLE) ? 3 : 4; }
-template <int LOG_D, bool NIBBLE>
-__host__ __device__ constexpr int enc2_max_warps() { return (LOG_D == 10 && !NIBBLE) ? 12 : 4; }
+// Rows per warp and warps per CTA of encode2 on inputs that fill the machine
+// (byte codes; see encode2_launch).  D = 1024 (168 registers) runs 3 rows per
+// warp in one CTA of 12 warps per SM, three warps per scheduler to hide the
+// serial reduction chains; shared memory holds 8 warps of 4 rows.  Everything
+// else: 4 rows per warp, CTAs of 4 warps.  Small inputs run one row per warp.
+template <int LOG_D>
+__host__ __device__ constexpr int enc2_rpw() { return LOG_D == 10 ? 3 : 4; }
+template <int LOG_D>
+__host__ __device__ constexpr int enc2_max_warps() { return LOG_D == 10 ? 12 : 4; }
 
 // Per-warp shared bytes of encode2: RPW padded vectors and the quantizer
 // indices of RPW vectors (D bytes each, one 32-bit word per lane and 4
@@ -539,7 +513,7 @@ __host__ __device__ constexpr int encode2_warp_bytes_c() {
 }
 
 template <int LOG_D, bool NIBBLE, int RPW>
-__global__ void __launch_bounds__(32 * enc2_max_warps<LOG_D, NIBBLE>()) encode2_kernel(
+__global__ void __launch_bounds__(32 * (NIBBLE ? 4 : enc2_max_warps<LOG_D>())) encode2_kernel(
     const float *__restrict__ X, size_t n, uint8_t *__restrict__ out, Params P, DevTables T) {
     constexpr int D = 1 << LOG_D;  // RPW: rows per warp
     constexpr int E = D / 32;
@@ -1829,8 +1803,16 @@ template <int LOG_D, bool NIBBLE>
 cudaError_t encode2_launch(const Params &P, const DevTables &T, const float *X, size_t n,
                            uint8_t *out, cudaStream_t st) {
     if (n <= encode_small_rows()) return encode2_run<LOG_D, NIBBLE, 1>(P, T, X, n, out, 2, st);
-    return encode2_run<LOG_D, NIBBLE, enc2_rpw<LOG_D, NIBBLE>()>(P, T, X, n, out,
-                                                                 enc2_max_warps<LOG_D, NIBBLE>(), st);
+    if constexpr (!NIBBLE) {
+        // Rows from shared memory: b = 9 (its 9-bit units and 256 levels are not the
+        // register kernel's), and at D = 1024 the inputs that fill one round of
+        // 36 rows a multiprocessor here but take the register kernel's 32 rows
+        // twice (4800 rows of 768: 22.6 and 24.8 us).
+        const size_t sms = sm_count();
+        if (P.qshift == 0 || (LOG_D == 10 && n > 32 * sms && n <= 36 * sms))
+            return encode2_run<LOG_D, false, enc2_rpw<LOG_D>()>(P, T, X, n, out, enc2_max_warps<LOG_D>(), st);
+    }
+    return launch_encode_regs(P, T, X, n, out, sm_count(), st);
 }
 
 template <int LOG_D, int VPW>

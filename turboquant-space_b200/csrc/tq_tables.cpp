@@ -147,4 +147,15 @@ bool build_quant_lut(const std::vector<float> &boundaries, int buckets, int max_
     return true;
 }
 
+int coarse_shift(const QuantLut &lut, int nb) {
+    for (int s = 8; s > 0; --s) {
+        const int step = 1 << s;
+        bool one = lut.buckets % step == 0;
+        for (int j = 0; one && j < lut.buckets; j += step)
+            one = (j + step < lut.buckets ? lut.lo[j + step] : nb) - lut.lo[j] <= 1;
+        if (one) return s;
+    }
+    return 0;
+}
+
 }  // namespace tq

@@ -25,5 +25,8 @@ struct QuantLut {
 };
 int quant_bucket(float z, float s, float c, int buckets);
 bool build_quant_lut(const std::vector<float> &boundaries, int buckets, int max_k, QuantLut &lut);
+// Largest shift (8 at most) for which 2^shift neighbouring buckets, from a
+// multiple of 2^shift on, hold one of the nb boundaries at most (0: none).
+int coarse_shift(const QuantLut &lut, int nb);
 
 }  // namespace tq
