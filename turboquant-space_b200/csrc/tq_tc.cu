@@ -74,22 +74,21 @@ constexpr uint32_t tc_idesc(uint32_t fmt) {
            ((uint32_t)(TC_BM >> 4) << 24);
 }
 
+// D (+)= A B of one K step, descriptors by their low words; issued by one lane
+// of a converged warp.
 template <bool TF32>
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc) {
+__device__ __forceinline__ void umma(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t acc) {
     if constexpr (TF32) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t"
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "mov.b64 da, {%1, %5};\n\t"
+            "mov.b64 db, {%2, %5};\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-            "l"(a), "l"(b), "r"(tc_idesc(2)), "r"(acc)
+            "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(b_lo), "r"(tc_idesc(2)), "r"(acc), "r"(kDescHi)
             : "memory");
     } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-            "l"(a), "l"(b), "r"(tc_idesc(1)), "r"(acc)
-            : "memory");
+        umma_f16(d_tmem, a_lo, b_lo, tc_idesc(1), acc);
     }
 }
 
@@ -142,7 +141,7 @@ __global__ void __launch_bounds__(tc_threads(SPLIT, DEC), 1) tcp_kernel(const __
     // DEC: cfull[2], cempty[2] (code tile buffers) follow; then the TMEM slot
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 9 + (DEC ? 4 : 0));
     const uint32_t cfull0 = smem_u32(bars + 2 * STAGES + 9), cempty0 = cfull0 + 16;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
     const uint32_t xfull0 = smem_u32(bars + 2 * STAGES), xempty0 = smem_u32(bars + 2 * STAGES + 2);
     const uint32_t drain = smem_u32(bars + 2 * STAGES + 4);
@@ -247,54 +246,64 @@ __global__ void __launch_bounds__(tc_threads(SPLIT, DEC), 1) tcp_kernel(const __
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            uint32_t it = 0, gc = 0;
-            bool ok = true;
-            for (int t = 0; t < ntiles && ok; ++t) {
-                for (int sg = 0; sg < sh.nseg && ok; ++sg) {
-                    const bool alo = !sh.a_exact[sg];
-                    const int chl = sh.whole[sg] ? sh.KB[sg] : CH;
-                    const int kbc = DEC ? dec.kbc : sh.KB[sg];
-                    for (int c0 = 0, c1 = 0; c0 < sh.KB[sg] && ok; c0 = c1, ++gc) {
-                        c1 = chunk_end(c0, chl, sh.KB[sg], kbc);
-                        const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
-                        if (!mbar_wait(xempty0 + 8 * b, xph ^ 1u, err, kErrTmemEmpty)) { ok = false; break; }
+        // The whole warp runs the loop and one elected lane issues, so that the
+        // descriptors are warp-uniform values: under a one-lane branch they are
+        // not, and an MMA took 120 to 250 clocks to issue.  Full QJL form on TF32,
+        // 2048 x 20k of 1536-d: 4018 -> 3528 us; 1024-row top-k pass over 1M of
+        // 384-d (tcw_kernel's, same change): 5.78 -> 4.53 ms, codes 8.67 -> 6.87.
+        const bool lead = elect_one();
+        constexpr uint32_t KSTEP = 32 >> 4;  // one MMA's K: 32 bytes
+        uint32_t it = 0, gc = 0;
+        bool ok = true;
+        for (int t = 0; t < ntiles && ok; ++t) {
+            for (int sg = 0; sg < sh.nseg && ok; ++sg) {
+                const bool alo = !sh.a_exact[sg];
+                const int chl = sh.whole[sg] ? sh.KB[sg] : CH;
+                const int kbc = DEC ? dec.kbc : sh.KB[sg];
+                for (int c0 = 0, c1 = 0; c0 < sh.KB[sg] && ok; c0 = c1, ++gc) {
+                    c1 = chunk_end(c0, chl, sh.KB[sg], kbc);
+                    const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
+                    if (!mbar_wait_warp(xempty0 + 8 * b, xph ^ 1u, err, kErrTmemEmpty)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t d_tmem = tmem_base + b * TC_BN;
+                    uint32_t acc = 0u;
+                    for (int kb = c0; kb < c1; ++kb, ++it) {
+                        const uint32_t s = it % STAGES, ph = (it / STAGES) & 1u;
+                        if (!mbar_wait_warp(full0 + 8 * s, ph, err, kErrFull)) { ok = false; break; }
                         tc_fence_after();
-                        const uint32_t d_tmem = tmem_base + b * TC_BN;
-                        uint32_t acc = 0u;
-                        for (int kb = c0; kb < c1; ++kb, ++it) {
-                            const uint32_t s = it % STAGES, ph = (it / STAGES) & 1u;
-                            if (!mbar_wait(full0 + 8 * s, ph, err, kErrFull)) { ok = false; break; }
-                            tc_fence_after();
-                            const bool blo = kb < sh.kbx[sg];
-                            const uint32_t base = smem_u32(smem + s * TC_STAGE_BYTES);
-                            const uint32_t ah = base, al = base + TC_A_BYTES;
-                            const uint32_t bh = base + 2 * TC_A_BYTES, bl = bh + TC_B_BYTES;
+                        const bool blo = kb < sh.kbx[sg];
+                        const uint32_t ah = sw128_desc_lo(smem_u32(smem + s * TC_STAGE_BYTES));
+                        const uint32_t al = ah + (TC_A_BYTES >> 4);
+                        const uint32_t bh = al + (TC_A_BYTES >> 4), bl = bh + (TC_B_BYTES >> 4);
+                        if (lead) {
 #pragma unroll
-                            for (int kk = 0; kk < 4; ++kk) {
-                                const uint32_t koff = kk * 32;  // one MMA's K: 32 bytes
+                            for (uint32_t kk = 0; kk < 4 * KSTEP; kk += KSTEP) {
                                 // the small products first, while the sum is smaller
                                 if (blo) {
-                                    umma<TF32>(d_tmem, sw128_desc(ah + koff), sw128_desc(bl + koff), acc);
+                                    umma<TF32>(d_tmem, ah + kk, bl + kk, acc);
                                     acc = 1u;
                                 }
                                 if (alo) {
-                                    umma<TF32>(d_tmem, sw128_desc(al + koff), sw128_desc(bh + koff), acc);
+                                    umma<TF32>(d_tmem, al + kk, bh + kk, acc);
                                     acc = 1u;
                                 }
-                                umma<TF32>(d_tmem, sw128_desc(ah + koff), sw128_desc(bh + koff), acc);
+                                umma<TF32>(d_tmem, ah + kk, bh + kk, acc);
                                 acc = 1u;
                             }
                             umma_commit(empty0 + 8 * s);  // stage free once these MMAs are done
                         }
-                        if (ok) umma_commit(xfull0 + 8 * b);  // chunk sum ready
+                        acc = 1u;
                     }
+                    if (ok && lead) umma_commit(xfull0 + 8 * b);  // chunk sum ready
                 }
             }
-            // every MMA issued must be complete before the tensor memory is freed
+        }
+        // every MMA issued must be complete before the tensor memory is freed
+        if (lead) {
             umma_commit(drain);
             mbar_drain(drain, 0);
         }
+        __syncwarp();
     } else if (!SPLIT || warp < 6) {
         // ---------------- promotion (warps 2..5, 128 threads) ----------------
         // (without SPLIT these warps also run the tile epilogue)
@@ -569,15 +578,6 @@ constexpr int TW_THREADS = 32 * (2 + TW_EPI_WARPS);
 constexpr uint32_t kIdescW = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TW_BN >> 3) << 17) |
                              ((uint32_t)(TC_BM >> 4) << 24);
 
-__device__ __forceinline__ void umma_w(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(kIdescW), "r"(acc)
-        : "memory");
-}
-
 template <int STAGES, int CH, class W>
 __global__ void __launch_bounds__(TW_THREADS, 1) tcw_kernel(const __grid_constant__ TcMaps maps,
                                                             const TcShape sh,
@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tcw_kernel(const __grid_constan
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * TW_STAGE_BYTES);
     // bars: full[STAGES], empty[STAGES], xfull[2], xempty[2], drain; then the TMEM slot
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 5);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
     const uint32_t xfull0 = smem_u32(bars + 2 * STAGES), xempty0 = smem_u32(bars + 2 * STAGES + 2);
     const uint32_t drain = smem_u32(bars + 2 * STAGES + 4);
@@ -646,45 +646,50 @@ __global__ void __launch_bounds__(TW_THREADS, 1) tcw_kernel(const __grid_constan
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            uint32_t it = 0, gc = 0;
-            bool ok = true;
-            for (int t = 0; t < ntiles && ok; ++t) {
-                for (int c0 = 0; c0 < KB && ok; c0 += CH, ++gc) {
-                    const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
-                    if (!mbar_wait(xempty0 + 8 * b, xph ^ 1u, err, kErrTmemEmpty)) { ok = false; break; }
+        // ---------------- MMA issuer (as tcp_kernel's) ----------------
+        const bool lead = elect_one();
+        constexpr uint32_t KSTEP = 32 >> 4;
+        uint32_t it = 0, gc = 0;
+        bool ok = true;
+        for (int t = 0; t < ntiles && ok; ++t) {
+            for (int c0 = 0; c0 < KB && ok; c0 += CH, ++gc) {
+                const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
+                if (!mbar_wait_warp(xempty0 + 8 * b, xph ^ 1u, err, kErrTmemEmpty)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + b * TW_BN;
+                const int c1 = c0 + CH < KB ? c0 + CH : KB;
+                uint32_t acc = 0u;
+                for (int kb = c0; kb < c1; ++kb, ++it) {
+                    const uint32_t s = it % STAGES, ph = (it / STAGES) & 1u;
+                    if (!mbar_wait_warp(full0 + 8 * s, ph, err, kErrFull)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + b * TW_BN;
-                    const int c1 = c0 + CH < KB ? c0 + CH : KB;
-                    uint32_t acc = 0u;
-                    for (int kb = c0; kb < c1; ++kb, ++it) {
-                        const uint32_t s = it % STAGES, ph = (it / STAGES) & 1u;
-                        if (!mbar_wait(full0 + 8 * s, ph, err, kErrFull)) { ok = false; break; }
-                        tc_fence_after();
-                        const bool blo = kb < kbx;
-                        const uint32_t base = smem_u32(smem + s * TW_STAGE_BYTES);
-                        const uint32_t ah = base, al = base + TC_A_BYTES;
-                        const uint32_t bh = base + 2 * TC_A_BYTES, bl = bh + TW_B_BYTES;
+                    const bool blo = kb < kbx;
+                    const uint32_t ah = sw128_desc_lo(smem_u32(smem + s * TW_STAGE_BYTES));
+                    const uint32_t al = ah + (TC_A_BYTES >> 4);
+                    const uint32_t bh = al + (TC_A_BYTES >> 4), bl = bh + (TW_B_BYTES >> 4);
+                    if (lead) {
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            const uint32_t koff = kk * 32;
+                        for (uint32_t kk = 0; kk < 4 * KSTEP; kk += KSTEP) {
                             if (blo) {
-                                umma_w(d_tmem, sw128_desc(ah + koff), sw128_desc(bl + koff), acc);
+                                umma_f16(d_tmem, ah + kk, bl + kk, kIdescW, acc);
                                 acc = 1u;
                             }
-                            umma_w(d_tmem, sw128_desc(al + koff), sw128_desc(bh + koff), acc);
-                            umma_w(d_tmem, sw128_desc(ah + koff), sw128_desc(bh + koff), 1u);
+                            umma_f16(d_tmem, al + kk, bh + kk, kIdescW, acc);
+                            umma_f16(d_tmem, ah + kk, bh + kk, kIdescW, 1u);
                             acc = 1u;
                         }
                         umma_commit(empty0 + 8 * s);
                     }
-                    if (ok) umma_commit(xfull0 + 8 * b);
+                    acc = 1u;
                 }
+                if (ok && lead) umma_commit(xfull0 + 8 * b);
             }
+        }
+        if (lead) {
             umma_commit(drain);
             mbar_drain(drain, 0);
         }
+        __syncwarp();
     } else {
         // ---------------- epilogue (warps 2..9, 256 threads) ----------------
         const int q = warp & 3, h = (warp - 2) >> 2;  // lane quadrant, column half

@@ -24,19 +24,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 }
 
 // Shared-memory matrix descriptor of a K-major, 128-byte-swizzled tile whose
-// rows are 128 bytes and whose 8-row groups are 1024 bytes apart.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFFu);  // start address
-    d |= (uint64_t)1u << 16;                  // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024u >> 4) << 32;        // stride byte offset: 8 rows x 128 B
-    d |= (uint64_t)1u << 46;                  // descriptor version (sm_100)
-    d |= (uint64_t)2u << 61;                  // layout: SWIZZLE_128B
-    return d;
-}
-
-// The same descriptor's low word (the high word is the constant kDescHi);
-// adding bytes / 16 moves the start address.
+// rows are 128 bytes and whose 8-row groups are 1024 bytes apart: bits 0-13 the
+// start address / 16, 16-29 the leading byte offset (unused here), 32-45 the
+// stride byte offset / 16, 46 the descriptor version, 61-63 the swizzle (2 = 128
+// bytes).  The high word is constant; adding bytes / 16 to the low word moves
+// the start address.
 constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t addr) {
     return ((addr >> 4) & 0x3FFFu) | (1u << 16);
