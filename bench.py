@@ -327,7 +327,8 @@ def bf16_peaks():
 
 
 def mton_result(args, sym, steps=10, cpu=True):
-    """Dense M x N contractions, FP32 CUDA cores vs split-BF16 tcgen05.
+    """Dense M x N contractions, FP32 accuracy (hi/lo FP16 pairs) vs split-BF16,
+    both on tcgen05 tensor cores.
 
     mton: 1,000,000 codes of normalised N(0,1) 768-d rows (4-bit), 4096
           normalised queries -> 4096 x 1,000,000 asymmetric distances.
@@ -428,7 +429,7 @@ def mton_result(args, sym, steps=10, cpu=True):
              "Gdist_s": round(m * n / (ms * 1e-3) / 1e9, 3),
              "max_rel_err_vs_fp64": err, "max_plain_rel_err_vs_fp64": plain, "reps": reps}
         if name != "fp32":
-            # issued tensor work: exact-sign asymmetric planes (or decoded tiles)
+            # issued tensor work: exact-sign asymmetric tiles
             # take 3 products over the D centroid columns and 2 over the D sign
             # columns; symmetric 3 over D
             issued = float(m) * n * 2 * (5 * D if not sym else 3 * D)
@@ -486,8 +487,8 @@ def run_symq(args):
     """QJL-corrected symmetric distances (light, full, full-prepared): 2048 row
     codes x 200,000 column codes of a 1024-centre Gaussian mixture at 1536-d
     (padded 2048), 4-bit, device-resident.  Each variant is timed on the GPU
-    (CUDA events) in both precisions (FP32 CUDA cores, split-TF32 tensor
-    cores) and checked against the FP64 evaluation of its formula on 2,000
+    (CUDA events) in both precisions (FP32: CUDA cores, light on tensor cores;
+    split-TF32: tensor cores) and checked against the FP64 evaluation of its formula on 2,000
     sampled pairs; the reference's own CPU code (oracle/_ref) is timed on a
     bounded sample (128 x 512 pairs) on the host cores."""
     import torch

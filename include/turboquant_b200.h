@@ -48,21 +48,22 @@ typedef enum tq_status {
 
 /* Arithmetic used by the M x N contractions. */
 typedef enum tq_precision {
-    TQ_PRECISION_FP32 = 0,       /* FP32 CUDA-core kernels: the drop-in */
-    TQ_PRECISION_SPLIT_BF16 = 1, /* tcgen05 tensor cores on hi+lo BF16 pairs, FP32 TMEM accumulators */
+    TQ_PRECISION_FP32 = 0,       /* the drop-in, FP32 accuracy: tcgen05 tensor cores on hi+lo FP16
+                                    pairs (22 bits) with the code tiles decoded in shared memory,
+                                    summed in FP32 every one or two K blocks; CUDA cores for
+                                    small calls, padded dims below 16 and the full QJL forms */
+    TQ_PRECISION_SPLIT_BF16 = 1, /* the same kernel on hi+lo BF16 pairs, summed every 4 or 8 K blocks */
     TQ_PRECISION_SPLIT_TF32 = 2, /* tcgen05 tensor cores on hi+lo TF32 pairs, FP32 TMEM accumulators
                                     (the QJL-corrected symmetric distances only) */
     TQ_PRECISION_REFERENCE = 3,  /* the reference's own FP32 arithmetic in its Release build's
                                     summation order, one pair per thread: bit-identical to
                                     distSearchScalarB4 / distSearchAVX (asymmetric M x N) and
                                     distBuildScalarB4 / distBuildAVX (symmetric M x N) */
-    TQ_PRECISION_SPLIT_BF16_DECODED = 4 /* as SPLIT_BF16, but the column tiles are decoded from
-                                    the codes in shared memory (128 x 128 tiles) instead of
-                                    being read from BF16 planes written to device memory
-                                    first: 16 bytes of per-code scalars instead of 3-6 KB of
-                                    planes per code.  Padded dims >= 64; a tile of 128 codes
-                                    must fit in shared memory beside the pipeline (nibble
-                                    codes up to padded dim 1024, byte codes up to 512);
+    TQ_PRECISION_SPLIT_BF16_DECODED = 4 /* the same arithmetic as SPLIT_BF16 (which decodes its
+                                    code tiles in shared memory, too), for callers that named
+                                    it; its limits are kept.  Padded dims >= 64; codes of
+                                    at most 756 bytes (nibble codes up to padded dim 1024,
+                                    byte codes up to 512);
                                     device codes 16-byte aligned.  Otherwise
                                     TQ_ERR_NOT_SUPPORTED.  Plain M x N entry points only. */
 } tq_precision;
@@ -225,9 +226,10 @@ tq_status tq_rotated_coords_batch_device(const tq_space *sp, const float *X, siz
  * bindings.cpp:221-266, 312-334): out[m, n] row-major.  Host pointers,
  * synchronous.  Each code is reconstructed and passed through the QJL
  * Hadamard once; the pair terms are two contractions on the GPU:
- * TQ_PRECISION_FP32 on CUDA cores (the drop-in), TQ_PRECISION_SPLIT_TF32 on
- * tcgen05 tensor cores (hi/lo TF32 operands, FP32 accumulators; padded dims
- * below 64 stay on CUDA cores).  TQ_PRECISION_SPLIT_BF16 is refused with
+ * TQ_PRECISION_FP32 (the drop-in) on CUDA cores, the light variant on tensor
+ * cores as in the M x N calls; TQ_PRECISION_SPLIT_TF32 on tcgen05 tensor cores
+ * (hi/lo TF32 operands, FP32 accumulators; padded dims below 64 stay on CUDA
+ * cores; light as with FP32).  TQ_PRECISION_SPLIT_BF16 is refused with
  * TQ_ERR_NOT_SUPPORTED: the operands are values of the small centroid table,
  * whose BF16-pair rounding errors add up instead of averaging out. */
 tq_status tq_distance_m_to_n_symmetric_qjl(const tq_space *sp, const uint8_t *codes_a, size_t m,
@@ -312,8 +314,9 @@ typedef enum tq_index_layout {
     TQ_INDEX_PLANES = 0, /* the codes plus their exact-sign hi/lo BF16 operand planes:
                             code_size + 6 * padded_dim + 8 bytes a code; the fastest pass */
     TQ_INDEX_CODES = 1   /* the codes plus four floats a code (code_size + 16 bytes): the pass
-                            decodes each tile of codes in shared memory (kernel variants 1..4),
-                            for corpora ~10x larger per GPU at a slower pass; padded dim >= 64 */
+                            decodes each tile of codes in shared memory (kernel variants 2 and
+                            4, or 6 by the tuner), for corpora ~10x larger per GPU; padded
+                            dim >= 64 */
 } tq_index_layout;
 
 /* Keep n codes (host or device memory) resident in HBM in the given layout. */
@@ -331,7 +334,8 @@ typedef struct tq_server_params {
                            free device memory) */
     int kernel_variant; /* -1: autotune the contraction's tile shape per batch-size bucket;
                            else fixed (tq_topk_variant_shape): 0..6 for a TQ_INDEX_PLANES
-                           index, 1..4 for TQ_INDEX_CODES */
+                           index, 1..4 for TQ_INDEX_CODES.  6 is the filter pass over
+                           the codes, which the tuner may pick for either layout */
     size_t queue_rows;  /* queued query rows beyond which submit returns TQ_ERR_BUSY
                            (0: no cap beyond the admission pool) */
     int candidates;     /* tensor-pass candidates per row that the exact stage rescores,

@@ -40,3 +40,24 @@ def test_tile_edges(cuda_ok, dim, bits, m, n):
                          o.distance_m_to_n_symmetric_qjl(rows, codes, "light"),
                          sym_term_scale(rows, codes, cs, cs - 12))
     assert ok, ("light", err.max())
+
+
+@pytest.mark.parametrize("dim,bits", [(16, 4), (20, 8), (64, 3), (128, 2), (384, 4), (768, 8), (1000, 9),
+                                      (1536, 4), (4096, 6)])
+@pytest.mark.parametrize("m,n", [(1, 1), (2, 130), (17, 128), (65, 257), (129, 300)])
+@pytest.mark.parametrize("variant", ["full", "full_prepared"])
+def test_full_form_tile_edges(cuda_ok, dim, bits, m, n, variant):
+    """The full QJL form as two passes (the correction's products, then the
+    distances with them clamped in)."""
+    rng = np.random.default_rng(dim * 5 + bits + 17 * m + n)
+    X = (rng.standard_normal((n, dim)) * rng.uniform(1e-2, 1e2, (n, 1))).astype(np.float32)
+    Q = (rng.standard_normal((m, dim)) * rng.uniform(1e-2, 1e2, (m, 1))).astype(np.float32)
+    X[n // 2], Q[m // 2] = (0.0, 0.0) if n > 1 else (X[0], Q[0])
+    Q[0] = X[0]  # a code against itself
+    s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    cs = s.code_size_bytes()
+    codes, rows = o.encode_batch(X), o.encode_batch(Q)
+    got = getattr(s, f"distance_m_to_n_symmetric_{variant}")(rows, codes)
+    err, ok = dist_close(got, o.distance_m_to_n_symmetric_qjl(rows, codes, variant),
+                         sym_term_scale(rows, codes, cs, cs - 12))
+    assert ok, (variant, err.max())

@@ -329,6 +329,7 @@ tq_status tq_space_create(size_t dim, int bits, uint64_t rot_seed, uint64_t qjl_
         // space_turbo_quant.h:265-266 and turbo_quant.h:69, in FP32 as written
         P.scale = std::sqrt(static_cast<float>(M_PI) / 2.0f) / std::sqrt(static_cast<float>(D));
         P.wht_scale = 1.0f / std::sqrt(static_cast<float>(D));
+        P.cent_scale = tq::cg_cent_scale(sp->centroids.data(), sp->levels);
         P.lutq = 0;
         P.qlut_k = 0;
         P.qflag = 0;
@@ -1036,7 +1037,7 @@ struct SymqRunner {
     float *A1 = nullptr, *A2 = nullptr;  // hi then lo, m_pad x K1p / K2p each
     int *err = nullptr;
     bool cg = false;
-    tq::CgRows cgr;
+    tq::CgRows cgr, corr;  // the light form's or the full form's MSE rows; the full form's correction
 
     SymqRunner(const tq_space *s, int md, bool split_tf32 = false)
         : sp(s), mode(md), tc(split_tf32 && s->D >= 64) {
@@ -1063,13 +1064,15 @@ struct SymqRunner {
                 "symmetric planes kernel");
         return TQ_OK;
     }
-    // Takes the light variant to the M x N kernel where the codes allow it
-    // (A, B: device pointers of the call).
+    // Takes a call to the M x N kernel where the codes allow it (A, B: device
+    // pointers of the call): the light variant, and the full ones at FP32.
     void choose(const void *A, const void *B) {
-        cg = light() && sp->D >= 16 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 3) == 0;
+        cg = sp->D >= 16 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 3) == 0 &&
+             (light() || !tc);
     }
     tq_status prepare_rows_cg(const uint8_t *A, size_t rows_, cudaStream_t s) {
         m = rows_;
+        if (!light()) return prepare_rows_full_cg(A, s);
         const size_t plane = m * tq::cg_row_k(sp->P, tq::kCgLight) * 2;  // a multiple of 128 bytes
         TQ_CUDA(rows.alloc(2 * plane + m * sizeof(float4) + sizeof(int), s), "cudaMallocAsync(row planes)");
         auto *base = static_cast<unsigned char *>(rows.p);
@@ -1081,6 +1084,29 @@ struct SymqRunner {
             TQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s), "memset");
         }
         TQ_CUDA(tq::launch_cg_rows_codes(sp->P, sp->T, A, m, tq::kCgLight, tq::kCgFP16, cgr, s), "row planes");
+        return TQ_OK;
+    }
+    // The full form: a symmetric pass for the MSE products after an asymmetric one
+    // for the correction, whose products wait in the output.  Against planes of
+    // both sides and an FP32 contraction over 4 D on CUDA cores, which also lost
+    // more bits: 1 x 1 of 384-d 4-bit 125 -> 42 us, 300 x 20k 962 -> 201 us,
+    // 2048 x 20k of 1536-d 15.3 -> 1.12 ms.
+    tq_status prepare_rows_full_cg(const uint8_t *A, cudaStream_t s) {
+        const size_t kc = m * tq::cg_row_k(sp->P, tq::kCgAsym) * 2, km = m * tq::cg_row_k(sp->P, tq::kCgSym) * 2;
+        const size_t vec = sizeof(float) * m * sp->D;  // D >= 16: every part a multiple of 16 bytes
+        TQ_CUDA(rows.alloc(2 * (kc + km) + 2 * m * sizeof(float4), s), "cudaMallocAsync(row planes)");
+        TQ_CUDA(rows_bf.alloc(2 * vec + 2 * sizeof(float) * m, s), "cudaMallocAsync(correction rows)");
+        auto *base = static_cast<unsigned char *>(rows.p);
+        corr.hi = base;
+        corr.lo = base + kc;
+        cgr.hi = base + 2 * kc;
+        cgr.lo = base + 2 * kc + km;
+        cgr.rs = reinterpret_cast<float4 *>(base + 2 * (kc + km));
+        corr.rs = cgr.rs + m;
+        float *q = static_cast<float *>(rows_bf.p), *sq = q + m * sp->D, *norms = sq + m * sp->D;
+        TQ_CUDA(tq::launch_symq_full_rows(sp->P, sp->T, A, m, q, sq, norms, s), "correction rows kernel");
+        TQ_CUDA(tq::launch_cg_rows_prepared(sp->P, q, sq, norms, m, tq::kCgFP16, corr, s), "row planes");
+        TQ_CUDA(tq::launch_cg_rows_codes(sp->P, sp->T, A, m, tq::kCgSym, tq::kCgFP16, cgr, s), "row planes");
         return TQ_OK;
     }
     // The space's status word carries this call's errors (host entry points read it).
@@ -1112,6 +1138,15 @@ struct SymqRunner {
     }
     // out[:, 0:n] (leading dimension ldo) for n column codes
     tq_status run_cols(const uint8_t *B, size_t n, float *out, size_t ldo, cudaStream_t s) {
+        if (cg && !light()) {
+            TQ_CUDA(tq::launch_cgemm(sp->P, sp->T, tq::kCgAsym, tq::kCgFP16, corr, m, B, n, out, ldo,
+                                     sp->T.status, s, tq::kCgProducts),
+                    "tcgen05 correction kernel");
+            TQ_CUDA(tq::launch_cgemm(sp->P, sp->T, tq::kCgSym, tq::kCgFP16, cgr, m, B, n, out, ldo,
+                                     sp->T.status, s, tq::kCgClampedSum),
+                    "tcgen05 full symmetric kernel");
+            return TQ_OK;
+        }
         if (cg) {
             TQ_CUDA(tq::launch_cgemm(sp->P, sp->T, tq::kCgLight, tq::kCgFP16, cgr, m, B, n, out, ldo,
                                      err ? err : sp->T.status, s),
@@ -1172,7 +1207,8 @@ struct SymqRunner {
     }
 };
 
-// The QJL-corrected symmetric contractions run in FP32 (CUDA cores) or
+// The QJL-corrected symmetric contractions run at FP32 accuracy (the M x N
+// kernel, or CUDA cores) or
 // split-TF32 (tensor cores).  A BF16 pair is refused: its planes' rounding
 // errors do not average out (see tc_symq_kernel) and exceed 1e-5.
 tq_status symq_precision_ok(tq_precision p) {

@@ -54,6 +54,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "tq_cgemm.h"
@@ -76,7 +77,11 @@ constexpr int kErrFull = 1, kErrEmpty = 2, kErrTmemFull = 3, kErrTmemEmpty = 4;
 
 // FP16 scalings: |q_rot|, |s_q| <= 1 and |c| < 5 (Lloyd-Max of N(0,1), at most
 // 9 bits), so hi stays below 65504 and lo of any value that matters is normal.
-constexpr float kRowScale = 16384.0f, kCentScale = 2048.0f;
+// The centroids' scale is P.cent_scale: few distinct values, whose rounding
+// errors do not average out over a row (40 x 20k symmetric distances of clustered
+// 384-d rows, error against FP64 with the FP32 chain / scale 2048 / chosen scale:
+// 3-bit 8.5 / 4.5 / 3.6e-8, 8-bit 3.5 / 3.7 / 3.4e-8).
+constexpr float kRowScale = 16384.0f;
 
 __device__ __forceinline__ void split16(float v, int fmt, uint32_t &h, uint32_t &l) {
     if (fmt == kCgFP16) {
@@ -95,7 +100,7 @@ struct CgArgs {
     size_t n;
     int cs, pb, nibble, levels;
     const float *centroids;
-    int fmt, form;
+    int fmt, form, post;
     int KBm, KB;         // K blocks of the centroid part, of all
     int chm, chs;        // K blocks per accumulation chunk: centroid part, sign part
     int NT, stages, ring;  // row columns per tile, pipeline stages, code-word ring slots
@@ -103,6 +108,7 @@ struct CgArgs {
     size_t m;
     const float4 *rs;    // per row: r1, r2, s1, s2
     float scale;         // sqrt(pi / 2D)
+    float cent;          // the centroids' FP16 scale
     float undo_c, undo_s;  // undo the operand scalings of the two parts
     float *out;
     size_t ldo;
@@ -191,7 +197,7 @@ __device__ __forceinline__ void chunk_pieces(uint32_t X, int cols, F f) {
 // DW: decoder warps (warps 4 .. 4 + DW - 1); the other 12 - DW warps are the
 // epilogue: two column halves of 128 (DW = 4), or one of 64 (DW = 8).  Batches
 // of few rows are bound by the decoders, wide ones by the MMAs.
-template <int DW, bool NIB, bool LIGHT, bool PAIR>
+template <int DW, bool NIB, bool LIGHT, bool PAIR, bool FULL>
 __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_constant__ CUtensorMap map_h,
                                                               const __grid_constant__ CUtensorMap map_l,
                                                               const CgArgs p) {
@@ -242,7 +248,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             const int v = i >> 5;
             uint32_t h, l;
             const float c = v < p.levels ? p.centroids[v] : 0.0f;
-            split16(p.fmt == kCgFP16 ? c * kCentScale : c, p.fmt, h, l);
+            split16(p.fmt == kCgFP16 ? c * p.cent : c, p.fmt, h, l);
             btab[i] = h | (l << 16);
         }
     }
@@ -413,7 +419,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             for (int v = 0; v < 8; ++v) {
                 uint32_t h, l;
                 const float cv = v < p.levels ? p.centroids[v] : 0.0f;
-                split16(p.fmt == kCgFP16 ? cv * kCentScale : cv, p.fmt, h, l);
+                split16(p.fmt == kCgFP16 ? cv * p.cent : cv, p.fmt, h, l);
                 const int sh = 8 * (v & 3);
                 tab.hl[v >> 2] |= (h & 0xFFu) << sh;
                 tab.hh[v >> 2] |= (h >> 8) << sh;
@@ -556,15 +562,40 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             float *o = p.out + col0 * p.ldo + row;
             const float4 *rs = p.rs + col0;
             const int live = (int)min((size_t)cpt, col0 < p.m ? p.m - col0 : 0);
+            if constexpr (FULL) {
+                // products, or distances with another pass's products clamped in (all
+                // loads of 16 columns in flight at once)
+                const bool add = p.post == kCgClampedSum;
 #pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                if (k % 16 == 0 && k >= live) break;
-                if (k < live) {
-                    const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + k));
-                    const float ipt = __fmul_rn(__fmul_rn(y[k], r.x), c1);
-                    __stcs(o, fmaxf(__fmaf_rn(-2.0f, ipt, __fadd_rn(r.y, c2)), 0.0f));
+                for (int k0 = 0; k0 < CPT; k0 += 16) {
+                    if (k0 >= live) break;
+                    float other[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) other[k] = add && k0 + k < live ? __ldcs(o + k * p.ldo) : 0.0f;
+#pragma unroll
+                    for (int k = k0; k < k0 + 16; ++k) {
+                        if (k < live) {
+                            const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + k));
+                            float ipt = __fmul_rn(__fmul_rn(y[k], r.x), c1);
+                            const float lim = fabsf(ipt);
+                            if (add) ipt = __fadd_rn(ipt, fmaxf(-lim, fminf(lim, other[k - k0])));
+                            const float d = fmaxf(__fmaf_rn(-2.0f, ipt, __fadd_rn(r.y, c2)), 0.0f);
+                            __stcs(o, add ? d : ipt);
+                        }
+                        o += p.ldo;
+                    }
                 }
-                o += p.ldo;
+            } else {
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) {
+                    if (k % 16 == 0 && k >= live) break;
+                    if (k < live) {
+                        const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + k));
+                        const float ipt = __fmul_rn(__fmul_rn(y[k], r.x), c1);
+                        __stcs(o, fmaxf(__fmaf_rn(-2.0f, ipt, __fadd_rn(r.y, c2)), 0.0f));
+                    }
+                    o += p.ldo;
+                }
             }
         }
     }
@@ -620,7 +651,7 @@ __global__ void __launch_bounds__(256) cg_rows_codes_kernel(const uint8_t *__res
                                                             float4 *__restrict__ rs) {
     const int half = KBm * CG_BK, K = form == kCgLight ? 2 * half : half, quads = K / 4;
     const size_t total = m * (size_t)quads;
-    const float f = fmt == kCgFP16 ? kCentScale : 1.0f;
+    const float f = fmt == kCgFP16 ? P.cent_scale : 1.0f;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (size_t)gridDim.x * blockDim.x) {
         const size_t r = t / quads;
@@ -656,6 +687,37 @@ unsigned rows_grid(size_t work) {
 
 }  // namespace
 
+float cg_cent_scale(const float *centroids, int levels) {
+    float best = 2048.0f;
+    double best_err = 1e300;
+    for (int i = 0; i < 256; ++i) {
+        const float a = 2048.0f - 4.0f * (float)i;
+        double sw = 0.0, d1 = 0.0, d2 = 0.0, l2 = 0.0;
+        for (int v = levels / 2; v < levels; ++v) {  // the others are their negatives
+            const double c = centroids[v], w = c * c * std::exp(-c * c / 3.0);  // c^2 times about its share
+            const float x = centroids[v] * a;
+            const float h = __half2float(__float2half_rn(x)), l = __half2float(__float2half_rn(x - h));
+            const double d = ((double)h + l) / (c * a) - 1.0, r = l / (c * a);
+            sw += w;
+            d1 += w * d;
+            d2 += w * d * d;
+            l2 += w * r * r;
+        }
+        // a product of two values is off by d + d' - r r', and the undoing factor by
+        // its rounding.  Over near rows, whose values agree, that is a bias; over
+        // others it averages out.
+        const double u2 = (double)(1.0f / (a * a)) * a * a - 1.0;
+        const double u1 = (double)(1.0f / (a * kRowScale)) * a * kRowScale - 1.0;
+        const double b2 = (2.0 * d1 - l2) / sw + u2, b1 = d1 / sw + u1;
+        const double err = b2 * b2 + b1 * b1 + (2.0 * d2 + l2 * l2 / sw) / sw / 64.0;
+        if (err < best_err) {
+            best = a;
+            best_err = err;
+        }
+    }
+    return best;
+}
+
 size_t cg_row_k(const Params &P, int form) {
     const size_t half = ((size_t)P.D + CG_BK - 1) / CG_BK * CG_BK;
     return form == kCgSym ? half : 2 * half;
@@ -682,7 +744,7 @@ cudaError_t launch_cg_rows_codes(const Params &P, const DevTables &T, const uint
 
 cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt, const CgRows &rows,
                          size_t m, const uint8_t *codes, size_t n, float *out, size_t ldo, int *err,
-                         cudaStream_t st) {
+                         cudaStream_t st, int post) {
     if (m == 0 || n == 0) return cudaSuccess;
     if (P.cs % 4 || (reinterpret_cast<uintptr_t>(codes) & 3)) return cudaErrorMisalignedAddress;
     if (!aligned16({rows.hi, rows.lo, rows.rs})) return cudaErrorMisalignedAddress;
@@ -696,6 +758,7 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.centroids = T.centroids;
     a.fmt = fmt;
     a.form = form;
+    a.post = post;
     a.KBm = (P.D + CG_BK - 1) / CG_BK;
     a.KB = form == kCgSym ? a.KBm : 2 * a.KBm;
     // Chunk lengths (K blocks).  FP16: 2 (1 where the whole part is 4 blocks or
@@ -707,9 +770,10 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.m = m;
     a.rs = rows.rs;
     a.scale = P.scale;
+    a.cent = P.cent_scale;
     a.undo_s = fmt == kCgFP16 && form == kCgAsym ? 1.0f / kRowScale : 1.0f;
     a.undo_c = fmt == kCgFP16
-                   ? 1.0f / (kCentScale * (form == kCgAsym ? kRowScale : kCentScale))
+                   ? 1.0f / (P.cent_scale * (form == kCgAsym ? kRowScale : P.cent_scale))
                    : 1.0f;
     a.out = out;
     a.ldo = ldo;
@@ -748,7 +812,9 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     const bool light = form == kCgLight;
     auto pick = [&](auto wide, auto nib) {
         constexpr bool W = decltype(wide)::value, N = decltype(nib)::value;
-        return light ? cgemm_kernel<W ? 4 : 8, N, true, W> : cgemm_kernel<W ? 4 : 8, N, false, W>;
+        return post != kCgDist ? cgemm_kernel<W ? 4 : 8, N, false, W, true>
+               : light         ? cgemm_kernel<W ? 4 : 8, N, true, W, false>
+                               : cgemm_kernel<W ? 4 : 8, N, false, W, false>;
     };
     using T_ = std::true_type;
     using F_ = std::false_type;

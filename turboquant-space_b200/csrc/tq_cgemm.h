@@ -6,6 +6,10 @@
 namespace tq {
 
 enum CgForm { kCgAsym = 0, kCgSym = 1, kCgLight = 2 };  // queries / codes / codes + light QJL term
+// What the epilogue does with the products ip |a| |b|: distances; the products
+// themselves; or distances with out's own values, such products of another pass,
+// added to ip after clamping them to +-|ip| (the full QJL form's correction).
+enum CgPost { kCgDist = 0, kCgProducts = 1, kCgClampedSum = 2 };
 enum CgFmt { kCgFP16 = 0, kCgBF16 = 1 };                // 16-bit type of the hi / lo pairs
 
 // The row operand: hi and lo planes of m x cg_row_k 16-bit values and four
@@ -15,6 +19,10 @@ struct CgRows {
     float4 *rs = nullptr;
 };
 size_t cg_row_k(const Params &P, int form);
+
+// P.cent_scale: the scale in (1024, 2048] at which products of the centroids' FP16
+// pairs (without lo lo) have the least bias and error.
+float cg_cent_scale(const float *centroids, int levels);
 
 // Prepared queries (kCgAsym) or codes (kCgSym, kCgLight) -> row operand.
 cudaError_t launch_cg_rows_prepared(const Params &P, const float *q_rot, const float *s_q,
@@ -28,6 +36,6 @@ cudaError_t launch_cg_rows_codes(const Params &P, const DevTables &T, const uint
 // set non-zero if a bounded wait in the kernel gave up.
 cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt, const CgRows &rows,
                          size_t m, const uint8_t *codes, size_t n, float *out, size_t ldo, int *err,
-                         cudaStream_t st);
+                         cudaStream_t st, int post = kCgDist);
 
 }  // namespace tq

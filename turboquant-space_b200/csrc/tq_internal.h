@@ -44,6 +44,7 @@ struct Params {
     float qlut_c;
     float scale;       // sqrt(pi/2)/sqrt(D)            space_turbo_quant.h:265
     float wht_scale;   // 1/sqrt(D)                     turbo_quant.h:69
+    float cent_scale;  // scale of the FP16 hi/lo centroids (cg_cent_scale)
 };
 
 // Device copies of the space's tables (one allocation per space).
@@ -89,6 +90,11 @@ int symq_k2(int mode, int D);   // columns of the correction plane
 cudaError_t launch_symq_planes(const Params &P, const DevTables &T, const uint8_t *codes,
                                size_t rows, int mode, bool row_side, float *P1, int ldk1,
                                float *P2, int ldk2, float *scal, cudaStream_t st);
+// The row codes of the full symmetric form as prepared queries whose asymmetric
+// products (q_rot, s_q: rows x D, norms: rows x 2) are the form's correction.
+// Codes 4-byte aligned.
+cudaError_t launch_symq_full_rows(const Params &P, const DevTables &T, const uint8_t *codes, size_t rows,
+                                  float *q_rot, float *s_q, float *norms, cudaStream_t st);
 // The same planes as hi/lo TF32 pairs in FP32 containers (hi = tf32(v),
 // lo = tf32(v - hi)): H1/L1 rows_pad x K1, H2/L2 rows_pad x K2, zero past the
 // planes' columns and past `rows`; L2 may be null for the light variant

@@ -11,6 +11,8 @@
 //              TQ_INDEX_CODES: four floats a code (c1, c2 and the chunk
 //                factors fc, fs of launch_dec_factors); the tensor pass decodes
 //                each B tile in shared memory from the codes.
+//              Either layout also serves the filter pass (variant 6,
+//              tq_filter.cu), which reads the codes and 4 bytes of factors each.
 //   slot       buffers for one batch of up to `max_rows` query rows and one CUDA
 //              graph per row bucket (128, 256, 512, ... max_rows) capturing
 //              rows gathered from the pool -> prepareQuery -> query planes ->
@@ -31,7 +33,8 @@
 //              do not fit in the pool's free space, which holds the rows of the
 //              queued and the in-flight requests.  A batch gathers its rows
 //              from the pool on the device.
-//   autotune   per bucket, each kernel variant (tile shape x stage depth) is
+//   autotune   per bucket, each kernel variant (tile shape x stage depth, or the
+//              filter pass) is
 //              timed on the index and the fastest is captured into the graph.
 //   exact      the tensor-core pass keeps `kc` candidates per row; the
 //              rescoring kernel recomputes them with the reference's own

@@ -15,6 +15,12 @@
 //                          fused: corr = clamp(corr, +-|ip_mse|),
 //                          ip = (ip_mse + corr) |a| |b|, d = max(0, ...).
 //
+//   symq_full_rows_kernel  the full variants' correction as the products of an
+//                          asymmetric query, for the M x N kernel (tq_cgemm.cu),
+//                          which runs the light and full variants wherever codes
+//                          are 4-byte aligned and D >= 16; the kernels above
+//                          serve the rest, split-TF32 and one prepared row.
+//
 // The reference evaluates the full variants pair by pair (two
 // reconstructions and two Hadamards per pair); here every code is
 // reconstructed and rotated once, and the four inner products of a pair
@@ -29,6 +35,7 @@
 #include "tq_internal.h"
 #include "tq_rht.cuh"
 
+#include <algorithm>
 #include <cstdint>
 
 namespace tq {
@@ -75,6 +82,79 @@ __global__ void __launch_bounds__(256) rotated_coords_kernel(const float *__rest
 __device__ __forceinline__ float round_tf32(float x) {
     const uint32_t b = __float_as_uint(x);
     return __uint_as_float((b + 0xFFFu + ((b >> 13) & 1u)) & ~0x1FFFu);
+}
+
+// ---------------------------------------------------------------------------
+// The full form's correction as the product of an asymmetric query.  With
+// recon = W S (c sigma) (S: the QJL signs, W: the scaled Hadamard matrix, which
+// is symmetric), <sgn_a, recon_b> = <S W sgn_a, c_b> sigma_b, so
+//   corr = sigma_b <r1, c_b> + s g_b <r2, sgn_b>,
+//   r1 = s g_a S W sgn_a,  r2 = recon_a + (p / s) g_a sgn_a,
+// which the M x N kernel takes from the codes b as they are: no planes of b.
+// Writes r1 and r2 times 2^-x (largest magnitude in [1/2, 1)) as prepared
+// queries with norms = [|a|^2, |a| 2^x].  W sgn is a sum of +-1, exact before its
+// scaling.  One warp per code.
+// ---------------------------------------------------------------------------
+template <int LOG_D>
+__global__ void __launch_bounds__(256) symq_full_rows_kernel(const uint8_t *__restrict__ codes, size_t rows,
+                                                             float *__restrict__ q_rot,
+                                                             float *__restrict__ s_q,
+                                                             float *__restrict__ norms, Params P,
+                                                             DevTables T) {
+    constexpr int D = 1 << LOG_D;
+    extern __shared__ __align__(16) unsigned char smem[];
+    load_tables(smem, P, T, true);
+    __syncthreads();
+    uint32_t *ones = reinterpret_cast<uint32_t *>(smem + kTabRotOff);  // the rotation's signs are not used
+    for (int i = threadIdx.x; i < (D + 31) / 32; i += blockDim.x) ones[i] = 0xffffffffu;
+    __syncthreads();
+    const float *s_cent = reinterpret_cast<const float *>(smem + kTabCentOff);
+    const uint32_t *s_qjl = reinterpret_cast<const uint32_t *>(smem + kTabQjlOff);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    float *buf = reinterpret_cast<float *>(smem + kTabBytes) + warp * (D + 8);
+    const float p2d = __fdiv_rn(kPi, __fmul_rn(2.0f, (float)D));
+    for (size_t r = (size_t)blockIdx.x * nw + warp; r < rows; r += (size_t)gridDim.x * nw) {
+        const uint8_t *c = codes + r * (size_t)P.cs;
+        const float *meta = reinterpret_cast<const float *>(c + P.pb);  // 4-byte aligned
+        const float norm = meta[0], gamma = meta[1], sigma = meta[2];
+        const float g1 = __fmul_rn(P.scale, gamma), g2 = __fmul_rn(__fdiv_rn(p2d, P.scale), gamma);
+        auto unit = [&](int i) -> unsigned {
+            return P.nibble ? ((i & 1) ? c[i >> 1] >> 4 : c[i >> 1] & 15u) : c[i];
+        };
+        float *o1 = q_rot + r * D, *o2 = s_q + r * D, top = 0.0f;
+        for (int i = lane; i < D; i += 32) buf[swz(i)] = (unit(i) & 1u) ? 1.0f : -1.0f;
+        __syncwarp();
+        fwht_from<LOG_D, 0, false>(buf, lane, 1.0f, ones, P.wht_scale);
+        for (int i = lane; i < D; i += 32) {
+            const float v = __fmul_rn(apply_sign(buf[swz(i)], s_qjl, i), g1);
+            o1[i] = v;
+            top = fmaxf(top, fabsf(v));
+        }
+        __syncwarp();
+        for (int i = lane; i < D; i += 32) buf[swz(i)] = __fmul_rn(s_cent[unit(i) >> 1], sigma);
+        __syncwarp();
+        fwht_from<LOG_D, 0, false>(buf, lane, 1.0f, s_qjl, P.wht_scale);
+        for (int i = lane; i < D; i += 32) {
+            const float v = __fadd_rn(buf[swz(i)], (unit(i) & 1u) ? g2 : -g2);
+            o2[i] = v;
+            top = fmaxf(top, fabsf(v));
+        }
+        __syncwarp();
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(kFull, top, off));
+        int x = 0;
+        if (top > 0.0f && top < 3e38f) frexpf(top, &x);
+        x = max(-100, min(100, x));
+        const float down = ldexpf(1.0f, -x);
+        for (int i = lane; i < D; i += 32) {  // each lane's own values
+            o1[i] *= down;
+            o2[i] *= down;
+        }
+        if (lane == 0) {
+            norms[2 * r] = __fmul_rn(norm, norm);
+            norms[2 * r + 1] = __fmul_rn(norm, ldexpf(1.0f, x));
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -504,7 +584,29 @@ struct PlanesRun {
     }
 };
 
+template <int LOG_D>
+struct FullRowsRun {
+    static cudaError_t run(const Params &P, const DevTables &T, const uint8_t *codes, size_t rows,
+                           float *q_rot, float *s_q, float *norms, cudaStream_t st) {
+        const int D = 1 << LOG_D, w = sq_warps(D);
+        const size_t smem = (size_t)kTabBytes + (size_t)w * 4 * (D + 8);
+        cudaError_t e = cudaFuncSetAttribute(symq_full_rows_kernel<LOG_D>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        const size_t blocks = std::min((rows + w - 1) / w, (size_t)sq_sm_count() * 8);
+        symq_full_rows_kernel<LOG_D><<<(unsigned)blocks, 32 * w, smem, st>>>(codes, rows, q_rot, s_q, norms,
+                                                                             P, T);
+        return cudaGetLastError();
+    }
+};
+
 }  // namespace
+
+cudaError_t launch_symq_full_rows(const Params &P, const DevTables &T, const uint8_t *codes, size_t rows,
+                                  float *q_rot, float *s_q, float *norms, cudaStream_t st) {
+    if (rows == 0) return cudaSuccess;
+    return dispatch_logd_sq<FullRowsRun>(P.log2D, P, T, codes, rows, q_rot, s_q, norms, st);
+}
 
 int symq_ldk(int K) { return (K + SQ_BK - 1) / SQ_BK * SQ_BK; }
 

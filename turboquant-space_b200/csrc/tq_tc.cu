@@ -1419,9 +1419,9 @@ int tc_topk_variants() { return (int)(sizeof(kTopkShapes) / sizeof(kTopkShapes[0
 // each K = 16 MMA is taken to add at most 2^-20 of (|accumulator| + sum |p|);
 // promotions, the planes' FP32 roundings and the reference's own sums add a
 // few 1e-7.  With n MMAs per accumulator (a chunk of ch K blocks: 12 per
-// block with a lo plane, 8 without; variant 6: every block of K) the sum is
+// block with a lo plane, 8 without; the whole-K threshold pass: every block of K) the sum is
 // 3 * 2^-16 + n * 2^-20 + 5e-7, taken with a factor 1.8 and at least 2.5e-4:
-// 2.5e-4 for the 8-block chunks (n = 96), 3.6e-4 for variant 6 at K = 1024,
+// 2.5e-4 for the 8-block chunks (n = 96), 3.6e-4 for the whole K at K = 1024,
 // K_lo = 512 (n = 160).
 float tc_topk_kappa(int variant, int K, int k_lo) {
     const int KB = K / TC_BK, kbx = k_lo / TC_BK;
@@ -1562,7 +1562,7 @@ cudaError_t launch_tc_thresh(const void *Ah, const void *Al, size_t rows_pad, co
     if (!aligned16({Bh, Bl})) return cudaErrorMisalignedAddress;
     if (!bf16_maps(mp, sh, Ah, Al, rows_pad, Bh, Bl, n_pad, K, k_lo)) return cudaErrorInvalidValue;
     if (n_pad % TW_BN == 0) {
-        // variant 6's shape: 128 x 256 tiles, the whole K in one accumulator
+        // 128 x 256 tiles, the whole K in one accumulator
         if (!make_map(&mp.m[0][2], Bh, K, n_pad, TW_BN) || !make_map(&mp.m[0][3], Bl, k_lo, n_pad, TW_BN))
             return cudaErrorInvalidValue;
         ThreshEpi::Params ew = ep;

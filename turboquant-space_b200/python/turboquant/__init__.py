@@ -420,11 +420,11 @@ class TurboQuantSpace:
     def distance_m_to_n(self, queries, codes, precision="fp32", out=None):
         """distanceBatchMToN: queries [m, dim] float32 x codes [n, cs] -> [m, n].
 
-        precision: "fp32" (CUDA cores, the drop-in), "split_bf16" (tcgen05
-        tensor cores on hi+lo BF16 operand planes), "split_bf16_decoded" (the
-        same arithmetic, column tiles decoded from the codes in shared memory:
-        less device memory, somewhat slower) or "reference" (the reference
-        build's own summation order, bit-identical distances)."""
+        precision: "fp32" (the drop-in: tcgen05 tensor cores on hi+lo FP16
+        pairs, FP32 accuracy; CUDA cores for small calls), "split_bf16" (the
+        same on hi+lo BF16 pairs), "split_bf16_decoded" (the same arithmetic
+        as "split_bf16", codes of at most 756 bytes) or "reference" (the
+        reference build's own summation order, bit-identical distances)."""
         cs = self.code_size_bytes()
         prec = _capi.PRECISION[precision]
         if _is_device(queries) or _is_device(codes):
@@ -518,8 +518,9 @@ class TurboQuantSpace:
                                                      prec))
         return out
 
-    # precision="fp32" is the drop-in (CUDA cores); "split_tf32" runs the two
-    # contractions on tcgen05 tensor cores (hi/lo TF32 operands, FP32 sums).
+    # precision="fp32" is the drop-in (CUDA cores; light on tcgen05 tensor cores,
+    # hi/lo FP16 operands); "split_tf32" runs the two contractions of the full
+    # forms on tensor cores (hi/lo TF32 operands, FP32 sums).
     def distance_m_to_n_symmetric_full(self, codes_a, codes_b, precision="fp32"):
         """distanceBatchMToNSymmetricFull: MSE + all four QJL terms (:618-631, 731-800)."""
         return self._symmetric_qjl(codes_a, codes_b, "full", precision)
