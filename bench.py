@@ -473,6 +473,7 @@ def mton_result(args, sym, steps=10, cpu=True):
         "speedup_split_bf16_decoded_vs_fp32": (
             round(res["fp32"]["ms"] / res["split_bf16_decoded"]["ms"], 2)
             if "ms" in res["split_bf16_decoded"] else None),
+        "fp32_form": "hi/lo FP16 pairs on the same tensor-core kernel (FP32 accuracy)",
         "target_speedup": 4.0,
         "cpu_baseline": cpu_base,
     }
