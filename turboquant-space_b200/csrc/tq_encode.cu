@@ -19,9 +19,9 @@
 //   - A group's rows arrive by cp.async while the previous group is encoded;
 //     its codes leave as one bulk store.
 //
-// What bounds it: the shared-memory pipe (about 540 wavefronts a row at D = 1024,
+// What bounds it: the shared-memory pipe (about 526 wavefronts a row at D = 1024,
 // 256 of them shuffles; encode2 had 694 and was 80% busy) and instruction issue
-// (1960 a row; 2334).  300k rows, encode2 -> this kernel: 256-d 4-bit 289 -> 174
+// (2024 a row; 2334).  300k rows, encode2 -> this kernel: 256-d 4-bit 289 -> 174
 // us, 384-d 4-bit 510 -> 372, 500-d 8-bit 492 -> 391, 768-d 4-bit 992 -> 897,
 // 768-d 8-bit 918 -> 866.  Eight lanes a row at D = 1024 leave 8 warps of 255
 // registers: 920 us.
