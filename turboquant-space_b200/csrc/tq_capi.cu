@@ -1026,6 +1026,8 @@ size_t sq_round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // planes (K padded to 32, rows to 128 / 256) for the tcgen05 kernel.  Padded
 // dims below 64 keep the FP32 kernel: a tile of so short a reduction is
 // mostly padding.
+constexpr size_t kCorrSlice = 32768;  // rows whose correction is prepared at a time
+
 struct SymqRunner {
     const tq_space *sp;
     int mode, ldk1, ldk2;
@@ -1093,9 +1095,11 @@ struct SymqRunner {
     // 2048 x 20k of 1536-d 15.3 -> 1.12 ms.
     tq_status prepare_rows_full_cg(const uint8_t *A, cudaStream_t s) {
         const size_t kc = m * tq::cg_row_k(sp->P, tq::kCgAsym) * 2, km = m * tq::cg_row_k(sp->P, tq::kCgSym) * 2;
-        const size_t vec = sizeof(float) * m * sp->D;  // D >= 16: every part a multiple of 16 bytes
+        // the correction's FP32 rows live for a slice of the rows at a time
+        const size_t slice = std::min(m, kCorrSlice), K = tq::cg_row_k(sp->P, tq::kCgAsym);
+        const size_t vec = sizeof(float) * slice * sp->D;  // D >= 16: every part a multiple of 16 bytes
         TQ_CUDA(rows.alloc(2 * (kc + km) + 2 * m * sizeof(float4), s), "cudaMallocAsync(row planes)");
-        TQ_CUDA(rows_bf.alloc(2 * vec + 2 * sizeof(float) * m, s), "cudaMallocAsync(correction rows)");
+        TQ_CUDA(rows_bf.alloc(2 * vec + 2 * sizeof(float) * slice, s), "cudaMallocAsync(correction rows)");
         auto *base = static_cast<unsigned char *>(rows.p);
         corr.hi = base;
         corr.lo = base + kc;
@@ -1103,9 +1107,17 @@ struct SymqRunner {
         cgr.lo = base + 2 * kc + km;
         cgr.rs = reinterpret_cast<float4 *>(base + 2 * (kc + km));
         corr.rs = cgr.rs + m;
-        float *q = static_cast<float *>(rows_bf.p), *sq = q + m * sp->D, *norms = sq + m * sp->D;
-        TQ_CUDA(tq::launch_symq_full_rows(sp->P, sp->T, A, m, q, sq, norms, s), "correction rows kernel");
-        TQ_CUDA(tq::launch_cg_rows_prepared(sp->P, q, sq, norms, m, tq::kCgFP16, corr, s), "row planes");
+        float *q = static_cast<float *>(rows_bf.p), *sq = q + slice * sp->D, *norms = sq + slice * sp->D;
+        for (size_t r0 = 0; r0 < m; r0 += slice) {
+            const size_t nr = std::min(slice, m - r0);
+            tq::CgRows part;
+            part.hi = static_cast<unsigned char *>(corr.hi) + r0 * K * 2;
+            part.lo = static_cast<unsigned char *>(corr.lo) + r0 * K * 2;
+            part.rs = corr.rs + r0;
+            TQ_CUDA(tq::launch_symq_full_rows(sp->P, sp->T, A + r0 * sp->code_size, nr, q, sq, norms, s),
+                    "correction rows kernel");
+            TQ_CUDA(tq::launch_cg_rows_prepared(sp->P, q, sq, norms, nr, tq::kCgFP16, part, s), "row planes");
+        }
         TQ_CUDA(tq::launch_cg_rows_codes(sp->P, sp->T, A, m, tq::kCgSym, tq::kCgFP16, cgr, s), "row planes");
         return TQ_OK;
     }

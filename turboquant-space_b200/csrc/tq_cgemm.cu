@@ -687,6 +687,9 @@ unsigned rows_grid(size_t work) {
 
 }  // namespace
 
+// What the truncation of the chunks takes off a sum of terms of one sign (near
+// rows of 32 to 2048 values at 2 to 8 bits: 1.6e-8 to 5e-8).
+constexpr double kTruncBias = 3e-8;
 float cg_cent_scale(const float *centroids, int levels) {
     float best = 2048.0f;
     double best_err = 1e300;
@@ -704,11 +707,11 @@ float cg_cent_scale(const float *centroids, int levels) {
             l2 += w * r * r;
         }
         // a product of two values is off by d + d' - r r', and the undoing factor by
-        // its rounding.  Over near rows, whose values agree, that is a bias; over
-        // others it averages out.
+        // its rounding.  Over near rows, whose values agree, that is a bias, to which
+        // the tensor core's truncation of the chunks adds; over others it averages out.
         const double u2 = (double)(1.0f / (a * a)) * a * a - 1.0;
         const double u1 = (double)(1.0f / (a * kRowScale)) * a * kRowScale - 1.0;
-        const double b2 = (2.0 * d1 - l2) / sw + u2, b1 = d1 / sw + u1;
+        const double b2 = (2.0 * d1 - l2) / sw + u2 - kTruncBias, b1 = d1 / sw + u1;
         const double err = b2 * b2 + b1 * b1 + (2.0 * d2 + l2 * l2 / sw) / sw / 64.0;
         if (err < best_err) {
             best = a;
@@ -762,10 +765,11 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.KBm = (P.D + CG_BK - 1) / CG_BK;
     a.KB = form == kCgSym ? a.KBm : 2 * a.KBm;
     // Chunk lengths (K blocks).  FP16: 2 (1 where the whole part is 4 blocks or
-    // fewer), so that the truncation of one chunk stays below the rounding of an
+    // fewer, and for few rows, whose tiles are bound by the decode: 8 x 200k of
+    // 384-d 95 -> 97 us, symmetric error 3.5e-8 -> 2.8e-8), so that the truncation of one chunk stays below the rounding of an
     // FP32 chain of the same length; BF16: 8 for queries and 4 for codes against
     // codes, whose terms share a sign more often.
-    a.chm = fmt == kCgFP16 ? (a.KBm <= 4 ? 1 : 2) : form == kCgAsym ? 8 : 4;
+    a.chm = fmt == kCgFP16 ? (a.KBm <= 4 || m < 32 ? 1 : 2) : form == kCgAsym ? 8 : 4;
     a.chs = form == kCgLight ? a.KBm : 16;  // +-1 by +-1 sums are exact integers
     a.m = m;
     a.rs = rows.rs;

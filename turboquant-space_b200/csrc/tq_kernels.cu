@@ -3,7 +3,8 @@
 //   encode_kernel   fused encodeVector (space_turbo_quant.h:339-396): norm,
 //                   sign flip + FWHT, sigma, Lloyd-Max quantize, residual,
 //                   gamma, QJL sign flip + FWHT, pack + trailer.  Bit-exact
-//                   with the reference's pinned Release build.
+//                   with the reference's pinned Release build (many rows of padded
+//                   dims 256 to 1024: tq_encode.cu).
 //   prepare_kernel  prepareQuery (:439-460).
 //   scan_kernel     asymmetric distSearch* (:659-686, 951-983) over a code
 //                   stream (distanceBatch1ToN/MToN :577-599) and the MSE-only
