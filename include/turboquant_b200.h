@@ -282,6 +282,12 @@ tq_status tq_space_scan_timer_read(tq_space *sp, double *total_ms, uint64_t *lau
  * stays usable), TQ_OK if it did not. */
 tq_status tq_selftest_bounded_wait(int device, int budget_ms);
 
+/* Self-test of the M x N kernel's index arithmetic, on the host alone: the
+ * largest row whose scalars the light QJL-corrected form of a call of m rows by
+ * n codes reads, over all tiles of the call.  Below m, or the kernel would read
+ * past them. */
+tq_status tq_selftest_mton_rows(const tq_space *sp, size_t m, size_t n, size_t *last_row);
+
 /* ---- serving: device-resident index + continuous-batching top-k server ---
  * The reference has no index or serving loop (README.md:81-83); these entry
  * points serve exact top-k asymmetric search over a corpus kept in HBM.  The

@@ -158,3 +158,17 @@ def test_precision_names_match_the_header():
     enum = {m.group(1).lower(): int(m.group(2))
             for m in re.finditer(r"\bTQ_PRECISION_([A-Z0-9_]+)\s*=\s*(\d+)", text)}
     assert enum == _capi.PRECISION, (enum, _capi.PRECISION)
+
+
+@pytest.mark.parametrize("dim,bits", [(64, 4), (384, 4), (384, 8), (1536, 4)])
+def test_mton_row_scalar_reads_stay_in_range(dim, bits):
+    """The light form's epilogue reads the scalars of its tile's rows before it
+    knows which columns are live.  Row counts just past a multiple of the wide
+    tiles leave a whole half of a tile past the rows; no read may follow it there."""
+    s = tq.TurboQuantSpace(dim, bits)
+    last = ctypes.c_size_t()
+    for n in (1, 1000, 20_000, 50_000, 1_000_000):
+        for m in (1, 2, 17, 33, 64, 65, 72, 127, 128, 129, 150, 255, 256, 257, 260, 300, 384, 385, 513, 520,
+                  640, 641, 1025, 1100):
+            _capi.check(_capi.lib().tq_selftest_mton_rows(s._h, m, n, ctypes.byref(last)))
+            assert last.value == m - 1, (m, n, last.value)

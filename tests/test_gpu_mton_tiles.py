@@ -61,3 +61,26 @@ def test_full_form_tile_edges(cuda_ok, dim, bits, m, n, variant):
     err, ok = dist_close(got, o.distance_m_to_n_symmetric_qjl(rows, codes, variant),
                          sym_term_scale(rows, codes, cs, cs - 12))
     assert ok, (variant, err.max())
+
+
+@pytest.mark.parametrize("dim,bits", [(64, 4), (100, 8), (384, 4)])
+@pytest.mark.parametrize("m,n", [(130, 6300), (257, 3801), (520, 2100)])
+def test_wide_tiles_with_few_live_columns(cuda_ok, dim, bits, m, n):
+    """Code counts at which 128-column tiles over CTA pairs are taken, with a
+    last row tile of 2 to 8 rows: its second half of columns lies past the rows."""
+    rng = np.random.default_rng(dim + bits + m + n)
+    X = (rng.standard_normal((n, dim)) * rng.uniform(1e-2, 1e2, (n, 1))).astype(np.float32)
+    Q = (rng.standard_normal((m, dim)) * rng.uniform(1e-2, 1e2, (m, 1))).astype(np.float32)
+    s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    cs = s.code_size_bytes()
+    codes, rows = o.encode_batch(X), o.encode_batch(Q)
+    scale = sym_term_scale(rows, codes, cs, cs - 12)
+    err, ok = dist_close(s.distance_m_to_n_symmetric_light(rows, codes),
+                         o.distance_m_to_n_symmetric_qjl(rows, codes, "light"), scale)
+    assert ok, ("light", err.max())
+    err, ok = dist_close(s.distance_m_to_n_symmetric(rows, codes),
+                         o.distance_m_to_n_symmetric(rows, codes), scale)
+    assert ok, ("symmetric", err.max())
+    err, ok = dist_close(s.distance_m_to_n(Q, codes), o.distance_m_to_n(Q, codes),
+                         asym_term_scale(Q, codes, cs, cs - 12))
+    assert ok, ("asymmetric", err.max())

@@ -631,6 +631,17 @@ tq_status tq_space_take_device_status(const tq_space *sp, int *code) {
     return take_status(sp, code);
 }
 
+tq_status tq_selftest_mton_rows(const tq_space *sp, size_t m, size_t n, size_t *last_row) {
+    if (!sp || !last_row || m == 0 || n == 0) return fail(TQ_ERR_INVALID_ARGUMENT, "NULL space or empty call");
+    const int nt = tq::cg_tile_cols(sp->P, tq::kCgLight, m, n), cpt = nt / tq::cg_tile_parts(nt);
+    *last_row = 0;
+    for (size_t col0 = 0; col0 < (m + nt - 1) / nt * nt; col0 += cpt) {
+        const tq::CgCols cols(col0, cpt, m);
+        for (int k = 0; k < cpt; ++k) *last_row = std::max(*last_row, cols.base + cols.offset(k));
+    }
+    return TQ_OK;
+}
+
 tq_status tq_distance_1_to_n_prepared_device(const tq_space *sp, const float *q_rot,
                                              const float *s_q, const float *norms,
                                              const uint8_t *codes, size_t n, float *out,

@@ -537,10 +537,10 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
                         else chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = __fmaf_rn(x, fx, y[k]); });
                     }
                 } else if (!ord.cent(c0)) {
-                    const float4 *rs = p.rs + col0;
-                    const int last = (int)min((size_t)cpt, p.m > col0 ? p.m - col0 : 1) - 1;
+                    const CgCols cols(col0, cpt, p.m);
+                    const float4 *rs = p.rs + cols.base;
                     chunk_pieces<CPT>(X, cpt, [&](int k, float x) {
-                        const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + min(k, last)) + 1);
+                        const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + cols.offset(k)) + 1);
                         const float ip = __fmul_rn(__fmul_rn(__fmul_rn(y[k], p.undo_c), r.x), sigma);
                         const float corr = __fmul_rn(__fmul_rn(x, r.y), gamma);
                         const float lim = fabsf(ip);
@@ -560,8 +560,9 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             const float c2 = __fmul_rn(norm, norm);
             const float c1 = p.form == kCgSym ? __fmul_rn(__fmul_rn(sigma, norm), p.undo_c) : norm;
             float *o = p.out + col0 * p.ldo + row;
-            const float4 *rs = p.rs + col0;
-            const int live = (int)min((size_t)cpt, col0 < p.m ? p.m - col0 : 0);
+            const CgCols cols(col0, cpt, p.m);
+            const float4 *rs = p.rs + cols.base;
+            const int live = cols.live;
             if constexpr (FULL) {
                 // products, or distances with another pass's products clamped in (all
                 // loads of 16 columns in flight at once)
@@ -745,6 +746,30 @@ cudaError_t launch_cg_rows_codes(const Params &P, const DevTables &T, const uint
     return cudaGetLastError();
 }
 
+// The tiles of the code side: 256 codes over a CTA pair for wide ones, 128 otherwise.
+static size_t code_tiles(size_t n, int NT) { return NT > 64 ? (n + 255) / 256 : (n + 127) / 128; }
+
+// Columns per tile: the width that takes the least time by a rough count of
+// clocks: waves of 148 CTAs times a tile's K blocks, each the slower of its
+// MMAs (10 per block on average over both parts, NT / 2 clocks each) and its
+// decode, plus the tile's epilogue.  Wide tiles (128, 256) run on CTA pairs.
+int cg_tile_cols(const Params &P, int form, size_t m, size_t n) {
+    const int KBm = (P.D + CG_BK - 1) / CG_BK, KB = form == kCgSym ? KBm : 2 * KBm;
+    int best = 256;
+    double best_t = 0.0;
+    for (int NT = 256; NT >= 16; NT >>= 1) {
+        const size_t tiles = code_tiles(n, NT) * ((m + NT - 1) / NT), slots = NT > 64 ? 74 : 148;
+        const double waves = (double)((tiles + slots - 1) / slots);
+        const double mma = 5.0 * NT, dec = NT <= 64 ? 600.0 : 1000.0;
+        const double t = waves * (KB * std::max(mma, dec) + 8.0 * NT + 1000.0);
+        if (NT == 256 || t < best_t) {
+            best = NT;
+            best_t = t;
+        }
+    }
+    return best;
+}
+
 cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt, const CgRows &rows,
                          size_t m, const uint8_t *codes, size_t n, float *out, size_t ldo, int *err,
                          cudaStream_t st, int post) {
@@ -782,23 +807,7 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.out = out;
     a.ldo = ldo;
     a.err = err;
-    // Columns per tile: the width that takes the least time by a rough count
-    // of clocks: waves of 148 CTAs times a tile's K blocks, each the slower of
-    // its MMAs (10 per block on average over both parts, NT / 2 clocks each)
-    // and its decode, plus the tile's epilogue.  Wide tiles (128, 256) run on
-    // CTA pairs, 256 codes a tile.
-    auto code_tiles = [&](int NT) { return (n + (NT > 64 ? 255 : 127)) / (NT > 64 ? 256 : 128); };
-    double best_t = 0.0;
-    for (int NT = 256; NT >= 16; NT >>= 1) {
-        const size_t tiles = code_tiles(NT) * ((m + NT - 1) / NT), slots = NT > 64 ? 74 : 148;
-        const double waves = (double)((tiles + slots - 1) / slots);
-        const double mma = 5.0 * NT, dec = NT <= 64 ? 600.0 : 1000.0;
-        const double tt = waves * (a.KB * std::max(mma, dec) + 8.0 * NT + 1000.0);
-        if (NT == 256 || tt < best_t) {
-            a.NT = NT;
-            best_t = tt;
-        }
-    }
+    a.NT = cg_tile_cols(P, form, m, n);
     const bool pair = a.NT > 64;
     const int stage_bytes = 2 * CG_A_BYTES + 2 * a.NT * (pair ? 64 : 128);
     const int tab = P.nibble ? 0 : CG_TAB_BYTES, ring_bytes = CG_BM * (P.nibble ? 32 : 64);
@@ -806,7 +815,7 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.stages = std::min(CG_MAX_STAGES, (avail - 2 * ring_bytes) / stage_bytes);
     a.ring = std::min(CG_MAX_RING, (avail - a.stages * stage_bytes) / ring_bytes);
     const size_t smem = (size_t)a.stages * stage_bytes + a.ring * ring_bytes + CG_FIXED + tab;
-    const size_t nt = code_tiles(a.NT), tiles = nt * ((m + a.NT - 1) / a.NT);
+    const size_t nt = code_tiles(n, a.NT), tiles = nt * ((m + a.NT - 1) / a.NT);
     if (tiles > 0x7FFFFFFFull || nt > 0x7FFFFFFFull) return cudaErrorInvalidValue;
     a.num_nt = (unsigned)nt;
     a.num_tiles = (unsigned)tiles;

@@ -20,6 +20,24 @@ struct CgRows {
 };
 size_t cg_row_k(const Params &P, int form);
 
+// The rows behind the columns [col0, col0 + cpt) of one part of a tile: `live` of
+// them (0 where the part lies past row m - 1, as the second half of a tile does
+// whose rows end in the first), and the row whose scalars column k may read: its
+// own, or for columns past the live ones, whose values are not used, one that exists.
+struct CgCols {
+    size_t base;
+    int live, last;
+    __host__ __device__ CgCols(size_t col0, int cpt, size_t m)
+        : base(col0 < m ? col0 : m - 1),
+          live(col0 >= m ? 0 : m - col0 < (size_t)cpt ? (int)(m - col0) : cpt),
+          last(live > 0 ? live - 1 : 0) {}
+    // column k reads row base + offset(k)
+    __host__ __device__ int offset(int k) const { return k < last ? k : last; }
+};
+// Columns per tile of a call, and the parts a tile's columns are split in.
+int cg_tile_cols(const Params &P, int form, size_t m, size_t n);
+inline int cg_tile_parts(int cols) { return cols > 64 ? 2 : 1; }
+
 // P.cent_scale: the scale in (1024, 2048] at which products of the centroids' FP16
 // pairs (without lo lo) have the least bias and error.
 float cg_cent_scale(const float *centroids, int levels);
