@@ -84,3 +84,38 @@ def test_wide_tiles_with_few_live_columns(cuda_ok, dim, bits, m, n):
     err, ok = dist_close(s.distance_m_to_n(Q, codes), o.distance_m_to_n(Q, codes),
                          asym_term_scale(Q, codes, cs, cs - 12))
     assert ok, ("asymmetric", err.max())
+
+
+def _near(dim, m, seed):
+    rng = np.random.default_rng(seed)
+    X = rng.standard_normal((2048, dim)).astype(np.float32)
+    X /= np.linalg.norm(X, axis=1, keepdims=True)
+    Q = X[:m] + (0.02 / dim ** 0.5) * rng.standard_normal((m, dim)).astype(np.float32)
+    return X, np.ascontiguousarray(Q, np.float32)
+
+
+def _near_errors(d, f64):
+    """Errors of each row's near pair, relative to |q|^2 + |x|^2 (about 2)."""
+    return (np.array([d[i, i] for i in range(len(f64))], np.float64) - f64) / 2.0
+
+
+@pytest.mark.parametrize("dim,bits", [(128, 8), (384, 4), (768, 2), (1024, 3), (1536, 2), (1536, 8)])
+def test_near_pairs_at_fp32_are_as_accurate_as_the_scan(cuda_ok, dim, bits):
+    """Near pairs, whose terms share a sign, are where truncating sums show.  Calls
+    of 16 rows (tensor cores) against calls of one row (the scan kernel's FP32
+    chains): at most 1.5 times its error, and half an ulp of the sum more.  64 rows
+    at once: at most the error of rounding an FP32 chain of 2 D terms, a random walk
+    of 2 D half-ulps of a sum that grows to its end."""
+    m = 64
+    X, Q = _near(dim, m, dim + bits)
+    s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    codes = o.encode_batch(X)
+    f64 = np.array([o.distance_f64(Q[i], codes[i]) for i in range(m)])
+    scan = np.concatenate([s.distance_m_to_n(Q[i:i + 1], codes) for i in range(m)])
+    few = np.concatenate([s.distance_m_to_n(Q[i:i + 16], codes) for i in range(0, m, 16)])
+    rms = lambda e: float(np.sqrt(np.mean(e * e)))  # noqa: E731
+    es, ef, ew = (_near_errors(d, f64) for d in (scan, few, s.distance_m_to_n(Q, codes)))
+    assert rms(ef) <= 1.5 * rms(es) + 2.0 ** -25, (rms(ef), rms(es))
+    assert abs(ef.mean()) <= abs(es.mean()) + 2.0 ** -24, (ef.mean(), es.mean())
+    D = 1 << (dim - 1).bit_length()
+    assert rms(ew) <= 2.0 ** -25 * (2 * D) ** 0.5, rms(ew)

@@ -30,11 +30,14 @@
 // a lane-replicated shared table (no bank conflicts).
 //
 // Accumulation: the MMAs of a chunk of K blocks accumulate from zero in one of
-// two tensor-memory buffers (the tensor core's FP32 accumulation truncates
+// two (four with split quarters) tensor-memory buffers (the tensor core's FP32 accumulation truncates
 // toward zero, about 2^-24 of the running sum an MMA; a block's small products
 // run before its hi hi ones, while the sum is small); the epilogue warps add
 // each finished chunk into FP32 registers with IEEE adds while the other
-// buffer fills.
+// buffer fills.  Calls of fewer than 32 rows at FP16 go further: each quarter of a
+// K block (one MMA's 16 values) has accumulators of its own, added in FP32, so that
+// no sum is truncated at its full size more than once a K block; narrow tiles leave
+// the tensor pipe and the columns idle that this takes.
 //
 // CTA pairs: wide tiles (NT > 64) run on clusters of two CTAs, 256 codes by NT
 // rows, tcgen05.mma.cta_group::2: each CTA decodes its 128 codes and loads half
@@ -194,16 +197,37 @@ __device__ __forceinline__ void chunk_pieces(uint32_t X, int cols, F f) {
     }
 }
 
+// The same for a chunk whose K-block quarters have accumulators of their own,
+// NT (16 or 32) columns each: f(k, their sum).
+template <class F>
+__device__ __forceinline__ void chunk_quarters(uint32_t X, int NT, F f) {
+#pragma unroll
+    for (int c0 = 0; c0 < 32; c0 += 16) {
+        if (c0 >= NT) break;
+        uint32_t x[4][16];
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tmem_ld16_nw(X + q * NT + c0, x[q]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            f(c0 + j, __fadd_rn(__fadd_rn(__uint_as_float(x[0][j]), __uint_as_float(x[1][j])),
+                                __fadd_rn(__uint_as_float(x[2][j]), __uint_as_float(x[3][j]))));
+    }
+}
+
 // DW: decoder warps (warps 4 .. 4 + DW - 1); the other 12 - DW warps are the
 // epilogue: two column halves of 128 (DW = 4), or one of 64 (DW = 8).  Batches
 // of few rows are bound by the decoders, wide ones by the MMAs.
-template <int DW, bool NIB, bool LIGHT, bool PAIR, bool FULL>
+// SPLIT: tiles of at most 32 columns, whose K-block quarters accumulate apart.
+template <int DW, bool NIB, bool LIGHT, bool PAIR, bool FULL, bool SPLIT>
 __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_constant__ CUtensorMap map_h,
                                                               const __grid_constant__ CUtensorMap map_l,
                                                               const CgArgs p) {
     constexpr int EW = 12 - DW;          // epilogue warps
+    constexpr uint32_t NB = SPLIT ? 4 : 2, BUF = 512 / NB;  // chunk buffers in tensor memory, columns of each
     constexpr int HALVES = EW / 4;       // column parts of a tile
-    constexpr int CPT = DW == 4 ? 128 : 64;  // columns per epilogue thread, at most
+    constexpr int CPT = SPLIT ? 32 : DW == 4 ? 128 : 64;  // columns per epilogue thread, at most
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const uint32_t rank = PAIR ? cluster_rank() : 0u;
@@ -211,12 +235,12 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
     const int stage_bytes = 2 * CG_A_BYTES + 2 * bt_bytes;
     const uint32_t tiles0 = smem_u32(smem);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + p.stages * stage_bytes);
-    // bars: full[6], empty[6], xfull[2], xempty[2], drain, cfull[8], cempty[8], pfull[6]; then the TMEM slot
+    // bars: full[6], empty[6], xfull[4], xempty[4], drain, cfull[8], cempty[8], pfull[6]; then the TMEM slot
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * CG_MAX_STAGES;
-    const uint32_t xfull0 = empty0 + 8 * CG_MAX_STAGES, xempty0 = xfull0 + 16, drain = xempty0 + 16;
+    const uint32_t xfull0 = empty0 + 8 * CG_MAX_STAGES, xempty0 = xfull0 + 32, drain = xempty0 + 32;
     const uint32_t cfull0 = drain + 8, cempty0 = cfull0 + 8 * CG_MAX_RING;
     const uint32_t pfull0 = cempty0 + 8 * CG_MAX_RING;  // PAIR, rank 0: the other CTA's stage is full
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * CG_MAX_STAGES + 5 + 2 * CG_MAX_RING);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * CG_MAX_STAGES + 9 + 2 * CG_MAX_RING);
     // the ring of code words, then the byte codes' table
     constexpr int WPI = NIB ? 1 : 2;                 // words of 8 coordinates
     constexpr int RING_BYTES = CG_BM * 32 * WPI;     // one K block's words
@@ -230,7 +254,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             mbar_init(empty0 + 8 * s, 1);
             mbar_init(pfull0 + 8 * s, 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (uint32_t b = 0; b < NB; ++b) {
             mbar_init(xfull0 + 8 * b, 1);
             mbar_init(xempty0 + 8 * b, PAIR ? 2 * EW : EW);  // PAIR: rank 0's counts both CTAs'
         }
@@ -314,17 +338,18 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             const uint32_t idesc = (1u << 4) | (f << 7) | (f << 10) | ((uint32_t)(p.NT >> 3) << 17) |
                                    ((uint32_t)((PAIR ? 2 * CG_BM : CG_BM) >> 4) << 24);
             constexpr bool one_sign = LIGHT;  // +-1 rows: their lo is zero
+            const uint32_t dk = SPLIT ? (uint32_t)p.NT : 0u;  // quarter kk's accumulator: d + kk dk
             const uint32_t ab = CG_A_BYTES >> 4, bb = (uint32_t)bt_bytes >> 4;
             uint32_t s = 0, ph = 0, gc = 0;
             bool ok = true;
             for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
                 for (int c0 = 0, c1 = 0; c0 < KB && ok; c0 = c1, ++gc) {
                     c1 = ord.chunk_end(p, c0);
-                    const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
+                    const uint32_t b = gc % NB, xph = (gc / NB) & 1u;
                     if (!(PAIR ? mbar_wait_cluster_warp(xempty0 + 8 * b, xph ^ 1u, p.err, kErrTmemEmpty)
                                : mbar_wait_warp(xempty0 + 8 * b, xph ^ 1u, p.err, kErrTmemEmpty))) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t d = tmem_base + b * 256u;
+                    const uint32_t d = tmem_base + b * BUF;
                     uint32_t acc = 0u;
                     for (int kb = c0; kb < c1; ++kb) {
                         if (!mbar_wait_warp(full0 + 8 * s, ph, p.err, kErrFull)) { ok = false; break; }
@@ -335,26 +360,25 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
                         if (lead) {
                             // one MMA's K: 32 bytes.  The block's small products first: each
                             // MMA truncates the sum, and it is small until hi hi joins.
+                            auto acc0 = [&](int kk) { return kk == 0 || dk ? acc : 1u; };
+                            bool fresh = true;  // no product of this block is in yet
                             if (ord.cent(kb)) {
 #pragma unroll
-                                for (int kk = 0; kk < 4; ++kk) {
-                                    umma_f16<PAIR>(d, al + 2 * kk, bh + 2 * kk, idesc, acc);
-                                    acc = 1u;
-                                }
+                                for (int kk = 0; kk < 4; ++kk)
+                                    umma_f16<PAIR>(d + kk * dk, al + 2 * kk, bh + 2 * kk, idesc, acc0(kk));
 #pragma unroll
-                                for (int kk = 0; kk < 4; ++kk) umma_f16<PAIR>(d, ah + 2 * kk, bl + 2 * kk, idesc, 1u);
+                                for (int kk = 0; kk < 4; ++kk)
+                                    umma_f16<PAIR>(d + kk * dk, ah + 2 * kk, bl + 2 * kk, idesc, 1u);
+                                fresh = false;
                             } else if (!one_sign) {
 #pragma unroll
-                                for (int kk = 0; kk < 4; ++kk) {
-                                    umma_f16<PAIR>(d, ah + 2 * kk, bl + 2 * kk, idesc, acc);
-                                    acc = 1u;
-                                }
+                                for (int kk = 0; kk < 4; ++kk)
+                                    umma_f16<PAIR>(d + kk * dk, ah + 2 * kk, bl + 2 * kk, idesc, acc0(kk));
+                                fresh = false;
                             }
 #pragma unroll
-                            for (int kk = 0; kk < 4; ++kk) {
-                                umma_f16<PAIR>(d, ah + 2 * kk, bh + 2 * kk, idesc, acc);
-                                acc = 1u;
-                            }
+                            for (int kk = 0; kk < 4; ++kk)
+                                umma_f16<PAIR>(d + kk * dk, ah + 2 * kk, bh + 2 * kk, idesc, fresh ? acc0(kk) : 1u);
                             commit<PAIR>(empty0 + 8 * s);
                         }
                         acc = 1u;
@@ -517,29 +541,33 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             }
             for (int c0 = 0, c1 = 0; c0 < KB; c0 = c1, ++gc) {
                 c1 = ord.chunk_end(p, c0);
-                const uint32_t b = gc & 1u, xph = (gc >> 1) & 1u;
+                const uint32_t b = gc % NB, xph = (gc / NB) & 1u;
                 if (!mbar_wait_warp(xfull0 + 8 * b, xph, p.err, kErrTmemFull)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t X = lanes + b * 256u;
+                const uint32_t X = lanes + b * BUF;
+                auto pieces = [&](auto f) {
+                    if constexpr (SPLIT) chunk_quarters(X, p.NT, f);
+                    else chunk_pieces<CPT>(X, cpt, f);
+                };
                 // How a chunk joins the running sum.  Symmetric and light: centroid
                 // chunks are added (the light form's last chunk is its clamped
                 // correction).  Asymmetric: fma(x, f, y) with f = scale gamma for
                 // the sign part and sigma for the centroid part.
                 if (LIGHT || p.form == kCgSym) {
-                    if (c0 == 0) chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = x; });
-                    else if (!LIGHT || ord.cent(c0)) chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = __fadd_rn(y[k], x); });
+                    if (c0 == 0) pieces([&](int k, float x) { y[k] = x; });
+                    else if (!LIGHT || ord.cent(c0)) pieces([&](int k, float x) { y[k] = __fadd_rn(y[k], x); });
                 }
                 if constexpr (!LIGHT) {
                     if (p.form == kCgAsym) {
                         const float fx = ord.cent(c0) ? __fmul_rn(sigma, p.undo_c)
                                                       : __fmul_rn(__fmul_rn(p.scale, gamma), p.undo_s);
-                        if (c0 == 0) chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = __fmul_rn(x, fx); });
-                        else chunk_pieces<CPT>(X, cpt, [&](int k, float x) { y[k] = __fmaf_rn(x, fx, y[k]); });
+                        if (c0 == 0) pieces([&](int k, float x) { y[k] = __fmul_rn(x, fx); });
+                        else pieces([&](int k, float x) { y[k] = __fmaf_rn(x, fx, y[k]); });
                     }
                 } else if (!ord.cent(c0)) {
                     const CgCols cols(col0, cpt, p.m);
                     const float4 *rs = p.rs + cols.base;
-                    chunk_pieces<CPT>(X, cpt, [&](int k, float x) {
+                    pieces([&](int k, float x) {
                         const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + cols.offset(k)) + 1);
                         const float ip = __fmul_rn(__fmul_rn(__fmul_rn(y[k], p.undo_c), r.x), sigma);
                         const float corr = __fmul_rn(__fmul_rn(x, r.y), gamma);
@@ -789,13 +817,21 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.post = post;
     a.KBm = (P.D + CG_BK - 1) / CG_BK;
     a.KB = form == kCgSym ? a.KBm : 2 * a.KBm;
-    // Chunk lengths (K blocks).  FP16: 2 (1 where the whole part is 4 blocks or
-    // fewer, and for few rows, whose tiles are bound by the decode: 8 x 200k of
-    // 384-d 95 -> 97 us, symmetric error 3.5e-8 -> 2.8e-8), so that the truncation of one chunk stays below the rounding of an
-    // FP32 chain of the same length; BF16: 8 for queries and 4 for codes against
-    // codes, whose terms share a sign more often.
+    // Chunk lengths (K blocks), so that what truncation takes off a chunk stays below
+    // the rounding of an FP32 sum.  FP16: 2 (1 where the whole part is 4 blocks or
+    // fewer).  BF16: 8 for queries and 4 for codes against codes, whose terms share a
+    // sign more often.  The sign part: +-1 by +-1 sums (light) are exact integers;
+    // otherwise 8, since its hi products are nearly exact in FP32 and its share of a
+    // near pair's sum is a third at most (near pairs of 1536-d 2-bit, mean error with
+    // 16 / 8 / 2 blocks 3.4 / 2.0 / 1.1e-7, and 2000 x 100k of 768-d 1.55 / 1.59 /
+    // 1.70 ms; an FP32 chain's largest error there is 3e-6, this one's 1.1e-6).
+    // Fewer than 32 rows, where the scan kernel's short FP32 chains stand for
+    // comparison: chunks of 1 and 4 blocks with the quarters apart, an error like the
+    // scan's (near pairs of 2-bit codes, 8 rows, largest 5.5e-7 -> 3.3e-7 against the
+    // scan's 2.9e-7) for 97 -> 102 us at 8 x 200k of 384-d, 245 -> 250 of 768-d 8-bit,
+    // 93 -> 100 at 24 x 200k.
     a.chm = fmt == kCgFP16 ? (a.KBm <= 4 || m < 32 ? 1 : 2) : form == kCgAsym ? 8 : 4;
-    a.chs = form == kCgLight ? a.KBm : 16;  // +-1 by +-1 sums are exact integers
+    a.chs = form == kCgLight ? a.KBm : fmt == kCgFP16 && m < 32 ? 4 : 8;
     a.m = m;
     a.rs = rows.rs;
     a.scale = P.scale;
@@ -808,6 +844,7 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.ldo = ldo;
     a.err = err;
     a.NT = cg_tile_cols(P, form, m, n);
+    const bool split = fmt == kCgFP16 && m < 32 && a.NT <= 32;
     const bool pair = a.NT > 64;
     const int stage_bytes = 2 * CG_A_BYTES + 2 * a.NT * (pair ? 64 : 128);
     const int tab = P.nibble ? 0 : CG_TAB_BYTES, ring_bytes = CG_BM * (P.nibble ? 32 : 64);
@@ -823,15 +860,19 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     const int K = a.KB * CG_BK, box = pair ? a.NT / 2 : a.NT;
     if (!make_map(&mh, rows.hi, K, m, box) || !make_map(&ml, rows.lo, K, m, box)) return cudaErrorInvalidValue;
     const bool light = form == kCgLight;
-    auto pick = [&](auto wide, auto nib) {
-        constexpr bool W = decltype(wide)::value, N = decltype(nib)::value;
-        return post != kCgDist ? cgemm_kernel<W ? 4 : 8, N, false, W, true>
-               : light         ? cgemm_kernel<W ? 4 : 8, N, true, W, false>
-                               : cgemm_kernel<W ? 4 : 8, N, false, W, false>;
+    // wide tiles, narrow ones, and narrow ones with split accumulators
+    auto pick = [&](auto nib, auto form_light, auto form_full) {
+        constexpr bool N = decltype(nib)::value, L = decltype(form_light)::value, F = decltype(form_full)::value;
+        return pair    ? cgemm_kernel<4, N, L, true, F, false>
+               : split ? cgemm_kernel<8, N, L, false, F, true>
+                       : cgemm_kernel<8, N, L, false, F, false>;
     };
     using T_ = std::true_type;
     using F_ = std::false_type;
-    auto kern = P.nibble ? (pair ? pick(T_{}, T_{}) : pick(F_{}, T_{})) : (pair ? pick(T_{}, F_{}) : pick(F_{}, F_{}));
+    auto by_form = [&](auto nib) {
+        return post != kCgDist ? pick(nib, F_{}, T_{}) : light ? pick(nib, T_{}, F_{}) : pick(nib, F_{}, F_{});
+    };
+    auto kern = P.nibble ? by_form(T_{}) : by_form(F_{});
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
