@@ -119,3 +119,21 @@ def test_near_pairs_at_fp32_are_as_accurate_as_the_scan(cuda_ok, dim, bits):
     assert abs(ef.mean()) <= abs(es.mean()) + 2.0 ** -24, (ef.mean(), es.mean())
     D = 1 << (dim - 1).bit_length()
     assert rms(ew) <= 2.0 ** -25 * (2 * D) ** 0.5, rms(ew)
+
+
+@pytest.mark.parametrize("dim", [128, 768, 1536])
+@pytest.mark.parametrize("bits", [2, 3, 4, 8])
+def test_near_pairs_at_split_bf16(cuda_ok, dim, bits):
+    """BF16 pairs round each of a few centroid values by up to 2^-17, the same way in
+    every term.  With the centroids' scale no such bias is left: near pairs are off
+    by 2e-6 on average at most, the truncation of a whole chunk (1.9e-6)."""
+    m = 64
+    X, Q = _near(dim, m, 3 * dim + bits)
+    s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    codes, rows = o.encode_batch(X), o.encode_batch(Q)
+    f64 = np.array([o.distance_f64(Q[i], codes[i]) for i in range(m)])
+    e = _near_errors(s.distance_m_to_n(Q, codes, precision="split_bf16"), f64)
+    assert abs(e.mean()) <= 2e-6, e.mean()
+    f64 = np.array([o.distance_symmetric_f64(rows[i], codes[i]) for i in range(m)])
+    e = _near_errors(s.distance_m_to_n_symmetric(rows, codes, precision="split_bf16"), f64)
+    assert abs(e.mean()) <= 2e-6, e.mean()

@@ -329,7 +329,7 @@ tq_status tq_space_create(size_t dim, int bits, uint64_t rot_seed, uint64_t qjl_
         // space_turbo_quant.h:265-266 and turbo_quant.h:69, in FP32 as written
         P.scale = std::sqrt(static_cast<float>(M_PI) / 2.0f) / std::sqrt(static_cast<float>(D));
         P.wht_scale = 1.0f / std::sqrt(static_cast<float>(D));
-        P.cent_scale = tq::cg_cent_scale(sp->centroids.data(), sp->levels);
+        for (int fmt : {tq::kCgFP16, tq::kCgBF16}) P.cent_scale[fmt] = tq::cg_cent_scale(sp->centroids.data(), sp->levels, fmt);
         P.lutq = 0;
         P.qlut_k = 0;
         P.qflag = 0;

@@ -83,7 +83,8 @@ constexpr int kErrFull = 1, kErrEmpty = 2, kErrTmemFull = 3, kErrTmemEmpty = 4;
 // The centroids' scale is P.cent_scale: few distinct values, whose rounding
 // errors do not average out over a row (40 x 20k symmetric distances of clustered
 // 384-d rows, error against FP64 with the FP32 chain / scale 2048 / chosen scale:
-// 3-bit 8.5 / 4.5 / 3.6e-8, 8-bit 3.5 / 3.7 / 3.4e-8).
+// 3-bit 8.5 / 4.5 / 3.6e-8, 8-bit 3.5 / 3.7 / 3.4e-8; near pairs at BF16, largest
+// error with no scale / the chosen one: 2-bit 4.4 / 2.0e-6, 8-bit 3.7 / 1.9e-6).
 constexpr float kRowScale = 16384.0f;
 
 __device__ __forceinline__ void split16(float v, int fmt, uint32_t &h, uint32_t &l) {
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             const int v = i >> 5;
             uint32_t h, l;
             const float c = v < p.levels ? p.centroids[v] : 0.0f;
-            split16(p.fmt == kCgFP16 ? c * p.cent : c, p.fmt, h, l);
+            split16(c * p.cent, p.fmt, h, l);
             btab[i] = h | (l << 16);
         }
     }
@@ -443,7 +444,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             for (int v = 0; v < 8; ++v) {
                 uint32_t h, l;
                 const float cv = v < p.levels ? p.centroids[v] : 0.0f;
-                split16(p.fmt == kCgFP16 ? cv * p.cent : cv, p.fmt, h, l);
+                split16(cv * p.cent, p.fmt, h, l);
                 const int sh = 8 * (v & 3);
                 tab.hl[v >> 2] |= (h & 0xFFu) << sh;
                 tab.hh[v >> 2] |= (h >> 8) << sh;
@@ -680,7 +681,7 @@ __global__ void __launch_bounds__(256) cg_rows_codes_kernel(const uint8_t *__res
                                                             float4 *__restrict__ rs) {
     const int half = KBm * CG_BK, K = form == kCgLight ? 2 * half : half, quads = K / 4;
     const size_t total = m * (size_t)quads;
-    const float f = fmt == kCgFP16 ? P.cent_scale : 1.0f;
+    const float f = P.cent_scale[fmt];
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (size_t)gridDim.x * blockDim.x) {
         const size_t r = t / quads;
@@ -716,19 +717,27 @@ unsigned rows_grid(size_t work) {
 
 }  // namespace
 
-// What the truncation of the chunks takes off a sum of terms of one sign (near
-// rows of 32 to 2048 values at 2 to 8 bits: 1.6e-8 to 5e-8).
-constexpr double kTruncBias = 3e-8;
-float cg_cent_scale(const float *centroids, int levels) {
-    float best = 2048.0f;
+// What the truncation of the chunks takes off a sum of terms of one sign, which a
+// scale may give back.  FP16: near rows of 32 to 2048 values at 2 to 8 bits, 1.6e-8
+// to 5e-8.  BF16: half an ulp, 0.72 2^-24 of the sum so far on average, an MMA, over
+// 12 MMAs a block: 44.5 of the whole sum in chunks of 8 blocks (queries), whose sum
+// grows evenly, 20.5 in chunks of 4 (codes
+// against codes).
+constexpr double kTruncBias[2][2] = {{0.0, 3e-8}, {1.9e-6, 8.8e-7}};  // [fmt][rows are codes]
+float cg_cent_scale(const float *centroids, int levels, int fmt) {
+    const bool h16 = fmt == kCgFP16;
+    const float top = h16 ? 2048.0f : 2.0f, step = h16 ? 4.0f : 1.0f / 256, rows = h16 ? kRowScale : 1.0f;
+    const double t1 = kTruncBias[fmt][0], t2 = kTruncBias[fmt][1];
+    float best = top;
     double best_err = 1e300;
     for (int i = 0; i < 256; ++i) {
-        const float a = 2048.0f - 4.0f * (float)i;
+        const float a = top - step * (float)i;
         double sw = 0.0, d1 = 0.0, d2 = 0.0, l2 = 0.0;
         for (int v = levels / 2; v < levels; ++v) {  // the others are their negatives
             const double c = centroids[v], w = c * c * std::exp(-c * c / 3.0);  // c^2 times about its share
             const float x = centroids[v] * a;
-            const float h = __half2float(__float2half_rn(x)), l = __half2float(__float2half_rn(x - h));
+            const float h = h16 ? __half2float(__float2half_rn(x)) : __bfloat162float(__float2bfloat16_rn(x));
+            const float l = h16 ? __half2float(__float2half_rn(x - h)) : __bfloat162float(__float2bfloat16_rn(x - h));
             const double d = ((double)h + l) / (c * a) - 1.0, r = l / (c * a);
             sw += w;
             d1 += w * d;
@@ -739,8 +748,8 @@ float cg_cent_scale(const float *centroids, int levels) {
         // its rounding.  Over near rows, whose values agree, that is a bias, to which
         // the tensor core's truncation of the chunks adds; over others it averages out.
         const double u2 = (double)(1.0f / (a * a)) * a * a - 1.0;
-        const double u1 = (double)(1.0f / (a * kRowScale)) * a * kRowScale - 1.0;
-        const double b2 = (2.0 * d1 - l2) / sw + u2 - kTruncBias, b1 = d1 / sw + u1;
+        const double u1 = (double)(1.0f / (a * rows)) * a * rows - 1.0;
+        const double b2 = (2.0 * d1 - l2) / sw + u2 - t2, b1 = d1 / sw + u1 - t1;
         const double err = b2 * b2 + b1 * b1 + (2.0 * d2 + l2 * l2 / sw) / sw / 64.0;
         if (err < best_err) {
             best = a;
@@ -835,11 +844,9 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.m = m;
     a.rs = rows.rs;
     a.scale = P.scale;
-    a.cent = P.cent_scale;
+    a.cent = P.cent_scale[fmt];
     a.undo_s = fmt == kCgFP16 && form == kCgAsym ? 1.0f / kRowScale : 1.0f;
-    a.undo_c = fmt == kCgFP16
-                   ? 1.0f / (P.cent_scale * (form == kCgAsym ? kRowScale : P.cent_scale))
-                   : 1.0f;
+    a.undo_c = 1.0f / (a.cent * (form != kCgAsym ? a.cent : fmt == kCgFP16 ? kRowScale : 1.0f));
     a.out = out;
     a.ldo = ldo;
     a.err = err;

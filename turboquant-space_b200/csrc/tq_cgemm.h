@@ -38,9 +38,9 @@ struct CgCols {
 int cg_tile_cols(const Params &P, int form, size_t m, size_t n);
 inline int cg_tile_parts(int cols) { return cols > 64 ? 2 : 1; }
 
-// P.cent_scale: the scale in (1024, 2048] at which products of the centroids' FP16
-// pairs (without lo lo) have the least bias and error.
-float cg_cent_scale(const float *centroids, int levels);
+// P.cent_scale[fmt]: the scale in (1024, 2048] (FP16) or (1, 2] (BF16) at which
+// products of the centroids' pairs (without lo lo) have the least bias and error.
+float cg_cent_scale(const float *centroids, int levels, int fmt);
 
 // Prepared queries (kCgAsym) or codes (kCgSym, kCgLight) -> row operand.
 cudaError_t launch_cg_rows_prepared(const Params &P, const float *q_rot, const float *s_q,

@@ -44,7 +44,7 @@ struct Params {
     float qlut_c;
     float scale;       // sqrt(pi/2)/sqrt(D)            space_turbo_quant.h:265
     float wht_scale;   // 1/sqrt(D)                     turbo_quant.h:69
-    float cent_scale;  // scale of the FP16 hi/lo centroids (cg_cent_scale)
+    float cent_scale[2];  // scale of the FP16 and BF16 hi/lo centroids (cg_cent_scale)
 };
 
 // Device copies of the space's tables (one allocation per space).
