@@ -137,3 +137,34 @@ def test_near_pairs_at_split_bf16(cuda_ok, dim, bits):
     f64 = np.array([o.distance_symmetric_f64(rows[i], codes[i]) for i in range(m)])
     e = _near_errors(s.distance_m_to_n_symmetric(rows, codes, precision="split_bf16"), f64)
     assert abs(e.mean()) <= 2e-6, e.mean()
+
+
+@pytest.mark.parametrize("dim,bits", [(128, 4), (100, 8), (1536, 3)])
+@pytest.mark.parametrize("m", [3, 16, 64])
+def test_rows_whose_norm_overflows(cuda_ok, dim, bits, m):
+    """Vectors whose squared norm overflows FP32 have the norm +inf; against them a
+    distance is +inf or 0 by the sign of the inner product, also where a correction
+    of the other sign is clamped in.  Rows of NaNs give 0."""
+    n = 300
+    rng = np.random.default_rng(dim + bits + m)
+    X = rng.standard_normal((n, dim)).astype(np.float32)
+    Q = rng.standard_normal((m, dim)).astype(np.float32)
+    X[::7] *= np.float32(1e25)
+    Q[1] *= np.float32(1e25)
+    X[5], Q[2] = np.nan, np.nan
+    s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    codes, rows = o.encode_batch(X), o.encode_batch(Q)
+    with np.errstate(all="ignore"):
+        calls = {
+            "asymmetric": (s.distance_m_to_n(Q, codes), o.distance_m_to_n(Q, codes)),
+            "symmetric": (s.distance_m_to_n_symmetric(rows, codes), o.distance_m_to_n_symmetric(rows, codes)),
+            "light": (s.distance_m_to_n_symmetric_light(rows, codes),
+                      o.distance_m_to_n_symmetric_qjl(rows, codes, "light")),
+            "full": (s.distance_m_to_n_symmetric_full(rows, codes),
+                     o.distance_m_to_n_symmetric_qjl(rows, codes, "full")),
+        }
+    for form, (got, ref) in calls.items():
+        finite = np.isfinite(ref)
+        assert (~finite).any(), form
+        np.testing.assert_array_equal(got[~finite], ref[~finite].astype(np.float32), err_msg=form)
+        np.testing.assert_allclose(got[finite], ref[finite], rtol=1e-4, atol=1e-2, err_msg=form)

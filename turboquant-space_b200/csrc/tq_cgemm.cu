@@ -594,7 +594,9 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             const int live = cols.live;
             if constexpr (FULL) {
                 // products, or distances with another pass's products clamped in (all
-                // loads of 16 columns in flight at once)
+                // loads of 16 columns in flight at once).  The norms join last: an
+                // infinite one times a sum of two signs gives what it does in the
+                // reference, where products that held it could cancel to a NaN.
                 const bool add = p.post == kCgClampedSum;
 #pragma unroll
                 for (int k0 = 0; k0 < CPT; k0 += 16) {
@@ -605,12 +607,15 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
 #pragma unroll
                     for (int k = k0; k < k0 + 16; ++k) {
                         if (k < live) {
-                            const float2 r = __ldg(reinterpret_cast<const float2 *>(rs + k));
-                            float ipt = __fmul_rn(__fmul_rn(y[k], r.x), c1);
-                            const float lim = fabsf(ipt);
-                            if (add) ipt = __fadd_rn(ipt, fmaxf(-lim, fminf(lim, other[k - k0])));
-                            const float d = fmaxf(__fmaf_rn(-2.0f, ipt, __fadd_rn(r.y, c2)), 0.0f);
-                            __stcs(o, add ? d : ipt);
+                            const float4 r = __ldg(rs + k);
+                            float v = __fmul_rn(y[k], r.x);
+                            if (add) {
+                                const float ip = __fmul_rn(__fmul_rn(__fmul_rn(y[k], p.undo_c), r.z), sigma);
+                                const float lim = fabsf(ip);
+                                const float sum = __fadd_rn(ip, fmaxf(-lim, fminf(lim, other[k - k0])));
+                                v = fmaxf(__fmaf_rn(-2.0f, __fmul_rn(__fmul_rn(sum, r.w), norm), __fadd_rn(r.y, c2)), 0.0f);
+                            }
+                            __stcs(o, v);
                         }
                         o += p.ldo;
                     }
@@ -673,7 +678,7 @@ __global__ void __launch_bounds__(256) cg_rows_prepared_kernel(
 }
 
 // Row codes: centroid values, for the light form followed by the +-1 signs.
-// rs: symmetric (sigma n, n^2, -, -); light (n, n^2, sigma, (pi / 2D) gamma).
+// rs: symmetric (sigma n, n^2, sigma, n); light (n, n^2, sigma, (pi / 2D) gamma).
 __global__ void __launch_bounds__(256) cg_rows_codes_kernel(const uint8_t *__restrict__ codes, size_t m,
                                                             Params P, DevTables T, int KBm, int form,
                                                             int fmt, __nv_bfloat16 *__restrict__ ph,
@@ -706,7 +711,7 @@ __global__ void __launch_bounds__(256) cg_rows_codes_kernel(const uint8_t *__res
             rs[r] = form == kCgLight
                         ? make_float4(norm, n2, sigma,
                                       __fmul_rn((float)(3.14159265358979323846 / (2.0 * P.D)), gamma))
-                        : make_float4(__fmul_rn(sigma, norm), n2, 0.0f, 0.0f);
+                        : make_float4(__fmul_rn(sigma, norm), n2, sigma, norm);
         }
     }
 }

@@ -6,9 +6,10 @@
 namespace tq {
 
 enum CgForm { kCgAsym = 0, kCgSym = 1, kCgLight = 2 };  // queries / codes / codes + light QJL term
-// What the epilogue does with the products ip |a| |b|: distances; the products
-// themselves; or distances with out's own values, such products of another pass,
-// added to ip after clamping them to +-|ip| (the full QJL form's correction).
+// What the epilogue does with the products: distances; the products ip themselves,
+// times the row's first scalar but neither norm (kCgAsym); or distances with out's
+// own values, such products of another pass, added to ip after clamping them to
+// +-|ip| (kCgSym: the full QJL form's correction).
 enum CgPost { kCgDist = 0, kCgProducts = 1, kCgClampedSum = 2 };
 enum CgFmt { kCgFP16 = 0, kCgBF16 = 1 };                // 16-bit type of the hi / lo pairs
 

@@ -92,8 +92,8 @@ __device__ __forceinline__ float round_tf32(float x) {
 //   r1 = s g_a S W sgn_a,  r2 = recon_a + (p / s) g_a sgn_a,
 // which the M x N kernel takes from the codes b as they are: no planes of b.
 // Writes r1 and r2 times 2^-x (largest magnitude in [1/2, 1)) as prepared
-// queries with norms = [|a|^2, |a| 2^x].  W sgn is a sum of +-1, exact before its
-// scaling.  One warp per code.
+// queries with norms = [0, 2^x] (the vectors' own join after the clamp).  W sgn is
+// a sum of +-1, exact before its scaling.  One warp per code.
 // ---------------------------------------------------------------------------
 template <int LOG_D>
 __global__ void __launch_bounds__(256) symq_full_rows_kernel(const uint8_t *__restrict__ codes, size_t rows,
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) symq_full_rows_kernel(const uint8_t *__re
     for (size_t r = (size_t)blockIdx.x * nw + warp; r < rows; r += (size_t)gridDim.x * nw) {
         const uint8_t *c = codes + r * (size_t)P.cs;
         const float *meta = reinterpret_cast<const float *>(c + P.pb);  // 4-byte aligned
-        const float norm = meta[0], gamma = meta[1], sigma = meta[2];
+        const float gamma = meta[1], sigma = meta[2];
         const float g1 = __fmul_rn(P.scale, gamma), g2 = __fmul_rn(__fdiv_rn(p2d, P.scale), gamma);
         auto unit = [&](int i) -> unsigned {
             return P.nibble ? ((i & 1) ? c[i >> 1] >> 4 : c[i >> 1] & 15u) : c[i];
@@ -151,8 +151,8 @@ __global__ void __launch_bounds__(256) symq_full_rows_kernel(const uint8_t *__re
             o2[i] *= down;
         }
         if (lane == 0) {
-            norms[2 * r] = __fmul_rn(norm, norm);
-            norms[2 * r + 1] = __fmul_rn(norm, ldexpf(1.0f, x));
+            norms[2 * r] = 0.0f;
+            norms[2 * r + 1] = ldexpf(1.0f, x);
         }
     }
 }
