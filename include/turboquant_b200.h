@@ -257,14 +257,16 @@ tq_status tq_distance_1_to_n_symmetric_full_device(const tq_space *sp, const flo
                                                    const uint8_t *codes, size_t n, float *out,
                                                    void *stream);
 
-/* The device status word of the space's stream-ordered kernels.  Every wait in
- * the staged 1->N scan is bounded; a wait that gives up (a copy that never
- * completes) writes a non-zero code here and the kernel returns without
- * finishing its codes.  Synchronise the streams the space's *_device calls ran
- * on, then call this: it reports the code in *code (0 = none), clears it, and
- * returns TQ_ERR_TIMEOUT when it was set.  The host-pointer entry points check
- * it themselves.  No counterpart in the reference (CPU code never waits on a
- * device). */
+/* The device status of the space's stream-ordered calls.  Every wait in the staged
+ * 1->N scan and in the M x N kernel (the M x N, symmetric and QJL-corrected
+ * entry points at TQ_PRECISION_FP32) is bounded; a wait that gives up (a copy or an
+ * arrival that never comes) leaves a non-zero code here and its kernel returns
+ * without finishing its distances.  Synchronise the streams the space's *_device
+ * calls ran on, then call this: it reports the code in *code (0 = none), clears it,
+ * and returns TQ_ERR_TIMEOUT when it was set.  One call's failure does not touch
+ * another M x N call.  The calls that wait themselves return TQ_ERR_TIMEOUT: the
+ * host-pointer entry points, and the *_device ones at the other precisions.  No
+ * counterpart in the reference (CPU code never waits on a device). */
 tq_status tq_space_take_device_status(const tq_space *sp, int *code);
 
 /* Kernel timer of the 1->N scan (no counterpart in the reference: a
@@ -276,11 +278,14 @@ tq_status tq_space_take_device_status(const tq_space *sp, int *code);
 tq_status tq_space_scan_timer(tq_space *sp, int enable);
 tq_status tq_space_scan_timer_read(tq_space *sp, double *total_ms, uint64_t *launches);
 
-/* Self-test of the device-side failure path: a kernel waits, with a limit of
- * about budget_ms, on a barrier that nothing signals.  Returns TQ_ERR_TIMEOUT
- * when the wait gave up and reported it (the expected outcome; the context
- * stays usable), TQ_OK if it did not. */
+/* Self-test of the device-side failure path: kernels wait, with a limit of about
+ * budget_ms each, on a barrier that nothing signals, by the wait within a block and
+ * by that of a cluster.  Returns TQ_ERR_TIMEOUT when both gave up and reported it
+ * (the expected outcome; the context stays usable), TQ_OK if they did not. */
 tq_status tq_selftest_bounded_wait(int device, int budget_ms);
+/* The same as an M x N call of the space on device pointers: the code is left for
+ * tq_space_take_device_status. */
+tq_status tq_selftest_space_wait(const tq_space *sp, int budget_ms);
 
 /* Self-test of the M x N kernel's index arithmetic, on the host alone: the
  * largest row whose scalars the light QJL-corrected form of a call of m rows by

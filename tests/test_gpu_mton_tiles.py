@@ -168,3 +168,35 @@ def test_rows_whose_norm_overflows(cuda_ok, dim, bits, m):
         assert (~finite).any(), form
         np.testing.assert_array_equal(got[~finite], ref[~finite].astype(np.float32), err_msg=form)
         np.testing.assert_allclose(got[finite], ref[finite], rtol=1e-4, atol=1e-2, err_msg=form)
+
+
+def test_a_call_that_gave_up_does_not_touch_others(cuda_ok):
+    """A wait that ran out in one call on device arrays shows in the space's device
+    status, and nowhere else: later calls give the same distances and no error."""
+    import torch
+    from turboquant import _capi
+
+    s = tq.TurboQuantSpace(384, 4)
+    X = torch.randn(4000, 384, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    codes, q = s.encode_batch(X), X[:70].contiguous()
+    hq, hc = q.cpu().numpy(), codes.cpu().numpy()
+    rows = codes[:70].contiguous()
+
+    def results():
+        out = [s.distance_m_to_n(q, codes), s.distance_m_to_n_symmetric(rows, codes),
+               s.distance_m_to_n_symmetric_light(rows, codes), s.distance_m_to_n_symmetric_full(rows, codes)]
+        torch.cuda.synchronize()
+        out = [t.cpu().numpy() for t in out]
+        out += [s.distance_m_to_n(hq, hc), s.distance_1_to_n(hq[0], hc),
+                s.distance_m_to_n_symmetric(hc[:70], hc), s.distance_m_to_n_symmetric_full(hc[:70], hc)]
+        return out
+
+    want = results()
+    s.take_device_status()
+    assert _capi.lib().tq_selftest_space_wait(s._h, 50) == _capi.TQ_ERR_TIMEOUT
+    for a, b in zip(results(), want):
+        np.testing.assert_array_equal(a, b)
+    with pytest.raises(tq.TQError) as e:
+        s.take_device_status()
+    assert e.value.status == _capi.TQ_ERR_TIMEOUT
+    s.take_device_status()  # taken

@@ -48,18 +48,26 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 
 // Bounded wait: true when the phase completed; false after the budget ran out
 // (error recorded) or when another thread already recorded an error.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err, int code) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err, int code,
+                                          long long budget = kWaitCycles) {
     const long long t0 = clock64();
     for (uint32_t it = 1;; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((it & 1023u) == 0) {
             if (*reinterpret_cast<volatile int *>(err) != 0) return false;
-            if (clock64() - t0 > kWaitCycles) {
+            if (clock64() - t0 > budget) {
                 atomicCAS(err, 0, code);
                 return false;
             }
         }
     }
+}
+
+// Hands a call's error on to the space's status word, for calls that return before
+// their kernels (status null: the caller reads err itself).  Only for threads whose
+// wait gave up, so that a call without errors pays nothing.
+__device__ __forceinline__ void report_wait(const int *err, int *status) {
+    if (status) atomicCAS(status, 0, *reinterpret_cast<const volatile int *>(err));
 }
 
 // Bounded wait that ignores the status word: used to drain this thread's own

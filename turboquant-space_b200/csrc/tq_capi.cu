@@ -86,15 +86,18 @@ tq_status check_dev(const void *p, size_t bytes, const char *name) {
     return TQ_OK;
 }
 
-// Reads and clears the space's device status word (after the caller's
-// synchronisation); TQ_ERR_TIMEOUT when a bounded device wait gave up.
-tq_status take_status(const tq_space *sp, int *code_out) {
-    int code = 0;
-    TQ_CUDA(cudaMemcpy(&code, sp->T.status, sizeof(int), cudaMemcpyDeviceToHost), "read status");
-    if (code_out) *code_out = code;
-    if (code == 0) return TQ_OK;
-    TQ_CUDA(cudaMemset(sp->T.status, 0, sizeof(int)), "clear status");
-    return fail(TQ_ERR_TIMEOUT, "a bounded device-side wait gave up (code %d)", code);
+// Reads and clears the first `words` of the space's device status words (after the
+// caller's synchronise).  Host entry points that scan look at the scan's own; the
+// other is left to tq_space_take_device_status, since it tells of device calls that
+// another thread may have made.
+tq_status take_status(const tq_space *sp, int *code_out, int words = 1) {
+    int code[2] = {0, 0};
+    TQ_CUDA(cudaMemcpy(code, sp->T.status, words * sizeof(int), cudaMemcpyDeviceToHost), "read status");
+    const int c = code[0] ? code[0] : code[1];
+    if (code_out) *code_out = c;
+    if (c == 0) return TQ_OK;
+    TQ_CUDA(cudaMemset(sp->T.status, 0, words * sizeof(int)), "clear status");
+    return fail(TQ_ERR_TIMEOUT, "a bounded device-side wait gave up (code %d)", c);
 }
 
 tq_status check_codes_align(const void *p, const char *name) {
@@ -153,10 +156,12 @@ class MtonRunner {
     }
 
     // n: all the columns of the call (run_cols may take them in parts)
-    MtonRunner(tq_space *sp, bool sym, tq_precision prec, size_t m, size_t n)
+    // host: the caller waits for the call and asks finish() for its errors
+    MtonRunner(tq_space *sp, bool sym, tq_precision prec, size_t m, size_t n, bool host)
         : sp_(sp), sym_(sym), prec_(prec), m_(m) {
         bf16_ = prec == TQ_PRECISION_SPLIT_BF16 || prec == TQ_PRECISION_SPLIT_BF16_DECODED;
         cg_ = bf16_ || (prec == TQ_PRECISION_FP32 && use_cg(n));
+        wait_ = cg_ && (bf16_ || host);
     }
 
     tq_status prepare_rows(const void *rows_dev, cudaStream_t s) {
@@ -193,10 +198,7 @@ class MtonRunner {
         r_.hi = base;
         r_.lo = base + plane;
         r_.rs = reinterpret_cast<float4 *>(base + 2 * plane);
-        if (bf16_) {  // reported by finish(); FP32 is stream-ordered and reports through the status word
-            err_ = reinterpret_cast<int *>(r_.rs + m_);
-            TQ_CUDA(cudaMemsetAsync(err_, 0, sizeof(int), s), "memset");
-        }
+        r_.err = reinterpret_cast<int *>(r_.rs + m_);
         if (!sym_)
             TQ_CUDA(tq::launch_cg_rows_prepared(sp_->P, q_rot_, s_q_, norms_, m_, fmt(), r_, s), "row planes");
         else
@@ -210,7 +212,7 @@ class MtonRunner {
             return fail(TQ_ERR_NOT_SUPPORTED, "decoded split-BF16 tiles need 16-byte aligned device codes");
         if (cg_)
             TQ_CUDA(tq::launch_cgemm(sp_->P, sp_->T, form(), fmt(), r_, m_, codes, n, out, ldo,
-                                     err_ ? err_ : sp_->T.status, s),
+                                     wait_ ? nullptr : sp_->T.status + 1, s),
                     "tcgen05 M x N kernel");
         else if (!sym_ && prec_ == TQ_PRECISION_REFERENCE)
             TQ_CUDA(tq::launch_exact_mton(sp_->P, sp_->T.centroids, q_rot_, s_q_, norms_, m_, codes,
@@ -230,17 +232,16 @@ class MtonRunner {
         return TQ_OK;
     }
 
-    // Reports a bounded wait that gave up inside the split-BF16 kernel.
+    // Reports a bounded wait that gave up inside the tensor-core kernel.  FP32 device
+    // calls are stream-ordered and report through the space's status word instead.
     tq_status finish(cudaStream_t s) {
-        if (!err_) return TQ_OK;
+        if (!wait_) return TQ_OK;
         int h = 0;
-        TQ_CUDA(cudaMemcpyAsync(&h, err_, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H status");
+        TQ_CUDA(cudaMemcpyAsync(&h, r_.err, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H status");
         TQ_CUDA(cudaStreamSynchronize(s), "sync");
         if (h != 0) return fail(TQ_ERR_TIMEOUT, "tensor-core kernel: a pipeline wait timed out (code %d)", h);
         return TQ_OK;
     }
-    // The space's status word carries this call's errors (host entry points read it).
-    bool uses_status_word() const { return cg_ && !err_; }
 
   private:
     // Code size up to which SPLIT_BF16_DECODED is offered: a tile of 128 codes
@@ -259,14 +260,13 @@ class MtonRunner {
     int form() const { return sym_ ? tq::kCgSym : tq::kCgAsym; }
     int fmt() const { return bf16_ ? tq::kCgBF16 : tq::kCgFP16; }
     tq_space *sp_;
-    bool sym_, bf16_ = false, cg_ = false;
+    bool sym_, bf16_ = false, cg_ = false, wait_ = false;
     tq_precision prec_;
     size_t m_;
     Scratch prep_, rows_;
     float *q_rot_ = nullptr, *s_q_ = nullptr, *norms_ = nullptr;
     const uint8_t *codes_a_ = nullptr;
     tq::CgRows r_;
-    int *err_ = nullptr;
 };
 
 }  // namespace
@@ -628,7 +628,7 @@ tq_status tq_space_take_device_status(const tq_space *sp, int *code) {
     tq_status st = need_device(sp);
     if (st != TQ_OK) return st;
     DeviceGuard g(sp->device);
-    return take_status(sp, code);
+    return take_status(sp, code, 2);
 }
 
 tq_status tq_selftest_mton_rows(const tq_space *sp, size_t m, size_t n, size_t *last_row) {
@@ -740,7 +740,7 @@ tq_status tq_distance_m_to_n_device(const tq_space *sp, const float *queries, si
     const size_t mchunk = MtonRunner::row_chunk(sp, false);
     for (size_t m0 = 0; m0 < m; m0 += mchunk) {
         const size_t mc = std::min(mchunk, m - m0);
-        MtonRunner r(const_cast<tq_space *>(sp), false, precision, mc, n);
+        MtonRunner r(const_cast<tq_space *>(sp), false, precision, mc, n, false);
         if ((st = r.prepare_rows(queries + m0 * sp->dim, s)) != TQ_OK) return st;
         if ((st = r.run_cols(codes, n, out + m0 * n, n, s)) != TQ_OK) return st;
         if ((st = r.finish(s)) != TQ_OK) return st;
@@ -765,7 +765,7 @@ tq_status tq_distance_m_to_n_symmetric_device(const tq_space *sp, const uint8_t 
     const size_t mchunk = MtonRunner::row_chunk(sp, true);
     for (size_t m0 = 0; m0 < m; m0 += mchunk) {
         const size_t mc = std::min(mchunk, m - m0);
-        MtonRunner r(const_cast<tq_space *>(sp), true, precision, mc, n);
+        MtonRunner r(const_cast<tq_space *>(sp), true, precision, mc, n, false);
         if ((st = r.prepare_rows(A + m0 * sp->code_size, s)) != TQ_OK) return st;
         if ((st = r.run_cols(B, n, out + m0 * n, n, s)) != TQ_OK) return st;
         if ((st = r.finish(s)) != TQ_OK) return st;
@@ -931,7 +931,7 @@ tq_status mton_host(tq_space *sp, bool sym, tq_precision prec, const void *rows_
     Scratch rows;
     TQ_CUDA(rows.alloc(row_bytes, sc), "cudaMallocAsync(rows)");
     TQ_CUDA(cudaMemcpyAsync(rows.p, rows_host, row_bytes, cudaMemcpyHostToDevice, sc), "H2D rows");
-    MtonRunner runner(sp, sym, prec, m, n);
+    MtonRunner runner(sp, sym, prec, m, n, true);
     tq_status st = runner.prepare_rows(rows.p, sc);
     if (st != TQ_OK) return st;
     const size_t cbytes = (per * cs + 15) & ~size_t(15);
@@ -976,7 +976,6 @@ tq_status mton_host(tq_space *sp, bool sym, tq_precision prec, const void *rows_
         if (e != cudaSuccess && result == TQ_OK) result = cuda_fail(e, "m_to_n");
     }
     if (result == TQ_OK) result = runner.finish(sc);
-    if (result == TQ_OK && runner.uses_status_word()) result = take_status(sp, nullptr);
     for (int k = 0; k < 2; ++k) {
         cudaEventDestroy(uploaded[k]);
         cudaEventDestroy(computed[k]);
@@ -1042,7 +1041,7 @@ constexpr size_t kCorrSlice = 32768;  // rows whose correction is prepared at a 
 struct SymqRunner {
     const tq_space *sp;
     int mode, ldk1, ldk2;
-    bool tc;
+    bool tc, host;
     int K1p = 0, K2p = 0;
     size_t m = 0, m_pad = 0, per = 0;
     Scratch rows, cols, rows_bf, cols_bf;
@@ -1052,8 +1051,9 @@ struct SymqRunner {
     bool cg = false;
     tq::CgRows cgr, corr;  // the light form's or the full form's MSE rows; the full form's correction
 
-    SymqRunner(const tq_space *s, int md, bool split_tf32 = false)
-        : sp(s), mode(md), tc(split_tf32 && s->D >= 64) {
+    // on_host: the caller waits for the call and asks finish() for its errors
+    SymqRunner(const tq_space *s, int md, bool split_tf32 = false, bool on_host = false)
+        : sp(s), mode(md), tc(split_tf32 && s->D >= 64), host(on_host) {
         ldk1 = tq::symq_ldk((int)s->D);
         ldk2 = tq::symq_ldk(tq::symq_k2(md, (int)s->D));
         K1p = (int)sq_round_up((size_t)ldk1, 32);
@@ -1092,10 +1092,8 @@ struct SymqRunner {
         cgr.hi = base;
         cgr.lo = base + plane;
         cgr.rs = reinterpret_cast<float4 *>(base + 2 * plane);
-        if (tc) {  // reported by finish(), as the TF32 kernel's; otherwise stream-ordered
-            err = reinterpret_cast<int *>(cgr.rs + m);
-            TQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s), "memset");
-        }
+        cgr.err = reinterpret_cast<int *>(cgr.rs + m);
+        if (tc || host) err = cgr.err;  // reported by finish(), as the TF32 kernel's; otherwise stream-ordered
         TQ_CUDA(tq::launch_cg_rows_codes(sp->P, sp->T, A, m, tq::kCgLight, tq::kCgFP16, cgr, s), "row planes");
         return TQ_OK;
     }
@@ -1109,7 +1107,7 @@ struct SymqRunner {
         // the correction's FP32 rows live for a slice of the rows at a time
         const size_t slice = std::min(m, kCorrSlice), K = tq::cg_row_k(sp->P, tq::kCgAsym);
         const size_t vec = sizeof(float) * slice * sp->D;  // D >= 16: every part a multiple of 16 bytes
-        TQ_CUDA(rows.alloc(2 * (kc + km) + 2 * m * sizeof(float4), s), "cudaMallocAsync(row planes)");
+        TQ_CUDA(rows.alloc(2 * (kc + km) + 2 * m * sizeof(float4) + sizeof(int), s), "cudaMallocAsync(row planes)");
         TQ_CUDA(rows_bf.alloc(2 * vec + 2 * sizeof(float) * slice, s), "cudaMallocAsync(correction rows)");
         auto *base = static_cast<unsigned char *>(rows.p);
         corr.hi = base;
@@ -1118,6 +1116,8 @@ struct SymqRunner {
         cgr.lo = base + 2 * kc + km;
         cgr.rs = reinterpret_cast<float4 *>(base + 2 * (kc + km));
         corr.rs = cgr.rs + m;
+        cgr.err = corr.err = reinterpret_cast<int *>(corr.rs + m);
+        if (host) err = cgr.err;
         float *q = static_cast<float *>(rows_bf.p), *sq = q + slice * sp->D, *norms = sq + slice * sp->D;
         for (size_t r0 = 0; r0 < m; r0 += slice) {
             const size_t nr = std::min(slice, m - r0);
@@ -1132,8 +1132,6 @@ struct SymqRunner {
         TQ_CUDA(tq::launch_cg_rows_codes(sp->P, sp->T, A, m, tq::kCgSym, tq::kCgFP16, cgr, s), "row planes");
         return TQ_OK;
     }
-    // The space's status word carries this call's errors (host entry points read it).
-    bool uses_status_word() const { return cg && !err; }
     // The row planes straight into hi/lo TF32 pairs (m_pad x K1p, m_pad x
     // K2p); the light variant's sign plane is exact and has no lo plane.
     tq_status prepare_rows_tc(const uint8_t *A, size_t rows_, cudaStream_t s) {
@@ -1163,16 +1161,16 @@ struct SymqRunner {
     tq_status run_cols(const uint8_t *B, size_t n, float *out, size_t ldo, cudaStream_t s) {
         if (cg && !light()) {
             TQ_CUDA(tq::launch_cgemm(sp->P, sp->T, tq::kCgAsym, tq::kCgFP16, corr, m, B, n, out, ldo,
-                                     sp->T.status, s, tq::kCgProducts),
+                                     err ? nullptr : sp->T.status + 1, s, tq::kCgProducts),
                     "tcgen05 correction kernel");
             TQ_CUDA(tq::launch_cgemm(sp->P, sp->T, tq::kCgSym, tq::kCgFP16, cgr, m, B, n, out, ldo,
-                                     sp->T.status, s, tq::kCgClampedSum),
+                                     err ? nullptr : sp->T.status + 1, s, tq::kCgClampedSum),
                     "tcgen05 full symmetric kernel");
             return TQ_OK;
         }
         if (cg) {
             TQ_CUDA(tq::launch_cgemm(sp->P, sp->T, tq::kCgLight, tq::kCgFP16, cgr, m, B, n, out, ldo,
-                                     err ? err : sp->T.status, s),
+                                     err ? nullptr : sp->T.status + 1, s),
                     "tcgen05 light symmetric kernel");
             return TQ_OK;
         }
@@ -1336,7 +1334,7 @@ tq_status tq_distance_m_to_n_symmetric_qjl(const tq_space *csp, const uint8_t *c
     Scratch dA;
     TQ_CUDA(dA.alloc(m * cs, s), "cudaMallocAsync(codes_a)");
     TQ_CUDA(cudaMemcpyAsync(dA.p, codes_a, m * cs, cudaMemcpyHostToDevice, s), "H2D codes_a");
-    SymqRunner r(sp, mode, precision == TQ_PRECISION_SPLIT_TF32);
+    SymqRunner r(sp, mode, precision == TQ_PRECISION_SPLIT_TF32, true);
     r.choose(nullptr, nullptr);  // staging buffers of our own, aligned
     if ((st = r.prepare_rows(static_cast<uint8_t *>(dA.p), m, s)) != TQ_OK) return st;
     size_t per = std::max<size_t>(1, std::min(kChunkBytes / cs, (kChunkBytes * 2) / (4 * m)));
@@ -1354,7 +1352,6 @@ tq_status tq_distance_m_to_n_symmetric_qjl(const tq_space *csp, const uint8_t *c
                 "D2H distances");
     }
     TQ_CUDA(cudaStreamSynchronize(s), "distance_m_to_n_symmetric (QJL)");
-    if (r.uses_status_word()) return take_status(sp, nullptr);
     return r.finish(s);
 }
 

@@ -116,7 +116,7 @@ struct CgArgs {
     float undo_c, undo_s;  // undo the operand scalings of the two parts
     float *out;
     size_t ldo;
-    int *err;
+    int *err, *status;   // the call's error word, and the space's (may be null)
 };
 
 // The K blocks of a tile in the order they run: the asymmetric form's sign part
@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
     const uint32_t tmem_base = *tmem_slot;
     const int KB = p.KB;
     const CgOrder<LIGHT> ord(p);
+    bool ok = true;  // no wait of this thread's has given up
     // tiles of this CTA (or pair): t0, t0 + grid, ...; this CTA's first code of tile t
     const unsigned grid = PAIR ? gridDim.x >> 1 : gridDim.x, t0 = PAIR ? blockIdx.x >> 1 : blockIdx.x;
     auto first_code = [&](unsigned t) {
@@ -298,7 +299,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             if (lane == 0) {
                 uint32_t s = 0, ph = 1;
                 uint32_t it = 0;
-                bool ok = true;
                 for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
                     const int row = (int)((t / p.num_nt) * p.NT + rank * (p.NT / 2));
                     for (int kb = 0; kb < KB; ++kb, ++it) {
@@ -319,7 +319,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         } else if (warp == 1 && rank != 0) {
             // ---------------- PAIR, rank 1: reports each full stage to rank 0 ----------------
             uint32_t s = 0, ph = 0;
-            bool ok = true;
             for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
                 for (int kb = 0; kb < KB; ++kb) {
                     if (!mbar_wait_warp(full0 + 8 * s, ph, p.err, kErrFull)) { ok = false; break; }
@@ -342,7 +341,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             const uint32_t dk = SPLIT ? (uint32_t)p.NT : 0u;  // quarter kk's accumulator: d + kk dk
             const uint32_t ab = CG_A_BYTES >> 4, bb = (uint32_t)bt_bytes >> 4;
             uint32_t s = 0, ph = 0, gc = 0;
-            bool ok = true;
             for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
                 for (int c0 = 0, c1 = 0; c0 < KB && ok; c0 = c1, ++gc) {
                     c1 = ord.chunk_end(p, c0);
@@ -402,7 +400,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             // proxy fence waits for its own loads in flight.
             const int r0 = (warp - 2) * 64 + (lane >> 3), c = lane & 7;
             uint32_t cs = 0, cph = 1;
-            bool ok = true;
             for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
                 const size_t j0 = min(first_code(t), p.n - 1);
                 const uint8_t *base = p.codes + j0 * (size_t)p.cs;
@@ -459,7 +456,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         // counts are 2 or more)
         const uint32_t group = GROUPS == 2 ? (uint32_t)(warp - 4) >> 2 : 0u;
         uint32_t s = group, ph = 1, cs = group, cph = 0, it = 0;
-        bool ok = true;
         for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
             for (int kb = 0; kb < KB; ++kb, ++it) {
                 if (GROUPS == 2 && (it & 1u) != group) continue;
@@ -528,7 +524,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
         const uint32_t lanes = tmem_base + ((uint32_t)(32 * quad) << 16) + (uint32_t)(half * cpt);
         float y[CPT];
         uint32_t gc = 0;
-        bool ok = true;
         for (unsigned t = t0; t < p.num_tiles && ok; t += grid) {
             const size_t row = first_code(t) + 32 * quad + lane;
             const size_t col0 = (size_t)(t / p.num_nt) * p.NT + half * cpt;
@@ -634,6 +629,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
             }
         }
     }
+    if (!ok) report_wait(p.err, p.status);
     tc_fence_before();
     // PAIR: no CTA leaves while the other may still arrive on its barriers or
     // read its shared memory
@@ -659,7 +655,8 @@ __device__ __forceinline__ void put4(const float (&v)[4], int fmt, __nv_bfloat16
 __global__ void __launch_bounds__(256) cg_rows_prepared_kernel(
     const float *__restrict__ q_rot, const float *__restrict__ s_q, const float *__restrict__ norms,
     size_t m, int D, int KBm, int fmt, __nv_bfloat16 *__restrict__ ph, __nv_bfloat16 *__restrict__ pl,
-    float4 *__restrict__ rs) {
+    float4 *__restrict__ rs, int *__restrict__ err) {
+    if (err && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     const int half = KBm * CG_BK, K = 2 * half, quads = K / 4;
     const size_t total = m * (size_t)quads;
     const float f = fmt == kCgFP16 ? kRowScale : 1.0f;
@@ -683,7 +680,8 @@ __global__ void __launch_bounds__(256) cg_rows_codes_kernel(const uint8_t *__res
                                                             Params P, DevTables T, int KBm, int form,
                                                             int fmt, __nv_bfloat16 *__restrict__ ph,
                                                             __nv_bfloat16 *__restrict__ pl,
-                                                            float4 *__restrict__ rs) {
+                                                            float4 *__restrict__ rs, int *__restrict__ err) {
+    if (err && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     const int half = KBm * CG_BK, K = form == kCgLight ? 2 * half : half, quads = K / 4;
     const size_t total = m * (size_t)quads;
     const float f = P.cent_scale[fmt];
@@ -775,7 +773,7 @@ cudaError_t launch_cg_rows_prepared(const Params &P, const float *q_rot, const f
     const int KBm = (P.D + CG_BK - 1) / CG_BK;
     cg_rows_prepared_kernel<<<rows_grid(m * (size_t)KBm * 32), 256, 0, st>>>(
         q_rot, s_q, norms, m, P.D, KBm, fmt, static_cast<__nv_bfloat16 *>(r.hi),
-        static_cast<__nv_bfloat16 *>(r.lo), r.rs);
+        static_cast<__nv_bfloat16 *>(r.lo), r.rs, r.err);
     return cudaGetLastError();
 }
 
@@ -784,7 +782,7 @@ cudaError_t launch_cg_rows_codes(const Params &P, const DevTables &T, const uint
     const int KBm = (P.D + CG_BK - 1) / CG_BK;
     cg_rows_codes_kernel<<<rows_grid(m * (size_t)KBm * 32), 256, 0, st>>>(
         codes, m, P, T, KBm, form, fmt, static_cast<__nv_bfloat16 *>(r.hi),
-        static_cast<__nv_bfloat16 *>(r.lo), r.rs);
+        static_cast<__nv_bfloat16 *>(r.lo), r.rs, r.err);
     return cudaGetLastError();
 }
 
@@ -813,11 +811,11 @@ int cg_tile_cols(const Params &P, int form, size_t m, size_t n) {
 }
 
 cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt, const CgRows &rows,
-                         size_t m, const uint8_t *codes, size_t n, float *out, size_t ldo, int *err,
+                         size_t m, const uint8_t *codes, size_t n, float *out, size_t ldo, int *status,
                          cudaStream_t st, int post) {
     if (m == 0 || n == 0) return cudaSuccess;
     if (P.cs % 4 || (reinterpret_cast<uintptr_t>(codes) & 3)) return cudaErrorMisalignedAddress;
-    if (!aligned16({rows.hi, rows.lo, rows.rs})) return cudaErrorMisalignedAddress;
+    if (!aligned16({rows.hi, rows.lo, rows.rs}) || !rows.err) return cudaErrorMisalignedAddress;
     CgArgs a{};
     a.codes = codes;
     a.n = n;
@@ -854,7 +852,8 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     a.undo_c = 1.0f / (a.cent * (form != kCgAsym ? a.cent : fmt == kCgFP16 ? kRowScale : 1.0f));
     a.out = out;
     a.ldo = ldo;
-    a.err = err;
+    a.err = rows.err;
+    a.status = status;
     a.NT = cg_tile_cols(P, form, m, n);
     const bool split = fmt == kCgFP16 && m < 32 && a.NT <= 32;
     const bool pair = a.NT > 64;

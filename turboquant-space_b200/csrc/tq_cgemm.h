@@ -14,10 +14,12 @@ enum CgPost { kCgDist = 0, kCgProducts = 1, kCgClampedSum = 2 };
 enum CgFmt { kCgFP16 = 0, kCgBF16 = 1 };                // 16-bit type of the hi / lo pairs
 
 // The row operand: hi and lo planes of m x cg_row_k 16-bit values and four
-// scalars a row, all 16-byte aligned.
+// scalars a row, all 16-byte aligned, and the error word of the call that they
+// belong to: a word of its own, since a wait gives up as soon as it sees a set one.
 struct CgRows {
     void *hi = nullptr, *lo = nullptr;
     float4 *rs = nullptr;
+    int *err = nullptr;
 };
 size_t cg_row_k(const Params &P, int form);
 
@@ -43,7 +45,8 @@ inline int cg_tile_parts(int cols) { return cols > 64 ? 2 : 1; }
 // products of the centroids' pairs (without lo lo) have the least bias and error.
 float cg_cent_scale(const float *centroids, int levels, int fmt);
 
-// Prepared queries (kCgAsym) or codes (kCgSym, kCgLight) -> row operand.
+// Prepared queries (kCgAsym) or codes (kCgSym, kCgLight) -> row operand; *r.err = 0
+// (r.err null: left alone).
 cudaError_t launch_cg_rows_prepared(const Params &P, const float *q_rot, const float *s_q,
                                     const float *norms, size_t m, int fmt, const CgRows &r,
                                     cudaStream_t st);
@@ -51,10 +54,10 @@ cudaError_t launch_cg_rows_codes(const Params &P, const DevTables &T, const uint
                                  int form, int fmt, const CgRows &r, cudaStream_t st);
 
 // out[i * ldo + j] = distance of row i to code j.  Codes 4-byte aligned, the
-// code size a multiple of 4 (every padded dim but 4).  `err` (device int) is
-// set non-zero if a bounded wait in the kernel gave up.
+// code size a multiple of 4 (every padded dim but 4).  *rows.err is set non-zero if
+// a bounded wait in the kernel gave up, and *status (device int, may be null) with it.
 cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt, const CgRows &rows,
-                         size_t m, const uint8_t *codes, size_t n, float *out, size_t ldo, int *err,
+                         size_t m, const uint8_t *codes, size_t n, float *out, size_t ldo, int *status,
                          cudaStream_t st, int post = kCgDist);
 
 }  // namespace tq

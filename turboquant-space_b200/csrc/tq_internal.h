@@ -56,7 +56,8 @@ struct DevTables {
                               // bucket (P.qflag); otherwise a copy of qlut
     const uint32_t *rot_mask; // [D/32 rounded up]: bit i set <=> rot sign +1
     const uint32_t *qjl_mask; // [D/32 rounded up]
-    int *status;              // stream-ordered kernels' error word (0 = ok)
+    int *status;              // stream-ordered kernels' error words (0 = ok): [0] the 1 -> N scan's,
+                              // [1] the M x N kernel's device calls'
 };
 
 // ---- kernel launchers (tq_kernels.cu); all stream-ordered -------------------

@@ -116,9 +116,11 @@ cudaError_t launch_tc_symq(const void *A1h, const void *A1l, const void *B1h, co
                            size_t n_pad, const float *sa, const float *sb, float *out, size_t ldo,
                            int *err, cudaStream_t st);
 
-// One thread waits on an mbarrier nothing arrives at; after budget_cycles the
-// wait gives up and writes a non-zero code to *err (the failure path of every
-// bounded wait in the tensor-core kernels).
-cudaError_t launch_bounded_wait_selftest(int *err, long long budget_cycles, cudaStream_t st);
+// One thread waits on an mbarrier nothing arrives at, by the wait within a CTA or
+// that of a cluster; after budget_cycles the wait gives up and writes a non-zero
+// code to *err and, if it is not null, *status (the failure path of every bounded
+// wait in the tensor-core kernels).
+cudaError_t launch_bounded_wait_selftest(int *err, int *status, bool cluster, long long budget_cycles,
+                                         cudaStream_t st);
 
 }  // namespace tq

@@ -708,6 +708,31 @@ void worker_loop(tq_server *sv) {
 
 }  // namespace
 
+namespace {
+
+// Both forms of the bounded wait, one after the other, on an error word of their own
+// and `status` (may be null).  Each must give up.
+tq_status bounded_wait_selftest(int device, int *status, int budget_ms) {
+    if (budget_ms < 1 || budget_ms > 10000) return fail(TQ_ERR_INVALID_ARGUMENT, "budget_ms must be in 1..10000");
+    int clock_khz = 0;
+    cudaDeviceGetAttribute(&clock_khz, cudaDevAttrClockRate, device);
+    if (clock_khz <= 0) clock_khz = 2000000;
+    int *err = nullptr, h[2] = {0, 0};
+    TQ_CUDA(cudaMalloc(&err, 2 * sizeof(int)), "cudaMalloc");
+    cudaError_t e = cudaMemset(err, 0, 2 * sizeof(int));
+    for (int form = 0; form < 2 && e == cudaSuccess; ++form)
+        e = tq::launch_bounded_wait_selftest(err + form, status, form == 1, (long long)clock_khz * budget_ms, nullptr);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(h, err, sizeof(h), cudaMemcpyDeviceToHost);
+    cudaFree(err);
+    if (e != cudaSuccess) return cuda_fail(e, "bounded-wait self-test");
+    if (h[0] != 0 && h[1] != 0)
+        return fail(TQ_ERR_TIMEOUT, "device waits gave up after ~%d ms each (codes %d, %d)", budget_ms, h[0], h[1]);
+    return TQ_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n, int codes_on_device,
@@ -1053,22 +1078,15 @@ tq_status tq_selftest_bounded_wait(int device, int budget_ms) {
         return fail(TQ_ERR_NO_DEVICE, "no CUDA device");
     }
     if (device < 0) cudaGetDevice(&device);
-    if (budget_ms < 1 || budget_ms > 10000) return fail(TQ_ERR_INVALID_ARGUMENT, "budget_ms must be in 1..10000");
     DeviceGuard g(device);
-    int clock_khz = 0;
-    cudaDeviceGetAttribute(&clock_khz, cudaDevAttrClockRate, device);
-    if (clock_khz <= 0) clock_khz = 2000000;
-    int *err = nullptr;
-    TQ_CUDA(cudaMalloc(&err, sizeof(int)), "cudaMalloc");
-    cudaError_t e = cudaMemset(err, 0, sizeof(int));
-    if (e == cudaSuccess) e = tq::launch_bounded_wait_selftest(err, (long long)clock_khz * budget_ms, nullptr);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    int h = 0;
-    if (e == cudaSuccess) e = cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost);
-    cudaFree(err);
-    if (e != cudaSuccess) return cuda_fail(e, "bounded-wait self-test");
-    if (h != 0) return fail(TQ_ERR_TIMEOUT, "device wait gave up after ~%d ms (code %d)", budget_ms, h);
-    return TQ_OK;
+    return bounded_wait_selftest(device, nullptr, budget_ms);
+}
+
+tq_status tq_selftest_space_wait(const tq_space *sp, int budget_ms) {
+    if (!sp) return fail(TQ_ERR_INVALID_ARGUMENT, "NULL space");
+    if (sp->device < 0) return fail(TQ_ERR_NO_DEVICE, "no CUDA device");
+    DeviceGuard g(sp->device);
+    return bounded_wait_selftest(sp->device, sp->T.status + 1, budget_ms);
 }
 
 void tq_server_destroy(tq_server *sv) {

@@ -1317,24 +1317,20 @@ __global__ void __launch_bounds__(256) topk_merge_kernel(const int *__restrict__
     }
 }
 
-// Self-test of the bounded wait: one thread waits on an mbarrier that nothing
-// arrives at, with a budget of `budget_cycles`; the wait must give up and
-// record kErrSelfTest in *err instead of hanging.
+// Self-test of the bounded waits: one thread waits on an mbarrier that nothing
+// arrives at, with a budget of `budget_cycles`, by the loop of the kernels' waits in
+// one CTA or in a cluster; the wait must give up and record kErrSelfTest in *err,
+// and in *status (may be null), instead of hanging.
 constexpr int kErrSelfTest = 9;
-__global__ void bounded_wait_selftest_kernel(int *err, long long budget_cycles) {
+__global__ void bounded_wait_selftest_kernel(int *err, int *status, bool cluster, long long budget_cycles) {
     __shared__ __align__(8) uint64_t bar;
     if (threadIdx.x != 0) return;
     const uint32_t b = smem_u32(&bar);
     mbar_init(b, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    const long long t0 = clock64();
-    for (uint32_t it = 1;; ++it) {
-        if (mbar_try_wait(b, 0)) return;  // cannot happen: no arrival
-        if ((it & 255u) == 0 && clock64() - t0 > budget_cycles) {
-            atomicCAS(err, 0, kErrSelfTest);
-            return;
-        }
-    }
+    mbar_init_fence();
+    const bool ok = cluster ? mbar_wait_cluster(b, 0, err, kErrSelfTest, budget_cycles)
+                            : mbar_wait(b, 0, err, kErrSelfTest, budget_cycles);
+    if (!ok) report_wait(err, status);
 }
 
 // FP32 planes (TF32 operands): K x rows, 32-value (128-byte) boxes, 128-byte swizzle.
@@ -1440,8 +1436,9 @@ bool tc_topk_shape(int variant, int out[4]) {
     return true;
 }
 
-cudaError_t launch_bounded_wait_selftest(int *err, long long budget_cycles, cudaStream_t st) {
-    bounded_wait_selftest_kernel<<<1, 32, 0, st>>>(err, budget_cycles);
+cudaError_t launch_bounded_wait_selftest(int *err, int *status, bool cluster, long long budget_cycles,
+                                         cudaStream_t st) {
+    bounded_wait_selftest_kernel<<<1, 32, 0, st>>>(err, status, cluster, budget_cycles);
     return cudaGetLastError();
 }
 

@@ -137,7 +137,8 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // As mbar_wait, for a barrier that the other CTA of the cluster arrives on.
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int *err, int code) {
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int *err, int code,
+                                                  long long budget = kWaitCycles) {
     const long long t0 = clock64();
     for (uint32_t it = 1;; ++it) {
         uint32_t ok;
@@ -151,7 +152,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
         if (ok) return true;
         if ((it & 1023u) == 0) {
             if (*reinterpret_cast<volatile int *>(err) != 0) return false;
-            if (clock64() - t0 > kWaitCycles) {
+            if (clock64() - t0 > budget) {
                 atomicCAS(err, 0, code);
                 return false;
             }

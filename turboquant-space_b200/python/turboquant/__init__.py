@@ -417,6 +417,13 @@ class TurboQuantSpace:
         check(lib().tq_distance_1_to_n(self._h, _ptr(q), _ptr(c), n, _ptr(out)))
         return out
 
+    def take_device_status(self):
+        """Raises TQError if a kernel of this space's calls on device arrays gave up on
+        one of its bounded waits since the last look, and left distances unfinished.
+        Such calls return before their kernels have run: synchronise their streams
+        first.  (Calls on host arrays raise it themselves.)"""
+        _capi.check(_capi.lib().tq_space_take_device_status(self._h, None))
+
     def distance_m_to_n(self, queries, codes, precision="fp32", out=None):
         """distanceBatchMToN: queries [m, dim] float32 x codes [n, cs] -> [m, n].
 
