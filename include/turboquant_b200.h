@@ -287,6 +287,10 @@ tq_status tq_selftest_bounded_wait(int device, int budget_ms);
  * tq_space_take_device_status. */
 tq_status tq_selftest_space_wait(const tq_space *sp, int budget_ms);
 
+/* Self-test of the serving filter's error bound, on the host alone: the share of
+ * sum |terms| that it allows for the FP32 sums of the exact stage. */
+tq_status tq_selftest_filter_sums(const tq_space *sp, float *share);
+
 /* Self-test of the M x N kernel's index arithmetic, on the host alone: the
  * largest row whose scalars the light QJL-corrected form of a call of m rows by
  * n codes reads, over all tiles of the call.  Below m, or the kernel would read

@@ -172,3 +172,33 @@ def test_mton_row_scalar_reads_stay_in_range(dim, bits):
                   640, 641, 1025, 1100):
             _capi.check(_capi.lib().tq_selftest_mton_rows(s._h, m, n, ctypes.byref(last)))
             assert last.value == m - 1, (m, n, last.value)
+
+
+def _chain_error(terms, lanes):
+    """FP32 sums of `lanes` running sums over the terms, relative to sum |terms|."""
+    t = terms.reshape(-1, lanes)
+    acc = np.zeros(lanes, np.float32)
+    for row in t:  # an FMA each: one rounding of the exact product plus the sum
+        acc = (acc.astype(np.float64) + row).astype(np.float32)
+    while acc.size > 1:
+        acc = acc[:acc.size // 2] + acc[acc.size // 2:]
+    return abs(float(acc[0]) - terms.sum()) / np.abs(terms).sum()
+
+
+@pytest.mark.parametrize("dim,bits", [(64, 4), (64, 8), (512, 4), (512, 8), (2048, 4), (2048, 8), (8192, 8)])
+def test_filter_bound_covers_the_exact_stage_sums(dim, bits):
+    """The serving filter's bound must cover the roundings of the exact stage's
+    running sums, 8 over byte codes and 32 over pairs of nibble codes.  Equal terms
+    whose low bits are just under half an ulp of the sum lose them at every add."""
+    s = tq.TurboQuantSpace(dim, bits)
+    share = ctypes.c_float()
+    _capi.check(_capi.lib().tq_selftest_filter_sums(s._h, ctypes.byref(share)))
+    lanes, steps = (32, dim // 64) if bits <= 4 else (8, dim // 8)
+    worst = 0.0
+    for cut in range(1, 16):
+        term = 1.0 + 2.0 ** -cut - 2.0 ** -26
+        low = np.float32(term)  # and one that loses half an ulp of the last binade's sums
+        step = 2.0 ** -23 * 2.0 ** int(np.log2(max(2, steps)))
+        for x in (float(low), 1.0 + 0.49 * step, 1.0 + 0.245 * step):
+            worst = max(worst, _chain_error(np.full(lanes * steps, x), lanes))
+    assert worst <= share.value, (worst, share.value)

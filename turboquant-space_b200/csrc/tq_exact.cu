@@ -383,11 +383,12 @@ struct RescoreArgs {
 // dropped lo*lo product and the pairs' residuals are below 3 * 2^-16 |a_i b_i|;
 // each 16-deep MMA step is assumed to add at most 2^-20 (|acc| + sum |p|), and
 // a chunk of at most 8 K blocks issues at most 96 MMAs into one accumulator
-// from zero (96 * 2^-20 of the chunk's |terms|); promotions, the planes' FP32
-// roundings and the reference's own FP32 sums (chains of at most D/64 + 8
-// adds) add a few 1e-7.  Their sum, 1.4e-4, is taken as kappa = 2.5e-4 of
-// sum_i |terms| (a pass with more MMAs per accumulator, as the whole-K
-// variant, brings a kappa grown with their count: tc_topk_kappa), and
+// from zero (96 * 2^-20 of the chunk's |terms|); promotions and the planes' FP32
+// roundings add a few 1e-7.  Their sum, 1.4e-4, is taken as kappa = 2.5e-4 of
+// sum_i |terms| (a pass with more MMAs per accumulator, as the whole-K variant,
+// brings a kappa grown with their count: tc_topk_kappa); its slack covers the
+// reference's own FP32 sums, chains of D/64 + 8 adds for nibble codes and D/8 + 8
+// for byte codes (6.2e-5 at D = 8192).  And
 //   sum_i |terms| <= |q| (cmax sigma_j |x_j| sum|q_rot| + scale gamma_j |x_j| sum|s_q|),
 // bounded with the index-wide maxima of sigma |x| and scale gamma |x|.  The
 // distance epilogues of both sides add kKappaEpi (|q|^2 + max |x|^2), and a
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(256) rescore_kernel(RescoreArgs a) {
                         M3 = a.filter.bound[3];
             const float e = w.x * M0 + 1.0001f * M1 + w.y * M2 + w.w * M3 +
                             (float)(a.filter.mmas + 1) * (1.0f / 1048576.0f) * (w.z * M0 + w.w * (M2 + M3)) +
-                            2e-6f * (M0 + M2);
+                            a.filter.sums * (M0 + M1 + M2);
             eps = a.bound_scale * (2.0f * qn * 1.001f * e + 2.0f * kKappaEpi * (qn2 + a.bound[2]));
             complete = a.filter.bad[row] == 0;
         }

@@ -54,7 +54,8 @@ struct RescoreFilter {
     const float4 *rowq = nullptr;
     const float *bound = nullptr;
     const int *bad = nullptr;
-    int mmas = 0;
+    int mmas = 0;      // filter_mmas
+    float sums = 0.0f; // filter_sums
 };
 cudaError_t launch_rescore(const Params &P, const float *centroids, float cmax, const int *m_dev,
                            int kc, int k, const float *cand_d, const long long *cand_i,

@@ -12,7 +12,7 @@
 // Cauchy-Schwarz the difference is at most |q| times
 //     |dq| M0 + |q| M1 + |ds| M2 + |s~| M3          (2-norms; dq = q_rot - q~ ...)
 //   + (mmas + 1) 2^-20 (|q~| M0 + |s~| (M2 + M3))   (accumulation, see rescore)
-//   + 2e-6 (M0 + M2)                                (FP32 sums on both sides)
+//   + sums (M0 + M1 + M2)                           (FP32 sums on both sides: filter_sums)
 // with the index-wide maxima
 //   M0 = sigma |x| |c~|, M1 = sigma |x| |c - c~|, M2 = g |x| sqrt(D),
 //   M3 = |g - sigma rho~| |x| sqrt(D).
@@ -786,6 +786,13 @@ cudaError_t launch_pass(const Params &P, const FlArgs &base, const CUtensorMap &
 
 size_t filter_k(const Params &P) { return 2 * (((size_t)P.D + FL_BK - 1) / FL_BK * FL_BK); }
 int filter_mmas(const Params &P) { return (int)(filter_k(P) / 16); }
+// Roundings of 2^-24 on the way of a term, as a share of sum |terms|.  The exact
+// stage's running sums (tq_exact.cu) are 32 over the bytes of nibble codes, D / 64
+// adds each, and 8 over byte codes, D / 8 FMAs each; what joins them (a tree of 5,
+// or 16 bytes in a row at D < 64) and both sides' scalar factors are at most 24 more.
+float filter_sums(const Params &P) {
+    return (float)((P.nibble ? P.D / 64 : P.D / 8) + 24) * (1.0f / 16777216.0f);
+}
 
 float filter_alpha(const float *centroids, int levels) {
     float best = 2048.0f;

@@ -42,6 +42,8 @@ size_t filter_k(const Params &P);  // values per query row: two parts of whole 6
 
 // MMAs into one accumulator (the bound's accumulation term).
 int filter_mmas(const Params &P);
+// The bound's term for the FP32 sums of both sides, a share of sum |terms|.
+float filter_sums(const Params &P);
 
 // Prepared queries -> the kc smallest approximate distances of each row,
 // ascending, cand_d / cand_i [rows][kc] (index -1 past the corpus), and bad.

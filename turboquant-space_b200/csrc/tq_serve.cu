@@ -317,7 +317,7 @@ cudaError_t enqueue_batch(tq_server *sv, Slot &sl, int rows_cap, int var, bool c
                            tq::tc_topk_kappa(var, (int)K, ix->K_lo),
                            tq::tc_topk_kappa(tq::tc_thresh_variant(!planes, ix->n_pad), (int)K, ix->K_lo),
                            filter ? tq::RescoreFilter{sl.flt.rowq, ix->filter.bound, sl.flt.bad,
-                                                      tq::filter_mmas(sp->P)}
+                                                      tq::filter_mmas(sp->P), tq::filter_sums(sp->P)}
                                   : tq::RescoreFilter{},
                            sv->bound_scale, sl.d_od,
                            sl.d_oi, sl.d_fail, sl.d_thr, sl.d_tthr, sl.d_cnt, rows_cap, st);
@@ -1080,6 +1080,12 @@ tq_status tq_selftest_bounded_wait(int device, int budget_ms) {
     if (device < 0) cudaGetDevice(&device);
     DeviceGuard g(device);
     return bounded_wait_selftest(device, nullptr, budget_ms);
+}
+
+tq_status tq_selftest_filter_sums(const tq_space *sp, float *share) {
+    if (!sp || !share) return fail(TQ_ERR_INVALID_ARGUMENT, "NULL");
+    *share = tq::filter_sums(sp->P);
+    return TQ_OK;
 }
 
 tq_status tq_selftest_space_wait(const tq_space *sp, int budget_ms) {

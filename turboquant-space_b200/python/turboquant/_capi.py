@@ -33,7 +33,7 @@ EXPORTS = (
     "tq_distance_m_to_n_symmetric_device", "tq_index_create", "tq_index_create_ex", "tq_index_destroy",
     "tq_server_create", "tq_server_create_ex", "tq_server_submit", "tq_request_wait", "tq_request_done",
     "tq_request_release", "tq_server_get_stats", "tq_server_reset_stats", "tq_server_tuning", "tq_server_tuning_times", "tq_topk_variant_shape",
-    "tq_server_destroy", "tq_selftest_bounded_wait", "tq_selftest_mton_rows", "tq_selftest_space_wait",
+    "tq_server_destroy", "tq_selftest_bounded_wait", "tq_selftest_mton_rows", "tq_selftest_space_wait", "tq_selftest_filter_sums",
     "tq_space_take_device_status", "tq_space_scan_timer",
     "tq_space_scan_timer_read",
     "tq_rotated_coords_batch", "tq_rotated_coords_batch_device",
@@ -165,6 +165,8 @@ def lib() -> C.CDLL:
     L.tq_selftest_bounded_wait.argtypes = [C.c_int, C.c_int]
     L.tq_selftest_space_wait.restype = st
     L.tq_selftest_space_wait.argtypes = [vp, C.c_int]
+    L.tq_selftest_filter_sums.restype = st
+    L.tq_selftest_filter_sums.argtypes = [vp, C.POINTER(C.c_float)]
     L.tq_selftest_mton_rows.restype = st
     L.tq_selftest_mton_rows.argtypes = [vp, sz, sz, C.POINTER(sz)]
     L.tq_space_scan_timer.restype = st
