@@ -40,3 +40,40 @@ def test_filter_edges(cuda_ok, dim, bits, n, m, k):
                                   np.take_along_axis(ref, idx, 1).astype(np.float32).view(np.uint32))
     assert np.all(I[:, w:] == -1)
     assert st["bound_violations"] == 0
+
+
+@pytest.mark.parametrize("order", ["by cluster", "round robin"])
+def test_storage_order_leaves_no_more_rows_open(cuda_ok, order):
+    """Fifty clusters of 6,000 codes, a query near each: the filter's thresholds come
+    from a sample that must not depend on the order the corpus is stored in.  Stored
+    by cluster or round robin, at most a tenth more of the rows take the exact
+    fallback than with the same corpus shuffled, and the results are the same."""
+    rng = np.random.default_rng(11)
+    dim, bits, per, groups, k = 64, 8, 6000, 50, 10
+    n = per * groups
+    centres = rng.standard_normal((groups, dim)).astype(np.float32)
+    label = np.repeat(np.arange(groups), per) if order == "by cluster" else np.tile(np.arange(groups), per)
+    X = (centres[label] + 0.3 * rng.standard_normal((n, dim))).astype(np.float32)
+    Q = (centres + 0.3 * rng.standard_normal((groups, dim))).astype(np.float32)
+    space, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    codes = space.encode_batch(X)
+    ref = o.distance_m_to_n(Q, codes)
+    idx = np.argsort(ref, axis=1, kind="stable")[:, :k]
+
+    def search(c):
+        ix = space.index(c)
+        try:
+            with ix.serve(k=k, max_rows=128, slots=1, kernel_variant=6) as sv:
+                D, I = sv.submit(Q).wait()
+                return D, I, sv.stats()["fallback_rows"]
+        finally:
+            ix.close()
+
+    D, I, stored = search(codes)
+    np.testing.assert_array_equal(I, idx)
+    np.testing.assert_array_equal(D, np.take_along_axis(ref, idx, 1).astype(np.float32))
+    perm = rng.permutation(n)
+    D2, _, shuffled = search(codes[perm])
+    np.testing.assert_array_equal(np.sort(D2, axis=1), np.sort(D, axis=1))
+    print(f"{order}: {stored} open rows, {shuffled} shuffled")
+    assert stored <= shuffled + groups // 10

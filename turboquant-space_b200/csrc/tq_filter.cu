@@ -21,9 +21,11 @@
 // no operand planes of the corpus.
 //
 // The kc smallest come from thresholds, not from lists kept per thread:
-//   1. the distances of kFilterSample codes (tiles spread evenly over the
-//      corpus) are written out; the kc-th smallest of a row is a threshold
-//      that at least kc codes meet;
+//   1. the distances of kFilterSample codes are written out, one code from each
+//      of as many equal runs of the corpus, at a hashed place in it: whatever the
+//      order that the corpus is stored in (by cluster, by time, round robin), a
+//      group of codes has about its share of the sample.  The kc-th smallest of a
+//      row is a threshold that at least kc codes meet;
 //   2. a larger spread sample, about sqrt(kFilterSample n) codes, lists the
 //      codes that meet it, and the kc-th smallest of the list is a closer one
 //      (larger corpora only);
@@ -77,7 +79,8 @@ struct FlArgs {
     const uint32_t *rho;
     int KBm;               // 64-value blocks of each part
     int box, stages, ring;
-    unsigned nt, stride;   // code tiles of this launch: i * stride, i < nt
+    unsigned nt;           // code tiles of this launch
+    unsigned long long step;  // codes per position of them, 32.32 fixed point (code_at)
     const int *m_dev;
     const float2 *uv, *r12;
     const float *thr;
@@ -131,6 +134,16 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
+}
+
+// Position `lin` of a pass over one code in step / 2^32 -> code: a hashed place in the
+// position's run of the corpus, [lin, lin + 1) step / 2^32.  step = 2^32: every code.
+__device__ __forceinline__ size_t code_at(unsigned long long step, uint32_t lin) {
+    if (step == 1ull << 32) return lin;
+    uint32_t h = lin * 0x9E3779B1u;
+    h = (h ^ (h >> 15)) * 0x85EBCA6Bu;
+    h ^= h >> 13;
+    return (size_t)((lin * step + __umul64hi(step, (unsigned long long)h << 32)) >> 32);
 }
 
 // The approximate distance of one pair: S the unscaled accumulator, c1 = sigma
@@ -194,7 +207,10 @@ __global__ void __launch_bounds__(FL_THREADS, 1) filter_kernel(const __grid_cons
     const int N = m >= FL_ROWS ? FL_ROWS : ((m + 31) & ~31);
     const unsigned mbs = (unsigned)((m + FL_ROWS - 1) / FL_ROWS);
     const unsigned tiles = m > 0 ? mbs * p.nt : 0u, grid = gridDim.x >> 1, t0 = blockIdx.x >> 1;
-    auto first_code = [&](unsigned t) { return (size_t)(t % p.nt) * p.stride * kFilterTile + rank * FL_BM; };
+    // code of row r of this CTA's half of tile t
+    auto code_of = [&](unsigned t, int r) {
+        return code_at(p.step, (t % p.nt) * (unsigned)kFilterTile + rank * FL_BM + r);
+    };
 
     if (warp == 0) {
         // ---------------- TMA producer: the rows' K blocks ----------------
@@ -269,12 +285,14 @@ __global__ void __launch_bounds__(FL_THREADS, 1) filter_kernel(const __grid_cons
         uint32_t cs = 0, cph = 1;
         bool ok = true;
         for (unsigned t = t0; t < tiles && ok; t += grid) {
-            const size_t j0 = min(first_code(t), p.n - 1);
+            // rows past n repeat the last code; a tile half's codes span at most a
+            // 64th of the corpus where it is sampled, so 32 bits hold their offsets
+            const size_t j0 = min(code_of(t, 0), p.n - 1);
             const uint8_t *base = p.codes + j0 * (size_t)p.cs + 4 * c;
-            const int last = (int)min((size_t)(FL_BM - 1), p.n - 1 - j0);  // rows past n repeat the last code
             uint32_t ro[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ro[i] = (uint32_t)(min(r0 + 4 * i, last) * p.cs);
+            for (int i = 0; i < 8; ++i)
+                ro[i] = (uint32_t)(min(code_of(t, r0 + 4 * i), p.n - 1) - j0) * (uint32_t)p.cs;
             for (int q = 0; q < KBm; ++q) {
                 if (!mbar_wait_warp(cempty0 + 8 * cs, cph, p.err, kErrEmpty)) { ok = false; break; }
                 const uint32_t dst = ring0 + cs * RING_BYTES + r0 * (32 * WPI) + 4 * c;
@@ -313,10 +331,9 @@ __global__ void __launch_bounds__(FL_THREADS, 1) filter_kernel(const __grid_cons
         for (unsigned t = t0; t < tiles && ok; t += grid) {
             uint32_t rho[8], pm[8];
             if (!cent) {
-                const size_t j0 = first_code(t);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const size_t j = j0 + r0 + 4 * i;
+                    const size_t j = code_of(t, r0 + 4 * i);
                     rho[i] = j < p.n ? __ldg(p.rho + j) : 0u;
                     pm[i] = sign_bytes(rho[i]);
                 }
@@ -416,7 +433,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) filter_kernel(const __grid_cons
                 __syncwarp();
                 mb_have = mb;
             }
-            const size_t code = first_code(t) + 32 * quad + lane;
+            const size_t code = code_of(t, 32 * quad + lane);
             const bool live = code < p.n;
             float norm = 0.0f, sigma = 0.0f;
             if (live) {
@@ -756,9 +773,10 @@ __global__ void __launch_bounds__(256) filter_index_kernel(Params P, DevTables T
 cudaError_t launch_pass(const Params &P, const FlArgs &base, const CUtensorMap &map, int mode, size_t tiles_all,
                         size_t want, cudaStream_t st) {
     FlArgs a = base;
-    // `want` tiles spread evenly over all of them
-    a.stride = (unsigned)std::max<size_t>(1, tiles_all / std::max<size_t>(1, want));
-    a.nt = (unsigned)std::min((tiles_all + a.stride - 1) / a.stride, want);
+    // the codes of `want` tiles spread evenly over the corpus, or all of them
+    const size_t total = want * kFilterTile;
+    a.nt = (unsigned)std::min(tiles_all, want);
+    a.step = total < a.n ? ((unsigned long long)a.n << 32) / total : 1ull << 32;
     const int stage_bytes = FL_A_BYTES + a.box * 128, ring_bytes = FL_BM * (P.nibble ? 32 : 64);
     const int tab = P.nibble ? 0 : FL_TAB_BYTES, avail = FL_SMEM_MAX - FL_FIXED - tab;
     a.stages = std::min(FL_MAX_STAGES, (avail - 4 * ring_bytes) / stage_bytes) & ~1;  // the decoder groups alternate
