@@ -327,8 +327,10 @@ typedef struct tq_server_stats {
 /* How an index keeps its corpus for the tensor-core pass. */
 typedef enum tq_index_layout {
     TQ_INDEX_PLANES = 0, /* the codes plus their exact-sign hi/lo BF16 operand planes:
-                            code_size + 6 * padded_dim + 8 bytes a code; the fastest pass */
-    TQ_INDEX_CODES = 1   /* the codes plus four floats a code (code_size + 16 bytes): the pass
+                            code_size + 6 * padded_dim + 8 bytes a code, and 4 more for the
+                            filter pass (kernel variant 6) if there is room */
+    TQ_INDEX_CODES = 1   /* the codes plus four floats a code (code_size + 16 bytes, and 4 more
+                            for the filter pass if there is room): the pass
                             decodes each tile of codes in shared memory (kernel variants 2 and
                             4, or 6 by the tuner), for corpora ~10x larger per GPU; padded
                             dim >= 64 */
@@ -346,7 +348,9 @@ typedef struct tq_server_params {
     int k;              /* results per query row, 1..16 */
     int max_rows;       /* query rows per batch, a positive multiple of 128 */
     int slots;          /* batches in flight, 1..8 (fewer if they do not fit in half of the
-                           free device memory) */
+                           free device memory).  The filter pass takes 64 KB a row and slot
+                           more; a server that tunes goes without it rather than with
+                           fewer slots */
     int kernel_variant; /* -1: autotune the contraction's tile shape per batch-size bucket;
                            else fixed (tq_topk_variant_shape): 0..6 for a TQ_INDEX_PLANES
                            index, 1..4 for TQ_INDEX_CODES.  6 is the filter pass over

@@ -77,3 +77,36 @@ def test_storage_order_leaves_no_more_rows_open(cuda_ok, order):
     np.testing.assert_array_equal(np.sort(D2, axis=1), np.sort(D, axis=1))
     print(f"{order}: {stored} open rows, {shuffled} shuffled")
     assert stored <= shuffled + groups // 10
+
+
+def test_only_servers_that_may_filter_hold_its_buffers(cuda_ok):
+    """The filter's buffers are 64 KB a query row: servers of another kernel variant
+    do not hold them, and a server that tunes gives up the filter rather than slots
+    where memory is short."""
+    import torch
+
+    rng = np.random.default_rng(2)
+    space = tq.TurboQuantSpace(64, 4)
+    codes = space.encode_batch(rng.standard_normal((3000, 64)).astype(np.float32))
+    ix = space.index(codes)
+    rows, slots = 4096, 8
+    used = {}
+    try:
+        for variant in (4, 6):
+            torch.cuda.synchronize()
+            before = torch.cuda.mem_get_info()[0]
+            with ix.serve(k=16, max_rows=rows, slots=2, kernel_variant=variant):
+                used[variant] = before - torch.cuda.mem_get_info()[0]
+        assert used[6] - used[4] >= 2 * rows * 64 * 1024, used
+        # room for the slots themselves, by the server's own estimate, but not for the
+        # filter's 270 MB each as well
+        per_slot = rows * (64 * 4 + 130 * 4 + 128 * 4 + 16 * 12 + 32 * 12 + 300 * 16 * 8) + (32 << 20)
+        leave = 2 * slots * per_slot + (512 << 20)
+        fill = torch.empty(max(0, torch.cuda.mem_get_info()[0] - leave), dtype=torch.uint8, device="cuda")
+        with ix.serve(k=16, max_rows=rows, slots=slots) as sv:
+            assert sv.stats()["slots"] == slots
+            assert all(b["variant"] != 6 for b in sv.tuning())
+        del fill
+    finally:
+        ix.close()
+        torch.cuda.empty_cache()

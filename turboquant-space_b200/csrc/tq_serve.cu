@@ -80,7 +80,7 @@ struct tq_index {
     uint8_t *codes = nullptr;  // the corpus itself (n x code_size), for the exact stages
     float *bound = nullptr;    // kBoundFloats index-wide maxima of the error bound
     float cmax = 0.0f;         // max |centroid|
-    tq::FilterIndex filter;    // the filter pass's per-code factors (variant 6)
+    tq::FilterIndex filter;    // the filter pass's per-code factors (variant 6; rho null: no room for them)
     int device = -1;
 };
 
@@ -141,7 +141,8 @@ struct Slot {
     int *d_rows = nullptr;
     void *d_ap = nullptr;  // query planes: max_rows x K x 2 BF16 planes
     long long *d_oi = nullptr;
-    tq::FilterBuffers flt;  // the filter pass's (variant 6)
+    void *d_filter = nullptr;  // the filter pass's buffers (variant 6), where a bucket may take it
+    tq::FilterBuffers flt;
     std::vector<int> bucket_rows;
     std::vector<cudaGraphExec_t> graphs;
     std::vector<tq_request *> batch;  // requests in flight in this slot
@@ -159,6 +160,7 @@ struct tq_server {
     int fb_ctas = 296;        // CTAs of the exact fallback pass
     int grid = 148;
     int max_rows = 1024;
+    bool filter = false;      // the slots have the filter pass's buffers
     size_t queue_rows_cap = 0;
     std::vector<Slot> slots;
     std::vector<int> bucket_variant;  // autotuned kernel variant per bucket
@@ -388,10 +390,6 @@ tq_status slot_alloc(tq_server *sv, Slot &sl) {
     const size_t o_colld = take(R * tq::kCollectCap * 4), o_colli = take(R * tq::kCollectCap * 4);
     const size_t o_scan = take(R * 4), o_list = take(R * 4), o_ap2 = take(R * K * 4);
     const size_t o_r1o = take(R * 4), o_r2o = take(R * 4), o_gthr = take(R * 8);
-    const size_t o_fp = take(R * tq::filter_k(sp->P) * 2), o_rowq = take(R * 16), o_r12 = take(R * 8);
-    const size_t o_uv = take(R * 8), o_fthr = take(R * 4), o_samp = take(R * tq::kFilterSample * 4);
-    const size_t o_fcnt = take(R * 4), o_fld = take(R * tq::kFilterCap * 4);
-    const size_t o_fli = take(R * tq::kFilterCap * 4), o_bad = take(R * 4);
     TQ_CUDA(cudaMalloc(&sl.d_block, off), "cudaMalloc(slot)");
     TQ_CUDA(cudaMemset(sl.d_block, 0, off), "cudaMemset(slot)");
     auto *base = static_cast<unsigned char *>(sl.d_block);
@@ -424,16 +422,26 @@ tq_status slot_alloc(tq_server *sv, Slot &sl) {
     sl.d_r1o = reinterpret_cast<float *>(base + o_r1o);
     sl.d_r2o = reinterpret_cast<float *>(base + o_r2o);
     sl.d_gthr = reinterpret_cast<unsigned long long *>(base + o_gthr);
-    sl.flt.planes = base + o_fp;
-    sl.flt.rowq = reinterpret_cast<float4 *>(base + o_rowq);
-    sl.flt.r12 = reinterpret_cast<float2 *>(base + o_r12);
-    sl.flt.uv = reinterpret_cast<float2 *>(base + o_uv);
-    sl.flt.thr = reinterpret_cast<float *>(base + o_fthr);
-    sl.flt.samp = reinterpret_cast<float *>(base + o_samp);
-    sl.flt.cnt = reinterpret_cast<int *>(base + o_fcnt);
-    sl.flt.list_d = reinterpret_cast<float *>(base + o_fld);
-    sl.flt.list_i = reinterpret_cast<int *>(base + o_fli);
-    sl.flt.bad = reinterpret_cast<int *>(base + o_bad);
+    if (sv->filter) {
+        off = 0;
+        const size_t o_fp = take(R * tq::filter_k(sp->P) * 2), o_rowq = take(R * 16), o_r12 = take(R * 8);
+        const size_t o_uv = take(R * 8), o_fthr = take(R * 4), o_samp = take(R * tq::kFilterSample * 4);
+        const size_t o_fcnt = take(R * 4), o_fld = take(R * tq::kFilterCap * 4);
+        const size_t o_fli = take(R * tq::kFilterCap * 4), o_bad = take(R * 4);
+        TQ_CUDA(cudaMalloc(&sl.d_filter, off), "cudaMalloc(slot, filter pass)");
+        TQ_CUDA(cudaMemset(sl.d_filter, 0, off), "cudaMemset(slot, filter pass)");
+        base = static_cast<unsigned char *>(sl.d_filter);
+        sl.flt.planes = base + o_fp;
+        sl.flt.rowq = reinterpret_cast<float4 *>(base + o_rowq);
+        sl.flt.r12 = reinterpret_cast<float2 *>(base + o_r12);
+        sl.flt.uv = reinterpret_cast<float2 *>(base + o_uv);
+        sl.flt.thr = reinterpret_cast<float *>(base + o_fthr);
+        sl.flt.samp = reinterpret_cast<float *>(base + o_samp);
+        sl.flt.cnt = reinterpret_cast<int *>(base + o_fcnt);
+        sl.flt.list_d = reinterpret_cast<float *>(base + o_fld);
+        sl.flt.list_i = reinterpret_cast<int *>(base + o_fli);
+        sl.flt.bad = reinterpret_cast<int *>(base + o_bad);
+    }
     for (int b = 128; b < sv->max_rows; b *= 2) sl.bucket_rows.push_back(b);
     sl.bucket_rows.push_back(sv->max_rows);
     return TQ_OK;
@@ -445,6 +453,7 @@ void slot_free(Slot &sl) {
     sl.graphs.clear();
     if (sl.stream) cudaStreamSynchronize(sl.stream);
     if (sl.d_block) cudaFree(sl.d_block);
+    if (sl.d_filter) cudaFree(sl.d_filter);
     if (sl.h_q) cudaFreeHost(sl.h_q);
     if (sl.h_m) cudaFreeHost(sl.h_m);
     if (sl.h_err) cudaFreeHost(sl.h_err);
@@ -467,14 +476,14 @@ void slot_free(Slot &sl) {
 // variant would otherwise be timed at a clock that real batches under the
 // power cap do not get.
 // Tuning results of this process, per (device, padded dim, bits, corpus size,
-// candidates, slots tuned together, bucket rows): the fastest variant and its
-// time.  A server whose key is present skips timing that bucket.
+// candidates, slots tuned together, bucket rows, filter pass on offer): the fastest
+// variant and its time.  A server whose key is present skips timing that bucket.
 struct TuneKey {
-    int device, D, bits, kc, ns, rows, layout;
+    int device, D, bits, kc, ns, rows, layout, filter;
     size_t n;
     bool operator<(const TuneKey &o) const {
-        return std::tie(device, D, bits, kc, ns, rows, layout, n) <
-               std::tie(o.device, o.D, o.bits, o.kc, o.ns, o.rows, o.layout, o.n);
+        return std::tie(device, D, bits, kc, ns, rows, layout, filter, n) <
+               std::tie(o.device, o.D, o.bits, o.kc, o.ns, o.rows, o.layout, o.filter, o.n);
     }
 };
 std::mutex g_tune_mu;
@@ -490,7 +499,7 @@ tq_status autotune(tq_server *sv, int fixed_variant) {
     sv->tune_ms.assign((size_t)nb * nv, 0.0f);
     const tq_index *ix = sv->index;
     auto key_of = [&](int rows) {
-        return TuneKey{ix->device, (int)ix->sp->D, ix->sp->bits, sv->kc, ns, rows, ix->layout, ix->n};
+        return TuneKey{ix->device, (int)ix->sp->D, ix->sp->bits, sv->kc, ns, rows, ix->layout, sv->filter, ix->n};
     };
     if (fixed_variant < 0) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -537,7 +546,7 @@ tq_status autotune(tq_server *sv, int fixed_variant) {
         double best = 1e30;
         for (int v = 0; v < nv; ++v) {
             if (fixed_variant >= 0 && v != fixed_variant) continue;
-            if (!variant_fits(sv->index, v) && v != kFilterVariant) continue;
+            if (v == kFilterVariant ? !sv->filter : !variant_fits(sv->index, v)) continue;
             TQ_CUDA(enqueue_batch(sv, s0, rows, v, false), "autotune warm-up");
             TQ_CUDA(cudaEventRecord(e0, s0.stream), "event");
             for (int si = 1; si < ns; ++si)
@@ -769,12 +778,15 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
     const size_t plane_bytes = planes ? ix->n_pad * (K + (size_t)ix->K_lo) * 2 : 0;
     const size_t code_bytes = round_up(n * sp->code_size, 256);
     const size_t nscal = planes ? 2 : 4;  // c1, c2 (+ fc, fs)
-    cudaError_t e = cudaMalloc(&ix->block, plane_bytes + (nscal + 1) * ix->n_pad * 4 + code_bytes +
-                                               (tq::kBoundFloats + tq::kFilterBound) * 4 + 256);
+    cudaError_t e = cudaMalloc(&ix->block, plane_bytes + nscal * ix->n_pad * 4 + code_bytes +
+                                               tq::kBoundFloats * 4 + 256);
     if (e != cudaSuccess) {
         delete ix;
         return cuda_fail(e, "cudaMalloc(index)");
     }
+    // the filter pass's factors, 4 bytes a code: an index without room for them goes without
+    void *factors = nullptr;
+    if (cudaMalloc(&factors, (ix->n_pad + tq::kFilterBound) * 4) != cudaSuccess) cudaGetLastError();
     auto *base = static_cast<unsigned char *>(ix->block);
     ix->planes = planes ? base : nullptr;
     ix->c1 = reinterpret_cast<float *>(base + plane_bytes);
@@ -783,12 +795,12 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
         ix->fc = ix->c2 + ix->n_pad;
         ix->fs = ix->fc + ix->n_pad;
     }
-    ix->filter.rho = reinterpret_cast<uint32_t *>(ix->c1 + nscal * ix->n_pad);
-    ix->codes = reinterpret_cast<uint8_t *>(ix->filter.rho + ix->n_pad);
+    ix->filter.rho = static_cast<uint32_t *>(factors);
+    ix->codes = reinterpret_cast<uint8_t *>(ix->c1 + nscal * ix->n_pad);
     ix->bound = reinterpret_cast<float *>(ix->codes + code_bytes);
     ix->filter.codes = ix->codes;
     ix->filter.n = n;
-    ix->filter.bound = ix->bound + tq::kBoundFloats;
+    ix->filter.bound = factors ? static_cast<float *>(factors) + ix->n_pad : nullptr;
     ix->filter.alpha = tq::filter_alpha(sp->centroids.data(), sp->levels);
     e = cudaMemcpy(ix->codes, codes, n * sp->code_size,
                    codes_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
@@ -809,10 +821,11 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
                                    nullptr);
     }
     if (e == cudaSuccess) e = tq::launch_index_bound(sp->P, ix->codes, n, ix->bound, nullptr);
-    if (e == cudaSuccess) e = tq::launch_filter_index(sp->P, sp->T, ix->filter, nullptr);
+    if (e == cudaSuccess && factors) e = tq::launch_filter_index(sp->P, sp->T, ix->filter, nullptr);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         cudaFree(ix->block);
+        cudaFree(factors);
         delete ix;
         return cuda_fail(e, "index build");
     }
@@ -829,6 +842,7 @@ void tq_index_destroy(tq_index *ix) {
     if (!ix) return;
     DeviceGuard g(ix->device);
     if (ix->block) cudaFree(ix->block);
+    if (ix->filter.rho) cudaFree(ix->filter.rho);
     delete ix;
 }
 
@@ -846,6 +860,9 @@ tq_status tq_server_create_ex(tq_index *ix, const tq_server_params *prm, tq_serv
     if (slots < 1 || slots > 8) return fail(TQ_ERR_INVALID_ARGUMENT, "slots must be in 1..8");
     if (kernel_variant >= 0 && !variant_fits(ix, kernel_variant))
         return fail(TQ_ERR_INVALID_ARGUMENT, "kernel variant %d does not serve this index layout",
+                    kernel_variant);
+    if (kernel_variant == kFilterVariant && !ix->filter.rho)
+        return fail(TQ_ERR_OUT_OF_MEMORY, "kernel variant %d: there was no memory for the index's filter factors",
                     kernel_variant);
     DeviceGuard g(ix->device);
     int sms = 148;
@@ -879,10 +896,17 @@ tq_status tq_server_create_ex(tq_index *ix, const tq_server_params *prm, tq_serv
     const size_t slot_bytes =
         R * (ix->sp->dim * 4 + (2 * D + 2) * 4 + K * 4 + 8 + (size_t)k * 12 + (size_t)kc * 12 + 4 +
              (size_t)sv->fb_ctas * k * 8) +
-        R * (tq::filter_k(ix->sp->P) * 2 + 4 * tq::kFilterSample + 8 * tq::kFilterCap + 64) +
         (size_t)sms * 128 * tq::kTopKListsMax * tq::kCandMax * 8 + 8192;
-    const size_t fit = std::max<size_t>(1, (free_b / 2) / slot_bytes);
-    slots = (int)std::min<size_t>((size_t)slots, fit);
+    // The filter pass's buffers (64 KB a row) come where the tuner may take it or it is
+    // asked for.  The tuner does without rather than have fewer slots for them.
+    const size_t filter_bytes = R * (tq::filter_k(ix->sp->P) * 2 + 4 * tq::kFilterSample + 8 * tq::kFilterCap + 64);
+    auto fit = [&](size_t bytes) { return (free_b / 2) / bytes; };
+    const size_t want = std::min<size_t>((size_t)slots, std::max<size_t>(1, fit(slot_bytes)));
+    sv->filter = kernel_variant == kFilterVariant ||
+                 (kernel_variant < 0 && ix->filter.rho && fit(slot_bytes + filter_bytes) >= want);
+    slots = (int)(kernel_variant == kFilterVariant
+                      ? std::min(want, std::max<size_t>(1, fit(slot_bytes + filter_bytes)))
+                      : want);
     sv->slots.resize(slots);
     tq_status st = TQ_OK;
     cudaError_t ce = cudaMalloc(&sv->pool, sv->pool_rows * row_bytes);
@@ -892,6 +916,14 @@ tq_status tq_server_create_ex(tq_index *ix, const tq_server_params *prm, tq_serv
     for (auto &sl : sv->slots)
         if (st == TQ_OK && (st = slot_alloc(sv, sl)) != TQ_OK) break;
     if (st == TQ_OK) st = autotune(sv, kernel_variant);
+    if (st == TQ_OK && sv->filter &&
+        std::find(sv->bucket_variant.begin(), sv->bucket_variant.end(), kFilterVariant) == sv->bucket_variant.end()) {
+        for (auto &sl : sv->slots) {  // no bucket took it
+            cudaFree(sl.d_filter);
+            sl.d_filter = nullptr;
+            sl.flt = tq::FilterBuffers();
+        }
+    }
     for (auto &sl : sv->slots) {
         if (st != TQ_OK) break;
         st = capture_graphs(sv, sl);
