@@ -86,9 +86,9 @@ def test_wide_tiles_with_few_live_columns(cuda_ok, dim, bits, m, n):
     assert ok, ("asymmetric", err.max())
 
 
-def _near(dim, m, seed):
+def _near(dim, m, seed, n=2048):
     rng = np.random.default_rng(seed)
-    X = rng.standard_normal((2048, dim)).astype(np.float32)
+    X = rng.standard_normal((n, dim)).astype(np.float32)
     X /= np.linalg.norm(X, axis=1, keepdims=True)
     Q = X[:m] + (0.02 / dim ** 0.5) * rng.standard_normal((m, dim)).astype(np.float32)
     return X, np.ascontiguousarray(Q, np.float32)
@@ -107,7 +107,7 @@ def test_near_pairs_at_fp32_are_as_accurate_as_the_scan(cuda_ok, dim, bits):
     at once: at most the error of rounding an FP32 chain of 2 D terms, a random walk
     of 2 D half-ulps of a sum that grows to its end."""
     m = 64
-    X, Q = _near(dim, m, dim + bits)
+    X, Q = _near(dim, m, dim + bits, n=20_000)  # enough codes that 16 rows do not run on the scan
     s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
     codes = o.encode_batch(X)
     f64 = np.array([o.distance_f64(Q[i], codes[i]) for i in range(m)])
@@ -200,3 +200,22 @@ def test_a_call_that_gave_up_does_not_touch_others(cuda_ok):
         s.take_device_status()
     assert e.value.status == _capi.TQ_ERR_TIMEOUT
     s.take_device_status()  # taken
+
+
+@pytest.mark.parametrize("dim,bits", [(16, 4), (384, 4), (768, 8), (1536, 4)])
+@pytest.mark.parametrize("m,pairs", [(3, 20_000), (12, 20_000), (12, 60_000), (31, 200_000), (32, 4_000)])
+def test_either_side_of_the_scan_rule(cuda_ok, dim, bits, m, pairs):
+    """Fewer than 32 rows run on the scan kernel or the tensor cores by a count of
+    their pairs (about 40,000 at wide dims, 170,000 at narrow ones)."""
+    n = pairs // m
+    rng = np.random.default_rng(dim + bits + m + n)
+    X, Q = (rng.standard_normal((r, dim)).astype(np.float32) for r in (n, m))
+    s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    cs = s.code_size_bytes()
+    codes, rows = o.encode_batch(X), o.encode_batch(Q)
+    err, ok = dist_close(s.distance_m_to_n(Q, codes), o.distance_m_to_n(Q, codes),
+                         asym_term_scale(Q, codes, cs, cs - 12))
+    assert ok, ("asymmetric", err.max())
+    err, ok = dist_close(s.distance_m_to_n_symmetric(rows, codes), o.distance_m_to_n_symmetric(rows, codes),
+                         sym_term_scale(rows, codes, cs, cs - 12))
+    assert ok, ("symmetric", err.max())

@@ -247,15 +247,21 @@ class MtonRunner {
     // Code size up to which SPLIT_BF16_DECODED is offered: a tile of 128 codes
     // beside two 64 KB stages in shared memory.
     static constexpr size_t kDecMaxCode = 756;
-    // FP32: the tensor-core kernel, except where the scan kernel's single launch
-    // per row is faster (us a call, scan / tensor-core): few rows, which do not
-    // pay for the decode of every code (200,000 codes: 384-d 4-bit 38 / 105 for
-    // one row, 111 / 105 for two, 394 / 107 for eight; 768-d 8-bit 113 / 252 for
-    // two, 378 / 252 for eight), and few rows against few codes, where the
-    // row-plane launch shows (8 x 1,000: 32 / 36; 8 x 30,000: 76 / 46).
+    // FP32: the tensor-core kernel, except where the scan kernel, a launch over rows and
+    // codes, is faster.  One or two rows (four of byte codes) do not pay for the decode
+    // of every code (200,000 codes, scan / tensor-core, us a call: 384-d 4-bit 38 / 105
+    // for one row, 111 / 105 for two, 394 / 107 for eight; 768-d 8-bit 113 / 252 for two,
+    // 378 / 252 for eight).  Fewer than 32 rows against few codes: a tile walks its K
+    // blocks one after the other, 0.55 us each, and the row planes are a launch of 4 us;
+    // the scan takes 0.5 us for 2^20 values (0.25 against codes).  12 rows by 1000
+    // codes: 768-d 8-bit 33 / 39, 1536-d 4-bit 50 / 66, 4096-d 8-bit 93 / 133; by 10,000
+    // codes 61 / 26, 150 / 66, 330 / 135.
     bool use_cg(size_t n) const {
         if (sp_->D < 16 || m_ <= (sp_->P.nibble ? 2 : 4)) return false;
-        return m_ > 8 || m_ * n * sp_->D > (size_t(1) << 25);
+        if (m_ >= 32) return true;
+        const double blocks = (sym_ ? 1.0 : 2.0) * (double)((sp_->D + 63) / 64), tiles = (double)((n + 127) / 128);
+        const double scan = (sym_ ? 0.25 : 0.5) / (1 << 20) * (double)m_ * (double)n * (double)sp_->D;
+        return scan > 4.0 + 0.55 * blocks * std::ceil(tiles / 148.0);
     }
     int form() const { return sym_ ? tq::kCgSym : tq::kCgAsym; }
     int fmt() const { return bf16_ ? tq::kCgBF16 : tq::kCgFP16; }
