@@ -1033,15 +1033,14 @@ constexpr size_t kSymqTcChunkBytes = size_t(2048) << 20;  // TF32 pairs: fewer, 
 
 size_t sq_round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// The light variant runs on the M x N kernel with in-kernel decoded code tiles
-// (tq_cgemm.cu, FP16 pairs; both precisions, padded dims of at least 16, 4-byte
-// aligned codes): no column planes.  Otherwise:
-// row planes built once (from row codes, or from a prepared code), column
-// planes built per chunk; one two-accumulator contraction per chunk: the FP32
-// CUDA-core kernel, or (split-TF32) the FP32 planes split into hi/lo TF32
-// planes (K padded to 32, rows to 128 / 256) for the tcgen05 kernel.  Padded
-// dims below 64 keep the FP32 kernel: a tile of so short a reduction is
-// mostly padding.
+// The light variant (both precisions, padded dims of at least 16) and the full ones
+// at FP32 (padded dims of at least 32) run on the M x N kernel with in-kernel decoded
+// code tiles (tq_cgemm.cu, FP16 pairs) where device codes are 4-byte aligned: no
+// column planes.  Otherwise: row planes built once (from row codes, or from a prepared
+// code), column planes built per chunk; one two-accumulator contraction per chunk: the
+// FP32 CUDA-core kernel, or (split-TF32) the FP32 planes split into hi/lo TF32 planes
+// (K padded to 32, rows to 128 / 256) for the tcgen05 kernel.  Padded dims below 64
+// keep the FP32 kernel: a tile of so short a reduction is mostly padding.
 constexpr size_t kCorrSlice = 32768;  // rows whose correction is prepared at a time
 
 struct SymqRunner {
@@ -1084,9 +1083,12 @@ struct SymqRunner {
         return TQ_OK;
     }
     // Takes a call to the M x N kernel where the codes allow it (A, B: device
-    // pointers of the call): the light variant, and the full ones at FP32.
+    // pointers of the call): the light variant, and the full ones at FP32.  The full
+    // form's two passes work on whole K blocks of 64 values, three quarters of them
+    // padding at D = 16: there the CUDA-core kernel is faster (64 x 10,000 42 us against
+    // 47, 1000 x 20,000 208 against 245), at D = 32 not (45 / 46 and 264 / 254).
     void choose(const void *A, const void *B) {
-        cg = sp->D >= 16 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 3) == 0 &&
+        cg = sp->D >= (light() ? 16 : 32) && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 3) == 0 &&
              (light() || !tc);
     }
     tq_status prepare_rows_cg(const uint8_t *A, size_t rows_, cudaStream_t s) {
@@ -1234,9 +1236,8 @@ struct SymqRunner {
     }
 };
 
-// The QJL-corrected symmetric contractions run at FP32 accuracy (the M x N
-// kernel, or CUDA cores) or
-// split-TF32 (tensor cores).  A BF16 pair is refused: its planes' rounding
+// The QJL-corrected symmetric contractions run at FP32 accuracy (the M x N kernel,
+// or CUDA cores) or split-TF32 (tensor cores).  A BF16 pair is refused: its planes' rounding
 // errors do not average out (see tc_symq_kernel) and exceed 1e-5.
 tq_status symq_precision_ok(tq_precision p) {
     if (p == TQ_PRECISION_FP32 || p == TQ_PRECISION_SPLIT_TF32) return TQ_OK;
