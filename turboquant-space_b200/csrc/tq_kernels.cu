@@ -1863,21 +1863,22 @@ struct PrepareRun {
             prepare2_kernel<LOG_D><<<(unsigned)std::max<size_t>(blocks, 1), 128, 0, st>>>(Q, m, q_rot, s_q, norms,
                                                                                           P, T);
             return cudaGetLastError();
+        } else {
+            const int D = 1 << LOG_D;
+            int warps = (kSmemBudget - kTabBytes) / (4 * (D + 8));
+            if (warps > 8) warps = 8;
+            if (warps < 1) return cudaErrorInvalidConfiguration;
+            const size_t smem = (size_t)kTabBytes + (size_t)warps * 4 * (D + 8);
+            cudaError_t e = cudaFuncSetAttribute(prepare_kernel<LOG_D>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+            size_t blocks = (m + warps - 1) / warps;
+            const size_t cap = (size_t)sm_count() * 4;
+            if (blocks > cap) blocks = cap;
+            if (blocks < 1) blocks = 1;
+            prepare_kernel<LOG_D><<<(unsigned)blocks, 32 * warps, smem, st>>>(Q, m, q_rot, s_q, norms, P, T);
+            return cudaGetLastError();
         }
-        const int D = 1 << LOG_D;
-        int warps = (kSmemBudget - kTabBytes) / (4 * (D + 8));
-        if (warps > 8) warps = 8;
-        if (warps < 1) return cudaErrorInvalidConfiguration;
-        const size_t smem = (size_t)kTabBytes + (size_t)warps * 4 * (D + 8);
-        cudaError_t e = cudaFuncSetAttribute(prepare_kernel<LOG_D>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        size_t blocks = (m + warps - 1) / warps;
-        const size_t cap = (size_t)sm_count() * 4;
-        if (blocks > cap) blocks = cap;
-        if (blocks < 1) blocks = 1;
-        prepare_kernel<LOG_D><<<(unsigned)blocks, 32 * warps, smem, st>>>(Q, m, q_rot, s_q, norms, P, T);
-        return cudaGetLastError();
     }
 };
 
