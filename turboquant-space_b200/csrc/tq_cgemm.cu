@@ -59,8 +59,10 @@
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
+#include <vector>
 
 #include "tq_cgemm.h"
+#include "tq_tables.h"
 #include "tq_tc.cuh"
 
 namespace tq {
@@ -724,28 +726,38 @@ unsigned rows_grid(size_t work) {
 // scale may give back.  FP16: near rows of 32 to 2048 values at 2 to 8 bits, 1.6e-8
 // to 5e-8.  BF16: half an ulp, 0.72 2^-24 of the sum so far on average, an MMA, over
 // 12 MMAs a block: 44.5 of the whole sum in chunks of 8 blocks (queries), whose sum
-// grows evenly, 20.5 in chunks of 4 (codes
-// against codes).
+// grows evenly, 20.5 in chunks of 4 (codes against codes).
 constexpr double kTruncBias[2][2] = {{0.0, 3e-8}, {1.9e-6, 8.8e-7}};  // [fmt][rows are codes]
 float cg_cent_scale(const float *centroids, int levels, int fmt) {
     const bool h16 = fmt == kCgFP16;
     const float top = h16 ? 2048.0f : 2.0f, step = h16 ? 4.0f : 1.0f / 256, rows = h16 ? kRowScale : 1.0f;
     const double t1 = kTruncBias[fmt][0], t2 = kTruncBias[fmt][1];
+    // the positive levels (the others are their negatives): value, 1 / c, and c^2 times
+    // about its share
+    struct Level {
+        float c;
+        double inv, w;
+    };
+    std::vector<Level> lv;
+    double sw = 0.0;
+    for (int v = levels / 2; v < levels; ++v) {
+        const double c = centroids[v];
+        lv.push_back({centroids[v], 1.0 / c, c * c * std::exp(-c * c / 3.0)});
+        sw += lv.back().w;
+    }
     float best = top;
     double best_err = 1e300;
     for (int i = 0; i < 256; ++i) {
         const float a = top - step * (float)i;
-        double sw = 0.0, d1 = 0.0, d2 = 0.0, l2 = 0.0;
-        for (int v = levels / 2; v < levels; ++v) {  // the others are their negatives
-            const double c = centroids[v], w = c * c * std::exp(-c * c / 3.0);  // c^2 times about its share
-            const float x = centroids[v] * a;
-            const float h = h16 ? __half2float(__float2half_rn(x)) : __bfloat162float(__float2bfloat16_rn(x));
-            const float l = h16 ? __half2float(__float2half_rn(x - h)) : __bfloat162float(__float2bfloat16_rn(x - h));
-            const double d = ((double)h + l) / (c * a) - 1.0, r = l / (c * a);
-            sw += w;
-            d1 += w * d;
-            d2 += w * d * d;
-            l2 += w * r * r;
+        const double ia = 1.0 / a;
+        double d1 = 0.0, d2 = 0.0, l2 = 0.0;
+        for (const Level &e : lv) {
+            const float x = e.c * a, h = h16 ? round_fp16(x) : round_bf16(x);
+            const float l = h16 ? round_fp16(x - h) : round_bf16(x - h);
+            const double s = e.inv * ia, d = ((double)h + l) * s - 1.0, r = l * s;
+            d1 += e.w * d;
+            d2 += e.w * d * d;
+            l2 += e.w * r * r;
         }
         // a product of two values is off by d + d' - r r', and the undoing factor by
         // its rounding.  Over near rows, whose values agree, that is a bias, to which

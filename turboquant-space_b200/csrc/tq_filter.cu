@@ -46,8 +46,10 @@
 
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "tq_filter.h"
+#include "tq_tables.h"
 #include "tq_tc.cuh"
 
 namespace tq {
@@ -813,16 +815,20 @@ float filter_sums(const Params &P) {
 }
 
 float filter_alpha(const float *centroids, int levels) {
+    // the levels below zero (the others are their negatives): value, and the density
+    // of N(0,1) at it
+    const int half = std::min(levels / 2, 128);
+    std::vector<double> w(half);
+    for (int v = 0; v < half; ++v) w[v] = std::exp(-0.5 * (double)centroids[v] * centroids[v]);
     float best = 2048.0f;
     double best_e = INFINITY;
     for (int t = 0; t < 1024; ++t) {
         const float alpha = 1024.0f + (float)t;
+        const double ia = 1.0 / alpha;
         double e = 0.0;
-        for (int v = 0; v < std::min(levels, 128); ++v) {
-            const double c = centroids[v];
-            // the weight of a level: the density of N(0,1) at it
-            const double x = (double)__half2float(__float2half_rn(centroids[v] * alpha)) / alpha - c;
-            e += x * x * std::exp(-0.5 * c * c);
+        for (int v = 0; v < half; ++v) {
+            const double x = (double)round_fp16(centroids[v] * alpha) * ia - centroids[v];
+            e += x * x * w[v];
         }
         if (e < best_e) {
             best_e = e;

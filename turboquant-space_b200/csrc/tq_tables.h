@@ -3,9 +3,30 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 namespace tq {
+
+// x rounded to the nearest FP16 or BF16 value, ties to even (finite values within
+// FP16's range), for tables that try many scales.
+inline float round_fp16(float x) {
+    uint32_t u;
+    std::memcpy(&u, &x, 4);
+    if ((u & 0x7FFFFFFFu) < 0x38800000u) return (x + 0.75f) - 0.75f;  // below 2^-14: steps of 2^-24
+    u += 0xFFFu + ((u >> 13) & 1u);
+    u &= ~0x1FFFu;
+    std::memcpy(&x, &u, 4);
+    return x;
+}
+inline float round_bf16(float x) {
+    uint32_t u;
+    std::memcpy(&u, &x, 4);
+    u += 0x7FFFu + ((u >> 16) & 1u);
+    u &= 0xFFFF0000u;
+    std::memcpy(&x, &u, 4);
+    return x;
+}
 
 // generateSigns (turbo_quant.h:74-86): splitmix64 draw i, bit 0 set -> +1.
 std::vector<float> sign_vector(size_t d, uint64_t seed);
