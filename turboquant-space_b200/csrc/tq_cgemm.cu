@@ -186,17 +186,24 @@ __device__ __forceinline__ uint4 byte_sign(uint32_t x0, uint32_t x1, uint32_t on
 }
 
 // f(k, x) for at least the first `cols` of CPT columns of a chunk buffer, in
-// pieces of 32 (a piece past `cols` holds values that are not used).
-template <int CPT, class F>
+// pieces of 32, or of 16 where f needs the registers (a piece past `cols` holds
+// values that are not used).
+template <int CPT, bool HALF, class F>
 __device__ __forceinline__ void chunk_pieces(uint32_t X, int cols, F f) {
+    constexpr int W = HALF ? 16 : 32;
 #pragma unroll
-    for (int pc = 0; pc < CPT / 32; ++pc) {
-        if (32 * pc >= cols) break;
-        uint32_t x[32];
+    for (int pc = 0; pc < CPT / W; ++pc) {
+        if (W * pc >= cols) break;
+        uint32_t x[W];
         __syncwarp();
-        tmem_ld32(X + 32 * pc, x);
+        if constexpr (HALF) {
+            tmem_ld16_nw(X + W * pc, x);
+            tmem_wait_ld();
+        } else {
+            tmem_ld32(X + W * pc, x);
+        }
 #pragma unroll
-        for (int j = 0; j < 32; ++j) f(32 * pc + j, __uint_as_float(x[j]));
+        for (int j = 0; j < W; ++j) f(W * pc + j, __uint_as_float(x[j]));
     }
 }
 
@@ -543,24 +550,25 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
                 if (!mbar_wait_warp(xfull0 + 8 * b, xph, p.err, kErrTmemFull)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t X = lanes + b * BUF;
-                auto pieces = [&](auto f) {
+                auto pieces = [&](auto f, auto small) {
                     if constexpr (SPLIT) chunk_quarters(X, p.NT, f);
-                    else chunk_pieces<CPT>(X, cpt, f);
+                    else chunk_pieces<CPT, decltype(small)::value>(X, cpt, f);
                 };
+                constexpr std::false_type wide{};
                 // How a chunk joins the running sum.  Symmetric and light: centroid
                 // chunks are added (the light form's last chunk is its clamped
                 // correction).  Asymmetric: fma(x, f, y) with f = scale gamma for
                 // the sign part and sigma for the centroid part.
                 if (LIGHT || p.form == kCgSym) {
-                    if (c0 == 0) pieces([&](int k, float x) { y[k] = x; });
-                    else if (!LIGHT || ord.cent(c0)) pieces([&](int k, float x) { y[k] = __fadd_rn(y[k], x); });
+                    if (c0 == 0) pieces([&](int k, float x) { y[k] = x; }, wide);
+                    else if (!LIGHT || ord.cent(c0)) pieces([&](int k, float x) { y[k] = __fadd_rn(y[k], x); }, wide);
                 }
                 if constexpr (!LIGHT) {
                     if (p.form == kCgAsym) {
                         const float fx = ord.cent(c0) ? __fmul_rn(sigma, p.undo_c)
                                                       : __fmul_rn(__fmul_rn(p.scale, gamma), p.undo_s);
-                        if (c0 == 0) pieces([&](int k, float x) { y[k] = __fmul_rn(x, fx); });
-                        else pieces([&](int k, float x) { y[k] = __fmaf_rn(x, fx, y[k]); });
+                        if (c0 == 0) pieces([&](int k, float x) { y[k] = __fmul_rn(x, fx); }, wide);
+                        else pieces([&](int k, float x) { y[k] = __fmaf_rn(x, fx, y[k]); }, wide);
                     }
                 } else if (!ord.cent(c0)) {
                     const CgCols cols(col0, cpt, p.m);
@@ -571,7 +579,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) cgemm_kernel(const __grid_const
                         const float corr = __fmul_rn(__fmul_rn(x, r.y), gamma);
                         const float lim = fabsf(ip);
                         y[k] = __fadd_rn(ip, fmaxf(-lim, fminf(lim, corr)));
-                    });
+                    }, std::true_type{});
                 }
                 __syncwarp();
                 tc_fence_before();
