@@ -853,17 +853,19 @@ cudaError_t launch_cgemm(const Params &P, const DevTables &T, int form, int fmt,
     // the rounding of an FP32 sum.  FP16: 2 (1 where the whole part is 4 blocks or
     // fewer).  BF16: 8 for queries and 4 for codes against codes, whose terms share a
     // sign more often.  The sign part: +-1 by +-1 sums (light) are exact integers;
-    // otherwise 8, since its hi products are nearly exact in FP32 and its share of a
-    // near pair's sum is a third at most (near pairs of 1536-d 2-bit, mean error with
-    // 16 / 8 / 2 blocks 3.4 / 2.0 / 1.1e-7, and 2000 x 100k of 768-d 1.55 / 1.59 /
-    // 1.70 ms; an FP32 chain's largest error there is 3e-6, this one's 1.1e-6).
+    // otherwise FP16 takes 8, since its hi products are nearly exact in FP32 and its
+    // share of a near pair's sum is a third at most (near pairs of 1536-d 2-bit, mean
+    // error with 16 / 8 / 2 blocks 3.4 / 2.0 / 1.1e-7, and 2000 x 100k of 768-d 1.40 /
+    // 1.44 / 1.49 ms; an FP32 chain's largest error there is 3e-6, this one's 1.1e-6),
+    // and BF16 16 (8 change its near pairs' mean error by 1e-7 of 0.7e-6; under the
+    // power cap 4096 x 500k of 768-d take 15.9 ms with 8 and 15.3 with 16).
     // Fewer than 32 rows, where the scan kernel's short FP32 chains stand for
     // comparison: chunks of 1 and 4 blocks with the quarters apart, an error like the
     // scan's (near pairs of 2-bit codes, 8 rows, largest 5.5e-7 -> 3.3e-7 against the
     // scan's 2.9e-7) for 97 -> 102 us at 8 x 200k of 384-d, 245 -> 250 of 768-d 8-bit,
     // 93 -> 100 at 24 x 200k.
     a.chm = fmt == kCgFP16 ? (a.KBm <= 4 || m < 32 ? 1 : 2) : form == kCgAsym ? 8 : 4;
-    a.chs = form == kCgLight ? a.KBm : fmt == kCgFP16 && m < 32 ? 4 : 8;
+    a.chs = form == kCgLight ? a.KBm : fmt != kCgFP16 ? 16 : m < 32 ? 4 : 8;
     a.m = m;
     a.rs = rows.rs;
     a.scale = P.scale;
