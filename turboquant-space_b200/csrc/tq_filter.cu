@@ -46,6 +46,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "tq_filter.h"
@@ -70,7 +71,9 @@ constexpr float kRowScale = 16384.0f;
 constexpr int kErrFull = 1, kErrEmpty = 2, kErrTmemFull = 3, kErrTmemEmpty = 4;
 constexpr unsigned kAll = 0xffffffffu;
 
-enum { kSample = 0, kCollect = 1 };
+// Passes: the distances of a spread sample; the codes of a larger one that meet the
+// thresholds; all codes that do.
+enum { kSample = 0, kCollect = 1, kCollectAll = 2 };
 
 struct FlArgs {
     const uint8_t *codes;
@@ -139,9 +142,8 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 }
 
 // Position `lin` of a pass over one code in step / 2^32 -> code: a hashed place in the
-// position's run of the corpus, [lin, lin + 1) step / 2^32.  step = 2^32: every code.
+// position's run of the corpus, [lin, lin + 1) step / 2^32.  (step = 2^32: every code.)
 __device__ __forceinline__ size_t code_at(unsigned long long step, uint32_t lin) {
-    if (step == 1ull << 32) return lin;
     uint32_t h = lin * 0x9E3779B1u;
     h = (h ^ (h >> 15)) * 0x85EBCA6Bu;
     h ^= h >> 13;
@@ -210,8 +212,9 @@ __global__ void __launch_bounds__(FL_THREADS, 1) filter_kernel(const __grid_cons
     const unsigned mbs = (unsigned)((m + FL_ROWS - 1) / FL_ROWS);
     const unsigned tiles = m > 0 ? mbs * p.nt : 0u, grid = gridDim.x >> 1, t0 = blockIdx.x >> 1;
     // code of row r of this CTA's half of tile t
-    auto code_of = [&](unsigned t, int r) {
-        return code_at(p.step, (t % p.nt) * (unsigned)kFilterTile + rank * FL_BM + r);
+    auto code_of = [&](unsigned t, int r) -> size_t {
+        const uint32_t lin = (t % p.nt) * (unsigned)kFilterTile + rank * FL_BM + r;
+        return MODE == kCollectAll ? lin : code_at(p.step, lin);
     };
 
     if (warp == 0) {
@@ -423,7 +426,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) filter_kernel(const __grid_cons
         for (unsigned t = t0; t < tiles && ok; t += grid, ++gc) {
             const unsigned mb = t / p.nt;
             const int row0 = (int)(mb * FL_ROWS) + half * cpt;  // this warp's rows row0 .. row0 + cpt - 1
-            if (MODE == kCollect && mb != mb_have) {
+            if (MODE != kSample && mb != mb_have) {
                 __syncwarp();
                 for (int i = lane; i < (cpt >> 1); i += 32) {
                     // rows past m never pass
@@ -520,7 +523,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) filter_kernel(const __grid_cons
             tc_fence_before();
             if (lane == 0) mbar_arrive_cluster(rank0_addr(xempty0 + 8 * b));
         }
-        if (MODE == kCollect && ok) flush();
+        if (MODE != kSample && ok) flush();
     }
     tc_fence_before();
     cluster_sync();  // no CTA leaves while the other may still arrive on its barriers or read its memory
@@ -784,8 +787,12 @@ cudaError_t launch_pass(const Params &P, const FlArgs &base, const CUtensorMap &
     a.stages = std::min(FL_MAX_STAGES, (avail - 4 * ring_bytes) / stage_bytes) & ~1;  // the decoder groups alternate
     a.ring = std::min(FL_MAX_RING, (avail - a.stages * stage_bytes) / ring_bytes);
     const size_t smem = (size_t)a.stages * stage_bytes + (size_t)a.ring * ring_bytes + FL_FIXED + tab;
-    auto kern = P.nibble ? (mode == kSample ? filter_kernel<true, kSample> : filter_kernel<true, kCollect>)
-                         : (mode == kSample ? filter_kernel<false, kSample> : filter_kernel<false, kCollect>);
+    auto pick = [&](auto nib) {
+        constexpr bool N = decltype(nib)::value;
+        return mode == kSample ? filter_kernel<N, kSample> : mode == kCollect ? filter_kernel<N, kCollect>
+                                                                              : filter_kernel<N, kCollectAll>;
+    };
+    auto kern = P.nibble ? pick(std::true_type{}) : pick(std::false_type{});
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
@@ -897,7 +904,7 @@ cudaError_t launch_filter(const Params &P, const DevTables &T, const FilterIndex
                                                                        b.r12, b.uv, b.thr);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = launch_pass(P, a, map, kCollect, tiles, tiles, st);
+    if (e == cudaSuccess) e = launch_pass(P, a, map, kCollectAll, tiles, tiles, st);
     if (e != cudaSuccess) return e;
     filter_select_kernel<<<(unsigned)rows, 256, 0, st>>>(m_dev, kc, ix.n, b.cnt, b.list_d, b.list_i, b.r12,
                                                          cand_d, cand_i, b.bad);
