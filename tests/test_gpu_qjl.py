@@ -217,3 +217,26 @@ def test_symmetric_qjl_shapes_and_errors(cuda_ok):
         s.distance_m_to_n_symmetric_light(codes.astype(np.float32), codes)
     with pytest.raises(ValueError, match="code: wrong byte size"):
         s.prepare_symmetric_query(codes[0][:-1])
+
+
+@pytest.mark.parametrize("dim,bits", [(64, 4), (384, 4), (768, 8)])
+@pytest.mark.parametrize("m,n", [(3, 200), (64, 129), (130, 300)])
+@pytest.mark.parametrize("variant", ["light", "full", "full_prepared"])
+def test_device_codes_off_four_bytes(cuda_ok, dim, bits, m, n, variant):
+    """Codes at any address: the CUDA-core kernels (64 x 64 tiles, and 128 x 128 from 64
+    rows on) take what the tensor-core kernel's 4-byte copies cannot."""
+    import torch
+
+    rng = np.random.default_rng(dim + bits + m + n)
+    s, o = tq.TurboQuantSpace(dim, bits), O.OracleSpace(dim, bits)
+    cs = s.code_size_bytes()
+    A, B = (o.encode_batch(rng.standard_normal((r, dim)).astype(np.float32)) for r in (m, n))
+    dev = []
+    for c, off in ((A, 1), (B, 3)):
+        buf = torch.zeros(c.size + off, dtype=torch.uint8, device="cuda")
+        buf[off:] = torch.from_numpy(c.reshape(-1)).cuda()
+        dev.append(buf[off:].view(-1, cs))
+        assert dev[-1].data_ptr() % 4
+    got = getattr(s, f"distance_m_to_n_symmetric_{variant}")(*dev).cpu().numpy()
+    err, ok = dist_close(got, o.distance_m_to_n_symmetric_qjl(A, B, variant), sym_term_scale(A, B, cs, cs - 12))
+    assert ok, err.max()

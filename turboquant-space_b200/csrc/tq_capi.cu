@@ -177,8 +177,8 @@ class MtonRunner {
                             D);
             if (sp_->code_size > kDecMaxCode)
                 return fail(TQ_ERR_NOT_SUPPORTED,
-                            "decoded split-BF16 tiles: a tile of 128 codes of %zu bytes does not fit in shared "
-                            "memory beside the pipeline (use split_bf16)", sp_->code_size);
+                            "decoded split-BF16 tiles take codes of at most %zu bytes, not %zu (use split_bf16)",
+                            kDecMaxCode, sp_->code_size);
         }
         if (!sym_) {  // prepared queries (the scan path uses them directly)
             TQ_CUDA(prep_.alloc(sizeof(float) * m_ * (2 * D + 2), s), "cudaMallocAsync(prepared)");
@@ -244,8 +244,8 @@ class MtonRunner {
     }
 
   private:
-    // Code size up to which SPLIT_BF16_DECODED is offered: a tile of 128 codes
-    // beside two 64 KB stages in shared memory.
+    // Code size up to which SPLIT_BF16_DECODED is offered: what its first kernel could
+    // hold in shared memory, kept as the precision's documented limit.
     static constexpr size_t kDecMaxCode = 756;
     // FP32: the tensor-core kernel, except where the scan kernel, a launch over rows and
     // codes, is faster.  One or two rows (four of byte codes) do not pay for the decode

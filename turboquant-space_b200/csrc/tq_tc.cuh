@@ -116,11 +116,16 @@ __device__ __forceinline__ uint32_t rank0_addr(uint32_t addr) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
     return r;
 }
-// Arrives on a barrier of the other CTA.  No wider release than the default:
-// what the arrival reports (operand tiles, tensor-memory reads) is complete in
-// the arriving CTA's own memories before it is sent (proxy fence and local
-// barrier, or tcgen05.wait and fence), and the MMAs that depend on it access
-// them there; a cluster-scope release costs about 1,000 clocks here.
+// Arrives on a barrier of the other CTA: a release at the default scope, which PTX
+// documents as this CTA's.  What the arrival reports is ordered for its readers
+// without a wider one: operand tiles are this CTA's shared memory, written through
+// the proxy fence and a local barrier (or by TMA on one) before it is sent, and read
+// by the MMA in this SM; tensor-memory reads end in tcgen05.wait::ld and
+// fence::before_thread_sync.  Nothing of it passes through a cache that another SM
+// would have to see flushed, which is what a cluster-scope release adds; CUTLASS's
+// two-SM pipelines arrive on the leader's barriers in the same form.  With
+// .release.cluster the relay took 1254 clocks a K block, and the filter pass's MMAs
+// waited for it 63% of their time (9.2 against 7.8 M clocks).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
