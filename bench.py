@@ -488,8 +488,8 @@ def run_symq(args):
     """QJL-corrected symmetric distances (light, full, full-prepared): 2048 row
     codes x 200,000 column codes of a 1024-centre Gaussian mixture at 1536-d
     (padded 2048), 4-bit, device-resident.  Each variant is timed on the GPU
-    (CUDA events) in both precisions (FP32: CUDA cores, light on tensor cores;
-    split-TF32: tensor cores) and checked against the FP64 evaluation of its formula on 2,000
+    (CUDA events) in both precisions (FP32 on FP16 pairs, and split-TF32, both on
+    tensor cores) and checked against the FP64 evaluation of its formula on 2,000
     sampled pairs; the reference's own CPU code (oracle/_ref) is timed on a
     bounded sample (128 x 512 pairs) on the host cores."""
     import torch

@@ -50,9 +50,11 @@ typedef enum tq_status {
 typedef enum tq_precision {
     TQ_PRECISION_FP32 = 0,       /* the drop-in, FP32 accuracy: tcgen05 tensor cores on hi+lo FP16
                                     pairs (22 bits) with the code tiles decoded in shared memory,
-                                    summed in FP32 every one or two K blocks; CUDA cores for
-                                    small calls, padded dims below 16 and the full QJL forms */
-    TQ_PRECISION_SPLIT_BF16 = 1, /* the same kernel on hi+lo BF16 pairs, summed every 4 or 8 K blocks */
+                                    summed in FP32 every one or two K blocks (the sign part every
+                                    8, or 4 below 32 rows); CUDA cores for small calls and padded
+                                    dims below 16 */
+    TQ_PRECISION_SPLIT_BF16 = 1, /* the same kernel on hi+lo BF16 pairs, summed every 4 or 8 K
+                                    blocks (the sign part every 16) */
     TQ_PRECISION_SPLIT_TF32 = 2, /* tcgen05 tensor cores on hi+lo TF32 pairs, FP32 TMEM accumulators
                                     (the QJL-corrected symmetric distances only) */
     TQ_PRECISION_REFERENCE = 3,  /* the reference's own FP32 arithmetic in its Release build's
@@ -225,9 +227,12 @@ tq_status tq_rotated_coords_batch_device(const tq_space *sp, const float *X, siz
 /* distanceBatchMToNSymmetric{Light,Full,FullPrepared} (:557-572, 618-647,
  * bindings.cpp:221-266, 312-334): out[m, n] row-major.  Host pointers,
  * synchronous.  Each code is reconstructed and passed through the QJL
- * Hadamard once; the pair terms are two contractions on the GPU:
- * TQ_PRECISION_FP32 (the drop-in) on CUDA cores, the light variant on tensor
- * cores as in the M x N calls; TQ_PRECISION_SPLIT_TF32 on tcgen05 tensor cores
+ * Hadamard once; the pair terms are contractions on the GPU:
+ * TQ_PRECISION_FP32 (the drop-in) on tensor cores as in the M x N calls, the full
+ * variants in two passes (CUDA cores for device codes that are not 4-byte aligned
+ * and padded dims below 16, full variants below 32); device calls are stream-ordered
+ * and report a wait that gave up through tq_space_take_device_status.
+ * TQ_PRECISION_SPLIT_TF32 runs the full variants on tcgen05 tensor cores
  * (hi/lo TF32 operands, FP32 accumulators; padded dims below 64 stay on CUDA
  * cores; light as with FP32).  TQ_PRECISION_SPLIT_BF16 is refused with
  * TQ_ERR_NOT_SUPPORTED: the operands are values of the small centroid table,
@@ -332,8 +337,8 @@ typedef enum tq_index_layout {
     TQ_INDEX_CODES = 1   /* the codes plus four floats a code (code_size + 16 bytes, and 4 more
                             for the filter pass if there is room): the pass
                             decodes each tile of codes in shared memory (kernel variants 2 and
-                            4, or 6 by the tuner), for corpora ~10x larger per GPU; padded
-                            dim >= 64 */
+                            4; 1 and 3 too where their tiles fit; 6 by the tuner), for
+                            corpora ~10x larger per GPU; padded dim >= 64 */
 } tq_index_layout;
 
 /* Keep n codes (host or device memory) resident in HBM in the given layout. */
@@ -353,8 +358,9 @@ typedef struct tq_server_params {
                            fewer slots */
     int kernel_variant; /* -1: autotune the contraction's tile shape per batch-size bucket;
                            else fixed (tq_topk_variant_shape): 0..6 for a TQ_INDEX_PLANES
-                           index, 1..4 for TQ_INDEX_CODES.  6 is the filter pass over
-                           the codes, which the tuner may pick for either layout */
+                           index, 2 and 4 (1 and 3 where their tiles fit) for
+                           TQ_INDEX_CODES.  6 is the filter pass over the codes, which the
+                           tuner may pick for either layout */
     size_t queue_rows;  /* queued query rows beyond which submit returns TQ_ERR_BUSY
                            (0: no cap beyond the admission pool) */
     int candidates;     /* tensor-pass candidates per row that the exact stage rescores,

@@ -1108,8 +1108,8 @@ struct SymqRunner {
     // The full form: a symmetric pass for the MSE products after an asymmetric one
     // for the correction, whose products wait in the output.  Against planes of
     // both sides and an FP32 contraction over 4 D on CUDA cores, which also lost
-    // more bits: 1 x 1 of 384-d 4-bit 125 -> 42 us, 300 x 20k 962 -> 201 us,
-    // 2048 x 20k of 1536-d 15.3 -> 1.12 ms.
+    // more bits: 1 x 1 of 384-d 4-bit 125 -> 41 us, 300 x 20k 962 -> 194 us,
+    // 2048 x 20k of 1536-d 15.3 -> 1.25 ms.
     tq_status prepare_rows_full_cg(const uint8_t *A, cudaStream_t s) {
         const size_t kc = m * tq::cg_row_k(sp->P, tq::kCgAsym) * 2, km = m * tq::cg_row_k(sp->P, tq::kCgSym) * 2;
         // the correction's FP32 rows live for a slice of the rows at a time

@@ -19,12 +19,13 @@
 //   - A group's rows arrive by cp.async while the previous group is encoded;
 //     its codes leave as one bulk store.
 //
-// What bounds it: the shared-memory pipe (about 526 wavefronts a row at D = 1024,
-// 256 of them shuffles; encode2 had 694 and was 80% busy) and instruction issue
-// (2024 a row; 2334).  300k rows, encode2 -> this kernel: 256-d 4-bit 289 -> 174
-// us, 384-d 4-bit 510 -> 372, 500-d 8-bit 492 -> 391, 768-d 4-bit 992 -> 897,
-// 768-d 8-bit 918 -> 866.  Eight lanes a row at D = 1024 leave 8 warps of 255
-// registers: 920 us.
+// What bounds it: no pipe alone.  Shared memory takes about 526 wavefronts a row at
+// D = 1024, 256 of them shuffles (encode2: 694), instruction issue 2024 a row (2334);
+// both are 64% busy, with instruction fetch of the straight-line code (64 elements a
+// lane) and the packed-FP32 pipe among the stalls.  300k rows, encode2 -> this kernel:
+// 256-d 4-bit 289 -> 174 us, 384-d 4-bit 510 -> 372, 500-d 8-bit 492 -> 391, 768-d
+// 4-bit 992 -> 897, 768-d 8-bit 918 -> 866.  Eight lanes a row at D = 1024 leave 8
+// warps of 255 registers: 920 us.
 #include "tq_internal.h"
 #include "tq_async.cuh"
 #include "tq_rht.cuh"

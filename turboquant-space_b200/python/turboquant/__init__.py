@@ -525,9 +525,9 @@ class TurboQuantSpace:
                                                      prec))
         return out
 
-    # precision="fp32" is the drop-in (CUDA cores; light on tcgen05 tensor cores,
-    # hi/lo FP16 operands); "split_tf32" runs the two contractions of the full
-    # forms on tensor cores (hi/lo TF32 operands, FP32 sums).
+    # precision="fp32" is the drop-in (tcgen05 tensor cores, hi/lo FP16 operands; the
+    # full forms in two passes); "split_tf32" runs the full forms on hi/lo TF32
+    # operands (FP32 sums).
     def distance_m_to_n_symmetric_full(self, codes_a, codes_b, precision="fp32"):
         """distanceBatchMToNSymmetricFull: MSE + all four QJL terms (:618-631, 731-800)."""
         return self._symmetric_qjl(codes_a, codes_b, "full", precision)
