@@ -778,15 +778,21 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
     const size_t plane_bytes = planes ? ix->n_pad * (K + (size_t)ix->K_lo) * 2 : 0;
     const size_t code_bytes = round_up(n * sp->code_size, 256);
     const size_t nscal = planes ? 2 : 4;  // c1, c2 (+ fc, fs)
-    cudaError_t e = cudaMalloc(&ix->block, plane_bytes + nscal * ix->n_pad * 4 + code_bytes +
-                                               tq::kBoundFloats * 4 + 256);
+    // the filter pass's factors, 4 bytes a code, come last: an index without room for
+    // them goes without
+    const size_t own_bytes = plane_bytes + nscal * ix->n_pad * 4 + code_bytes + round_up(tq::kBoundFloats * 4, 256);
+    const size_t factor_bytes = (ix->n_pad + tq::kFilterBound) * 4;
+    bool factors = true;
+    cudaError_t e = cudaMalloc(&ix->block, own_bytes + factor_bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        factors = false;
+        e = cudaMalloc(&ix->block, own_bytes);
+    }
     if (e != cudaSuccess) {
         delete ix;
         return cuda_fail(e, "cudaMalloc(index)");
     }
-    // the filter pass's factors, 4 bytes a code: an index without room for them goes without
-    void *factors = nullptr;
-    if (cudaMalloc(&factors, (ix->n_pad + tq::kFilterBound) * 4) != cudaSuccess) cudaGetLastError();
     auto *base = static_cast<unsigned char *>(ix->block);
     ix->planes = planes ? base : nullptr;
     ix->c1 = reinterpret_cast<float *>(base + plane_bytes);
@@ -795,12 +801,12 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
         ix->fc = ix->c2 + ix->n_pad;
         ix->fs = ix->fc + ix->n_pad;
     }
-    ix->filter.rho = static_cast<uint32_t *>(factors);
+    ix->filter.rho = factors ? reinterpret_cast<uint32_t *>(base + own_bytes) : nullptr;
     ix->codes = reinterpret_cast<uint8_t *>(ix->c1 + nscal * ix->n_pad);
     ix->bound = reinterpret_cast<float *>(ix->codes + code_bytes);
     ix->filter.codes = ix->codes;
     ix->filter.n = n;
-    ix->filter.bound = factors ? static_cast<float *>(factors) + ix->n_pad : nullptr;
+    ix->filter.bound = factors ? reinterpret_cast<float *>(ix->filter.rho + ix->n_pad) : nullptr;
     ix->filter.alpha = tq::filter_alpha(sp->centroids.data(), sp->levels);
     e = cudaMemcpy(ix->codes, codes, n * sp->code_size,
                    codes_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
@@ -825,7 +831,6 @@ tq_status tq_index_create_ex(const tq_space *csp, const uint8_t *codes, size_t n
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         cudaFree(ix->block);
-        cudaFree(factors);
         delete ix;
         return cuda_fail(e, "index build");
     }
@@ -842,7 +847,6 @@ void tq_index_destroy(tq_index *ix) {
     if (!ix) return;
     DeviceGuard g(ix->device);
     if (ix->block) cudaFree(ix->block);
-    if (ix->filter.rho) cudaFree(ix->filter.rho);
     delete ix;
 }
 
